@@ -235,7 +235,8 @@ typedef struct skw_walk_params {
  * {prob, neighbour-if-kept, its offset, its usable degree, neighbour-via-alias, its offset, its
  * usable degree, alias} (32 B x E of device memory, plus 8 B x V), so that a step is a single
  * random 32-byte access.  Once built, skw_walk* use it for offline DeepWalk and PPR; walks are
- * bit-identical with and without it.  Must be rebuilt after the table changes. */
+ * bit-identical with and without it.  Must be rebuilt after the table changes; the memory is kept
+ * for that, until skw_walk_records_free, another graph, or an online call that builds tables. */
 int skw_walk_records_build(skw_ctx* ctx, float* ms);
 int skw_walk_records_free(skw_ctx* ctx);
 

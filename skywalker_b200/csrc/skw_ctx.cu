@@ -43,9 +43,19 @@ int ensure_bytes(skw_ctx* ctx, void** p, size_t* cap, size_t want) {
   *p = nullptr;
   *cap = 0;
   if (want == 0) want = 256;
-  SKW_CUDA(ctx, cudaMalloc(p, want));
+  SKW_CUDA(ctx, dev_malloc(ctx, p, want));
   *cap = want;
   return SKW_OK;
+}
+
+cudaError_t dev_malloc(skw_ctx* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->records && !ctx->records_ready) {
+    cudaGetLastError();
+    drop_records(ctx);
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
 }
 
 int err_reset(skw_ctx* ctx) {
@@ -273,7 +283,7 @@ void drop_records(skw_ctx* ctx) {
 int alloc_table(skw_ctx* ctx) {
   // kSlotSlack spare entries let a multi-GPU caller all-gather the table in equal chunks in place
   if (!ctx->slots) {
-    SKW_CUDA(ctx, cudaMalloc(&ctx->slots, sizeof(Slot) * (ctx->E + kSlotSlack)));
+    SKW_CUDA(ctx, dev_malloc(ctx, reinterpret_cast<void**>(&ctx->slots), sizeof(Slot) * (ctx->E + kSlotSlack)));
     fill_unbuilt_slots_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->slots, (size_t)ctx->E + kSlotSlack);
     SKW_LAUNCHED(ctx);
   }
@@ -736,7 +746,7 @@ int skw_alias_import(skw_ctx* ctx, const float* h_prob, const uint32_t* h_alias,
   if (!ctx->xadj) return fail(ctx, SKW_ERR_STATE, "skw_alias_import: no graph resident");
   if (!h_prob || !h_alias || !h_valid) return fail(ctx, SKW_ERR_ARG, "skw_alias_import: null array");
   DeviceGuard g(ctx->device);
-  drop_records(ctx);
+  ctx->records_ready = false;  // derived from the old table
   int rc = alloc_table(ctx);
   if (rc != SKW_OK) return rc;
   std::vector<Slot> tmp(ctx->E ? ctx->E : 1);
@@ -828,7 +838,7 @@ int skw_alias_load(skw_ctx* ctx, const char* path) {
   if (rc != SKW_OK) return rc;
   if (hdr[4] != fp)
     return fail(ctx, SKW_ERR_IO, "skw_alias_load: %s was written for another graph (same V and E, different offsets)", path);
-  drop_records(ctx);
+  ctx->records_ready = false;  // derived from the old table
   rc = alloc_table(ctx);
   if (rc != SKW_OK) return rc;
   ctx->table_ready = false;

@@ -108,8 +108,10 @@ int fail(skw_ctx* ctx, int code, const char* fmt, ...);
 int finish_graph(skw_ctx* ctx);
 // allocate slots[E] / valid[V] if absent
 int alloc_table(skw_ctx* ctx);
-// forget the fused walk records (they are derived from the table and die with it)
+// forget the fused walk records (they are derived from the table and die with it) and free their memory
 void drop_records(skw_ctx* ctx);
+// cudaMalloc that gives up the memory of records that are no longer valid before it fails
+cudaError_t dev_malloc(skw_ctx* ctx, void** p, size_t bytes);
 int fail_cuda(skw_ctx* ctx, cudaError_t e, const char* what, const char* file, int line);
 void set_global_error(const char* msg);
 

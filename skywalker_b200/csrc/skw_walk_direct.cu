@@ -467,7 +467,7 @@ int launch_walk_online_direct(skw_ctx* ctx, const WalkArgs& a, uint32_t app) {
   PrepMemo* memo = nullptr;
   if (ctx->max_degree >= kMemoMinDegree) {
     if (!ctx->prep_memo) {
-      SKW_CUDA(ctx, cudaMalloc(&ctx->prep_memo, sizeof(PrepMemo) * ((size_t)ctx->V + 1)));
+      SKW_CUDA(ctx, dev_malloc(ctx, &ctx->prep_memo, sizeof(PrepMemo) * ((size_t)ctx->V + 1)));
       SKW_CUDA(ctx, cudaMemsetAsync(ctx->prep_memo, 0, sizeof(PrepMemo) * ((size_t)ctx->V + 1), st));
       ctx->prep_stamp = 0;
     }
@@ -479,7 +479,7 @@ int launch_walk_online_direct(skw_ctx* ctx, const WalkArgs& a, uint32_t app) {
   }
   Ckpt* ck_all = nullptr;
   if (memo != nullptr && ctx->max_degree >= kCkMinDegree) {
-    if (!ctx->prep_ckpt) SKW_CUDA(ctx, cudaMalloc(&ctx->prep_ckpt, sizeof(Ckpt) * ((size_t)(ctx->E / kCkChunk) + 2)));
+    if (!ctx->prep_ckpt) SKW_CUDA(ctx, dev_malloc(ctx, &ctx->prep_ckpt, sizeof(Ckpt) * ((size_t)(ctx->E / kCkChunk) + 2)));
     ck_all = static_cast<Ckpt*>(ctx->prep_ckpt);  // validated by the memo's stamp: no clearing needed
   }
   const u32 stamp = ctx->prep_stamp;
