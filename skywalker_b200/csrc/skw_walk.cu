@@ -31,55 +31,66 @@ namespace skw {
 int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 cells, u32 offs,
                      const u32* alive_lengths, bool new_round);
 
+// One edge list of the CSR: its first edge and its length.
+struct EdgeList {
+  u32 off, deg;
+};
+__device__ __forceinline__ EdgeList edge_list(const WalkArgs& a, u32 v) {
+  const u32 off = __ldg(a.xadj + v);
+  return EdgeList{off, __ldg(a.xadj + v + 1) - off};
+}
+
+// The neighbour that random words r draw from the list of `cur`.  Returns false when there is none.
+__device__ __forceinline__ bool walk_draw(const WalkArgs& a, u32 cur, EdgeList here, Rand4 r, u32& next) {
+  const u32 col = __umulhi(r.x, here.deg);
+  u32 cand = col;
+  if (!a.unbiased) {
+    const Slot s = load_slot(a.slots + (u64)here.off + col);
+    if (s.prob < 0.0f) return false;  // vertex without usable weight
+    cand = u01(r.y) < s.prob ? col : s.alias;
+    if (cand >= here.deg) {  // a table that does not belong to this graph
+      dev_fail(a.err, DEV_ERR_INDEX, cur, cand, 20);
+      return false;
+    }
+  }
+  next = ldg_once(a.adjncy + (u64)here.off + cand);
+  return true;
+}
+
 // One step of one walker standing on `cur`.  Returns false when the walk ends here.
 // r: the random words of (walker, step, trial 0).
 template <int APP>
-__device__ __forceinline__ bool walk_step(const WalkArgs& a, u64 gw, u32 step, u32 cur, u32 prev,
-                                          u32& next, Rand4 r) {
+__device__ __forceinline__ bool walk_step(const WalkArgs& a, u32 step, u64 gw, u32 cur, u32& next, Rand4 r) {
   if (APP == SKW_APP_PPR && u01(r.z) < a.tp) return false;
   if (cur >= a.V) {
     dev_fail(a.err, DEV_ERR_INDEX, cur, step, (u32)gw);
     return false;
   }
-  const u32 off = __ldg(a.xadj + cur);
-  const u32 deg = __ldg(a.xadj + cur + 1) - off;
-  if (deg == 0) return false;
-  if (APP == SKW_APP_NODE2VEC && prev != kNoVertex) {
-    for (u32 trial = 0;;) {
-      const u32 col = __umulhi(r.x, deg);
-      u32 cand = col;
-      if (!a.unbiased) {
-        const Slot s = load_slot(a.slots + (u64)off + col);
-        if (s.prob < 0.0f) return false;  // vertex without usable weight
-        cand = u01(r.y) < s.prob ? col : s.alias;
-        if (cand >= deg) {  // a table that does not belong to this graph
-          dev_fail(a.err, DEV_ERR_INDEX, cur, cand, 20);
-          return false;
-        }
-      }
-      next = ldg_once(a.adjncy + (u64)off + cand);
-      const float f = next == prev ? a.inv_p : (connected(a.xadj, a.adjncy, prev, next) ? 1.0f : a.inv_q);
-      if (__fmul_rn(u01(r.w), a.fmax) < f) break;
-      if (++trial == kN2vMaxTrials) break;  // keep the last proposal
-      r = philox_tagged(a.seed, TAG_WALK, gw, step, trial);
-    }
-    return true;
-  }
-  const u32 col = __umulhi(r.x, deg);
-  u32 cand = col;
-  if (!a.unbiased) {
-    const Slot s = load_slot(a.slots + (u64)off + col);
-    if (s.prob < 0.0f) return false;
-    cand = u01(r.y) < s.prob ? col : s.alias;
-    if (cand >= deg) {
-      dev_fail(a.err, DEV_ERR_INDEX, cur, cand, 20);
-      return false;
-    }
-  }
-  next = ldg_once(a.adjncy + (u64)off + cand);
-  return true;
+  const EdgeList here = edge_list(a, cur);
+  return here.deg != 0 && walk_draw(a, cur, here, r, next);
 }
 
+// The same for node2vec, which also needs the list of the vertex it came from (there, deg 0 on the first
+// step).  A step is a chain of dependent accesses -- slot, neighbour, search of that list -- so the list of
+// the proposed vertex is fetched beside the search instead of at the start of the next step, and the list
+// of the vertex that is left is handed on.
+__device__ __forceinline__ bool walk_step_n2v(const WalkArgs& a, u32 step, u64 gw, u32 cur, u32 prev, EdgeList here,
+                                              EdgeList there, u32& next, EdgeList& next_list, Rand4 r) {
+  if (here.deg == 0) return false;
+  for (u32 trial = 0;;) {
+    if (!walk_draw(a, cur, here, r, next)) return false;
+    if (next >= a.V) {
+      dev_fail(a.err, DEV_ERR_INDEX, next, step, (u32)gw);
+      return false;
+    }
+    next_list = edge_list(a, next);
+    if (prev == kNoVertex || n2v_keep(__fmul_rn(u01(r.w), a.fmax), next == prev, a.inv_p, a.inv_q,
+                                      [&] { return connected(a.adjncy, there.off, there.off + there.deg, next, a.V); }))
+      return true;
+    if (++trial == kN2vMaxTrials) return true;  // keep the last proposal
+    r = philox_tagged(a.seed, TAG_WALK, gw, step, trial);
+  }
+}
 
 // All steps of all walkers in one launch.  Each lane owns walkers tid, tid + T, tid + 2T ...;
 // the loop body is one step, so lanes of a warp stay converged although their walkers differ.
@@ -89,15 +100,17 @@ __global__ void __launch_bounds__(256) walk_offline_kernel(const WalkArgs a) {
   u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   u64 edges = 0;
   bool have = w < a.n;
-  u32 cur = 0, prev = kNoVertex, step = 0;
+  u32 cur = 0, step = 0;
   u32* row = nullptr;
   Rand4 r{0, 0, 0, 0};  // random words of the walker's current step
-  if (have) {
+  auto begin = [&]() {
     cur = __ldg(a.starts + w);
     row = a.paths + w * a.hop_num;
     row[0] = cur;
+    step = 0;
     if (APP != SKW_APP_PPR) r = philox_tagged(a.seed, TAG_WALK, a.walker_base + w * a.walker_stride, 0, 0);
-  }
+  };
+  if (have) begin();
   while (have) {
     u32 next = 0;
     const u64 gw = a.walker_base + w * a.walker_stride;
@@ -109,15 +122,14 @@ __global__ void __launch_bounds__(256) walk_offline_kernel(const WalkArgs a) {
     bool go;
     if (APP == SKW_APP_PPR) {
       go = step + 1 < a.hop_num &&
-           walk_step<APP>(a, gw, step, cur, prev, next, philox_tagged(a.seed, TAG_WALK, gw, step, 0));
+           walk_step<APP>(a, step, gw, cur, next, philox_tagged(a.seed, TAG_WALK, gw, step, 0));
     } else {
       rn = philox_tagged(a.seed, TAG_WALK, gw, step + 1, 0);
-      go = step + 1 < a.hop_num && walk_step<APP>(a, gw, step, cur, prev, next, r);
+      go = step + 1 < a.hop_num && walk_step<APP>(a, step, gw, cur, next, r);
     }
     if (go) {
       ++step;
       row[step] = next;
-      prev = cur;
       cur = next;
       if (APP != SKW_APP_PPR) r = rn;
     } else {
@@ -125,13 +137,140 @@ __global__ void __launch_bounds__(256) walk_offline_kernel(const WalkArgs a) {
       edges += step;
       w += T;
       have = w < a.n;
-      if (have) {
+      if (have) begin();
+    }
+  }
+  add_edges(a.sum, edges);
+}
+
+// node2vec over the table.  A step is a chain of dependent accesses of varying length: slot and neighbour of
+// every proposal, the list of the proposed vertex, and for about half of the proposals a search of the list the
+// walk came from.  With one STEP per iteration every lane of a warp waits for the one with the most rejections
+// and the longest search; here an iteration is one ACCESS of whatever each lane is at (the loads of all lanes
+// are issued before any is used), so a walker takes as long as its own accesses.  The neighbour of the drawn
+// column is fetched beside its slot, since the draw mostly keeps it, and the words of the next proposal and of
+// the next step are computed while the loads are in flight.
+// Bound by the latency of dependent DRAM accesses for small batches, by the rate of random accesses for large
+// ones.  On the power-law graph of 117 M undirected edges, p = 2, q = 0.5, 80 steps, 40,000 / 400,000 walkers:
+// 1.18 / 6.35 ms with a step per iteration, a binary search for every proposal and offsets loaded where they are
+// used; with an access per iteration and searches only where they decide (n2v_keep) 0.60 / 7.2 ms when a round
+// of the search probes eight places (short chain, many accesses), 0.47 / 3.1 ms when it goes by the values
+// (ListSearch).  CTAs of two warps spread small batches evenly over the SMs (0.62 ms with eight); fewer
+// walkers a warp than lanes gained nothing.
+constexpr u32 kN2vCta = 64;
+struct Draw {
+  u32 x, y, w;  // column, acceptance, rejection
+};
+__device__ __forceinline__ Draw n2v_draw(const WalkArgs& a, u64 gw, u32 step, u32 trial) {
+  const Rand4 r = philox_tagged(a.seed, TAG_WALK, gw, step, trial);
+  return Draw{r.x, r.y, r.w};
+}
+__global__ void __launch_bounds__(kN2vCta) walk_n2v_kernel(const WalkArgs a) {
+  const u64 T = (u64)gridDim.x * blockDim.x;
+  u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  u64 edges = 0;
+  enum : u32 { kStart, kDraw, kNeighbour, kList, kSearch, kEnd };  // what the lane does next
+  u32 at = kStart;
+  u32 cur = 0, prev = kNoVertex, next = 0, cand = 0, step = 0, trial = 0;
+  EdgeList here{0, 0}, there{0, 0}, next_list{0, 0};  // of the vertex stood on, the one before, the one proposed
+  ListSearch find;
+  const bool wide = on_sector_boundary(a.adjncy);
+  bool searching = false;
+  Draw r{0, 0, 0}, r_retry{0, 0, 0}, r_step{0, 0, 0};  // of this proposal, the next one, the next step
+  bool live = true;
+  // The vote brings the lanes together again, whatever way they took through the last iteration.
+  while (__any_sync(0xFFFFFFFFu, live)) {
+    if (at == kEnd) {
+      a.lengths[w] = step;
+      edges += step;
+      w += T;
+      at = kStart;
+    }
+    if (live && at == kStart) {
+      live = w < a.n;
+      if (live) {
         cur = __ldg(a.starts + w);
-        row = a.paths + w * a.hop_num;
-        row[0] = cur;
+        a.paths[w * a.hop_num] = cur;
         prev = kNoVertex;
-        step = 0;
-        if (APP != SKW_APP_PPR) r = philox_tagged(a.seed, TAG_WALK, a.walker_base + w * a.walker_stride, 0, 0);
+        step = trial = 0;
+        here = EdgeList{0, 0};
+        if (cur < a.V) here = edge_list(a, cur);
+        else dev_fail(a.err, DEV_ERR_INDEX, cur, 0, (u32)w);
+        r = n2v_draw(a, a.walker_base + w * a.walker_stride, 0, 0);
+        at = a.hop_num > 1 && here.deg != 0 ? kDraw : kEnd;
+      }
+    }
+    // one access for every lane: slot and neighbour of the drawn column, neighbour of the alias, or a pair of
+    // offsets (a lane that only searches re-reads)
+    if (at == kDraw) cand = __umulhi(r.x, here.deg);
+    const u32* nb = a.adjncy + (u64)here.off + cand;
+    const u32* p = at == kDraw && !a.unbiased ? reinterpret_cast<const u32*>(a.slots + (u64)here.off + cand)
+                                              : a.xadj + next;
+    u32 w0 = 0, w1 = 0, w2 = 0, found[8], sector = 0;
+    if (live && at <= kNeighbour) w2 = ldg_once(nb);
+    if (live && at != kNeighbour && at != kEnd) {
+      w0 = ldg_once(p);
+      w1 = ldg_once(p + 1);
+    }
+    if (searching) {
+      sector = find.sector(next);
+      load_sector(a.adjncy, sector, find.lo, find.hi, wide, found);
+    }
+    if (at == kDraw) {
+      const u64 gw = a.walker_base + w * a.walker_stride;
+      r_retry = n2v_draw(a, gw, step, trial + 1);
+      if (trial == 0) r_step = n2v_draw(a, gw, step + 1, 0);
+    }
+    bool proposed = at == kNeighbour;  // whether `next` becomes known
+    bool judged = false, keep = true;  // whether the proposal is decided, and how
+    if (at == kDraw) {
+      const float prob = __uint_as_float(w0);
+      proposed = a.unbiased || u01(r.y) < prob;
+      at = kNeighbour;
+      if (!proposed) cand = w1;
+      if (!a.unbiased && prob < 0.0f) {  // vertex without usable weight
+        at = kEnd;
+      } else if (cand >= here.deg) {  // a table that does not belong to this graph
+        dev_fail(a.err, DEV_ERR_INDEX, cur, cand, 20);
+        at = kEnd;
+      }
+    } else if (at == kList || at == kSearch) {
+      if (at == kList) next_list = EdgeList{w0, w1 - w0};
+      judged = true;
+      if (searching) {
+        bool hit;
+        at = kSearch;
+        judged = find.advance(found, sector, next, hit);
+        keep = __fmul_rn(u01(r.w), a.fmax) < (hit ? 1.0f : a.inv_q);
+        searching = !judged;
+      }
+    }
+    if (proposed && at != kEnd) {
+      next = w2;
+      at = kList;
+      if (next >= a.V) {
+        dev_fail(a.err, DEV_ERR_INDEX, next, step, (u32)w);
+        at = kEnd;
+      } else if (prev != kNoVertex) {
+        keep = n2v_keep(__fmul_rn(u01(r.w), a.fmax), next == prev, a.inv_p, a.inv_q, [&] { return searching = true; });
+        find = ListSearch(there.off, there.off + there.deg, a.V);  // not empty: the walk left that vertex
+        judged = !keep && !searching;
+      }
+    }
+    if (judged) {
+      if (!keep && ++trial < kN2vMaxTrials) {
+        r = r_retry;
+        at = kDraw;
+      } else if (keep || at == kSearch) {  // out of trials: the last proposal is kept, once its list is here
+        ++step;
+        a.paths[w * a.hop_num + step] = next;
+        prev = cur;
+        cur = next;
+        there = here;
+        here = next_list;
+        trial = 0;
+        r = r_step;
+        at = step + 1 < a.hop_num && here.deg != 0 ? kDraw : kEnd;
       }
     }
   }
@@ -154,10 +293,19 @@ __global__ void __launch_bounds__(256) walk_online_step_kernel(const WalkArgs a,
     if (a.lengths[w] != kAlive) continue;
     u32* row = a.paths + w * a.hop_num;
     const u32 cur = row[step];
-    const u32 prev = (APP == SKW_APP_NODE2VEC && step) ? row[step - 1] : kNoVertex;
     u32 next = 0;
     const u64 gw = a.walker_base + w * a.walker_stride;
-    if (walk_step<APP>(a, gw, step, cur, prev, next, philox_tagged(a.seed, TAG_WALK, gw, step, 0))) {
+    const Rand4 r = philox_tagged(a.seed, TAG_WALK, gw, step, 0);
+    bool go;
+    if (APP == SKW_APP_NODE2VEC && cur < a.V) {
+      const u32 prev = step ? row[step - 1] : kNoVertex;
+      EdgeList next_list;
+      go = walk_step_n2v(a, step, gw, cur, prev, edge_list(a, cur), step ? edge_list(a, prev) : EdgeList{0, 0}, next,
+                         next_list, r);
+    } else {
+      go = walk_step<APP>(a, step, gw, cur, next, r);
+    }
+    if (go) {
       row[step + 1] = next;
       if (step + 2 == a.hop_num) {
         a.lengths[w] = step + 1;
@@ -810,7 +958,9 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     switch (prm->app) {
       case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<grid, 256, 0, st>>>(a); break;
       case SKW_APP_PPR: walk_offline_kernel<SKW_APP_PPR><<<grid, 256, 0, st>>>(a); break;
-      default: walk_offline_kernel<SKW_APP_NODE2VEC><<<grid, 256, 0, st>>>(a); break;
+      default:
+        walk_n2v_kernel<<<(unsigned)std::min<u64>((n + kN2vCta - 1) / kN2vCta, 0x7FFFFFFFull), kN2vCta, 0, st>>>(a);
+        break;
     }
     SKW_LAUNCHED(ctx);
   } else if (!build_tables) {
