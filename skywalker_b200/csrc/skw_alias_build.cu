@@ -23,41 +23,40 @@
 // Every quantity is an integer or a single correctly rounded IEEE operation, so the table is a
 // pure function of the weight list: no atomics on masses, no dependence on scheduling.
 //
-// Work distribution: vertices are binned by degree into nine classes with warp ballots and
-// shared-memory prefix sums (classify_* kernels); classes of degree <= 32 run one sub-warp
-// group of 4/8/16/32 lanes per vertex entirely in registers; degree <= 256 and <= 1024 one warp
-// per vertex, degree <= 4096 one CTA of 256 threads and degree <= 16384 one CTA of 1024 threads per
-// vertex, with the two prefix lists in shared memory; larger vertices one CTA of 1024 threads with
-// the lists in a global scratch slab, merged through shared-memory windows.
+// Work distribution: vertices are binned by degree with warp ballots and shared-memory prefix sums (classify_*
+// kernels), one work list per class.  Lists of up to 4096 weights are built in double precision by a lane, a group of
+// lanes, a warp or a CTA that holds the whole list in registers (skw_alias_f64.cuh); longer ones by CTAs that work
+// through it in tiles of 64-bit integers (build_vertex_merge).
 #include <math_constants.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
 
+#include "skw_alias_f64.cuh"
 #include "skw_alias_math.cuh"
 #include "skw_ctx.h"
 
 namespace skw {
 
-// degree classes: groups of 4/8/16/32 lanes; one warp per vertex (two capacities); one CTA of
-// 256 threads with its lists in shared memory; one CTA of 1024 threads with its lists in a
-// global scratch slab, merged through shared-memory windows
-enum { K_G1 = 0, K_G2, K_G4, K_G8, K_G16, K_G32, K_W1K, K_C, K_C2A, K_C2, K_H, K_CLASSES };
-constexpr u32 kGroupEpt = 8;          // list elements a lane of a sub-warp group keeps in registers
-constexpr u32 kWarpSmallMax = 32 * kGroupEpt;  // 256: the largest list a whole warp holds in registers
-constexpr u32 kWarpMax = 1024;
-constexpr u32 kLargeMax = kCtaSmemMaxDegree;  // 4096: 12 bytes of list state per edge, 4 CTAs per SM
+// Degree classes.  Up to 4096 weights a list is one tile in the registers of NT threads, EPT weights each
+// (skw_alias_f64.cuh): one lane with 8 or 16; groups of 2 to 32 lanes and CTAs of 64 to 256 threads with 16.  What a
+// thread spends on scans, the division and its way into the merge (some 300 instructions) is shared by its weights,
+// so few threads with many weights beat many with few.  Longer lists are worked through in tiles: CTAs with the two
+// prefix lists in shared memory up to 16384, one CTA of 1024 threads with the lists in a global scratch slab, merged
+// through shared-memory windows, beyond.
+enum { K_1A = 0, K_1B, K_2, K_4, K_8, K_16, K_32, K_C64, K_C128, K_C256, K_C2A, K_C2, K_H, K_CLASSES };
+constexpr u32 kListEpt = 16;
+constexpr u32 kGroupMax = 32 * kListEpt;      // 512: the longest list of a group of lanes
 constexpr u32 kMidSmemMax = 8192;             // two 512-thread CTAs per SM with 96 KB of lists each
 constexpr u32 kHugeSmemMax = 16384;           // one 1024-thread CTA per SM with 192 KB of lists
+static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
+static_assert(4 * K_CLASSES <= 64, "class counters");
 
 __device__ __forceinline__ int degree_class(u32 deg) {
-  if (deg <= kWarpSmallMax) {  // groups of 1, 2, 4 ... 32 lanes, kGroupEpt elements per lane
-    if (deg <= kGroupEpt) return K_G1;
-    return K_G1 + (32 - __clz((int)((deg - 1) / kGroupEpt)));
-  }
-  if (deg <= kWarpMax) return K_W1K;
-  if (deg <= kLargeMax) return K_C;
+  if (deg <= 8) return K_1A;
+  if (deg <= kF64Max) return deg <= kListEpt ? K_1B : K_1B + (32 - __clz((int)((deg - 1) / kListEpt)));
   if (deg <= kMidSmemMax) return K_C2A;
   if (deg <= kHugeSmemMax) return K_C2;
   return K_H;
@@ -646,357 +645,127 @@ __device__ void build_vertex_merge(u32 t, u32 v, u32 off, u32 n, const float* w,
   if (t == 0) valid[v] = 1;
 }
 
-// ------------------------------------------------------------------ packed lists (n <= 4096) --
-// Lists of at most 4096 elements get a leaner form of the same construction.
-//   * One list entry is one 64-bit word: (prefix key << 12) | position.  With n <= 4096 the bucket
-//     has 40 bits, every prefix stays below 2^52 and a position needs 12 bits, so the merge reads
-//     and compares single words (8 instead of 12 bytes of shared memory per edge).
-//   * Only the deficit prefix D is scanned, with the number of smalls riding in bits 52..63 of the
-//     same word (there is always at least one large, so the count is at most 4095).  The excess prefix
-//     follows from the cumulative mass: sum over k <= p of (M_k - C) = X(p) - D(p), hence
-//     X(p) = D(p) + g(Q_(p+1)) - (p + 1) * C, with g(Q_(p+1)) already at hand.
-//   * Each thread owns EPT consecutive elements of a tile, so the prefix sums are short serial
-//     loops plus one cross-thread scan per tile; when the whole list fits one tile (SINGLE) the
-//     weights are loaded and quantised once and stay in registers, and the scan of the quantised
-//     weights yields their total as well.
-//   * The merge keeps the heads of both lists in registers: one shared-memory load per output.
-constexpr int kPosBits = 12;
-constexpr u64 kPosMask = (1ull << kPosBits) - 1;
-constexpr int kCntShift = 52;
-constexpr u64 kKeyMask = (1ull << kCntShift) - 1;
-constexpr u64 kListEnd = ~0ull;  // stands for "no entry left": its key exceeds every real key
-constexpr u32 kPackedMax = 1u << kPosBits;
-
-// Cooperation inside a group of G lanes of one warp (G = 1, 2, 4 ... 32).  Groups of a warp work on
-// different vertices and may diverge, so every shuffle names only the lanes of its own group.
-template <int G>
-struct GroupCoop {
-  static constexpr int NT = G;
-  u32 mask, t;
-  __device__ __forceinline__ GroupCoop() {
-    const u32 lane = threadIdx.x & 31;
-    t = lane & (G - 1);
-    mask = G == 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(u32)(G - 1)));
+// ------------------------------------------------------------------ lists of up to 4096 ----
+// The vertices of one class that a group, warp or CTA works through: items first, first + stride ... of the class's
+// work list.  A vertex is reached by a chain of three dependent accesses (work list, offsets, weights), which is
+// longer than the building of a short list: so the list is read three items ahead, the offsets two, and the
+// weights of the next item are on their way to L2 while this one is built.
+struct ClassItems {
+  const u32* list;  // at the current item
+  const u32* xadj;
+  u32 left, stride;        // items from the current one on
+  u32 v, off, end;         // the current item
+  u32 v1, off1, end1, v2;  // the next one; the vertex after it
+  struct After {
+    u32 off2, end2, v3;
+  };
+  __device__ __forceinline__ u32 vertex(u32 steps) const { return left > steps * stride ? __ldg(list + steps * stride) : 0u; }
+  __device__ __forceinline__ ClassItems(const u32* worklist, const u32* cls, int k, const u32* x, u32 first, u32 step)
+      : list(worklist + cls[2 * K_CLASSES + k] + first), xadj(x), left(cls[k] - min(cls[k], first)), stride(step) {
+    v = vertex(0);
+    v1 = vertex(1);
+    v2 = vertex(2);
+    off = __ldg(xadj + v);
+    end = __ldg(xadj + v + 1);
+    off1 = __ldg(xadj + v1);
+    end1 = __ldg(xadj + v1 + 1);
   }
-  __device__ __forceinline__ void sync() const { __syncwarp(mask); }
-  __device__ __forceinline__ float max(float v) const {
-#pragma unroll
-    for (int o = G / 2; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(mask, v, o, G));
-    return v;
+  __device__ __forceinline__ bool more() const { return left != 0; }
+  // Called before the current item is built; advance() takes what it returns.  Thread t brings in the weights of
+  // the next item from per_thread * t on.
+  __device__ __forceinline__ After look_ahead(const float* wgt, u32 t, u32 per_thread) const {
+    if (left > stride && t * per_thread < end1 - off1)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(wgt + off1 + t * per_thread));
+    return After{__ldg(xadj + v2), __ldg(xadj + v2 + 1), vertex(3)};
   }
-  __device__ __forceinline__ u64 sum(u64 x) const {
-#pragma unroll
-    for (int o = G / 2; o; o >>= 1) x += __shfl_xor_sync(mask, x, o, G);
-    return x;
-  }
-  // v becomes the exclusive prefix over the group, total the group's sum
-  __device__ __forceinline__ void scan(u64& v, u64& total) const {
-    u64 inc = v;
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-      const u64 x = __shfl_up_sync(mask, inc, o, G);
-      if (t >= (u32)o) inc += x;
-    }
-    total = __shfl_sync(mask, inc, G - 1, G);
-    v = inc - v;
+  __device__ __forceinline__ void advance(const After& a) {
+    left -= min(left, stride);
+    list += stride;
+    v = v1;
+    off = off1;
+    end = end1;
+    v1 = v2;
+    off1 = a.off2;
+    end1 = a.end2;
+    v2 = a.v3;
   }
 };
 
-// Cooperation inside a CTA of NTHREADS threads (s_tmp: NTHREADS / 32 + 1 words of shared memory).
-template <int NTHREADS>
-struct CtaCoop {
-  static constexpr int NT = NTHREADS;
-  u32 t;
-  u64* s_tmp;
-  __device__ __forceinline__ explicit CtaCoop(u64* tmp) : t(threadIdx.x), s_tmp(tmp) {}
-  __device__ __forceinline__ void sync() const { __syncthreads(); }
-  __device__ __forceinline__ float max(float v) const { return coop_max<NTHREADS>(v, reinterpret_cast<float*>(s_tmp)); }
-  __device__ __forceinline__ u64 sum(u64 x) const {
-    u64 total;
-    coop_scan_u64<NTHREADS>(x, total, s_tmp);
-    return total;
-  }
-  __device__ __forceinline__ void scan(u64& v, u64& total) const { coop_scan_u64<NTHREADS>(v, total, s_tmp); }
+// Up to G * EPT weights: one group of G lanes per vertex, 32 / G vertices per warp side by side.
+template <int G, int EPT>
+struct GroupShared {
+  // an odd number of words a group; the slots also hold the staged weights (G >= 8: n + n / EPT words of 4 bytes)
+  static constexpr u32 kWords = (G * EPT + 1) | 1;
+  uint2 lists[32 / G][kWords], slots[32 / G][kWords];
 };
-
-// Merge of the packed lists: S smalls at A[0 .. S) with key = inclusive deficit prefix, L = n - S
-// larges from the back (large j at A[n - 1 - j]) with key = inclusive excess prefix.  Thread t emits
-// an equal share of the merged order.  Keys are compared and subtracted where they sit, in bits 12
-// and up of an entry (a mass times 2^12 rounds to the same float as the mass, the scale being a
-// power of two).  A step of the loop has no branch: the entry that leaves, the entry that names the
-// alias and the two keys that make up the mass are selected, and one load refills the window of
-// three entries (the small at the head, the large at the head, the large behind it).
-template <int NT>
-__device__ __forceinline__ void merge_packed(u32 t, u32 n, u32 S, const u64* A, u64 C, int B, u32 off,
-                                             Slot* __restrict__ slots, u32 v, u32* err) {
-  constexpr u64 kKeyBits = ~kPosMask;
-  const u32 L = n - S;
-  const u32 VT = (n + NT - 1) / NT;
-  const u32 k0 = min(t * VT, n), k1 = min(k0 + VT, n);
-  if (k0 >= k1) return;
-  u32 i;
-  {
-    u32 lo = k0 > L ? k0 - L : 0, hi = min(k0, S);
-    while (lo < hi) {  // small mid precedes large k0-1-mid iff its key (deficit before it) <= that large's key
-      const u32 mid = (lo + hi) >> 1;
-      const u64 a = mid ? (A[mid - 1] & kKeyBits) : 0;
-      const u64 b = A[n - 1 - (k0 - 1 - mid)] & kKeyBits;
-      if (a <= b) lo = mid + 1;
-      else hi = mid;
-    }
-    i = lo;
-  }
-  // i <= S and j <= L hold from here on, and i + j = k < n: the entry that leaves always exists
-  u32 j = k0 - i;
-  u64 dsx = i ? (A[i - 1] & kKeyBits) : 0;  // deficit of the smalls before small i
-  u64 hs = i < S ? A[i] : kListEnd;
-  u64 hl = j < L ? A[n - 1 - j] : kListEnd;
-  u64 hl2 = j + 1 < L ? A[n - 2 - j] : kListEnd;
-  const u64 Cs = C << kPosBits;
-  const int Bs = B + kPosBits;
-  Slot* __restrict__ out = slots + off;
-  bool bad = false;
-  for (u32 k = k0; k < k1; ++k) {
-    const u64 ks = hs & kKeyBits, kl = hl & kKeyBits;
-    const bool fits = dsx <= kl;           // the large at the head still has room for a small
-    const bool take = i < S && fits;       // a small leaves; else a large
-    const bool full = !take && fits;       // only once every small is placed: the large owns its bucket
-    const u64 e = take ? hs : hl;
-    const u64 a = take ? hl : hl2;         // a small's alias is the large at the head, a large's the next one
-    const u32 p = (u32)e & (u32)kPosMask;
-    // mass conservation puts the last large after every small and leaves no large short of a
-    // successor; an entry that is missing all the same is recorded and the slot made self-contained
-    const bool none = (u32)(a >> 32) == 0xFFFFFFFFu;  // a key stays below 2^52 - 2^40: only kListEnd has these bits
-    bad |= none && !full;
-    const bool self = full || none;
-    const u64 x = take ? dsx : kl, y = take ? ks : dsx;  // small: C - (ks - dsx); large: kl + C - dsx
-    Slot o;
-    o.prob = self ? 1.0f : mass_to_prob_fast(Cs + x - y, Bs);
-    o.alias = self ? p : ((u32)a & (u32)kPosMask);
-    out[p] = o;
-    i += take ? 1u : 0u;
-    j += take ? 0u : 1u;
-    const u32 idx = take ? i : n - 2 - j;
-    const bool more = take ? i < S : j + 1 < L;
-    const u64 nx = more ? A[idx] : kListEnd;
-    dsx = take ? ks : dsx;
-    hl = take ? hl : hl2;
-    hl2 = take ? hl2 : nx;
-    hs = take ? nx : hs;
-  }
-  if (bad) dev_fail(err, DEV_ERR_INTERNAL, v, k0, 8);
-}
-
-// Table of one vertex (degree n <= 4096) by the threads of `co`; A holds n packed list entries.
-// SINGLE: n <= NT * EPT.  STAGED: w points at a copy of the weights in shared memory.
-template <class Coop, int EPT, bool SINGLE, bool STAGED>
-__device__ __forceinline__ void build_vertex_packed(const Coop& co, u32 v, u32 off, u32 n, const float* w,
-                                                    Slot* __restrict__ slots, uint8_t* __restrict__ valid,
-                                                    u64* A, u32* err) {
-  constexpr int NT = Coop::NT;
-  const u32 t = co.t;
-  auto weight = [&](u32 p) { return sane_weight(STAGED ? w[p] : __ldg(w + p)); };
-  float wr[EPT];
-  float wmax = 0.0f;
-  // SINGLE: the list is one tile, spread evenly over the threads (ceil(n / NT) <= EPT elements each)
-  const u32 ept1 = (n + NT - 1) / NT;
-  if constexpr (SINGLE) {
-    const u32 p1 = t * ept1;
-    const u32 cnt1 = p1 < n ? min(ept1, n - p1) : 0u;
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) {
-      wr[k] = (u32)k < cnt1 ? weight(p1 + k) : 0.0f;
-      wmax = fmaxf(wmax, wr[k]);
-    }
-  } else {
-    for (u32 p = t; p < n; p += NT) wmax = fmaxf(wmax, weight(p));
-  }
-  wmax = co.max(wmax);
-  if (!(wmax > 0.0f)) {
-    for (u32 p = t; p < n; p += NT) slots[(u64)off + p] = Slot{-1.0f, p};
-    if (t == 0) valid[v] = 0;
-    return;
-  }
-  const int B = bucket_bits(n);
-  const u64 C = (u64)1 << B;
-  const int sh = weight_shift(wmax, B);
-  u64 m[EPT];
-  u64 W = 0, Qex = 0;
-  if constexpr (SINGLE) {
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) {
-      m[k] = quantise_bits(wr[k], sh);
-      Qex += m[k];
-    }
-    co.scan(Qex, W);  // one scan gives the prefix of this thread and the total
-  } else {
-    u64 acc = 0;
-    for (u32 p = t; p < n; p += NT) acc += quantise_bits(weight(p), sh);
-    W = co.sum(acc);
-  }
-  const u64 nC = (u64)n << B;
-  const double K = mass_factor(n, B, W);
-  u64 cQ = 0, cPK = 0;  // carries between tiles (the same value in every thread)
-  for (u32 base = 0; base < (SINGLE ? 1u : n); base += NT * EPT) {
-    // A ragged last tile spreads its elements over all threads (ept of them each, the same in every
-    // thread) instead of filling the first threads with EPT each: a list of 278 weights then costs a
-    // warp one tile of 8 elements per lane plus one of 1, not two of 8.
-    const u32 ept = SINGLE ? ept1 : min((u32)EPT, (n - base + NT - 1) / NT);
-    const u32 p0 = base + t * ept;
-    const u32 cnt = p0 < n ? min(ept, n - p0) : 0u;  // elements of this thread in this tile
-    if constexpr (!SINGLE) {
-      Qex = 0;
-#pragma unroll
-      for (int k = 0; k < EPT; ++k) {
-        m[k] = 0;
-        if ((u32)k < cnt) m[k] = quantise_bits(weight(p0 + k), sh);
-        Qex += m[k];
-      }
-      u64 tq;
-      co.scan(Qex, tq);
-      Qex += cQ;
-      cQ += tq;
-    }
-    const u64 gex = cum_mass(Qex, W, nC, K);  // cumulative mass before this thread's elements
-    u64 g_prev = gex, Q = Qex, pk = 0;
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) {
-      if ((u32)k < cnt) {
-        Q += m[k];
-        const u64 g = cum_mass(Q, W, nC, K);
-        m[k] = g - g_prev;
-        g_prev = g;
-        if (m[k] < C) pk += (C - m[k]) + (1ull << kCntShift);
-      }
-    }
-    u64 tpk;
-    co.scan(pk, tpk);
-    pk += cPK;
-    cPK += tpk;
-    u64 Dr = pk & kKeyMask, gc = gex;
-    u32 Sr = (u32)(pk >> kCntShift);  // smalls before this thread's elements
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) {
-      const u32 p = p0 + k;
-      if ((u32)k < cnt) {
-        gc += m[k];
-        const bool small = m[k] < C;
-        Dr += small ? C - m[k] : 0ull;
-        // a small carries the inclusive deficit prefix, a large the inclusive excess prefix
-        const u64 key = small ? Dr : Dr + gc - ((u64)(p + 1) << B);
-        const u32 at = small ? Sr : n - 1 - (p - Sr);
-        Sr += small ? 1u : 0u;
-        A[at] = (key << kPosBits) | p;
-      }
-    }
-  }
-  co.sync();
-  const u32 S = (u32)(cPK >> kCntShift);
-  if (S >= n) {  // mass conservation guarantees a large
-    if (t == 0) dev_fail(err, DEV_ERR_INTERNAL, v, S, 7);
-    for (u32 p = t; p < n; p += NT) slots[(u64)off + p] = Slot{1.0f, p};
-    if (t == 0) valid[v] = 1;
-    return;
-  }
-  merge_packed<NT>(t, n, S, A, C, B, off, slots, v, err);
-  if (t == 0) valid[v] = 1;
-}
-
-// Degrees up to 8 * G: one group of G lanes per vertex, 32 / G vertices per warp side by side, the
-// whole list in registers.  Every warp owns 256 list words of shared memory, 8 * G per group.
-template <int G>
-__global__ void __launch_bounds__(256) build_small_kernel(const u32* __restrict__ worklist,
-                                                          const u32* __restrict__ cls, int k,
-                                                          const u32* __restrict__ xadj,
-                                                          const float* __restrict__ wgt,
-                                                          Slot* __restrict__ slots,
-                                                          uint8_t* __restrict__ valid,
-                                                          u32* __restrict__ err) {
-  __shared__ u64 s_lists[8][32 * kGroupEpt];
-  const u32 count = cls[k], base = cls[2 * K_CLASSES + k];
-  const u32 lane = threadIdx.x & 31;
-  constexpr u32 GPW = 32 / G;  // groups per warp
-  const u32 warp_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const u32 nwarps = (gridDim.x * blockDim.x) >> 5;
-  u64* A = s_lists[threadIdx.x >> 5] + (lane / G) * (G * kGroupEpt);
+constexpr int kGroupWarps = 4, kGroupCtas = 6;  // warps a CTA, CTAs an SM: what registers and shared memory allow
+// bytes of shared memory a warp has, whatever class it is at
+constexpr size_t kGroupBytes =
+    std::max({sizeof(GroupShared<32, 16>), sizeof(GroupShared<16, 16>), sizeof(GroupShared<8, 16>),
+              sizeof(GroupShared<4, 16>), sizeof(GroupShared<2, 16>), sizeof(GroupShared<1, 16>)});
+template <int G, int EPT>
+__device__ __forceinline__ void build_groups(unsigned char* smem, int k, const u32* worklist, const u32* cls, const u32* xadj,
+                                             const float* wgt, Slot* slots, uint8_t* valid, u32* err) {
+  GroupShared<G, EPT>* sh = reinterpret_cast<GroupShared<G, EPT>*>(smem);  // this warp's
+  const u32 in_warp = (threadIdx.x & 31) / G;
   const GroupCoop<G> co;
-  for (u64 it0 = (u64)warp_id * GPW; it0 < count; it0 += (u64)nwarps * GPW) {
-    const u64 it = it0 + lane / G;
-    if (it < count) {
-      const u32 v = worklist[base + it];
-      const u32 off = xadj[v], n = xadj[v + 1] - off;
-      if (n > G * kGroupEpt || n == 0) {  // classification and kernel disagree: record and skip
-        if (co.t == 0) dev_fail(err, DEV_ERR_INTERNAL, v, n, G);
-      } else {
-        build_vertex_packed<GroupCoop<G>, (int)kGroupEpt, true, false>(co, v, off, n, wgt + off, slots, valid, A, err);
-      }
-      co.sync();  // the group's list words are reused by its next vertex
+  for (ClassItems c(worklist, cls, k, xadj, (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / G,
+                    gridDim.x * (kGroupWarps * 32 / G)); c.more();) {
+    const ClassItems::After after = c.look_ahead(wgt, co.t, G >= 8 ? 32 : EPT);
+    const u32 n = c.end - c.off;
+    if (n > G * EPT || n == 0) {  // classification and kernel disagree: record and skip
+      if (co.t == 0) dev_fail(err, DEV_ERR_INTERNAL, c.v, n, G);
+    } else {
+      build_list_f64<GroupCoop<G>, EPT>(co, c.v, c.off, n, wgt + c.off, slots, valid, sh->lists[in_warp],
+                                        sh->slots[in_warp], err);
     }
+    co.sync();  // the group's words are reused by its next vertex
+    c.advance(after);
   }
+  __syncwarp();
+}
+// All group classes in one launch, every warp taking its share of one class after the other: nothing orders them,
+// and as launches of their own they cost a small graph 9 us each.
+__global__ void __launch_bounds__(kGroupWarps * 32, kGroupCtas)
+    build_groups_kernel(const u32* __restrict__ worklist, const u32* __restrict__ cls, const u32* __restrict__ xadj,
+                        const float* __restrict__ wgt, Slot* __restrict__ slots, uint8_t* __restrict__ valid,
+                        u32* __restrict__ err) {
+  extern __shared__ __align__(16) unsigned char cta_smem[];
+  unsigned char* smem = cta_smem + (threadIdx.x >> 5) * kGroupBytes;
+  build_groups<32, 16>(smem, K_32, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<16, 16>(smem, K_16, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<8, 16>(smem, K_8, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<4, 16>(smem, K_4, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<2, 16>(smem, K_2, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<1, 16>(smem, K_1B, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<1, 8>(smem, K_1A, worklist, cls, xadj, wgt, slots, valid, err);
 }
 
-// Degrees 257 .. 1024: one warp per vertex (tiles of 256 elements), WPB warps per CTA, vertices
-// handed out by an atomic cursor because their cost varies with the degree.
-template <int CAP, int WPB>
-__global__ void __launch_bounds__(WPB * 32) build_warp_packed_kernel(const u32* __restrict__ worklist,
-                                                                     u32* __restrict__ cls, int k,
-                                                                     const u32* __restrict__ xadj,
-                                                                     const float* __restrict__ wgt,
-                                                                     Slot* __restrict__ slots,
-                                                                     uint8_t* __restrict__ valid,
-                                                                     u32* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const u32 count = cls[k], base = cls[2 * K_CLASSES + k];
-  const u32 lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  u64* A = reinterpret_cast<u64*>(smem) + (size_t)wib * CAP;
-  u32* cursor = cls + 3 * K_CLASSES + k;
-  const GroupCoop<32> co;
-  for (;;) {
-    u32 it = 0;
-    if (lane == 0) it = atomicAdd(cursor, 1u);
-    it = __shfl_sync(0xFFFFFFFFu, it, 0);
-    if (it >= count) break;
-    const u32 v = worklist[base + it];
-    const u32 off = xadj[v], n = xadj[v + 1] - off;
-    if (n > CAP || n == 0) {
-      if (lane == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, CAP);
-      continue;
-    }
-    build_vertex_packed<GroupCoop<32>, 8, false, false>(co, v, off, n, wgt + off, slots, valid, A, err);
-    __syncwarp();
-  }
-}
-
-// Degrees 1025 .. 4096 when the weight array cannot be bulk-copied (not 16-byte aligned): one CTA
-// of NT threads per vertex, weights read from global memory.
+// 513 .. 4096 weights: one CTA of NT = 64, 128 or 256 threads per vertex.
 template <int NT>
-__global__ void __launch_bounds__(NT) build_cta_packed_kernel(const u32* __restrict__ worklist,
-                                                              u32* __restrict__ cls, int k,
-                                                              const u32* __restrict__ xadj,
-                                                              const float* __restrict__ wgt,
-                                                              Slot* __restrict__ slots,
-                                                              uint8_t* __restrict__ valid,
-                                                              u32* __restrict__ err) {
+struct ListShared {
+  static constexpr u32 kMost = NT * kListEpt;
+  uint2 list[kMost + 2], slots[kMost];
+  typename CtaCoop<NT>::Words words;
+};
+template <int NT>
+__global__ void __launch_bounds__(NT, 768 / NT) build_cta_kernel(const u32* __restrict__ worklist, const u32* __restrict__ cls,
+                                                       int k, const u32* __restrict__ xadj,
+                                                       const float* __restrict__ wgt, Slot* __restrict__ slots,
+                                                       uint8_t* __restrict__ valid, u32* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ u64 s_tmp[NT / 32 + 1];
-  __shared__ u32 s_it;
-  u64* A = reinterpret_cast<u64*>(smem);
-  const u32 count = cls[k], base = cls[2 * K_CLASSES + k];
-  const CtaCoop<NT> co(s_tmp);
-  for (;;) {
-    if (threadIdx.x == 0) s_it = atomicAdd(cls + 3 * K_CLASSES + k, 1u);
-    __syncthreads();
-    const u32 it = s_it;
-    __syncthreads();
-    if (it >= count) break;
-    const u32 v = worklist[base + it];
-    const u32 off = xadj[v], n = xadj[v + 1] - off;
-    if (n > kPackedMax || n == 0) {
-      if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, kPackedMax);
-      continue;
+  ListShared<NT>* sh = reinterpret_cast<ListShared<NT>*>(smem);
+  const CtaCoop<NT> co(&sh->words);
+  for (ClassItems c(worklist, cls, k, xadj, blockIdx.x, gridDim.x); c.more();) {
+    const ClassItems::After after = c.look_ahead(wgt, co.t, 32);
+    const u32 n = c.end - c.off;
+    if (n > ListShared<NT>::kMost || n == 0) {
+      if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, c.v, n, ListShared<NT>::kMost);
+    } else {
+      build_list_f64<CtaCoop<NT>, (int)kListEpt>(co, c.v, c.off, n, wgt + c.off, slots, valid, sh->list, sh->slots, err);
     }
-    build_vertex_packed<CtaCoop<NT>, 8, false, false>(co, v, off, n, wgt + off, slots, valid, A, err);
     __syncthreads();
+    c.advance(after);
   }
 }
 
@@ -1050,76 +819,6 @@ __global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restri
     build_vertex_merge<NT, 8, WIN, false, NBUF>(threadIdx.x, v, off, n, wgt + off, slots, valid, A, P, s_tmp,
                                                       smem, err, &pipe);
     if (pipe.failed) break;  // the same in every thread
-    __syncthreads();
-  }
-}
-
-// The 1025..CAP class with the weight list staged in shared memory by the bulk-copy engine: one
-// cp.async.bulk per vertex brings the 16-byte-aligned middle of the list (the up to 3 floats
-// before the first and after the last boundary come with plain loads), the three passes over the
-// weights then read shared memory.  The packed lists (8 B/edge) precede the weights in dynamic
-// shared memory.
-template <int NT, int CAP>
-__global__ void __launch_bounds__(NT) build_cta_staged_kernel(const u32* __restrict__ worklist,
-                                                              u32* __restrict__ cls, int k,
-                                                              const u32* __restrict__ xadj,
-                                                              const float* __restrict__ wgt,
-                                                              Slot* __restrict__ slots,
-                                                              uint8_t* __restrict__ valid,
-                                                              u32* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ u64 s_tmp[NT / 32 + 1];
-  __shared__ __align__(8) u64 s_bar;
-  __shared__ u32 s_it;
-  u64* A = reinterpret_cast<u64*>(smem);
-  float* sW = reinterpret_cast<float*>(A + CAP);  // CAP + 8 floats, 16-byte aligned
-  const CtaCoop<NT> co(s_tmp);
-  const u32 count = cls[k], base = cls[2 * K_CLASSES + k];
-  if (threadIdx.x == 0) mbar_init(&s_bar, 1);
-  __syncthreads();
-  u32 parity = 0;
-  for (;;) {
-    if (threadIdx.x == 0) s_it = atomicAdd(cls + 3 * K_CLASSES + k, 1u);
-    __syncthreads();
-    const u32 it = s_it;
-    __syncthreads();
-    if (it >= count) break;
-    const u32 v = worklist[base + it];
-    const u32 off = xadj[v], n = xadj[v + 1] - off;
-    if (n > (u32)CAP || n == 0) {
-      if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, CAP);
-      continue;
-    }
-    const float* w = wgt + off;
-    const u32 head = (u32)((reinterpret_cast<uintptr_t>(w) & 15u) >> 2);            // floats before w in its 16-byte group
-    const float* first = w - head;                                                 // aligned start
-    const u32 body = ((head + n) & ~3u);                                           // floats up to the last boundary
-    const u32 lead = head ? 4 - head : 0;                                          // list elements before the first boundary
-    // elements [lead_start .. ) layout in sW: element i of the list lives at sW[head + i]
-    bool mine_ok = true;
-    const u32 skip = head ? 4u : 0u;  // floats from `first` to the first boundary inside the list
-    const bool bulk = body > skip;
-    if (bulk) {
-      // whole 16-byte groups that lie inside the list: [first + skip, first + body)
-      if (threadIdx.x == 0) bulk_copy_g2s(sW + skip, first + skip, (body - skip) * 4u, &s_bar);
-      // ragged ends by plain loads
-      if (threadIdx.x < lead) sW[head + threadIdx.x] = __ldg(w + threadIdx.x);
-      const u32 tail = head + n - body;  // elements after the last boundary
-      if (threadIdx.x < tail) sW[body + threadIdx.x] = __ldg(first + body + threadIdx.x);
-      mine_ok = mbar_wait(&s_bar, parity, 1u << 16);
-    } else {
-      for (u32 i = threadIdx.x; i < n; i += NT) sW[head + i] = __ldg(w + i);
-    }
-    // the same outcome in every thread (and the barrier that publishes the plain stores)
-    if (!__syncthreads_and(mine_ok ? 1 : 0)) {
-      // the copy did not report completion in time: record it, give it one more bounded chance to
-      // land so that nothing still writes this CTA's shared memory when it leaves, and stop
-      if (threadIdx.x == 0) dev_fail(err, DEV_ERR_WAIT, v, n, 12);
-      if (!mine_ok) mbar_wait(&s_bar, parity, 1u << 16);
-      break;
-    }
-    if (bulk) parity ^= 1u;
-    build_vertex_packed<CtaCoop<NT>, 8, false, true>(co, v, off, n, sW + head, slots, valid, A, err);
     __syncthreads();
   }
 }
@@ -1302,23 +1001,22 @@ __device__ void build_vertex_cta(u32 v, u32 off, u32 n, const float* __restrict_
 // bases at [2K + k]).
 static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
   cudaStream_t st = ctx->stream;
-  static_assert(kLargeMax <= kPackedMax, "the 1025+ CTA class uses packed list entries");
-  constexpr int kCtaSmem = kLargeMax * 8;
   constexpr int kCta2Smem = kHugeSmemMax * 12 + tile_pipe_bytes(1024) / 2;  // lists + one weight tile
   constexpr int kCta2aSmem = kMidSmemMax * 12 + tile_pipe_bytes(512) / 2;  // lists + one weight tile
-  constexpr int kCtaStagedSmem = kLargeMax * 8 + (kLargeMax + 8) * 4;
-  constexpr int kW1KSmem = 8 * kWarpMax * 8;
   constexpr int kWin = 8192;                        // merged outputs per window of the scratch class
   constexpr int kWinSmem = win_smem_bytes(1024, kWin) + tile_pipe_bytes(1024);
+  constexpr size_t kGroupSmem = kGroupWarps * kGroupBytes;
   static bool attr_set[64] = {false};
   if (!attr_set[ctx->device & 63]) {
     SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_merge_kernel<1024, kWin>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWinSmem));
     SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_merge_kernel<1024, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCta2Smem));
     SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_merge_kernel<512, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCta2aSmem));
-    SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_staged_kernel<256, kLargeMax>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kCtaStagedSmem));
-    SKW_CUDA(ctx, cudaFuncSetAttribute(build_warp_packed_kernel<kWarpMax, 8>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kW1KSmem));
+#define SMEM(BYTES, ...) \
+  SKW_CUDA(ctx, cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)))
+    SMEM(sizeof(ListShared<256>), build_cta_kernel<256>);
+    SMEM(sizeof(ListShared<128>), build_cta_kernel<128>);
+    SMEM(kGroupSmem, build_groups_kernel);
+#undef SMEM
     attr_set[ctx->device & 63] = true;
   }
   // one slab per CTA of the scratch class, sized by the largest degree; fewer CTAs when a giant hub
@@ -1340,16 +1038,15 @@ static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
   // so they run side by side: the large classes (few, long-running CTAs, whose last vertices would
   // otherwise leave most SMs idle) start first on streams of their own, the small classes fill in
   // on the caller's stream.
-  const bool fork = ctx->max_degree > kWarpSmallMax;
-  cudaStream_t s_w1k = st, s_c = st, s_c2 = st, s_c2a = st, s_h = st;
+  const bool fork = ctx->max_degree > kGroupMax;
+  cudaStream_t s_h = st, s_a = st, s_b = st, s_c = st;
   if (fork) {
     SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
     for (int i = 0; i < skw_ctx::kBuilderStreams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
     s_h = ctx->bstream[0];
-    s_c2 = ctx->bstream[1];
-    s_c = ctx->bstream[2];
-    s_w1k = ctx->bstream[3];
-    s_c2a = ctx->bstream[3];  // behind the 257-1024 class on its stream
+    s_a = ctx->bstream[1];
+    s_b = ctx->bstream[2];
+    s_c = ctx->bstream[3];
   }
   if (slab_elems) {
     build_cta_merge_kernel<1024, kWin><<<gmem_ctas, 1024, kWinSmem, s_h>>>(
@@ -1358,44 +1055,30 @@ static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
     SKW_LAUNCHED(ctx);
   }
   if (ctx->max_degree > kMidSmemMax) {
-    build_cta_merge_kernel<1024, 0><<<ctx->sm_count, 1024, kCta2Smem, s_c2>>>(
+    build_cta_merge_kernel<1024, 0><<<ctx->sm_count, 1024, kCta2Smem, s_a>>>(
         worklist, cls, K_C2, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, nullptr, kHugeSmemMax, ctx->d_err);
     SKW_LAUNCHED(ctx);
   }
-  if (ctx->max_degree > kWarpMax) {
-    if ((reinterpret_cast<uintptr_t>(ctx->adjwgt) & 15u) == 0) {
-      build_cta_staged_kernel<256, kLargeMax><<<ctx->sm_count * 4, 256, kCtaStagedSmem, s_c>>>(
-          worklist, cls, K_C, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);
-    } else {  // a borrowed weight array that is not 16-byte aligned cannot be bulk-copied
-      build_cta_packed_kernel<256><<<ctx->sm_count * 6, 256, kCtaSmem, s_c>>>(
-          worklist, cls, K_C, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);
-    }
-    SKW_LAUNCHED(ctx);
-  }
-  if (ctx->max_degree > kWarpSmallMax) {
-    build_warp_packed_kernel<kWarpMax, 8><<<ctx->sm_count * 3, 256, kW1KSmem, s_w1k>>>(
-        worklist, cls, K_W1K, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);
-    SKW_LAUNCHED(ctx);
-  }
-  if (ctx->max_degree > kLargeMax) {
-    build_cta_merge_kernel<512, 0><<<ctx->sm_count * 2, 512, kCta2aSmem, s_c2a>>>(
+  if (ctx->max_degree > kF64Max) {
+    build_cta_merge_kernel<512, 0><<<ctx->sm_count * 2, 512, kCta2aSmem, s_b>>>(
         worklist, cls, K_C2A, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, nullptr, kMidSmemMax, ctx->d_err);
     SKW_LAUNCHED(ctx);
   }
-  const int ggrid = ctx->sm_count * 8;
-#define GROUP(GSZ, KCLS)                                                                          \
-  if (ctx->max_degree > (GSZ) * kGroupEpt / 2 || (GSZ) == 1) {                                    \
-    build_small_kernel<GSZ><<<ggrid, 256, 0, st>>>(worklist, cls, KCLS, ctx->xadj, ctx->adjwgt,   \
-                                                   ctx->slots, ctx->valid, ctx->d_err);           \
-    SKW_LAUNCHED(ctx);                                                                            \
+  // 24 warps an SM: what the registers and the shared memory of these kernels allow, all of them resident at once
+  // (the vertices are dealt out by a stride over the grid: a second wave of CTAs would start when the first is done)
+#define LISTS(MORE_THAN, KCLS, NT, STREAM)                                                                      \
+  if (ctx->max_degree > (MORE_THAN)) {                                                                          \
+    build_cta_kernel<NT><<<ctx->sm_count * (768 / (NT)), NT, sizeof(ListShared<NT>), STREAM>>>(                 \
+        worklist, cls, KCLS, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);                       \
+    SKW_LAUNCHED(ctx);                                                                                          \
   }
-  GROUP(32, K_G32)
-  GROUP(16, K_G16)
-  GROUP(8, K_G8)
-  GROUP(4, K_G4)
-  GROUP(2, K_G2)
-  GROUP(1, K_G1)
-#undef GROUP
+  LISTS(2048, K_C256, 256, s_c)
+  LISTS(1024, K_C128, 128, s_a)
+  LISTS(512, K_C64, 64, s_b)
+#undef LISTS
+  build_groups_kernel<<<ctx->sm_count * kGroupCtas, kGroupWarps * 32, kGroupSmem, st>>>(
+      worklist, cls, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);
+  SKW_LAUNCHED(ctx);
   if (fork) {
     for (int i = 0; i < skw_ctx::kBuilderStreams; ++i) {
       SKW_CUDA(ctx, cudaEventRecord(ctx->bjoin[i], ctx->bstream[i]));

@@ -1,0 +1,62 @@
+"""Tables at the edges of every degree class, for weights at the edges of the arithmetic, against the oracle."""
+import numpy as np
+import pytest
+
+SIZES = sorted({max(1, b + d) for b in (1, 8, 16, 32, 64, 128, 256, 512, 1024, 2048, 4096, 8192, 16384) for d in (-1, 0, 1)}
+               | {3, 100, 300, 777, 1500, 3000, 5000, 12000, 20001, 40000})
+
+
+def _weights(kind, n, rng):
+    if kind == "uniform":
+        return rng.uniform(1, 10, n)
+    if kind == "equal":
+        return np.full(n, 3.0)
+    if kind == "one_heavy":           # nearly all mass in one bucket
+        w = np.full(n, 1e-6)
+        w[rng.integers(0, n)] = 1e6
+        return w
+    if kind == "one_light":           # many larges, each a little over a bucket
+        w = np.ones(n)
+        w[rng.integers(0, n)] = 1e-7
+        return w
+    if kind == "lognormal":
+        return rng.lognormal(0, 3, n)
+    if kind == "pareto":
+        return rng.pareto(0.5, n) + 1e-3
+    if kind == "tiny":                # largest weight below 2^-87, denormals among them
+        return rng.uniform(0, 1, n) * 10.0 ** rng.integers(-45, -30, n)
+    if kind == "unusable":            # zeros, negatives, infinities and NaNs between usable ones, zeros at the end
+        w = rng.uniform(1, 10, n)
+        w[rng.random(n) < 0.3] = 0.0
+        for x in (-1.0, -0.0, np.inf, -np.inf, np.nan):
+            w[rng.random(n) < 0.05] = x
+        w[n - n // 5:] = 0.0
+        return w
+    raise ValueError(kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["uniform", "equal", "one_heavy", "one_light", "lognormal", "pareto", "tiny", "unusable"])
+@pytest.mark.parametrize("shift", [0, 3])
+def test_alias_class_edges(ctx, oracle, kind, shift):
+    import torch
+    rng = np.random.default_rng(len(kind) + shift)
+    sizes = SIZES + [2, 5, 300, 900]
+    x = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    E = int(x[-1])
+    V = len(sizes)
+    with np.errstate(over="ignore"):
+        w = np.concatenate([_weights(kind, n, rng) for n in sizes]).astype(np.float32)
+    a = np.concatenate([np.arange(n) % V for n in sizes]).astype(np.uint32)
+    d_w = torch.zeros(E + 4, device="cuda")[shift:shift + E]      # borrowed, not on a 16-byte boundary
+    d_w.copy_(torch.from_numpy(w))
+    d_x, d_a = (torch.from_numpy(v.view(np.int32)).cuda() for v in (x, a))
+    torch.cuda.synchronize()
+    ctx.adopt_device(V, E, d_x, d_a, d_w)
+    ctx.alias_build_offline()
+    prob, alias, valid = ctx.alias_export()
+    want_prob, want_alias, want_valid = oracle.alias_build(x, w)
+    assert np.array_equal(valid, want_valid)
+    usable = np.repeat(want_valid.astype(bool), sizes)
+    bad = np.flatnonzero(usable & ((prob != want_prob) | (alias != want_alias)))
+    assert bad.size == 0, "list lengths that differ: %s" % sorted({sizes[np.searchsorted(x, b, "right") - 1] for b in bad})
