@@ -228,6 +228,8 @@ typedef struct skw_walk_params {
  * position -- never a table entry).  SKW_WALK_CACHE_TABLES implies BUILD_TABLES. */
 #define SKW_WALK_BUILD_TABLES 4u
 #define SKW_WALK_DIRECT_SLOTS 8u
+/* skw_walk only: the whole h_paths matrix is written, cells past a walk's end with SKW_INVALID_VERTEX. */
+#define SKW_WALK_FILL_ROWS 16u
 
 /* Optional wider layout of the same table for offline DeepWalk / PPR.  No counterpart in the
  * reference (whose step reads xadj, prob_array, alias_array and adjncy separately,

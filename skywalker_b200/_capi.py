@@ -17,6 +17,7 @@ WALK_CACHE_TABLES = 1
 WALK_UNBIASED = 2
 WALK_BUILD_TABLES = 4
 WALK_DIRECT_SLOTS = 8
+WALK_FILL_ROWS = 16
 KHOP_UNBIASED = 2
 KHOP_DISTINCT = 4
 INVALID_VERTEX = 0xFFFFFFFF

@@ -15,12 +15,14 @@ Buffers may be numpy arrays (host entry points; copies happen inside the call) o
 `data_ptr()` method such as a CUDA torch tensor (device entry points; no copies).
 """
 import ctypes as C
+import threading
+import weakref
 
 import numpy as np
 
 from . import _capi
 from ._capi import (APP_DEEPWALK, APP_NODE2VEC, APP_PPR, INVALID_VERTEX, KHOP_TAKE_ALL,
-                    MODE_OFFLINE, MODE_ONLINE, WALK_CACHE_TABLES, WALK_UNBIASED, KHOP_UNBIASED, KHOP_DISTINCT, KhopParams,
+                    MODE_OFFLINE, MODE_ONLINE, WALK_CACHE_TABLES, WALK_FILL_ROWS, WALK_UNBIASED, KHOP_UNBIASED, KHOP_DISTINCT, KhopParams,
                     WalkParams)
 
 
@@ -44,6 +46,68 @@ def _ptr(x):
 
 def _is_device(x):
     return hasattr(x, "data_ptr") and getattr(x, "is_cuda", False)
+
+
+def _host_u32(x):
+    """x as contiguous 32-bit words on the host: itself where it already is (a numpy array or a CPU tensor of
+    32-bit integers, pinned ones included), else a converted copy."""
+    if isinstance(x, np.ndarray):
+        if x.flags.c_contiguous and x.dtype.kind in "iu" and x.dtype.itemsize == 4 and x.dtype.isnative:
+            return x
+    elif hasattr(x, "data_ptr") and x.element_size() == 4 and not x.is_floating_point() and x.is_contiguous():
+        return x
+    return np.ascontiguousarray(x, np.uint32)
+
+
+class _ResultPool:
+    """Pinned host memory for the results of calls that were given no arrays for them.  The GPU writes such memory
+    directly, where fresh pageable memory costs a page fault every 4 KiB and a copy through the driver's staging (a
+    batch of 4,096 x 80 walks spent half of its 0.46 ms there).  A block returns here when the last array that
+    views it is gone; at most OUT bytes are lent at a time and KEEP wait for reuse.  Safe with threads."""
+    LARGEST, OUT, KEEP = 64 << 20, 256 << 20, 128 << 20
+
+    def __init__(self):
+        # re-entrant: a collection inside a locked region may give blocks back
+        self.lock, self.waiting, self.kept, self.out = threading.RLock(), {}, 0, 0
+
+    def array(self, shape, dtype=np.uint32):
+        """An array with undefined contents."""
+        count = int(np.prod(shape, dtype=np.int64))
+        nbytes = count * np.dtype(dtype).itemsize
+        if not 0 < nbytes <= self.LARGEST:
+            return np.empty(shape, dtype)
+        size = max(4096, 1 << (nbytes - 1).bit_length())
+        with self.lock:
+            if self.out + size > self.OUT:  # the caller keeps many results: those stay pageable
+                return np.empty(shape, dtype)
+            blocks = self.waiting.get(size)
+            ptr = blocks.pop() if blocks else None
+            if ptr:
+                self.kept -= size
+            self.out += size
+        if not ptr:
+            p = C.c_void_p()
+            if _capi.load().skw_host_alloc(size, C.byref(p)):
+                with self.lock:
+                    self.out -= size
+                return np.empty(shape, dtype)
+            ptr = p.value
+        block = (C.c_ubyte * size).from_address(ptr)
+        weakref.finalize(block, self._give_back, ptr, size).atexit = False
+        return np.frombuffer(block, dtype, count).reshape(shape)
+
+    def _give_back(self, ptr, size):
+        with self.lock:
+            self.out -= size
+            keep = self.kept + size <= self.KEEP
+            if keep:
+                self.kept += size
+                self.waiting.setdefault(size, []).append(ptr)
+        if not keep:
+            _capi.load().skw_host_free(ptr)
+
+
+_results = _ResultPool()
 
 
 class DeviceArray:
@@ -209,22 +273,23 @@ class Context:
     # -- walks
     def walk(self, starts, hop_num, app=APP_DEEPWALK, mode=MODE_OFFLINE, tp=0.0, p=2.0, q=0.5, seed=42,
              walker_base=0, paths=None, lengths=None, n=None, walker_stride=1, enqueue_only=False, flags=0):
-        """Host arrays (numpy) or device buffers.  Returns (paths, lengths, ms, sampled_edges).
+        """Host arrays (numpy) or device buffers.  Returns (paths, lengths, ms, sampled_edges); in host rows
+        made here, cells past a walk's end hold INVALID_VERTEX.
         enqueue_only (device buffers only): queue the kernels and return at once with ms = edges = None;
         collect the edge count later with take_sampled_edges()."""
-        prm = WalkParams(app, mode, hop_num, tp, p, q, seed, walker_base, walker_stride, flags)
         ms, edges = C.c_float(), C.c_uint64()
         if _is_device(starts):
             n = int(starts.numel()) if n is None else n
             fn = self._lib.skw_walk_device
         else:
-            starts = np.ascontiguousarray(starts, np.uint32)
+            starts = _host_u32(starts)
             n = len(starts) if n is None else n
             if paths is None:
-                paths = np.full((n, hop_num), INVALID_VERTEX, np.uint32)
+                paths, flags = _results.array((n, hop_num)), flags | WALK_FILL_ROWS
             if lengths is None:
-                lengths = np.zeros(n, np.uint32)
+                lengths = _results.array((n,))
             fn = self._lib.skw_walk
+        prm = WalkParams(app, mode, hop_num, tp, p, q, seed, walker_base, walker_stride, flags)
         if enqueue_only:
             if fn is not self._lib.skw_walk_device:
                 raise ValueError("enqueue_only needs device buffers")
@@ -242,12 +307,12 @@ class Context:
         numpy array or a pinned buffer; without one a buffer of n * hop_num cells is allocated.
         lengths_u8: the lengths come back as bytes (skw_walk_packed_u8; hop_num <= 256)."""
         prm = WalkParams(app, mode, hop_num, tp, p, q, seed, walker_base, walker_stride, flags)
-        starts = starts if _is_device(starts) else np.ascontiguousarray(starts, np.uint32)
+        starts = starts if _is_device(starts) else _host_u32(starts)
         n = (int(starts.numel()) if _is_device(starts) else len(starts)) if n is None else n
         if packed is None:
-            packed = np.empty(max(n * hop_num, 1), np.uint32)
+            packed = _results.array((max(n * hop_num, 1),))
         if lengths is None:
-            lengths = np.zeros(max(n, 1), np.uint8 if lengths_u8 else np.uint32)[:n]
+            lengths = _results.array((max(n, 1),), np.uint8 if lengths_u8 else np.uint32)[:n]
         cap = int(packed.numel()) if hasattr(packed, "numel") else int(packed.size)
         ms, edges, cells = C.c_float(), C.c_uint64(), C.c_uint64()
         fn = self._lib.skw_walk_packed_u8 if lengths_u8 else self._lib.skw_walk_packed
@@ -284,12 +349,12 @@ class Context:
             n = int(seeds.numel()) if n is None else n
             fn = self._lib.skw_sample_khop_device
         else:
-            seeds = np.ascontiguousarray(seeds, np.uint32)
+            seeds = _host_u32(seeds)
             n = len(seeds) if n is None else n
             if data is None:
-                data = np.zeros((n, cells), np.uint32)
+                data = _results.array((n, cells))
             if sample_lengths is None:
-                sample_lengths = np.zeros((n, lens), np.uint32)
+                sample_lengths = _results.array((n, lens))
             fn = self._lib.skw_sample_khop
         self._ck(fn(self._h, C.byref(prm), _ptr(seeds) if n else None, n, _ptr(data) if n else None,
                     _ptr(sample_lengths) if n else None, C.byref(ms), C.byref(edges)))
@@ -302,12 +367,12 @@ class Context:
         cells_per, lens = self.khop_layout(fanout)
         prm = KhopParams(mode, len(fanout), (C.c_uint32 * 4)(*(list(fanout) + [0] * (4 - len(fanout)))),
                          flags, seed, instance_base, instance_stride)
-        seeds = np.ascontiguousarray(seeds, np.uint32)
+        seeds = _host_u32(seeds)
         n = len(seeds) if n is None else n
         if packed is None:
-            packed = np.empty(max(n * cells_per, 1), np.uint32)
+            packed = _results.array((max(n * cells_per, 1),))
         if sample_lengths is None:
-            sample_lengths = np.zeros((n, lens), np.uint32)
+            sample_lengths = _results.array((n, lens))
         cap = int(packed.numel()) if hasattr(packed, "numel") else int(packed.size)
         ms, edges, cells = C.c_float(), C.c_uint64(), C.c_uint64()
         self._ck(self._lib.skw_sample_khop_packed(self._h, C.byref(prm), _ptr(seeds) if n else None, n, _ptr(packed),

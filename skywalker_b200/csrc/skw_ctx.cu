@@ -58,15 +58,31 @@ cudaError_t dev_malloc(skw_ctx* ctx, void** p, size_t bytes) {
   return e;
 }
 
+// The status words of a context: 16 x u32 on the device (error records, then the four 64-bit sums at word 8) and the
+// same 16 words in mapped host memory.  A synchronous call ends with this kernel, which hands them to the host and
+// leaves them cleared for the next call: one small launch where two memsets before a call and two copies after it
+// took about 14 us of a call of 65.
+__global__ void report_status_kernel(uint32_t* __restrict__ d, uint32_t* __restrict__ h, uint32_t sums_to_clear) {
+  const uint32_t t = threadIdx.x;
+  h[t] = d[t];
+  if (t < 4 || (t >= 8 && ((sums_to_clear >> ((t - 8) >> 1)) & 1u))) d[t] = 0;
+}
+
 int err_reset(skw_ctx* ctx) {
-  SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, 4 * sizeof(uint32_t), ctx->stream));
+  if (!ctx->status_clean) {
+    SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, 4 * sizeof(uint32_t), ctx->stream));
+    SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum, 0, sizeof(uint64_t), ctx->stream));
+    SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum + 3, 0, sizeof(uint64_t), ctx->stream));
+  }
+  ctx->status_clean = false;
   return SKW_OK;
 }
 
-int err_check(skw_ctx* ctx, const char* where) {
-  SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_err, ctx->d_err, 4 * sizeof(uint32_t),
-                                cudaMemcpyDeviceToHost, ctx->stream));
+int err_check(skw_ctx* ctx, const char* where, uint32_t sums_to_clear) {
+  report_status_kernel<<<1, 16, 0, ctx->stream>>>(ctx->d_err, ctx->h_err, sums_to_clear);
+  SKW_LAUNCHED(ctx);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->status_clean = true;
   if (ctx->h_err[0] != DEV_OK) {
     static const char* names[] = {"ok", "index out of range", "bounded wait ran out",
                                   "capacity exceeded", "construction invariant broken"};
@@ -252,6 +268,7 @@ static int xadj_fingerprint(skw_ctx* ctx, uint64_t* out) {
   SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum, ctx->d_sum, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   *out = *ctx->h_sum;
+  ctx->status_clean = false;
   return SKW_OK;
 }
 
@@ -266,6 +283,7 @@ int finish_graph(skw_ctx* ctx) {
                                 ctx->stream));
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->max_degree = (uint32_t)*ctx->h_sum;
+  ctx->status_clean = false;
   return SKW_OK;
 }
 
@@ -347,23 +365,18 @@ int skw_ctx_create(int device, skw_ctx** out) {
   CK(cudaEventCreateWithFlags(&ctx->bfork, cudaEventDisableTiming));
   CK(cudaEventCreate(&ctx->ev0));
   CK(cudaEventCreate(&ctx->ev1));
-  // two error records of four words: [0..4) reset and checked by every call, [4..8) owned by the
-  // packing pipeline of skw_walk_packed, which spans several such calls
-  CK(cudaMalloc(&ctx->d_err, 8 * sizeof(uint32_t)));
-  CK(cudaMemset(ctx->d_err, 0, 8 * sizeof(uint32_t)));
-  CK(cudaMallocHost(&ctx->h_err, 8 * sizeof(uint32_t)));
+  CK(cudaMalloc(&ctx->d_err, 64));
+  CK(cudaMemset(ctx->d_err, 0, 64));
+  CK(cudaMallocHost(&ctx->h_err, 64));
+  ctx->d_sum = reinterpret_cast<uint64_t*>(ctx->d_err + 8);
+  ctx->h_sum = reinterpret_cast<uint64_t*>(ctx->h_err + 8);
   for (int i = 0; i < skw_ctx::kPackSlices; ++i) {
     CK(cudaEventCreateWithFlags(&ctx->pk_ready[i], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ctx->pk_in[i], cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&ctx->pk_tot[i], cudaEventDisableTiming));
     CK(cudaEventCreate(&ctx->pk_t0[i]));
     CK(cudaEventCreate(&ctx->pk_t1[i]));
   }
-  CK(cudaMalloc(&ctx->d_tot, skw_ctx::kPackSlices * sizeof(uint64_t)));
   CK(cudaMallocHost(&ctx->h_tot, skw_ctx::kPackSlices * sizeof(uint64_t)));
-  CK(cudaMalloc(&ctx->d_sum, 4 * sizeof(uint64_t)));
-  CK(cudaMemset(ctx->d_sum, 0, 4 * sizeof(uint64_t)));
-  CK(cudaMallocHost(&ctx->h_sum, 4 * sizeof(uint64_t)));
   CK(cudaMalloc(&ctx->cls_counts, 64 * sizeof(uint32_t)));
   CK(cudaMalloc(&ctx->frontier_cls, 64 * sizeof(uint32_t)));
 #undef CK
@@ -378,8 +391,6 @@ void skw_ctx_destroy(skw_ctx* ctx) {
   free_graph(ctx);
   cudaFree(ctx->d_err);
   cudaFreeHost(ctx->h_err);
-  cudaFree(ctx->d_sum);
-  cudaFreeHost(ctx->h_sum);
   cudaFree(ctx->worklist);
   cudaFree(ctx->cls_counts);
   cudaFree(ctx->cta_scratch);
@@ -388,7 +399,6 @@ void skw_ctx_destroy(skw_ctx* ctx) {
   for (int i = 0; i < skw_ctx::kStages; ++i) cudaFree(ctx->stage[i]);
   if (ctx->h_pack) cudaFreeHost(ctx->h_pack);
   delete static_cast<skw::HostPool*>(ctx->host_pool);
-  cudaFree(ctx->d_tot);
   cudaFreeHost(ctx->h_tot);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -403,7 +413,6 @@ void skw_ctx_destroy(skw_ctx* ctx) {
   for (int i = 0; i < skw_ctx::kPackSlices; ++i) {
     if (ctx->pk_ready[i]) cudaEventDestroy(ctx->pk_ready[i]);
     if (ctx->pk_in[i]) cudaEventDestroy(ctx->pk_in[i]);
-    if (ctx->pk_tot[i]) cudaEventDestroy(ctx->pk_tot[i]);
     if (ctx->pk_t0[i]) cudaEventDestroy(ctx->pk_t0[i]);
     if (ctx->pk_t1[i]) cudaEventDestroy(ctx->pk_t1[i]);
   }

@@ -27,12 +27,11 @@ struct skw_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t side_stream = nullptr;  // result copies that overlap kernels of `stream`
   cudaStream_t copy_stream = nullptr;  // skw_walk_packed: the packed rows of each slice
-  // skw_walk_packed, per slice: rows packed; cell count on the host; start and end of the walk
+  // skw_walk_packed, per slice: rows packed (and their count on the host); start and end of the walk
   static constexpr int kPackSlices = 8;
-  cudaEvent_t pk_ready[kPackSlices] = {}, pk_tot[kPackSlices] = {}, pk_t0[kPackSlices] = {}, pk_t1[kPackSlices] = {},
+  cudaEvent_t pk_ready[kPackSlices] = {}, pk_t0[kPackSlices] = {}, pk_t1[kPackSlices] = {},
               pk_in[kPackSlices] = {};
-  uint64_t* d_tot = nullptr;  // cells each slice's packed result needs
-  uint64_t* h_tot = nullptr;  // pinned mirror
+  uint64_t* h_tot = nullptr;  // cells each slice's packed result needs: mapped, written by the packing kernel
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // the degree-class builders of one build run side by side: classes 257+ on streams of their own,
   // forked from and joined back into `stream` by events
@@ -63,12 +62,13 @@ struct skw_ctx {
   bool records_ready = false;  // set once records, vinfo and vbits were all written
   bool records_all_usable = false;  // ... and no vertex with out-edges lacks a usable table
 
-  // device error word (4 x u32) and its pinned host mirror
+  // status words on the device and in mapped host memory: the error record (4 words, 4 spare) and four 64-bit sums
+  // (edges of a synchronous call, of enqueued calls, of packed calls; vertices without a usable table)
   uint32_t* d_err = nullptr;
   uint32_t* h_err = nullptr;
-  // pinned scalar for 64-bit reductions read back after a launch
   uint64_t* d_sum = nullptr;
   uint64_t* h_sum = nullptr;
+  bool status_clean = true;  // error record and sums 0 and 3 are zero
 
   // builder scratch, grown on demand
   uint32_t* worklist = nullptr;      // V entries, vertices grouped by degree class
@@ -117,9 +117,10 @@ void set_global_error(const char* msg);
 
 // Grow-only device buffer.
 int ensure_bytes(skw_ctx* ctx, void** p, size_t* cap, size_t want);
-// Zero the device error word before a group of launches / check it after synchronising.
+// Bracket of a synchronous call: the error record and sums 0 and 3 are zero after err_reset; err_check brings all
+// status words to the host, waits for the stream, clears the record and the given sums and reports an error.
 int err_reset(skw_ctx* ctx);
-int err_check(skw_ctx* ctx, const char* where);
+int err_check(skw_ctx* ctx, const char* where, uint32_t sums_to_clear = 1u | 8u);
 
 struct DeviceGuard {
   int prev = -1;

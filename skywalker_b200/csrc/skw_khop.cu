@@ -336,11 +336,9 @@ int skw_sample_khop_device(skw_ctx* ctx, const skw_khop_params* prm, const uint3
   DeviceGuard g(ctx->device);
   cudaStream_t st = ctx->stream;
   if ((rc = err_reset(ctx)) != SKW_OK) return rc;
-  SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum, 0, sizeof(uint64_t), st));
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
   if ((rc = khop_launch(ctx, prm, d_seeds, n, d_data, d_sample_lengths, prm->instance_base, true)) != SKW_OK) return rc;
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
-  SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum, ctx->d_sum, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   if ((rc = err_check(ctx, "skw_sample_khop")) != SKW_OK) return rc;
   if (ms) SKW_CUDA(ctx, cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1));
   if (sampled_edges) *sampled_edges = *ctx->h_sum;
@@ -374,7 +372,6 @@ int skw_sample_khop(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t* h_
   const uint64_t per = (n + slices - 1) / slices;
   const uint64_t stride = prm->instance_stride ? prm->instance_stride : 1;
   if ((rc = err_reset(ctx)) != SKW_OK) return rc;
-  SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum, 0, sizeof(uint64_t), st));
   if (n) SKW_CUDA(ctx, cudaMemcpyAsync(d_seeds, h_seeds, nb, cudaMemcpyHostToDevice, st));
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
   for (uint32_t c = 0; c < slices; ++c) {
@@ -396,7 +393,6 @@ int skw_sample_khop(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t* h_
                                   sizeof(uint32_t) * (size_t)nc * lens, cudaMemcpyDeviceToHost, side));
   }
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
-  SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum, ctx->d_sum, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
   const int rc_side = cudaStreamSynchronize(side) == cudaSuccess ? SKW_OK : SKW_ERR_CUDA;
   if ((rc = err_check(ctx, "skw_sample_khop")) != SKW_OK) return rc;
   if (rc_side != SKW_OK) return fail(ctx, SKW_ERR_CUDA, "skw_sample_khop: copying the result failed");
@@ -468,17 +464,14 @@ int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint3
       SKW_LAUNCHED(ctx);
     }
     khop_pack_kernel<<<grid, 256, 0, st>>>(d_data + base * cells, nc, cells, d_offs,
-                                           static_cast<u32*>(ctx->stage[4 + c]), cap[c], ctx->d_tot + c);
+                                           static_cast<u32*>(ctx->stage[4 + c]), cap[c], ctx->h_tot + c);
     SKW_LAUNCHED(ctx);
     SKW_CUDA(ctx, cudaEventRecord(ctx->pk_ready[c], st));
     SKW_CUDA(ctx, cudaStreamWaitEvent(side, ctx->pk_ready[c], 0));
-    SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_tot + c, ctx->d_tot + c, sizeof(u64), cudaMemcpyDeviceToHost, side));
-    SKW_CUDA(ctx, cudaEventRecord(ctx->pk_tot[c], side));
     return SKW_OK;
   };
   auto body = [&]() -> int {
-    SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum, 0, sizeof(uint64_t), st));
-    SKW_CUDA(ctx, cudaMemcpyAsync(d_seeds, h_seeds, nb, cudaMemcpyHostToDevice, st));
+      SKW_CUDA(ctx, cudaMemcpyAsync(d_seeds, h_seeds, nb, cudaMemcpyHostToDevice, st));
     SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
     for (uint32_t c = 0; c < slices && nc_of[c]; ++c) {
       const uint64_t base = (uint64_t)c * per, nc = nc_of[c];
@@ -493,7 +486,7 @@ int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint3
     uint64_t total_cells = 0;
     bool fits = h_packed != nullptr;
     for (uint32_t c = 0; c < slices && nc_of[c]; ++c) {
-      SKW_CUDA(ctx, cudaEventSynchronize(ctx->pk_tot[c]));
+      SKW_CUDA(ctx, cudaEventSynchronize(ctx->pk_ready[c]));
       uint64_t slice_cells = ctx->h_tot[c];
       if (fits && total_cells + slice_cells > capacity_cells) fits = false;  // keep going: the caller gets the size
       if (fits && slice_cells > cap[c]) {
@@ -503,7 +496,7 @@ int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint3
         if (r != SKW_OK) return r;
         cap[c] = nc_of[c] * cells;
         if ((r = count_and_pack(c, true)) != SKW_OK) return r;
-        SKW_CUDA(ctx, cudaEventSynchronize(ctx->pk_tot[c]));
+        SKW_CUDA(ctx, cudaEventSynchronize(ctx->pk_ready[c]));
         slice_cells = ctx->h_tot[c];
       }
       if (fits) {
@@ -513,7 +506,6 @@ int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint3
       }
       total_cells += slice_cells;
     }
-    SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum, ctx->d_sum, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     SKW_CUDA(ctx, cudaStreamSynchronize(side));
     SKW_CUDA(ctx, cudaStreamSynchronize(ctx->copy_stream));
     int r = err_check(ctx, "skw_sample_khop_packed");  // synchronises the context's stream
