@@ -222,10 +222,12 @@ typedef struct skw_walk_params {
  * distinct frontier vertices are built at every step, as OnlineWalkShMem does
  * (src/online_walk.cu:82-166), and the walkers draw from them.  DIRECT_SLOTS: every walker computes
  * the one slot it draws straight from the weight list of its vertex (one warp per walker, all steps
- * in one launch, no table memory touched) -- the same (prob, alias) bits a built table holds, so
- * the walks are identical.  With neither flag the library computes slots directly (for the duration
- * of a call it memoises, per vertex, the largest weight, the total and prefix sums at every 64th list
- * position -- never a table entry).  SKW_WALK_CACHE_TABLES implies BUILD_TABLES. */
+ * in one launch; for the duration of a call it memoises, per vertex, the largest weight, the total and
+ * prefix sums at every 64th list position -- never a table entry).  With neither flag the library
+ * takes the cheaper of DIRECT_SLOTS and, for batches that are large for the graph, the tables of the
+ * whole graph built for the call, in memory of their own (8 bytes an edge, kept until the graph
+ * changes): the table of skw_alias_build_offline and its walk records stay as they are.  All ways give
+ * identical walks.  SKW_WALK_CACHE_TABLES implies BUILD_TABLES. */
 #define SKW_WALK_BUILD_TABLES 4u
 #define SKW_WALK_DIRECT_SLOTS 8u
 /* skw_walk only: the whole h_paths matrix is written, cells past a walk's end with SKW_INVALID_VERTEX. */

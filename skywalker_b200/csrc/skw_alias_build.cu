@@ -52,7 +52,7 @@ constexpr u32 kGroupMax = 32 * kListEpt;      // 512: the longest list of a grou
 constexpr u32 kMidSmemMax = 8192;             // two 512-thread CTAs per SM with 96 KB of lists each
 constexpr u32 kHugeSmemMax = 16384;           // one 1024-thread CTA per SM with 192 KB of lists
 static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
-static_assert(4 * K_CLASSES <= 64, "class counters");
+static_assert(2 * K_CLASSES <= 64, "class counters");
 
 __device__ __forceinline__ int degree_class(u32 deg) {
   if (deg <= 8) return K_1A;
@@ -62,83 +62,60 @@ __device__ __forceinline__ int degree_class(u32 deg) {
   return K_H;
 }
 
-// cls[0..K) counts, cls[K..2K) fill cursors, cls[2K..3K) bases of the classes in the work list,
-// cls[3K..4K) cursors from which the builder kernels take their next vertex.
-__global__ void __launch_bounds__(256) classify_count_kernel(const u32* __restrict__ xadj,
-                                                             u32 v_begin, u32 v_end,
-                                                             u32* __restrict__ cls,
-                                                             uint8_t* __restrict__ valid) {
-  __shared__ u32 s_cnt[K_CLASSES];
-  if (threadIdx.x < K_CLASSES) s_cnt[threadIdx.x] = 0;
-  __syncthreads();
+// The work list of every class: vertices of that class in no particular order, cls[k] of them; cls[K + k] is the
+// cursor from which the kernels of the long lists take their next vertex.
+struct ClassLists {
+  u32* list[K_CLASSES];
+};
+
+// One pass over the offsets: a tile of 1024 vertices is binned with ballots, its counts reserve room in the lists with
+// one atomic per class and tile, and the vertices are written there.  Each list has room for as many vertices of its
+// least degree as there can be edges for (class_room), so nothing has to be counted first: reading the offsets once
+// instead of twice took the classification of 16.8 M vertices from 304 to 120 us.
+constexpr u32 kClassifyVertices = 4;  // per thread
+__global__ void __launch_bounds__(256) classify_kernel(const u32* __restrict__ xadj, u32 v_begin, u32 v_end,
+                                                       u32* __restrict__ cls, const ClassLists lists,
+                                                       uint8_t* __restrict__ valid) {
+  __shared__ u32 s_cnt[K_CLASSES], s_base[K_CLASSES];
   const u32 lane = threadIdx.x & 31;
-  for (u64 v0 = v_begin + (u64)blockIdx.x * blockDim.x; v0 < v_end; v0 += (u64)gridDim.x * blockDim.x) {
-    const u64 v = v0 + threadIdx.x;
-    int c = -1;
-    if (v < v_end) {
-      const u32 deg = xadj[v + 1] - xadj[v];
-      if (deg == 0) valid[v] = 0;
-      else c = degree_class(deg);
-    }
+  constexpr u32 kTile = 256 * kClassifyVertices;
+  for (u64 v0 = v_begin + (u64)blockIdx.x * kTile; v0 < v_end; v0 += (u64)gridDim.x * kTile) {
+    if (threadIdx.x < K_CLASSES) s_cnt[threadIdx.x] = 0;
+    int c[kClassifyVertices];
+    u32 rank[kClassifyVertices];
 #pragma unroll
-    for (int k = 0; k < K_CLASSES; ++k) {
-      const u32 m = __ballot_sync(0xFFFFFFFFu, c == k);
-      if (lane == 0 && m) atomicAdd(&s_cnt[k], __popc(m));
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < K_CLASSES && s_cnt[threadIdx.x]) atomicAdd(&cls[threadIdx.x], s_cnt[threadIdx.x]);
-}
-
-__global__ void classify_bases_kernel(u32* __restrict__ cls) {
-  if (threadIdx.x == 0) {
-    u32 run = 0;
-    for (int k = 0; k < K_CLASSES; ++k) {
-      cls[2 * K_CLASSES + k] = run;
-      cls[K_CLASSES + k] = 0;
-      run += cls[k];
-    }
-  }
-}
-
-// Ordered compaction inside a block (ballot + shared prefix), one atomic per class per block
-// tile to reserve the output range.
-__global__ void __launch_bounds__(256) classify_fill_kernel(const u32* __restrict__ xadj,
-                                                            u32 v_begin, u32 v_end,
-                                                            u32* __restrict__ cls,
-                                                            u32* __restrict__ worklist) {
-  __shared__ u32 s_warp[K_CLASSES][8];
-  __shared__ u32 s_base[K_CLASSES];
-  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (u64 v0 = v_begin + (u64)blockIdx.x * blockDim.x; v0 < v_end; v0 += (u64)gridDim.x * blockDim.x) {
-    const u64 v = v0 + threadIdx.x;
-    int c = -1;
-    if (v < v_end) {
-      const u32 deg = xadj[v + 1] - xadj[v];
-      if (deg) c = degree_class(deg);
-    }
-    u32 my_rank = 0;
-#pragma unroll
-    for (int k = 0; k < K_CLASSES; ++k) {
-      const u32 m = __ballot_sync(0xFFFFFFFFu, c == k);
-      if (c == k) my_rank = __popc(m & ((1u << lane) - 1u));
-      if (lane == 0) s_warp[k][warp] = __popc(m);
-    }
-    __syncthreads();
-    if (threadIdx.x < K_CLASSES) {
-      u32 run = 0;
-      for (int w = 0; w < 8; ++w) {
-        const u32 t = s_warp[threadIdx.x][w];
-        s_warp[threadIdx.x][w] = run;
-        run += t;
+    for (u32 j = 0; j < kClassifyVertices; ++j) {
+      const u64 v = v0 + j * 256 + threadIdx.x;
+      c[j] = -1;
+      if (v < v_end) {
+        const u32 deg = __ldg(xadj + v + 1) - __ldg(xadj + v);
+        if (deg == 0) valid[v] = 0;
+        else c[j] = degree_class(deg);
       }
-      s_base[threadIdx.x] =
-          run ? cls[2 * K_CLASSES + threadIdx.x] + atomicAdd(&cls[K_CLASSES + threadIdx.x], run) : 0;
     }
     __syncthreads();
-    if (c >= 0) worklist[s_base[c] + s_warp[c][warp] + my_rank] = (u32)v;
+#pragma unroll
+    for (u32 j = 0; j < kClassifyVertices; ++j) {
+      const u32 same = __match_any_sync(0xFFFFFFFFu, c[j]);
+      const int first = __ffs(same) - 1;
+      u32 at = 0;
+      if (c[j] >= 0 && lane == (u32)first) at = atomicAdd(&s_cnt[c[j]], (u32)__popc(same));
+      rank[j] = __shfl_sync(0xFFFFFFFFu, at, first) + __popc(same & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (threadIdx.x < K_CLASSES && s_cnt[threadIdx.x]) s_base[threadIdx.x] = atomicAdd(&cls[threadIdx.x], s_cnt[threadIdx.x]);
+    __syncthreads();
+#pragma unroll
+    for (u32 j = 0; j < kClassifyVertices; ++j)
+      if (c[j] >= 0) lists.list[c[j]][s_base[c[j]] + rank[j]] = (u32)(v0 + j * 256 + threadIdx.x);
     __syncthreads();
   }
+}
+
+// Vertices that class k can have at most, with E edges on V vertices.
+static u64 class_room(int k, u64 V, u64 E) {
+  static const u32 least[K_CLASSES] = {1, 9, 17, 33, 65, 129, 257, 513, 1025, 2049, kF64Max + 1, kMidSmemMax + 1, kHugeSmemMax + 1};
+  return std::min<u64>(V, E / least[k]) + 1;
 }
 
 // ------------------------------------------------------------------ bulk copy (TMA unit) ---
@@ -660,8 +637,8 @@ struct ClassItems {
     u32 off2, end2, v3;
   };
   __device__ __forceinline__ u32 vertex(u32 steps) const { return left > steps * stride ? __ldg(list + steps * stride) : 0u; }
-  __device__ __forceinline__ ClassItems(const u32* worklist, const u32* cls, int k, const u32* x, u32 first, u32 step)
-      : list(worklist + cls[2 * K_CLASSES + k] + first), xadj(x), left(cls[k] - min(cls[k], first)), stride(step) {
+  __device__ __forceinline__ ClassItems(const u32* all, u32 count, const u32* x, u32 first, u32 step)
+      : list(all + first), xadj(x), left(count - min(count, first)), stride(step) {
     v = vertex(0);
     v1 = vertex(1);
     v2 = vertex(2);
@@ -704,12 +681,12 @@ constexpr size_t kGroupBytes =
     std::max({sizeof(GroupShared<32, 16>), sizeof(GroupShared<16, 16>), sizeof(GroupShared<8, 16>),
               sizeof(GroupShared<4, 16>), sizeof(GroupShared<2, 16>), sizeof(GroupShared<1, 16>)});
 template <int G, int EPT>
-__device__ __forceinline__ void build_groups(unsigned char* smem, int k, const u32* worklist, const u32* cls, const u32* xadj,
+__device__ __forceinline__ void build_groups(unsigned char* smem, const u32* list, u32 count, const u32* xadj,
                                              const float* wgt, Slot* slots, uint8_t* valid, u32* err) {
   GroupShared<G, EPT>* sh = reinterpret_cast<GroupShared<G, EPT>*>(smem);  // this warp's
   const u32 in_warp = (threadIdx.x & 31) / G;
   const GroupCoop<G> co;
-  for (ClassItems c(worklist, cls, k, xadj, (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / G,
+  for (ClassItems c(list, count, xadj, (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / G,
                     gridDim.x * (kGroupWarps * 32 / G)); c.more();) {
     const ClassItems::After after = c.look_ahead(wgt, co.t, G >= 8 ? 32 : EPT);
     const u32 n = c.end - c.off;
@@ -727,18 +704,18 @@ __device__ __forceinline__ void build_groups(unsigned char* smem, int k, const u
 // All group classes in one launch, every warp taking its share of one class after the other: nothing orders them,
 // and as launches of their own they cost a small graph 9 us each.
 __global__ void __launch_bounds__(kGroupWarps * 32, kGroupCtas)
-    build_groups_kernel(const u32* __restrict__ worklist, const u32* __restrict__ cls, const u32* __restrict__ xadj,
+    build_groups_kernel(const ClassLists lists, const u32* __restrict__ cls, const u32* __restrict__ xadj,
                         const float* __restrict__ wgt, Slot* __restrict__ slots, uint8_t* __restrict__ valid,
                         u32* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char cta_smem[];
   unsigned char* smem = cta_smem + (threadIdx.x >> 5) * kGroupBytes;
-  build_groups<32, 16>(smem, K_32, worklist, cls, xadj, wgt, slots, valid, err);
-  build_groups<16, 16>(smem, K_16, worklist, cls, xadj, wgt, slots, valid, err);
-  build_groups<8, 16>(smem, K_8, worklist, cls, xadj, wgt, slots, valid, err);
-  build_groups<4, 16>(smem, K_4, worklist, cls, xadj, wgt, slots, valid, err);
-  build_groups<2, 16>(smem, K_2, worklist, cls, xadj, wgt, slots, valid, err);
-  build_groups<1, 16>(smem, K_1B, worklist, cls, xadj, wgt, slots, valid, err);
-  build_groups<1, 8>(smem, K_1A, worklist, cls, xadj, wgt, slots, valid, err);
+  build_groups<32, 16>(smem, lists.list[K_32], cls[K_32], xadj, wgt, slots, valid, err);
+  build_groups<16, 16>(smem, lists.list[K_16], cls[K_16], xadj, wgt, slots, valid, err);
+  build_groups<8, 16>(smem, lists.list[K_8], cls[K_8], xadj, wgt, slots, valid, err);
+  build_groups<4, 16>(smem, lists.list[K_4], cls[K_4], xadj, wgt, slots, valid, err);
+  build_groups<2, 16>(smem, lists.list[K_2], cls[K_2], xadj, wgt, slots, valid, err);
+  build_groups<1, 16>(smem, lists.list[K_1B], cls[K_1B], xadj, wgt, slots, valid, err);
+  build_groups<1, 8>(smem, lists.list[K_1A], cls[K_1A], xadj, wgt, slots, valid, err);
 }
 
 // 513 .. 4096 weights: one CTA of NT = 64, 128 or 256 threads per vertex.
@@ -749,14 +726,14 @@ struct ListShared {
   typename CtaCoop<NT>::Words words;
 };
 template <int NT>
-__global__ void __launch_bounds__(NT, 768 / NT) build_cta_kernel(const u32* __restrict__ worklist, const u32* __restrict__ cls,
-                                                       int k, const u32* __restrict__ xadj,
+__global__ void __launch_bounds__(NT, 768 / NT) build_cta_kernel(const u32* __restrict__ list, const u32* __restrict__ count,
+                                                       const u32* __restrict__ xadj,
                                                        const float* __restrict__ wgt, Slot* __restrict__ slots,
                                                        uint8_t* __restrict__ valid, u32* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem[];
   ListShared<NT>* sh = reinterpret_cast<ListShared<NT>*>(smem);
   const CtaCoop<NT> co(&sh->words);
-  for (ClassItems c(worklist, cls, k, xadj, blockIdx.x, gridDim.x); c.more();) {
+  for (ClassItems c(list, *count, xadj, blockIdx.x, gridDim.x); c.more();) {
     const ClassItems::After after = c.look_ahead(wgt, co.t, 32);
     const u32 n = c.end - c.off;
     if (n > ListShared<NT>::kMost || n == 0) {
@@ -778,7 +755,7 @@ __host__ __device__ constexpr int tile_pipe_bytes(int nt) { return 2 * (nt * 8 +
 // WIN > 0: lists in this CTA's slab of global scratch (cap entries of 12 bytes), merged through
 // windows of WIN outputs staged in dynamic shared memory.
 template <int NT, int WIN>
-__global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restrict__ worklist,
+__global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restrict__ list,
                                                              u32* __restrict__ cls, int k,
                                                              const u32* __restrict__ xadj,
                                                              const float* __restrict__ wgt,
@@ -792,7 +769,7 @@ __global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restri
   unsigned char* store = WIN ? scratch + (u64)blockIdx.x * cap * 12ull : smem;
   u64* A = reinterpret_cast<u64*>(store);
   u32* P = reinterpret_cast<u32*>(A + cap);
-  const u32 count = cls[k], base = cls[2 * K_CLASSES + k];
+  const u32 count = cls[k];
   __shared__ u32 s_it;
   // Weight tiles brought in by the bulk-copy engine: two buffers behind the merge windows (WIN > 0), one
   // buffer behind the lists of the shared-memory classes (two 512-thread CTAs with 96 KB of lists and a
@@ -805,12 +782,12 @@ __global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restri
   }
   __syncthreads();
   for (;;) {  // next vertex from the class's atomic cursor (degrees, hence costs, vary widely)
-    if (threadIdx.x == 0) s_it = atomicAdd(cls + 3 * K_CLASSES + k, 1u);
+    if (threadIdx.x == 0) s_it = atomicAdd(cls + K_CLASSES + k, 1u);
     __syncthreads();
     const u32 it = s_it;
     __syncthreads();
     if (it >= count) break;
-    const u32 v = worklist[base + it];
+    const u32 v = list[it];
     const u32 off = xadj[v], n = xadj[v + 1] - off;
     if (n > cap) {
       if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, (u32)cap);
@@ -997,9 +974,8 @@ __device__ void build_vertex_cta(u32 v, u32 off, u32 n, const float* __restrict_
   if (tid == 0) valid[v] = 1;
 }
 
-// Launch the class builders over work lists laid out as cls describes (counts at [k],
-// bases at [2K + k]).
-static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
+// Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`.
+static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot* slots, uint8_t* valid) {
   cudaStream_t st = ctx->stream;
   constexpr int kCta2Smem = kHugeSmemMax * 12 + tile_pipe_bytes(1024) / 2;  // lists + one weight tile
   constexpr int kCta2aSmem = kMidSmemMax * 12 + tile_pipe_bytes(512) / 2;  // lists + one weight tile
@@ -1050,18 +1026,18 @@ static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
   }
   if (slab_elems) {
     build_cta_merge_kernel<1024, kWin><<<gmem_ctas, 1024, kWinSmem, s_h>>>(
-        worklist, cls, K_H, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid,
+        lists.list[K_H], cls, K_H, ctx->xadj, ctx->adjwgt, slots, valid,
         static_cast<unsigned char*>(ctx->cta_scratch), slab_elems, ctx->d_err);
     SKW_LAUNCHED(ctx);
   }
   if (ctx->max_degree > kMidSmemMax) {
     build_cta_merge_kernel<1024, 0><<<ctx->sm_count, 1024, kCta2Smem, s_a>>>(
-        worklist, cls, K_C2, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, nullptr, kHugeSmemMax, ctx->d_err);
+        lists.list[K_C2], cls, K_C2, ctx->xadj, ctx->adjwgt, slots, valid, nullptr, kHugeSmemMax, ctx->d_err);
     SKW_LAUNCHED(ctx);
   }
   if (ctx->max_degree > kF64Max) {
     build_cta_merge_kernel<512, 0><<<ctx->sm_count * 2, 512, kCta2aSmem, s_b>>>(
-        worklist, cls, K_C2A, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, nullptr, kMidSmemMax, ctx->d_err);
+        lists.list[K_C2A], cls, K_C2A, ctx->xadj, ctx->adjwgt, slots, valid, nullptr, kMidSmemMax, ctx->d_err);
     SKW_LAUNCHED(ctx);
   }
   // 24 warps an SM: what the registers and the shared memory of these kernels allow, all of them resident at once
@@ -1069,7 +1045,7 @@ static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
 #define LISTS(MORE_THAN, KCLS, NT, STREAM)                                                                      \
   if (ctx->max_degree > (MORE_THAN)) {                                                                          \
     build_cta_kernel<NT><<<ctx->sm_count * (768 / (NT)), NT, sizeof(ListShared<NT>), STREAM>>>(                 \
-        worklist, cls, KCLS, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);                       \
+        lists.list[KCLS], cls + KCLS, ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err);                       \
     SKW_LAUNCHED(ctx);                                                                                          \
   }
   LISTS(2048, K_C256, 256, s_c)
@@ -1077,7 +1053,7 @@ static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
   LISTS(512, K_C64, 64, s_b)
 #undef LISTS
   build_groups_kernel<<<ctx->sm_count * kGroupCtas, kGroupWarps * 32, kGroupSmem, st>>>(
-      worklist, cls, ctx->xadj, ctx->adjwgt, ctx->slots, ctx->valid, ctx->d_err);
+      lists, cls, ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err);
   SKW_LAUNCHED(ctx);
   if (fork) {
     for (int i = 0; i < skw_ctx::kBuilderStreams; ++i) {
@@ -1094,19 +1070,10 @@ static int launch_builders(skw_ctx* ctx, const u32* worklist, u32* cls) {
 // units still running.  A vertex is claimed by the first unit that stamps it in the current collection.
 constexpr u32 kAliveMark = 0xFFFFFFFFu;
 
-__global__ void frontier_reset_kernel(u32* __restrict__ cls, u32 cap) {
-  if (threadIdx.x < K_CLASSES) {
-    cls[threadIdx.x] = 0;
-    cls[K_CLASSES + threadIdx.x] = 0;
-    cls[2 * K_CLASSES + threadIdx.x] = threadIdx.x * cap;
-    cls[3 * K_CLASSES + threadIdx.x] = 0;
-  }
-}
-
 __global__ void __launch_bounds__(256) frontier_collect_kernel(
     const u32* __restrict__ verts, u64 units, u32 width, u32 cells, u32 offs,
     const u32* __restrict__ alive, const u32* __restrict__ xadj, u32 V, u32* __restrict__ stamp,
-    u32 round, u32* __restrict__ cls, u32* __restrict__ lists, u32 cap, u32* __restrict__ err) {
+    u32 round, u32* __restrict__ cls, const ClassLists lists, u32 cap, u32* __restrict__ err) {
   const u32 lane = threadIdx.x & 31;
   const u64 T = (u64)gridDim.x * blockDim.x;
   for (u64 u0 = (u64)blockIdx.x * blockDim.x; u0 < units; u0 += T) {
@@ -1135,7 +1102,7 @@ __global__ void __launch_bounds__(256) frontier_collect_kernel(
       base = __shfl_sync(0xFFFFFFFFu, base, __ffs(m) - 1);
       if (c == k) {
         const u32 idx = base + __popc(m & ((1u << lane) - 1u));
-        if (idx < cap) lists[(u64)k * cap + idx] = v;
+        if (idx < cap) lists.list[k][idx] = v;
         else dev_fail(err, DEV_ERR_CAPACITY, idx, cap, 11);
       }
     }
@@ -1163,17 +1130,18 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
     ctx->stamp_round = 1;
   }
   cudaStream_t st = ctx->stream;
-  frontier_reset_kernel<<<1, 32, 0, st>>>(ctx->frontier_cls, cap);
-  SKW_LAUNCHED(ctx);
+  SKW_CUDA(ctx, cudaMemsetAsync(ctx->frontier_cls, 0, 2 * K_CLASSES * sizeof(u32), st));
   if (units) {
     // the claim is a chain of dependent accesses (vertex, offsets, stamp): fill every thread slot of the GPU
     const u64 want = (units + 255) / 256;
     const int grid = (int)(want < (u64)ctx->sm_count * 16 ? want : (u64)ctx->sm_count * 16);
+    ClassLists lists;
+    for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->frontier_lists + (size_t)k * cap;
     frontier_collect_kernel<<<grid, 256, 0, st>>>(verts, units, width, cells, offs, alive_lengths,
                                                   ctx->xadj, ctx->V, ctx->stamp, ctx->stamp_round,
-                                                  ctx->frontier_cls, ctx->frontier_lists, cap, ctx->d_err);
+                                                  ctx->frontier_cls, lists, cap, ctx->d_err);
     SKW_LAUNCHED(ctx);
-    rc = launch_builders(ctx, ctx->frontier_lists, ctx->frontier_cls);
+    rc = launch_builders(ctx, lists, ctx->frontier_cls, ctx->slots, ctx->valid);
     if (rc != SKW_OK) return rc;
   }
   return SKW_OK;
@@ -1203,6 +1171,30 @@ extern "C" int skw_selftest_bounded_wait(skw_ctx* ctx) {
   return err_check(ctx, "skw_selftest_bounded_wait");
 }
 
+namespace skw {
+// Queue the construction of the tables of vertices [v_begin, v_end) into `slots` and `valid`.
+int enqueue_tables(skw_ctx* ctx, u32 v_begin, u32 v_end, Slot* slots, uint8_t* valid) {
+  if (v_end <= v_begin) return SKW_OK;
+  u64 words = 0, at[K_CLASSES];
+  for (int k = 0; k < K_CLASSES; ++k) {
+    at[k] = words;
+    words += class_room(k, v_end - v_begin, ctx->E);
+  }
+  void* wl = ctx->worklist;
+  int rc = ensure_bytes(ctx, &wl, &ctx->worklist_cap, sizeof(u32) * words);
+  ctx->worklist = static_cast<u32*>(wl);
+  if (rc != SKW_OK) return rc;
+  ClassLists lists;
+  for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->worklist + at[k];
+  SKW_CUDA(ctx, cudaMemsetAsync(ctx->cls_counts, 0, 2 * K_CLASSES * sizeof(u32), ctx->stream));
+  const u64 tiles = ((u64)(v_end - v_begin) + 256 * kClassifyVertices - 1) / (256 * kClassifyVertices);
+  classify_kernel<<<(unsigned)std::min<u64>(tiles, (u64)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
+      ctx->xadj, v_begin, v_end, ctx->cls_counts, lists, valid);
+  SKW_LAUNCHED(ctx);
+  return launch_builders(ctx, lists, ctx->cls_counts, slots, valid);
+}
+}  // namespace skw
+
 extern "C" int skw_alias_build_offline(skw_ctx* ctx, uint32_t v_begin, uint32_t v_end, float* ms) {
   if (!ctx) return SKW_ERR_ARG;
   if (!ctx->xadj) return fail(ctx, SKW_ERR_STATE, "skw_alias_build_offline: no graph resident");
@@ -1218,26 +1210,11 @@ extern "C" int skw_alias_build_offline(skw_ctx* ctx, uint32_t v_begin, uint32_t 
   ctx->records_ready = false;
   int rc = alloc_table(ctx);
   if (rc != SKW_OK) return rc;
-  void* wl = ctx->worklist;
-  rc = ensure_bytes(ctx, &wl, &ctx->worklist_cap, sizeof(uint32_t) * ((size_t)ctx->V + 1));
-  ctx->worklist = static_cast<uint32_t*>(wl);
-  if (rc != SKW_OK) return rc;
   rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
   cudaStream_t st = ctx->stream;
-  SKW_CUDA(ctx, cudaMemsetAsync(ctx->cls_counts, 0, 4 * K_CLASSES * sizeof(uint32_t), st));
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
-  if (v_end > v_begin) {
-    const int cgrid = ctx->sm_count * 8;
-    classify_count_kernel<<<cgrid, 256, 0, st>>>(ctx->xadj, v_begin, v_end, ctx->cls_counts, ctx->valid);
-    SKW_LAUNCHED(ctx);
-    classify_bases_kernel<<<1, 32, 0, st>>>(ctx->cls_counts);
-    SKW_LAUNCHED(ctx);
-    classify_fill_kernel<<<cgrid, 256, 0, st>>>(ctx->xadj, v_begin, v_end, ctx->cls_counts, ctx->worklist);
-    SKW_LAUNCHED(ctx);
-    rc = launch_builders(ctx, ctx->worklist, ctx->cls_counts);
-    if (rc != SKW_OK) return rc;
-  }
+  if ((rc = enqueue_tables(ctx, v_begin, v_end, ctx->slots, ctx->valid)) != SKW_OK) return rc;
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   rc = err_check(ctx, "skw_alias_build_offline");
   if (rc != SKW_OK) return rc;

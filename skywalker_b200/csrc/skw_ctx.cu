@@ -104,6 +104,10 @@ static void free_graph(skw_ctx* ctx) {
   ctx->owns_graph = ctx->owns_weights = false;
   cudaFree(ctx->slots);
   cudaFree(ctx->valid);
+  cudaFree(ctx->online_slots);
+  cudaFree(ctx->online_valid);
+  ctx->online_slots = nullptr;
+  ctx->online_valid = nullptr;
   cudaFree(ctx->stamp);
   cudaFree(ctx->prep_memo);
   cudaFree(ctx->prep_ckpt);

@@ -55,6 +55,9 @@ struct skw_ctx {
   skw::Slot* slots = nullptr;
   uint8_t* valid = nullptr;
   bool table_ready = false;
+  // tables of one online call (the table above stays as it is)
+  skw::Slot* online_slots = nullptr;
+  uint8_t* online_valid = nullptr;
   // optional fused walk records (32 B per edge slot) and per-vertex {offset, usable degree}
   void* records = nullptr;
   void* vinfo = nullptr;
@@ -71,9 +74,9 @@ struct skw_ctx {
   bool status_clean = true;  // error record and sums 0 and 3 are zero
 
   // builder scratch, grown on demand
-  uint32_t* worklist = nullptr;      // V entries, vertices grouped by degree class
+  uint32_t* worklist = nullptr;      // vertices by degree class, one list per class
   size_t worklist_cap = 0;
-  uint32_t* cls_counts = nullptr;    // per degree class: count, fill cursor, base in the work list
+  uint32_t* cls_counts = nullptr;    // per degree class: count, then cursor
   void* cta_scratch = nullptr;       // slabs of the global-memory CTA builder
   size_t cta_scratch_bytes = 0;
 
@@ -108,6 +111,8 @@ int fail(skw_ctx* ctx, int code, const char* fmt, ...);
 int finish_graph(skw_ctx* ctx);
 // allocate slots[E] / valid[V] if absent
 int alloc_table(skw_ctx* ctx);
+// queue the construction of the tables of vertices [v_begin, v_end)
+int enqueue_tables(skw_ctx* ctx, uint32_t v_begin, uint32_t v_end, Slot* slots, uint8_t* valid);
 // forget the fused walk records (they are derived from the table and die with it) and free their memory
 void drop_records(skw_ctx* ctx);
 // cudaMalloc that gives up the memory of records that are no longer valid before it fails

@@ -14,6 +14,7 @@
 // word x -> column (multiply-high by the degree), y -> acceptance uniform, z -> PPR stop test,
 // w -> node2vec rejection uniform.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <thread>
@@ -877,20 +878,48 @@ static int walk_check(skw_ctx* ctx, const skw_walk_params* prm) {
   return SKW_OK;
 }
 
+// Whether an online batch is better served by building the tables of the whole graph (into memory of its own, for this
+// call) than by computing its slots one by one.  A slot computed from the weights costs 2.7 ns of a full GPU and 7.5 us
+// of a walker's time, and the first visit of a list 25 ns a weight of it (a batch that makes enough steps to meet the
+// longest list waits for that); a table costs 10 ps an edge of the graph and some 60 us to launch, and a step over it 0.15 ns or
+// 1.2 us.  40,000 x 80 node2vec on 204 M edges: 8.7 ms computed, 2.6 ms with tables; 256 x 80 on 4 M edges: 0.61
+// against 0.2 ms; 256 x 5 on 117 M edges is 0.04 ms computed.  The figures are those of a B200; where the line
+// lies exactly matters little, since near it both ways take the same time.
+static bool tables_pay(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
+  double longest = prm->hop_num - 1.0, steps = longest;
+  if (prm->app == SKW_APP_PPR && prm->tp > 0.0f) {
+    longest = std::min(longest, (log((double)n) + 1.0) / prm->tp);
+    steps = std::min(steps, 1.0 / prm->tp);
+  }
+  steps *= (double)n;
+  const double hub = steps * ctx->max_degree >= (double)ctx->E ? 25e-9 * ctx->max_degree : 0.0;
+  const double computed = std::max(7.5e-6 * longest + hub, 2.7e-9 * steps);
+  const double tables = 60e-6 + 10e-12 * (double)ctx->E + std::max(1.2e-6 * longest, 0.15e-9 * steps);
+  return tables < computed;
+}
+
+// Memory for such tables: 8 bytes an edge, kept until the graph changes.  False when there is none to be had.
+static bool online_table_memory(skw_ctx* ctx) {
+  if (ctx->online_slots) return true;
+  if (dev_malloc(ctx, reinterpret_cast<void**>(&ctx->online_slots), sizeof(Slot) * (ctx->E ? ctx->E : 1)) == cudaSuccess &&
+      dev_malloc(ctx, reinterpret_cast<void**>(&ctx->online_valid), ctx->V ? ctx->V : 1) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  cudaFree(ctx->online_slots);
+  ctx->online_slots = nullptr;
+  return false;
+}
+
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
-// No reset, no readback, no synchronisation (the online table path allocates on first use).
+// No reset, no readback, no synchronisation (the online paths allocate on first use).
 static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n,
                        uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum) {
   const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
   const bool online = prm->mode == SKW_MODE_ONLINE && !unbiased;
   int rc;
-  // Online walks evaluate the slot they draw straight from the weights; on request they build the
-  // tables of the frontier at every step instead (same walks).  With the per-vertex memo and the
-  // prefix checkpoints a slot evaluation costs two or three tiles of weights whatever the degree,
-  // while a table costs its whole list once per distinct frontier vertex and step, so the direct path
-  // is the default for every batch shape.
-  bool build_tables = false;
-  if (online) build_tables = (prm->flags & (SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES)) != 0;
+  // Online walks make one launch over tables of the whole graph or one that computes every slot it draws, whichever
+  // pays; on request they build the tables of the frontier at every step (same walks).
+  const bool build_tables = online && (prm->flags & (SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES)) != 0;
   if (build_tables) {
     drop_records(ctx);  // online builds overwrite table slots
     if ((rc = alloc_table(ctx)) != SKW_OK) return rc;
@@ -917,6 +946,12 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   a.inv_q = prm->app == SKW_APP_NODE2VEC ? 1.0f / prm->q : 1.0f;
   a.fmax = fmaxf(1.0f, fmaxf(a.inv_p, a.inv_q));
   cudaStream_t st = ctx->stream;
+  const bool whole_table = online && !build_tables && !(prm->flags & SKW_WALK_DIRECT_SLOTS) && tables_pay(ctx, prm, n) &&
+                           online_table_memory(ctx);
+  if (whole_table) {
+    if ((rc = enqueue_tables(ctx, 0, ctx->V, ctx->online_slots, ctx->online_valid)) != SKW_OK) return rc;
+    a.slots = ctx->online_slots;
+  }
   // Walk records serve unbiased walks as well (the record of column c names the c-th neighbour with its
   // offset and degree: one access per step instead of two), as long as every vertex with out-edges has
   // a usable table, i.e. the degrees in the records are the graph's own.
@@ -946,7 +981,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     } else if (prm->app == SKW_APP_PPR) walk_records_walk_kernel<SKW_APP_PPR><<<grid, 256, 0, st>>>(ra);
     else walk_records_walk_kernel<SKW_APP_DEEPWALK><<<grid, 256, 0, st>>>(ra);
     SKW_LAUNCHED(ctx);
-  } else if (!online) {
+  } else if (!online || whole_table) {
     const int grid = walk_grid(prm->app, n);
     switch (prm->app) {
       case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<grid, 256, 0, st>>>(a); break;
