@@ -15,6 +15,7 @@ Buffers may be numpy arrays (host entry points; copies happen inside the call) o
 `data_ptr()` method such as a CUDA torch tensor (device entry points; no copies).
 """
 import ctypes as C
+import functools
 import threading
 import weakref
 
@@ -329,6 +330,11 @@ class Context:
     # -- k-hop
     @staticmethod
     def khop_layout(fanout):
+        return Context._khop_layout(tuple(fanout))
+
+    @staticmethod
+    @functools.lru_cache(maxsize=64)
+    def _khop_layout(fanout):
         if not 1 <= len(fanout) <= 4:
             raise SkwError(-1, "k-hop sampling takes 1 to 4 hops, got %d" % len(fanout))
         prm = KhopParams(0, len(fanout), (C.c_uint32 * 4)(*(list(fanout) + [0] * (4 - len(fanout)))), 0, 0, 0, 1)

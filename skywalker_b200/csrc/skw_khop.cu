@@ -5,10 +5,10 @@
 // writing the Jobs_result<NS> tree (include/sampler_result.cuh:226-260, 334-352, 421-426).
 //
 // The reference drains per-hop job queues with one thread (offline) or one warp (online) per
-// frontier vertex.  Here a hop is one launch with one thread per OUTPUT cell: thread
+// frontier vertex.  Here one thread works on an OUTPUT cell: thread
 // (seed s, parent idx, child j) reads the parent vertex, makes its own Philox draw keyed by
 // (seed id, child cell, hop) and stores one coalesced word; no queues and no atomics on the data
-// path.  Online mode first builds the tables of the distinct vertices of the hop's frontier with
+// path.  Offline a CTA makes the whole trees of a few seeds; online mode goes hop by hop, and first builds the tables of the distinct vertices of the hop's frontier with
 // the degree-bucketed builders, then runs the same draw kernel.
 #include <algorithm>
 #include <string>
@@ -22,10 +22,13 @@ namespace skw {
 int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 cells, u32 offs,
                      const u32* alive_lengths, bool new_round);
 
+constexpr u32 kDistinctMaxFanout = 256, kDistinctRounds = 11;
+
 struct KhopArgs {
   const u32* xadj;
   const u32* adjncy;
   const Slot* slots;
+  const u32* seeds;
   u32* data;
   u32* lens;
   unsigned long long* sum;
@@ -36,67 +39,40 @@ struct KhopArgs {
   u64 instance_stride;
   u32 V;
   u32 cells, lens_per;
-  u32 offs_parent, offs_child, width_parent, fanout, hop, flags;
+  u32 flags;
+  u32 nhops;
+  u32 fanout[4], width[5], offs[5];  // per hop: samples a vertex, vertices a seed, their first cell in a row
 };
 
-__global__ void __launch_bounds__(256) khop_init_kernel(const u32* __restrict__ seeds, u64 n,
-                                                        u32 cells, u32* __restrict__ data) {
-  for (u64 s = (u64)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (u64)gridDim.x * blockDim.x)
-    data[s * cells] = seeds[s];
-}
-
-__global__ void __launch_bounds__(256) khop_hop_kernel(const KhopArgs a) {
-  const u64 per_seed = (u64)a.width_parent * a.fanout;
-  const u64 total = a.n * per_seed;
-  u64 got_sum = 0;
-  for (u64 u = (u64)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (u64)gridDim.x * blockDim.x) {
-    const u64 s = u / per_seed;
-    const u32 rem = (u32)(u - s * per_seed);
-    const u32 idx = rem / a.fanout, j = rem - idx * a.fanout;
-    u32* row = a.data + s * a.cells;
-    const u32 v = row[a.offs_parent + idx];
-    u32 out = SKW_INVALID_VERTEX, got = 0;
-    if (v != SKW_INVALID_VERTEX) {
-      if (v >= a.V) {
-        dev_fail(a.err, DEV_ERR_INDEX, v, idx, a.hop);
-      } else {
-        const u32 off = __ldg(a.xadj + v), deg = __ldg(a.xadj + v + 1) - off;
-        if (deg) {
-          if ((a.flags & SKW_KHOP_TAKE_ALL) && a.fanout >= deg) {
-            got = deg;
-            if (j < deg) out = __ldg(a.adjncy + (u64)off + j);
-          } else {
-            const Rand4 r = philox_tagged(a.seed, TAG_KHOP, a.instance_base + s * a.instance_stride, rem, a.hop);
-            const u32 col = __umulhi(r.x, deg);
-            if (a.flags & SKW_KHOP_UNBIASED) {
-              out = ldg_once(a.adjncy + (u64)off + col);
-              got = a.fanout;
-              goto store;
-            }
-            const Slot sl = load_slot(a.slots + (u64)off + col);
-            if (!(sl.prob < 0.0f)) {
-              const u32 cand = u01(r.y) < sl.prob ? col : sl.alias;
-              if (cand >= deg) {  // a table that does not belong to this graph
-                dev_fail(a.err, DEV_ERR_INDEX, v, cand, 23);
-              } else {
-                out = ldg_once(a.adjncy + (u64)off + cand);
-                got = a.fanout;
-              }
-            }
-          }
-        }
-      }
-    }
-  store:
-    row[a.offs_child + rem] = out;
-    if (j == 0) {
-      a.lens[s * a.lens_per + a.offs_parent + idx] = got;
-      got_sum += got;
+// Child j of the vertex v at place idx of hop h of seed s: the cell's value, and in `got` how many children v has.
+__device__ __forceinline__ u32 khop_child(const KhopArgs& a, u64 s, u32 v, u32 h, u32 idx, u32 j, u32& got) {
+  got = 0;
+  if (v == SKW_INVALID_VERTEX) return SKW_INVALID_VERTEX;
+  if (v >= a.V) {
+    dev_fail(a.err, DEV_ERR_INDEX, v, idx, h + 1);
+    return SKW_INVALID_VERTEX;
+  }
+  const u32 fanout = a.fanout[h];
+  const u32 off = __ldg(a.xadj + v), deg = __ldg(a.xadj + v + 1) - off;
+  if (deg == 0) return SKW_INVALID_VERTEX;
+  if ((a.flags & SKW_KHOP_TAKE_ALL) && fanout >= deg) {
+    got = deg;
+    return j < deg ? __ldg(a.adjncy + (u64)off + j) : SKW_INVALID_VERTEX;
+  }
+  const Rand4 r = philox_tagged(a.seed, TAG_KHOP, a.instance_base + s * a.instance_stride, idx * fanout + j, h + 1);
+  const u32 col = __umulhi(r.x, deg);
+  u32 cand = col;
+  if (!(a.flags & SKW_KHOP_UNBIASED)) {
+    const Slot sl = load_slot(a.slots + (u64)off + col);
+    if (sl.prob < 0.0f) return SKW_INVALID_VERTEX;
+    cand = u01(r.y) < sl.prob ? col : sl.alias;
+    if (cand >= deg) {  // a table that does not belong to this graph
+      dev_fail(a.err, DEV_ERR_INDEX, v, cand, 23);
+      return SKW_INVALID_VERTEX;
     }
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) got_sum += __shfl_xor_sync(0xFFFFFFFFu, got_sum, o);
-  if ((threadIdx.x & 31) == 0 && got_sum) atomicAdd(a.sum, (unsigned long long)got_sum);
+  got = fanout;
+  return ldg_once(a.adjncy + (u64)off + cand);
 }
 
 // SKW_KHOP_DISTINCT: one warp per parent vertex.  A parent whose degree is <= the fan-out hands over
@@ -105,71 +81,157 @@ __global__ void __launch_bounds__(256) khop_hop_kernel(const KhopArgs a) {
 // (seed id, parent index, trial, hop); a draw counts when its column was not drawn by an earlier trial.
 // "Earlier" is decided without atomics: columns accepted in earlier rounds sit in a per-warp list in
 // shared memory, and inside a round the lowest lane holding a column wins (match_any), so the result
-// is the one a sequential pass over the trials gives.
-constexpr u32 kDistinctMaxFanout = 256, kDistinctRounds = 11;
-__global__ void __launch_bounds__(256) khop_distinct_kernel(const KhopArgs a) {
-  __shared__ u32 s_seen[8][kDistinctMaxFanout];
-  const u32 lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const u64 warp = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5;
-  const u64 parents = a.n * a.width_parent;
-  const u32 f = a.fanout;
-  u32* seen = s_seen[wib];
+// is the one a sequential pass over the trials gives.  Returns the number of children.
+__device__ __forceinline__ u32 khop_distinct_children(const KhopArgs& a, u64 s, u32 v, u32 h, u32 idx, u32* child, u32* seen) {
+  const u32 lane = threadIdx.x & 31, f = a.fanout[h];
+  u32 got = 0, off = 0, deg = 0;
+  if (v != SKW_INVALID_VERTEX) {
+    if (v >= a.V) {
+      if (lane == 0) dev_fail(a.err, DEV_ERR_INDEX, v, idx, h + 1);
+    } else {
+      off = __ldg(a.xadj + v);
+      deg = __ldg(a.xadj + v + 1) - off;
+    }
+  }
+  if (deg && f >= deg) {
+    for (u32 j = lane; j < deg; j += 32) child[j] = __ldg(a.adjncy + (u64)off + j);
+    got = deg;
+  } else if (deg) {
+    const u64 gi = a.instance_base + s * a.instance_stride;
+    for (u32 round = 0; round < kDistinctRounds && got < f; ++round) {
+      const u32 t = round * 32 + lane;
+      const Rand4 r = philox_tagged(a.seed, TAG_KHOP, gi, idx, (t << 8) | 0x80u | (h + 1));
+      const u32 col = __umulhi(r.x, deg);
+      const Slot sl = load_slot(a.slots + (u64)off + col);
+      if (sl.prob < 0.0f) break;  // vertex without usable weight: the same in every lane
+      u32 cand = u01(r.y) < sl.prob ? col : sl.alias;
+      if (cand >= deg) {  // a table that does not belong to this graph
+        dev_fail(a.err, DEV_ERR_INDEX, v, cand, 24);
+        cand = 0;
+      }
+      bool fresh = true;
+      for (u32 i = 0; i < got; ++i) fresh = fresh && seen[i] != cand;
+      const u32 same = __match_any_sync(0xFFFFFFFFu, cand);
+      fresh = fresh && lane == (u32)(__ffs(same) - 1);
+      const u32 acc = __ballot_sync(0xFFFFFFFFu, fresh);
+      const u32 at = got + __popc(acc & ((1u << lane) - 1u));
+      if (fresh && at < f) {
+        seen[at] = cand;
+        child[at] = ldg_once(a.adjncy + (u64)off + cand);
+      }
+      got = min(f, got + (u32)__popc(acc));
+      __syncwarp();
+    }
+  }
+  for (u32 j = got + lane; j < f; j += 32) child[j] = SKW_INVALID_VERTEX;
+  return got;
+}
+
+__device__ __forceinline__ void khop_add(unsigned long long* sum, u64 mine) {
+  __shared__ unsigned long long s_sum;
+  if (threadIdx.x == 0) s_sum = 0;
+  __syncthreads();
+#pragma unroll
+  for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xFFFFFFFFu, mine, o);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&s_sum, (unsigned long long)mine);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_sum) atomicAdd(sum, s_sum);
+}
+
+// Whole trees, per_cta seeds a CTA, hop after hop with a barrier in between: one launch where the hops as launches of
+// their own are a chain of four for three hops.  1,000 seeds x 15, 10, 5: 54 -> 46 us a call; 65,536 x 25, 10: 201 ->
+// 159 us, the parents being in cache and the cell numbers 32-bit.  A
+// hop's parents were written by this CTA, so they are read with plain loads.
+template <bool DISTINCT>
+__global__ void __launch_bounds__(256) khop_tree_kernel(const KhopArgs a, u32 per_cta) {
+  __shared__ u32 s_seen[DISTINCT ? 8 : 1][DISTINCT ? kDistinctMaxFanout : 1];
+  const u64 s0 = (u64)blockIdx.x * per_cta;
+  const u32 ns = (u32)min((u64)per_cta, a.n - s0);
+  u32* rows = a.data + s0 * a.cells;
   u64 got_sum = 0;
-  for (u64 u = warp; u < parents; u += nwarps) {
-    const u64 s = u / a.width_parent;
-    const u32 idx = (u32)(u - s * a.width_parent);
+  for (u32 i = threadIdx.x; i < ns; i += 256) rows[(u64)i * a.cells] = __ldg(a.seeds + s0 + i);
+  for (u32 h = 0; h < a.nhops; ++h) {
+    __syncthreads();
+    const u32 f = a.fanout[h], wp = a.width[h], wc = a.width[h + 1];
+    if constexpr (DISTINCT) {
+      u32* seen = s_seen[threadIdx.x >> 5];
+      for (u32 u = threadIdx.x >> 5; u < ns * wp; u += 8) {
+        const u32 i = u / wp, idx = u - i * wp;
+        u32* row = rows + (u64)i * a.cells;
+        const u32 got = khop_distinct_children(a, s0 + i, row[a.offs[h] + idx], h, idx, row + a.offs[h + 1] + (u64)idx * f, seen);
+        if ((threadIdx.x & 31) == 0) {
+          a.lens[(s0 + i) * a.lens_per + a.offs[h] + idx] = got;
+          got_sum += got;
+        }
+        __syncwarp();  // the list is reused by the next parent
+      }
+    } else {
+      for (u32 u = threadIdx.x; u < ns * wc; u += 256) {
+        const u32 i = u / wc, rem = u - i * wc, idx = rem / f, j = rem - idx * f;
+        u32* row = rows + (u64)i * a.cells;
+        u32 got;
+        row[a.offs[h + 1] + rem] = khop_child(a, s0 + i, row[a.offs[h] + idx], h, idx, j, got);
+        if (j == 0) {
+          a.lens[(s0 + i) * a.lens_per + a.offs[h] + idx] = got;
+          got_sum += got;
+        }
+      }
+    }
+  }
+  khop_add(a.sum, got_sum);
+}
+
+// One hop of every tree (online mode, whose tables are built hop by hop, and trees that are too large for a CTA).
+__global__ void __launch_bounds__(256) khop_init_kernel(const u32* __restrict__ seeds, u64 n,
+                                                        u32 cells, u32* __restrict__ data) {
+  for (u64 s = (u64)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (u64)gridDim.x * blockDim.x)
+    data[s * cells] = seeds[s];
+}
+
+__global__ void __launch_bounds__(256) khop_hop_kernel(const KhopArgs a, u32 h) {
+  const u32 per_seed = a.width[h + 1], f = a.fanout[h];
+  const u64 total = a.n * per_seed, T = (u64)gridDim.x * blockDim.x;
+  u64 got_sum = 0;
+  // (seed, cell) of this thread, moved on by the stride: a 64-bit division a cell is a third of the instructions
+  u64 s = ((u64)blockIdx.x * blockDim.x + threadIdx.x) / per_seed;
+  u32 rem = (u32)(((u64)blockIdx.x * blockDim.x + threadIdx.x) - s * per_seed);
+  const u64 ds = T / per_seed;
+  const u32 dr = (u32)(T - ds * per_seed);
+  for (u64 u = (u64)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += T) {
+    const u32 idx = rem / f, j = rem - idx * f;
     u32* row = a.data + s * a.cells;
-    u32* child = row + a.offs_child + (u64)idx * f;
-    const u32 v = row[a.offs_parent + idx];
-    u32 got = 0;
-    u32 off = 0, deg = 0;
-    if (v != SKW_INVALID_VERTEX) {
-      if (v >= a.V) {
-        if (lane == 0) dev_fail(a.err, DEV_ERR_INDEX, v, idx, a.hop);
-      } else {
-        off = __ldg(a.xadj + v);
-        deg = __ldg(a.xadj + v + 1) - off;
-      }
-    }
-    if (deg && f >= deg) {
-      for (u32 j = lane; j < deg; j += 32) child[j] = __ldg(a.adjncy + (u64)off + j);
-      got = deg;
-    } else if (deg) {
-      const u64 gi = a.instance_base + s * a.instance_stride;
-      for (u32 round = 0; round < kDistinctRounds && got < f; ++round) {
-        const u32 t = round * 32 + lane;
-        const Rand4 r = philox_tagged(a.seed, TAG_KHOP, gi, idx, (t << 8) | 0x80u | a.hop);
-        const u32 col = __umulhi(r.x, deg);
-        const Slot sl = load_slot(a.slots + (u64)off + col);
-        if (sl.prob < 0.0f) break;  // vertex without usable weight: the same in every lane
-        u32 cand = u01(r.y) < sl.prob ? col : sl.alias;
-        if (cand >= deg) {  // a table that does not belong to this graph
-          dev_fail(a.err, DEV_ERR_INDEX, v, cand, 24);
-          cand = 0;
-        }
-        bool fresh = true;
-        for (u32 i = 0; i < got; ++i) fresh = fresh && seen[i] != cand;
-        const u32 same = __match_any_sync(0xFFFFFFFFu, cand);
-        fresh = fresh && lane == (u32)(__ffs(same) - 1);
-        const u32 acc = __ballot_sync(0xFFFFFFFFu, fresh);
-        const u32 at = got + __popc(acc & ((1u << lane) - 1u));
-        if (fresh && at < f) {
-          seen[at] = cand;
-          child[at] = ldg_once(a.adjncy + (u64)off + cand);
-        }
-        got = min(f, got + (u32)__popc(acc));
-        __syncwarp();
-      }
-    }
-    for (u32 j = got + lane; j < f; j += 32) child[j] = SKW_INVALID_VERTEX;
-    if (lane == 0) {
-      a.lens[s * a.lens_per + a.offs_parent + idx] = got;
+    u32 got;
+    row[a.offs[h + 1] + rem] = khop_child(a, s, row[a.offs[h] + idx], h, idx, j, got);
+    if (j == 0) {
+      a.lens[s * a.lens_per + a.offs[h] + idx] = got;
       got_sum += got;
     }
-    __syncwarp();  // the list is reused by the next parent
+    s += ds;
+    const u64 r = (u64)rem + dr;
+    s += r >= per_seed ? 1 : 0;
+    rem = (u32)(r >= per_seed ? r - per_seed : r);
   }
-  if (lane == 0 && got_sum) atomicAdd(a.sum, (unsigned long long)got_sum);
+  khop_add(a.sum, got_sum);
+}
+
+__global__ void __launch_bounds__(256) khop_distinct_kernel(const KhopArgs a, u32 h) {
+  __shared__ u32 s_seen[8][kDistinctMaxFanout];
+  const u32 wp = a.width[h];
+  const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5, parents = a.n * wp;
+  u64 got_sum = 0;
+  for (u64 u = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < parents; u += nwarps) {
+    const u64 s = u / wp;
+    const u32 idx = (u32)(u - s * wp);
+    u32* row = a.data + s * a.cells;
+    const u32 got = khop_distinct_children(a, s, row[a.offs[h] + idx], h, idx, row + a.offs[h + 1] + (u64)idx * a.fanout[h],
+                                           s_seen[threadIdx.x >> 5]);
+    if ((threadIdx.x & 31) == 0) {
+      a.lens[s * a.lens_per + a.offs[h] + idx] = got;
+      got_sum += got;
+    }
+    __syncwarp();
+  }
+  khop_add(a.sum, got_sum);
 }
 
 static int khop_check(skw_ctx* ctx, const skw_khop_params* prm) {
@@ -274,17 +336,19 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
     if ((rc = alloc_table(ctx)) != SKW_OK) return rc;
   }
   if (!n) return SKW_OK;
-  uint32_t width[6], offs[6], cells = 0, w = 1;
+  KhopArgs a;
+  uint32_t cells = 0, w = 1;
   for (uint32_t h = 0; h <= prm->nhops; ++h) {
     if (h) w *= prm->fanout[h - 1];
-    width[h] = w;
-    offs[h] = cells;
+    a.width[h] = w;
+    a.offs[h] = cells;
+    if (h < prm->nhops) a.fanout[h] = prm->fanout[h];
     cells += w;
   }
-  KhopArgs a;
   a.xadj = ctx->xadj;
   a.adjncy = ctx->adjncy;
   a.slots = ctx->slots;
+  a.seeds = d_seeds;
   a.data = d_data;
   a.lens = d_sample_lengths;
   a.sum = reinterpret_cast<unsigned long long*>(ctx->d_sum);
@@ -295,9 +359,25 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
   a.instance_stride = prm->instance_stride ? prm->instance_stride : 1;
   a.V = ctx->V;
   a.cells = cells;
-  a.lens_per = offs[prm->nhops];
+  a.lens_per = a.offs[prm->nhops];
   a.flags = prm->flags;
+  a.nhops = prm->nhops;
   cudaStream_t st = ctx->stream;
+  const bool distinct = (prm->flags & SKW_KHOP_DISTINCT) && !unbiased;
+  // Trees of up to 8192 cells: as many seeds a CTA as keep its threads busy at the first hop, as long as every SM has
+  // eight CTAs.
+  if (!online && cells <= 8192) {
+    const uint64_t first = distinct ? 8 : 256 / a.width[1];
+    const uint64_t spread = n / ((uint64_t)ctx->sm_count * 8);
+    const uint32_t per_cta = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({first, spread, 8192 / cells}));
+    const uint64_t ctas = (n + per_cta - 1) / per_cta;
+    if (ctas <= 0x7FFFFFFFull) {
+      if (distinct) khop_tree_kernel<true><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
+      else khop_tree_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
+      SKW_LAUNCHED(ctx);
+      return SKW_OK;
+    }
+  }
   const uint64_t cap = (uint64_t)ctx->sm_count * 16;
   uint64_t want = (n + 255) / 256;
   khop_init_kernel<<<(int)(want < cap ? want : cap), 256, 0, st>>>(d_seeds, n, cells, d_data);
@@ -306,20 +386,15 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
     // A table built earlier in this call (an earlier hop, an earlier slice of the seeds) stays good:
     // only the first collection of a call opens a new round of claims, every later one skips the
     // vertices that already hold one.
-    if (online && (rc = frontier_collect(ctx, d_data, n * width[h], width[h], cells, offs[h], nullptr,
+    if (online && (rc = frontier_collect(ctx, d_data, n * a.width[h], a.width[h], cells, a.offs[h], nullptr,
                                          first_of_call && h == 0)) != SKW_OK)
       return rc;
-    a.offs_parent = offs[h];
-    a.offs_child = offs[h + 1];
-    a.width_parent = width[h];
-    a.fanout = prm->fanout[h];
-    a.hop = h + 1;
-    if ((prm->flags & SKW_KHOP_DISTINCT) && !unbiased) {
-      want = (n * width[h] + 7) / 8;  // one warp per parent vertex
-      khop_distinct_kernel<<<(int)(want < cap ? want : cap), 256, 0, st>>>(a);
+    if (distinct) {
+      want = (n * a.width[h] + 7) / 8;  // one warp per parent vertex
+      khop_distinct_kernel<<<(int)(want < cap ? want : cap), 256, 0, st>>>(a, h);
     } else {
-      want = (n * width[h + 1] + 255) / 256;
-      khop_hop_kernel<<<(int)(want < cap ? want : cap), 256, 0, st>>>(a);
+      want = (n * a.width[h + 1] + 255) / 256;
+      khop_hop_kernel<<<(int)(want < cap ? want : cap), 256, 0, st>>>(a, h);
     }
     SKW_LAUNCHED(ctx);
   }
