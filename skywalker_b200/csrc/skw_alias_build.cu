@@ -35,6 +35,7 @@
 #include <mutex>
 
 #include "skw_alias_f64.cuh"
+#include "skw_alias_long.cuh"
 #include "skw_alias_math.cuh"
 #include "skw_ctx.h"
 
@@ -118,27 +119,11 @@ static u64 class_room(int k, u64 V, u64 E) {
   return std::min<u64>(V, E / least[k]) + 1;
 }
 
-// ------------------------------------------------------------------ bulk copy (TMA unit) ---
-// Untiled cp.async.bulk global -> shared with completion on an mbarrier.  Both addresses must be
-// 16-byte aligned and the size a multiple of 16 bytes; the caller rounds the window inwards and
-// fetches ragged ends with plain loads.  No multicast, local memory only.
+// ------------------------------------------------------------------ bounded wait ----------
 __device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(u64* bar, u32 arrivals) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, u32 bytes, u64* bar) {
-  // order earlier generic-proxy accesses of the destination before the async-proxy writes
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-// One arrival without bytes to wait for (a phase that no bulk copy feeds).
-__device__ __forceinline__ void mbar_arrive(u64* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 // Poll (without blocking) for the phase with the given parity, at most `limit` times with a short
 // sleep in between: a few milliseconds in total.  Returns false if the copy did not complete.
@@ -154,472 +139,6 @@ __device__ __forceinline__ bool mbar_wait(u64* bar, u32 parity, u32 limit) {
     __nanosleep(32);
   }
   return false;
-}
-
-// ------------------------------------------------------------------ merge-path builders ----
-// NT cooperating threads (one warp, or a CTA) build one vertex.
-//
-// The sweep "smalls in index order are topped up by larges in index order" is a MERGE of two
-// sorted lists: small i (key = deficit of the smalls before it) comes before large j (key = excess
-// of the larges up to and including it) iff its key is <= the large's key.  When small i is
-// emitted at state (i, j) its donor is large j; when large j is emitted while smalls remain it
-// has fallen below one bucket, keeps X(j) + C - D(i-1) of it and is topped up by large j+1; larges
-// emitted after the last small own exactly one bucket.  So after the two prefix lists are in
-// memory, every thread takes an equal slice of the merged order (merge-path partition by one
-// bisection per thread) and runs the sweep serially on it: the same number of steps in every
-// lane, no per-element searches.
-//
-// Phase 1 walks the weight list in tiles of NT*4 elements (4 consecutive elements per thread, so a
-// prefix sum is a short serial scan plus one cross-thread scan) and writes
-//   A[i] = inclusive deficit prefix of small i,   P[i] = its position        (smalls from the front)
-//   A[n-1-j] = inclusive excess prefix of large j, P[n-1-j] = its position   (larges from the back)
-template <int NT>
-__device__ __forceinline__ void coop_sync() {
-  if constexpr (NT == 32) __syncwarp();
-  else __syncthreads();
-}
-
-// Exclusive cross-thread prefix and total of one u64 per thread.  In a CTA the warp totals are
-// scanned by the first warp (s_tmp: NT/32 + 1 entries).
-template <int NT>
-__device__ __forceinline__ void coop_scan_u64(u64& v, u64& total, u64* s_tmp) {
-  const u32 lane = threadIdx.x & 31;
-  u64 inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const u64 t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-    if (lane >= (u32)o) inc += t;
-  }
-  if constexpr (NT == 32) {
-    total = __shfl_sync(0xFFFFFFFFu, inc, 31);
-    v = inc - v;
-  } else {
-    constexpr int NW = NT / 32;
-    const u32 warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 31) s_tmp[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      u64 x = lane < NW ? s_tmp[lane] : 0, xi = x;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const u64 t = __shfl_up_sync(0xFFFFFFFFu, xi, o);
-        if (lane >= (u32)o) xi += t;
-      }
-      if (lane < NW) s_tmp[lane] = xi - x;
-      if (lane == 31) s_tmp[NW] = xi;
-    }
-    __syncthreads();
-    total = s_tmp[NW];
-    v = s_tmp[warp] + inc - v;
-  }
-}
-
-// The same for a 64-bit and a 32-bit value at once (s_tmp: 2 * (NT/32 + 1) entries).
-template <int NT>
-__device__ __forceinline__ void coop_scan2(u64& a, u32& c, u64& ta, u32& tc, u64* s_tmp) {
-  const u32 lane = threadIdx.x & 31;
-  u64 ia = a;
-  u32 ic = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const u64 xa = __shfl_up_sync(0xFFFFFFFFu, ia, o);
-    const u32 xc = __shfl_up_sync(0xFFFFFFFFu, ic, o);
-    if (lane >= (u32)o) {
-      ia += xa;
-      ic += xc;
-    }
-  }
-  if constexpr (NT == 32) {
-    ta = __shfl_sync(0xFFFFFFFFu, ia, 31);
-    tc = __shfl_sync(0xFFFFFFFFu, ic, 31);
-    a = ia - a;
-    c = ic - c;
-  } else {
-    constexpr int NW = NT / 32, ST = NW + 1;
-    const u32 warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 31) {
-      s_tmp[warp] = ia;
-      s_tmp[ST + warp] = ic;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      u64 xa = lane < NW ? s_tmp[lane] : 0;
-      u32 xc = lane < NW ? (u32)s_tmp[ST + lane] : 0;
-      u64 ya = xa;
-      u32 yc = xc;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const u64 pa = __shfl_up_sync(0xFFFFFFFFu, ya, o);
-        const u32 pc = __shfl_up_sync(0xFFFFFFFFu, yc, o);
-        if (lane >= (u32)o) {
-          ya += pa;
-          yc += pc;
-        }
-      }
-      if (lane < NW) {
-        s_tmp[lane] = ya - xa;
-        s_tmp[ST + lane] = yc - xc;
-      }
-      if (lane == 31) {
-        s_tmp[NW] = ya;
-        s_tmp[ST + NW] = yc;
-      }
-    }
-    __syncthreads();
-    ta = s_tmp[NW];
-    tc = (u32)s_tmp[ST + NW];
-    a = s_tmp[warp] + ia - a;
-    c = (u32)s_tmp[ST + warp] + ic - c;
-  }
-}
-
-template <int NT>
-__device__ __forceinline__ float coop_max(float v, float* s_tmp) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  if constexpr (NT != 32) {
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) s_tmp[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float t = 0.0f;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) t = fmaxf(t, s_tmp[w]);
-    v = t;
-  }
-  return v;
-}
-
-// Merge phase over one window: nl = Sl + Ll list entries (Sl smalls in sA[0..Sl), Ll larges from
-// the back: large j' at nl-1-j'), positions in sP alike.  dsx_in = deficit of all smalls before
-// the window, next_pos = position of the first large after the window (kNoNext if none).  Thread
-// t emits an equal share of the window's merged order.
-constexpr u32 kNoNext = 0xFFFFFFFFu;
-template <int NT>
-__device__ __forceinline__ void merge_window(u32 t, u32 nl, u32 Sl, const u64* sA, const u32* sP, u64 dsx_in,
-                                             u32 next_pos, u64 C, int B, u32 off, Slot* __restrict__ slots,
-                                             u32 v, u32* err) {
-  const u32 Ll = nl - Sl;
-  const u32 VT = (nl + NT - 1) / NT;
-  const u32 k0 = min(t * VT, nl), k1 = min(k0 + VT, nl);
-  if (k0 >= k1) return;
-  u32 i, j;
-  {
-    u32 lo = k0 > Ll ? k0 - Ll : 0, hi = min(k0, Sl);
-    while (lo < hi) {
-      const u32 mid = (lo + hi) >> 1;
-      const u64 a = mid ? sA[mid - 1] : dsx_in;    // key of small mid
-      const u64 b = sA[nl - 1 - (k0 - 1 - mid)];   // key of large k0-1-mid
-      if (a <= b) lo = mid + 1;
-      else hi = mid;
-    }
-    i = lo;
-    j = k0 - lo;
-  }
-  // i <= Sl and j <= Ll hold from here on, and i + j = k < nl: the entry that leaves always exists.
-  // A step has no branch (see merge_packed): a window of three entries stays in registers, the
-  // small at the head, the large at the head and the large behind it; past the window's last large
-  // the key is "never full" and the position that of the next window's first large.
-  constexpr u64 kNever = ~0ull;
-  u64 dsx = i ? sA[i - 1] : dsx_in;  // deficit of the smalls before small i
-  u64 sk = 0, lk = kNever, lk2 = kNever;
-  u32 sp = 0, lp = next_pos, lp2 = next_pos;
-  if (i < Sl) {
-    sk = sA[i];
-    sp = sP[i];
-  }
-  if (j < Ll) {
-    lk = sA[nl - 1 - j];
-    lp = sP[nl - 1 - j];
-  }
-  if (j + 1 < Ll) {
-    lk2 = sA[nl - 2 - j];
-    lp2 = sP[nl - 2 - j];
-  }
-  Slot* __restrict__ out = slots + off;
-  bool bad = false;
-  for (u32 k = k0; k < k1; ++k) {
-    const bool fits = dsx <= lk;
-    const bool take = i < Sl && fits;              // a small leaves; else a large
-    const bool full = !take && fits;               // only once every small is placed
-    const u32 p = take ? sp : lp;
-    const u32 a = take ? lp : lp2;                 // a small's alias: the large at the head; a large's: the next one
-    const bool none = a == kNoNext;
-    bad |= none && !full;                          // mass conservation rules it out
-    const bool self = full || none;
-    const u64 x = take ? dsx : lk, y = take ? sk : dsx;  // small: C - (sk - dsx); large: lk + C - dsx
-    Slot o;
-    o.prob = self ? 1.0f : mass_to_prob_fast(C + x - y, B);
-    o.alias = self ? p : a;
-    out[p] = o;
-    i += take ? 1u : 0u;
-    j += take ? 0u : 1u;
-    const u32 idx = take ? i : nl - 2 - j;
-    const bool more = take ? i < Sl : j + 1 < Ll;
-    const u64 nk = more ? sA[idx] : kNever;
-    const u32 np = more ? sP[idx] : next_pos;
-    dsx = take ? sk : dsx;
-    lk = take ? lk : lk2;
-    lp = take ? lp : lp2;
-    lk2 = take ? lk2 : nk;
-    lp2 = take ? lp2 : np;
-    sk = take ? nk : sk;
-    sp = take ? np : sp;
-  }
-  if (bad) dev_fail(err, DEV_ERR_INTERNAL, v, k0, 8);
-}
-
-// WIN == 0: the lists A / P are in shared memory and are merged in place.  WIN > 0: they are in
-// global scratch and win_smem holds WIN * 12 + (NT + 1) * 4 bytes of shared memory for staging.
-// NBUF > 0: the tiles of the weight list come through `pipe` (see TilePipe) instead of global loads, with
-// two buffers one tile ahead of the one being worked on, with one buffer refilled as soon as a tile's
-// weights are quantised.
-// STAGED: w points at a copy of the weight list in shared memory, else at the list in global memory.
-// Weight tiles of the scratch class brought into shared memory by the bulk-copy engine, one tile
-// ahead of the one being worked on: two buffers of tile + 8 floats and one mbarrier each.  The parity
-// of each barrier's current phase lives in `parity` (bit b for buffer b) across the vertices of a CTA.
-struct TilePipe {
-  float* buf;   // 2 x (tile + 8) floats, 16-byte aligned
-  u64* bars;    // 2 mbarriers, initialised with one arrival
-  u32 parity;
-  bool failed;  // a copy did not report completion in time: the CTA stops taking vertices
-};
-
-template <int NT, int EPT, int WIN, bool STAGED, int NBUF = 0>
-__device__ void build_vertex_merge(u32 t, u32 v, u32 off, u32 n, const float* w,
-                                   Slot* __restrict__ slots, uint8_t* __restrict__ valid, u64* A,
-                                   u32* P, u64* s_tmp, unsigned char* win_smem, u32* err,
-                                   TilePipe* pipe = nullptr) {
-  auto weight = [&](u32 p) { return sane_weight(STAGED ? w[p] : __ldg(w + p)); };
-  float wmax = 0.0f;
-  for (u32 p = t; p < n; p += NT) wmax = fmaxf(wmax, weight(p));
-  wmax = coop_max<NT>(wmax, reinterpret_cast<float*>(s_tmp));
-  if (!(wmax > 0.0f)) {
-    for (u32 p = t; p < n; p += NT) slots[(u64)off + p] = Slot{-1.0f, p};
-    if (t == 0) valid[v] = 0;
-    return;
-  }
-  const int B = bucket_bits(n);
-  const u64 C = (u64)1 << B;
-  const int sh = weight_shift(wmax, B);
-  u64 W = 0;
-  {
-    u64 acc = 0;
-    for (u32 p = t; p < n; p += NT) acc += quantise_bits(weight(p), sh);
-    // total only: the exclusive prefix is not needed here
-    u64 x = acc;
-    coop_scan_u64<NT>(x, W, s_tmp);
-  }
-  const u64 nC = (u64)n << B;
-  const double K = mass_factor(n, B, W);
-
-  // Only the deficit prefix D and the count of larges are scanned; the excess prefix follows from the
-  // cumulative mass: sum over k <= p of (M_k - C) = X(p) - D(p), so X(p) = D(p) + g(Q_(p+1)) - (p + 1) * C.
-  u64 cQ = 0, cD = 0;  // carries between tiles (the same value in every thread)
-  u32 cL = 0;
-  constexpr u32 kTile = NT * EPT;
-  constexpr bool BULK = NBUF > 0;
-  // BULK: element i of a tile sits at buffer[head + i]; the list starts `head` floats after a 16-byte
-  // boundary and tiles are whole multiples of 16 bytes, so every tile has the same head.  The copy
-  // engine brings the 16-byte groups that lie inside the tile, up to three floats at either end come
-  // with plain loads.
-  const u32 head = BULK ? (u32)((reinterpret_cast<uintptr_t>(w) & 15u) >> 2) : 0u;
-  auto stage_tile = [&](u32 base, u32 b) {
-    if constexpr (BULK) {
-      const u32 tile_n = min(kTile, n - base);
-      const float* src = w + base;
-      float* dst = pipe->buf + b * (kTile + 8);
-      const u32 skip = head ? 4u : 0u;                 // floats from the aligned start to the first boundary inside
-      const u32 body = (head + tile_n) & ~3u;          // ... and to the last boundary inside
-      const u32 lead = head ? min(4u - head, tile_n) : 0u;
-      if (t < lead) dst[head + t] = __ldg(src + t);
-      if (body > skip) {
-        if (t == 0) bulk_copy_g2s(dst + skip, src - head + skip, (body - skip) * 4u, pipe->bars + b);
-        const u32 tail = head + tile_n - body;         // elements after the last boundary
-        if (t < tail) dst[body + t] = __ldg(src + (body - head) + t);
-      } else {
-        for (u32 i = lead + t; i < tile_n; i += NT) dst[head + i] = __ldg(src + i);
-        if (t == 0) mbar_arrive(pipe->bars + b);       // the phase still has to complete
-      }
-    }
-  };
-  if constexpr (BULK) stage_tile(0, 0);
-  for (u32 base = 0; base < n; base += NT * EPT) {
-    // a ragged last tile spreads its elements over all threads (ept each) instead of filling the first ones
-    const u32 ept = min((u32)EPT, (n - base + NT - 1) / NT);
-    const u32 p0 = base + t * ept;
-    const float* tw = nullptr;  // BULK: this tile's weights in shared memory, tw[i] = weight base + i
-    if constexpr (BULK) {
-      const u32 b = NBUF == 2 ? (base / kTile) & 1u : 0u;
-      // two buffers: the other one was last read in the tile before this one, which ended with a barrier
-      if (NBUF == 2 && base + kTile < n) stage_tile(base + kTile, b ^ 1u);
-      const bool ok = mbar_wait(pipe->bars + b, (pipe->parity >> b) & 1u, 1u << 16);
-      // the same outcome in every thread (and the barrier that publishes the plain stores)
-      if (!__syncthreads_and(ok ? 1 : 0)) {
-        // record it, give the copies in flight one more bounded chance to land so that nothing still
-        // writes this CTA's shared memory when it leaves, and stop
-        if (t == 0) dev_fail(err, DEV_ERR_WAIT, v, base, 13);
-        if (!ok) mbar_wait(pipe->bars + b, (pipe->parity >> b) & 1u, 1u << 16);
-        if (NBUF == 2 && base + kTile < n) mbar_wait(pipe->bars + (b ^ 1u), (pipe->parity >> (b ^ 1u)) & 1u, 1u << 16);
-        pipe->failed = true;
-        return;
-      }
-      pipe->parity ^= 1u << b;
-      tw = pipe->buf + b * (kTile + 8) + head;
-    }
-    u64 m[EPT];
-    u64 Qex = 0;
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) {
-      m[k] = 0;
-      if ((u32)k < ept && p0 + k < n)
-        m[k] = quantise_bits(BULK ? sane_weight(tw[p0 + k - base]) : weight(p0 + k), sh);
-      Qex += m[k];
-    }
-    u64 tq;
-    coop_scan_u64<NT>(Qex, tq, s_tmp);
-    // one buffer: every thread has passed the scan's barriers, so nobody reads this tile's weights any
-    // more and the next tile can come in under the rest of this one's work
-    if (NBUF == 1 && base + kTile < n) stage_tile(base + kTile, 0);
-    Qex += cQ;
-    cQ += tq;
-    const u64 gex = cum_mass(Qex, W, nC, K);
-    u64 g_prev = gex, Q = Qex;
-    u64 sd = 0;
-    u32 sl = 0;
-#pragma unroll
-    for (int k = 0; k < EPT; ++k) {
-      if ((u32)k < ept && p0 + k < n) {
-        Q += m[k];
-        const u64 g = cum_mass(Q, W, nC, K);
-        m[k] = g - g_prev;
-        g_prev = g;
-        if (m[k] < C) sd += C - m[k];
-        else ++sl;
-      }
-    }
-    u64 td;
-    u32 tl;
-    coop_scan2<NT>(sd, sl, td, tl, s_tmp);
-    u64 Dr = sd + cD, gc = gex;
-    u32 Lr = sl + cL;
-    const u32 L0 = cL;  // larges before this tile
-    cD += td;
-    cL += tl;
-    if constexpr (WIN == 0) {
-#pragma unroll
-      for (int k = 0; k < EPT; ++k) {
-        const u32 p = p0 + k;
-        if ((u32)k < ept && p < n) {
-          gc += m[k];
-          if (m[k] < C) {
-            Dr += C - m[k];
-            const u32 i = p - Lr;  // smalls before p
-            A[i] = Dr;
-            P[i] = p;
-          } else {
-            const u32 j = Lr++;    // larges before p
-            A[n - 1 - j] = Dr + gc - ((u64)(p + 1) << B);
-            P[n - 1 - j] = p;
-          }
-        }
-      }
-    } else {
-      // The lists live in global memory.  A thread's eight entries would go out as eight scattered
-      // 8-byte stores per warp instruction; instead the tile's entries are laid out in shared memory
-      // first (its smalls from the front, its larges from the back, as in the lists themselves) and
-      // copied out with consecutive lanes on consecutive addresses.
-      static_assert(WIN == 0 || WIN >= NT * EPT, "the window buffer doubles as the tile's staging area");
-      u64* tA = reinterpret_cast<u64*>(win_smem);
-      u32* tP = reinterpret_cast<u32*>(tA + WIN);
-      const u32 tile_n = min((u32)(NT * EPT), n - base);
-#pragma unroll
-      for (int k = 0; k < EPT; ++k) {
-        const u32 p = p0 + k;
-        if ((u32)k < ept && p < n) {
-          gc += m[k];
-          if (m[k] < C) {
-            Dr += C - m[k];
-            const u32 i = (p - base) - (Lr - L0);  // smalls of this tile before p
-            tA[i] = Dr;
-            tP[i] = p;
-          } else {
-            const u32 j = Lr++ - L0;               // larges of this tile before p
-            tA[tile_n - 1 - j] = Dr + gc - ((u64)(p + 1) << B);
-            tP[tile_n - 1 - j] = p;
-          }
-        }
-      }
-      coop_sync<NT>();
-      const u32 ts = tile_n - tl;          // smalls in this tile
-      const u32 S0 = base - L0;            // smalls before this tile
-      for (u32 x = t; x < ts; x += NT) {
-        A[S0 + x] = tA[x];
-        P[S0 + x] = tP[x];
-      }
-      for (u32 x = t; x < tl; x += NT) {   // large L0 + x sits at n - 1 - (L0 + x)
-        A[n - 1 - (L0 + x)] = tA[tile_n - 1 - x];
-        P[n - 1 - (L0 + x)] = tP[tile_n - 1 - x];
-      }
-      coop_sync<NT>();
-    }
-  }
-  coop_sync<NT>();
-  const u32 L = cL, S = n - L;
-  if (L == 0) {  // mass conservation guarantees a large
-    if (t == 0) dev_fail(err, DEV_ERR_INTERNAL, v, L, 7);
-    for (u32 p = t; p < n; p += NT) slots[(u64)off + p] = Slot{1.0f, p};
-    if (t == 0) valid[v] = 1;
-    return;
-  }
-  if constexpr (WIN == 0) {
-    merge_window<NT>(t, n, S, A, P, 0, kNoNext, C, B, off, slots, v, err);
-  } else {
-    // Lists live in global scratch: cut the merged order into windows of WIN outputs, stage each
-    // window's two list slices in shared memory with coalesced copies and merge it from there.
-    u64* sA = reinterpret_cast<u64*>(win_smem);
-    u32* sP = reinterpret_cast<u32*>(sA + WIN);
-    u32* bnd = sP + WIN;  // smalls before the start of each window of one round (NT + 1 entries)
-    const u32 nwin = (n + WIN - 1) / WIN;
-    for (u32 w0 = 0; w0 < nwin; w0 += NT - 1) {  // a round of cnt windows needs cnt + 1 boundaries
-      const u32 cnt = min((u32)NT - 1, nwin - w0);
-      coop_sync<NT>();
-      if (t <= cnt) {  // one bisection per window boundary, all in parallel
-        const u32 k0 = min((w0 + t) * (u32)WIN, n);
-        u32 lo = k0 > L ? k0 - L : 0, hi = min(k0, S);
-        while (lo < hi) {
-          const u32 mid = (lo + hi) >> 1;
-          const u64 a = mid ? A[mid - 1] : 0;
-          const u64 b = A[n - 1 - (k0 - 1 - mid)];
-          if (a <= b) lo = mid + 1;
-          else hi = mid;
-        }
-        bnd[t] = lo;
-      }
-      coop_sync<NT>();
-      for (u32 wi = 0; wi < cnt; ++wi) {
-        const u32 k0 = (w0 + wi) * (u32)WIN, k1 = min(k0 + (u32)WIN, n);
-        const u32 i0 = bnd[wi], i1 = bnd[wi + 1];
-        const u32 j0 = k0 - i0, j1 = k1 - i1;
-        const u32 Sl = i1 - i0, Ll = j1 - j0, nl = Sl + Ll;
-        for (u32 x = t; x < Sl; x += NT) {
-          sA[x] = A[i0 + x];
-          sP[x] = P[i0 + x];
-        }
-        for (u32 x = t; x < Ll; x += NT) {  // larges j0..j1-1 sit at global n-j1 .. n-j0-1
-          sA[Sl + x] = A[n - j1 + x];
-          sP[Sl + x] = P[n - j1 + x];
-        }
-        const u64 dsx_in = i0 ? A[i0 - 1] : 0;
-        const u32 next_pos = j1 < L ? P[n - 1 - j1] : kNoNext;
-        coop_sync<NT>();
-        merge_window<NT>(t, nl, Sl, sA, sP, dsx_in, next_pos, C, B, off, slots, v, err);
-        coop_sync<NT>();
-      }
-    }
-  }
-  if (t == 0) valid[v] = 1;
 }
 
 // ------------------------------------------------------------------ lists of up to 4096 ----
@@ -746,42 +265,22 @@ __global__ void __launch_bounds__(NT, 768 / NT) build_cta_kernel(const u32* __re
   }
 }
 
-// Dynamic shared memory of the scratch class: the merge windows (WIN keys and positions, NT + 1
-// window boundaries), rounded up to 16 bytes, then two weight tiles of NT * 8 + 8 floats.
-__host__ __device__ constexpr int win_smem_bytes(int nt, int win) { return (win * 12 + (nt + 1) * 4 + 15) & ~15; }
-__host__ __device__ constexpr int tile_pipe_bytes(int nt) { return 2 * (nt * 8 + 8) * 4; }
-
-// One CTA of NT threads per vertex of degree <= cap.  WIN == 0: lists in dynamic shared memory.
-// WIN > 0: lists in this CTA's slab of global scratch (cap entries of 12 bytes), merged through
-// windows of WIN outputs staged in dynamic shared memory.
-template <int NT, int WIN>
-__global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restrict__ list,
-                                                             u32* __restrict__ cls, int k,
-                                                             const u32* __restrict__ xadj,
-                                                             const float* __restrict__ wgt,
-                                                             Slot* __restrict__ slots,
-                                                             uint8_t* __restrict__ valid,
-                                                             unsigned char* __restrict__ scratch,
-                                                             u64 cap, u32* __restrict__ err) {
+// More than 4096 weights: one CTA per vertex, handed out by the class's cursor (degrees, hence costs, vary widely).
+// GLOBAL: lists in this CTA's slab of global scratch (cap + 2 entries of 12 bytes), else in shared memory.
+template <int NT, int CAP, bool GLOBAL>
+__global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __restrict__ list, u32* __restrict__ cls, int k,
+                                                                   const u32* __restrict__ xadj,
+                                                                   const float* __restrict__ wgt, Slot* __restrict__ slots,
+                                                                   uint8_t* __restrict__ valid,
+                                                                   unsigned char* __restrict__ scratch, u64 cap,
+                                                                   u32* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ u64 s_tmp[2 * (NT / 32 + 1)];
-  __shared__ __align__(8) u64 s_bars[2];
-  unsigned char* store = WIN ? scratch + (u64)blockIdx.x * cap * 12ull : smem;
-  u64* A = reinterpret_cast<u64*>(store);
-  u32* P = reinterpret_cast<u32*>(A + cap);
+  LongShared<NT, CAP>* sh = reinterpret_cast<LongShared<NT, CAP>*>(smem);
+  u64* A = GLOBAL ? reinterpret_cast<u64*>(scratch + (u64)blockIdx.x * (cap + 2) * 12ull) : nullptr;
+  u32* P = GLOBAL ? reinterpret_cast<u32*>(A + cap + 2) : nullptr;
   const u32 count = cls[k];
   __shared__ u32 s_it;
-  // Weight tiles brought in by the bulk-copy engine: two buffers behind the merge windows (WIN > 0), one
-  // buffer behind the lists of the shared-memory classes (two 512-thread CTAs with 96 KB of lists and a
-  // 16 KB tile each still share an SM)
-  constexpr int NBUF = WIN > 0 ? 2 : 1;
-  TilePipe pipe{reinterpret_cast<float*>(WIN ? smem + win_smem_bytes(NT, WIN) : smem + cap * 12ull), s_bars, 0u, false};
-  if (NBUF && threadIdx.x == 0) {
-    mbar_init(&s_bars[0], 1);
-    mbar_init(&s_bars[1], 1);
-  }
-  __syncthreads();
-  for (;;) {  // next vertex from the class's atomic cursor (degrees, hence costs, vary widely)
+  for (;;) {
     if (threadIdx.x == 0) s_it = atomicAdd(cls + K_CLASSES + k, 1u);
     __syncthreads();
     const u32 it = s_it;
@@ -793,9 +292,7 @@ __global__ void __launch_bounds__(NT) build_cta_merge_kernel(const u32* __restri
       if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, (u32)cap);
       continue;
     }
-    build_vertex_merge<NT, 8, WIN, false, NBUF>(threadIdx.x, v, off, n, wgt + off, slots, valid, A, P, s_tmp,
-                                                      smem, err, &pipe);
-    if (pipe.failed) break;  // the same in every thread
+    build_list_long<NT, CAP, GLOBAL>(v, off, n, wgt + off, slots, valid, sh, A, P, err);
     __syncthreads();
   }
 }
@@ -977,21 +474,20 @@ __device__ void build_vertex_cta(u32 v, u32 off, u32 n, const float* __restrict_
 // Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`.
 static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot* slots, uint8_t* valid) {
   cudaStream_t st = ctx->stream;
-  constexpr int kCta2Smem = kHugeSmemMax * 12 + tile_pipe_bytes(1024) / 2;  // lists + one weight tile
-  constexpr int kCta2aSmem = kMidSmemMax * 12 + tile_pipe_bytes(512) / 2;  // lists + one weight tile
-  constexpr int kWin = 8192;                        // merged outputs per window of the scratch class
-  constexpr int kWinSmem = win_smem_bytes(1024, kWin) + tile_pipe_bytes(1024);
   constexpr size_t kGroupSmem = kGroupWarps * kGroupBytes;
+  constexpr size_t kLongA = sizeof(LongShared<512, kMidSmemMax>), kLongB = sizeof(LongShared<1024, kHugeSmemMax>),
+                   kLongC = sizeof(LongShared<1024, 8192>);
+  static_assert(2 * (kLongA + 1024) <= 228 * 1024, "two CTAs an SM");
   static bool attr_set[64] = {false};
   if (!attr_set[ctx->device & 63]) {
-    SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_merge_kernel<1024, kWin>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWinSmem));
-    SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_merge_kernel<1024, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCta2Smem));
-    SKW_CUDA(ctx, cudaFuncSetAttribute(build_cta_merge_kernel<512, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCta2aSmem));
 #define SMEM(BYTES, ...) \
   SKW_CUDA(ctx, cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)))
     SMEM(sizeof(ListShared<256>), build_cta_kernel<256>);
     SMEM(sizeof(ListShared<128>), build_cta_kernel<128>);
     SMEM(kGroupSmem, build_groups_kernel);
+    SMEM(kLongA, (build_long_kernel<512, kMidSmemMax, false>));
+    SMEM(kLongB, (build_long_kernel<1024, kHugeSmemMax, false>));
+    SMEM(kLongC, (build_long_kernel<1024, 8192, true>));
 #undef SMEM
     attr_set[ctx->device & 63] = true;
   }
@@ -1001,13 +497,14 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   // every SM busy either way, but 0.23 ms instead of about 0.15 ms for the largest vertex of an online
   // frontier, which a hop has to wait for; so one vertex gets the 1024 threads.)
   const uint64_t slab_elems = ctx->max_degree > kHugeSmemMax ? (((uint64_t)ctx->max_degree + 1) & ~1ull) : 0;
+  const uint64_t slab_bytes = (slab_elems + 2) * 12ull;
   int gmem_ctas = ctx->sm_count;
   if (slab_elems) {
-    const uint64_t fit = (4ull << 30) / (slab_elems * 12ull);
+    const uint64_t fit = (4ull << 30) / slab_bytes;
     if (fit < (uint64_t)gmem_ctas) gmem_ctas = (int)(fit < 8 ? 8 : fit);
   }
   if (slab_elems) {
-    int rc = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, slab_elems * 12ull * gmem_ctas);
+    int rc = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, slab_bytes * gmem_ctas);
     if (rc != SKW_OK) return rc;
   }
   // The classes are independent and each kernel drains its own work list through an atomic cursor,
@@ -1024,22 +521,16 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
     s_b = ctx->bstream[2];
     s_c = ctx->bstream[3];
   }
-  if (slab_elems) {
-    build_cta_merge_kernel<1024, kWin><<<gmem_ctas, 1024, kWinSmem, s_h>>>(
-        lists.list[K_H], cls, K_H, ctx->xadj, ctx->adjwgt, slots, valid,
-        static_cast<unsigned char*>(ctx->cta_scratch), slab_elems, ctx->d_err);
-    SKW_LAUNCHED(ctx);
+#define LONG(MORE_THAN, KCLS, NT, CAP, GLOBAL, CTAS, BYTES, SCRATCH, MOST, STREAM)                                       \
+  if (ctx->max_degree > (MORE_THAN)) {                                                                                 \
+    build_long_kernel<NT, CAP, GLOBAL><<<CTAS, NT, BYTES, STREAM>>>(lists.list[KCLS], cls, KCLS, ctx->xadj,            \
+                                                                   ctx->adjwgt, slots, valid, SCRATCH, MOST, ctx->d_err); \
+    SKW_LAUNCHED(ctx);                                                                                                 \
   }
-  if (ctx->max_degree > kMidSmemMax) {
-    build_cta_merge_kernel<1024, 0><<<ctx->sm_count, 1024, kCta2Smem, s_a>>>(
-        lists.list[K_C2], cls, K_C2, ctx->xadj, ctx->adjwgt, slots, valid, nullptr, kHugeSmemMax, ctx->d_err);
-    SKW_LAUNCHED(ctx);
-  }
-  if (ctx->max_degree > kF64Max) {
-    build_cta_merge_kernel<512, 0><<<ctx->sm_count * 2, 512, kCta2aSmem, s_b>>>(
-        lists.list[K_C2A], cls, K_C2A, ctx->xadj, ctx->adjwgt, slots, valid, nullptr, kMidSmemMax, ctx->d_err);
-    SKW_LAUNCHED(ctx);
-  }
+  LONG(kHugeSmemMax, K_H, 1024, 8192, true, gmem_ctas, kLongC, static_cast<unsigned char*>(ctx->cta_scratch), slab_elems, s_h)
+  LONG(kMidSmemMax, K_C2, 1024, kHugeSmemMax, false, ctx->sm_count, kLongB, nullptr, kHugeSmemMax, s_a)
+  LONG(kF64Max, K_C2A, 512, kMidSmemMax, false, ctx->sm_count * 2, kLongA, nullptr, kMidSmemMax, s_b)
+#undef LONG
   // 24 warps an SM: what the registers and the shared memory of these kernels allow, all of them resident at once
   // (the vertices are dealt out by a stride over the grid: a second wave of CTAs would start when the first is done)
 #define LISTS(MORE_THAN, KCLS, NT, STREAM)                                                                      \
