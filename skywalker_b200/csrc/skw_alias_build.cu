@@ -699,7 +699,8 @@ extern "C" int skw_alias_build_offline(skw_ctx* ctx, uint32_t v_begin, uint32_t 
   // took 4 to 20 ms a rebuild at 67 M edges, against 1.7 ms for everything the GPU does.  skw_walk_records_free
   // returns the memory, and so does any allocation of the context that would fail without it (dev_malloc).
   ctx->records_ready = false;
-  int rc = alloc_table(ctx);
+  const bool whole = v_begin == 0 && v_end == ctx->V;
+  int rc = alloc_table(ctx, whole ? TableUse::kAll : TableUse::kSome);
   if (rc != SKW_OK) return rc;
   rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
@@ -708,7 +709,10 @@ extern "C" int skw_alias_build_offline(skw_ctx* ctx, uint32_t v_begin, uint32_t 
   if ((rc = enqueue_tables(ctx, v_begin, v_end, ctx->slots, ctx->valid)) != SKW_OK) return rc;
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   rc = err_check(ctx, "skw_alias_build_offline");
-  if (rc != SKW_OK) return rc;
+  if (rc != SKW_OK) {
+    if (whole && !ctx->table_ready) ctx->slots_marked = false;
+    return rc;
+  }
   if (ms) SKW_CUDA(ctx, cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1));
   ctx->table_ready = true;
   return SKW_OK;

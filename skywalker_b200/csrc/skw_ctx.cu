@@ -302,12 +302,19 @@ void drop_records(skw_ctx* ctx) {
   ctx->vbits = nullptr;
 }
 
-int alloc_table(skw_ctx* ctx) {
+int alloc_table(skw_ctx* ctx, TableUse use) {
   // kSlotSlack spare entries let a multi-GPU caller all-gather the table in equal chunks in place
+  const size_t n = (size_t)ctx->E + kSlotSlack;
   if (!ctx->slots) {
-    SKW_CUDA(ctx, dev_malloc(ctx, reinterpret_cast<void**>(&ctx->slots), sizeof(Slot) * (ctx->E + kSlotSlack)));
-    fill_unbuilt_slots_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->slots, (size_t)ctx->E + kSlotSlack);
+    SKW_CUDA(ctx, dev_malloc(ctx, reinterpret_cast<void**>(&ctx->slots), sizeof(Slot) * n));
+    ctx->slots_marked = false;
+  }
+  if (!ctx->slots_marked && use != TableUse::kFrontier) {
+    // what this call leaves out must read as "no usable table here"
+    const size_t from = use == TableUse::kAll ? (size_t)ctx->E : 0;
+    fill_unbuilt_slots_kernel<<<from ? 4 : ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->slots + from, n - from);
     SKW_LAUNCHED(ctx);
+    ctx->slots_marked = true;
   }
   if (!ctx->valid) {
     SKW_CUDA(ctx, cudaMalloc(&ctx->valid, ctx->V ? ctx->V : 1));
@@ -355,9 +362,7 @@ int skw_ctx_create(int device, skw_ctx** out) {
     }                                                                            \
   } while (0)
   CK(cudaSetDevice(device));
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, device));
-  ctx->sm_count = prop.multiProcessorCount;
+  CK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
   CK(cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
@@ -760,7 +765,7 @@ int skw_alias_import(skw_ctx* ctx, const float* h_prob, const uint32_t* h_alias,
   if (!h_prob || !h_alias || !h_valid) return fail(ctx, SKW_ERR_ARG, "skw_alias_import: null array");
   DeviceGuard g(ctx->device);
   ctx->records_ready = false;  // derived from the old table
-  int rc = alloc_table(ctx);
+  int rc = alloc_table(ctx, TableUse::kAll);
   if (rc != SKW_OK) return rc;
   std::vector<Slot> tmp(ctx->E ? ctx->E : 1);
   for (uint64_t i = 0; i < ctx->E; ++i) {
@@ -852,7 +857,7 @@ int skw_alias_load(skw_ctx* ctx, const char* path) {
   if (hdr[4] != fp)
     return fail(ctx, SKW_ERR_IO, "skw_alias_load: %s was written for another graph (same V and E, different offsets)", path);
   ctx->records_ready = false;  // derived from the old table
-  rc = alloc_table(ctx);
+  rc = alloc_table(ctx, TableUse::kAll);
   if (rc != SKW_OK) return rc;
   ctx->table_ready = false;
   const size_t chunk = 64u << 20;

@@ -54,6 +54,7 @@ struct skw_ctx {
   // alias table
   skw::Slot* slots = nullptr;
   uint8_t* valid = nullptr;
+  bool slots_marked = false;  // slots that no build has reached hold prob = -1
   bool table_ready = false;
   // tables of one online call (the table above stays as it is)
   skw::Slot* online_slots = nullptr;
@@ -109,8 +110,13 @@ namespace skw {
 int fail(skw_ctx* ctx, int code, const char* fmt, ...);
 // after the CSR pointers are set: compute max_degree
 int finish_graph(skw_ctx* ctx);
-// allocate slots[E] / valid[V] if absent
-int alloc_table(skw_ctx* ctx);
+// allocate slots[E] / valid[V] if absent; a call that writes only a part of the table has the rest marked unusable
+enum class TableUse {
+  kAll,      // writes every slot
+  kSome,     // a range of vertices, the others may be drawn from later
+  kFrontier  // draws only from the slots that it writes
+};
+int alloc_table(skw_ctx* ctx, TableUse use);
 // queue the construction of the tables of vertices [v_begin, v_end)
 int enqueue_tables(skw_ctx* ctx, uint32_t v_begin, uint32_t v_end, Slot* slots, uint8_t* valid);
 // forget the fused walk records (they are derived from the table and die with it) and free their memory

@@ -333,7 +333,7 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
   int rc;
   if (online) {
     drop_records(ctx);  // online builds overwrite table slots
-    if ((rc = alloc_table(ctx)) != SKW_OK) return rc;
+    if ((rc = alloc_table(ctx, TableUse::kFrontier)) != SKW_OK) return rc;
   }
   if (!n) return SKW_OK;
   KhopArgs a;

@@ -343,13 +343,16 @@ __device__ __forceinline__ void load_record(const WalkRecord* p, u32 (&w)[8]) {
                : "l"(p));
 }
 
+constexpr u32 kRecTile = 2048, kRecSpan = 2048;  // slots of a tile of the records build, offsets it keeps at hand
+constexpr u32 kRecCta = kRecTile / 8;
+
 // vinfo[v] = {first-edge offset, usable degree}; vbits = one bit per vertex, set when the usable
 // degree is not zero.  The bitmap is V/8 bytes and stays in L2, so a walker that starts on a dead
 // end (most uniformly random starts of a directed R-MAT graph) never touches DRAM for it.
 __global__ void __launch_bounds__(256) vertex_info_kernel(const u32* __restrict__ xadj,
                                                           const Slot* __restrict__ slots, u32 V,
                                                           uint2* __restrict__ vinfo, u32* __restrict__ vbits,
-                                                          u32* __restrict__ unusable) {
+                                                          u32* __restrict__ unusable, u32* __restrict__ tile_first) {
   const u64 T = (u64)gridDim.x * blockDim.x;
   const u64 rounds = ((u64)V + T - 1) / T;
   for (u64 it = 0; it < rounds; ++it) {  // whole warps stay in the loop: the ballot needs them
@@ -363,19 +366,24 @@ __global__ void __launch_bounds__(256) vertex_info_kernel(const u32* __restrict_
         atomicAdd(unusable, 1u);  // has out-edges but no table (all weights unusable, or not built yet): rare
       }
       vinfo[v] = make_uint2(off, eff);
+      // the tiles of the records build whose first slot lies in this list
+      for (u64 t = ((u64)off + kRecTile - 1) / kRecTile; t * kRecTile < (u64)off + deg; ++t) tile_first[t] = (u32)v;
     }
     const u32 word = __ballot_sync(0xFFFFFFFFu, eff != 0);
     if ((threadIdx.x & 31) == 0 && v < V) vbits[v >> 5] = word;
   }
 }
 
-// One thread per edge slot, a CTA per tile of kRecTile consecutive slots.  The source vertex of a
-// slot is found in two levels: two threads bisect the whole offset array for the tile's first and
-// last slot, the offsets of the vertices in between are copied to shared memory (a tile of 2048
-// slots spans 75 vertices on average on the R-MAT graphs, empty ones included), and every thread
-// bisects that copy.  A tile that spans more vertices than the copy holds (long runs of empty
-// vertices) bisects the global array inside the tile's vertex range instead.
-constexpr u32 kRecTile = 2048, kRecSpan = 4096;
+// A CTA per tile of kRecTile consecutive slots, neighbouring lanes on neighbouring slots.  The vertex of a tile's first
+// slot is at hand (tile_first); the offsets of the vertices of the tile are copied to shared memory (75 on average on the
+// R-MAT graphs, empty ones included), where every list also marks its first slot: a warp bisects the offsets for the
+// first of its 32 slots and goes by the marks from there.  A tile that spans more vertices (long runs of empty ones)
+// bisects the global array for every slot.  A neighbour's {offset, degree} is a random access; the one reached through the
+// alias mostly belongs to a slot of the same tile, whose thread has fetched it already.
+// Bound by the wavefronts of the L1 cache: a random access takes one, and so would every record if its thread's
+// records lay side by side (a warp's records side by side take a quarter), and by L2 traffic.  R-MAT 22, 65 M slots: 1.10 ms
+// with two random lookups a slot and every tile's vertices bisected from the whole offset array, 1.09 with eight
+// neighbouring slots a thread, 0.91 with a bisection per slot, 0.84 here; R-MAT 24, 457 M slots: 9.0 -> 7.5 ms.
 __device__ __forceinline__ u32 last_vertex_at_or_before(const u32* __restrict__ xadj, u32 lo, u32 hi, u32 e) {
   while (lo < hi) {  // last v in [lo, hi] with xadj[v] <= e
     const u32 mid = lo + ((hi - lo + 1) >> 1);
@@ -384,68 +392,94 @@ __device__ __forceinline__ u32 last_vertex_at_or_before(const u32* __restrict__ 
   }
   return lo;
 }
-__global__ void __launch_bounds__(256) walk_records_kernel(const u32* __restrict__ xadj,
-                                                           const u32* __restrict__ adjncy,
-                                                           const Slot* __restrict__ slots,
-                                                           const uint2* __restrict__ vinfo, u32 V,
-                                                           u64 E, WalkRecord* __restrict__ rec,
-                                                           u32* __restrict__ err) {
+__global__ void __launch_bounds__(kRecCta, 1024 / kRecCta) walk_records_kernel(const u32* __restrict__ xadj,
+                                                              const u32* __restrict__ adjncy,
+                                                              const Slot* __restrict__ slots,
+                                                              const uint2* __restrict__ vinfo,
+                                                              const u32* __restrict__ tile_first, u32 V, u64 E,
+                                                              WalkRecord* __restrict__ rec, u32* __restrict__ err) {
   __shared__ u32 s_x[kRecSpan + 1];
-  __shared__ u32 s_v[2];
+  __shared__ __align__(16) u32 s_nbr[kRecTile];
+  __shared__ __align__(16) uint2 s_info[kRecTile];
+  __shared__ __align__(16) uint16_t s_head[kRecTile];  // place of the list that starts here, plus 1
   const u64 tiles = (E + kRecTile - 1) / kRecTile;
   for (u64 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const u64 e0 = tile * kRecTile;
-    const u64 e1 = e0 + kRecTile < E ? e0 + kRecTile : E;
-    if (threadIdx.x < 2)
-      s_v[threadIdx.x] = last_vertex_at_or_before(xadj, 0, V - 1, threadIdx.x ? (u32)(e1 - 1) : (u32)e0);
-    __syncthreads();
-    const u32 v0 = s_v[0], v1 = s_v[1];
+    const u32 here = (u32)min((u64)kRecTile, E - e0);
+    const u32 v0 = __ldg(tile_first + tile), v1 = tile + 1 < tiles ? __ldg(tile_first + tile + 1) : V - 1;
+    u32 nbr[8];
+    Slot sl[8];
+#pragma unroll
+    for (u32 k = 0; k < 8; ++k) {  // (past the end: the last slot again)
+      const u32 e = (u32)e0 + min(threadIdx.x + kRecCta * k, here - 1);
+      sl[k] = load_slot(slots + e);
+      nbr[k] = __ldg(adjncy + e);
+    }
     const bool staged = v1 - v0 < kRecSpan;
-    if (staged)
-      for (u32 i = threadIdx.x; i <= v1 - v0 + 1; i += blockDim.x) s_x[i] = __ldg(xadj + v0 + i);
+    *reinterpret_cast<uint4*>(s_head + threadIdx.x * 8) = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    for (u64 e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      u32 off, deg;
-      if (staged) {
-        u32 lo = 0, hi = v1 - v0;
-        while (lo < hi) {
-          const u32 mid = lo + ((hi - lo + 1) >> 1);
-          if (s_x[mid] <= (u32)e) lo = mid;
-          else hi = mid - 1;
+    if (staged) {
+      for (u32 i = threadIdx.x; i <= v1 - v0 + 1; i += kRecCta) {
+        const u32 x = __ldg(xadj + v0 + i);
+        s_x[i] = x;
+        if (i <= v1 - v0 && x - (u32)e0 < here && __ldg(xadj + v0 + i + 1) != x) s_head[x - (u32)e0] = (uint16_t)(i + 1);
+      }
+    }
+    uint2 info[8];
+#pragma unroll
+    for (u32 k = 0; k < 8; ++k) {
+      info[k] = make_uint2(0u, 0u);
+      if (nbr[k] < V) info[k] = __ldg(vinfo + nbr[k]);
+      else dev_fail(err, DEV_ERR_INDEX, (u32)e0 + k, nbr[k], 22);
+    }
+#pragma unroll
+    for (u32 k = 0; k < 8; ++k) {
+      s_nbr[threadIdx.x + kRecCta * k] = nbr[k];
+      s_info[threadIdx.x + kRecCta * k] = info[k];
+    }
+    __syncthreads();
+    // the vertex (relative to v0) of the first slot of each of the warp's eight runs of 32, by one lane each
+    const u32 lane = threadIdx.x & 31;
+    u32 first = 0;
+    if (staged && lane < 8) {
+      const u32 e = (u32)e0 + min(threadIdx.x - lane + kRecCta * lane, here - 1);
+      for (u32 hi = v1 - v0; first < hi;) {
+        const u32 mid = (first + hi + 1) >> 1;
+        if (s_x[mid] <= e) first = mid;
+        else hi = mid - 1;
+      }
+    }
+#pragma unroll
+    for (u32 k = 0; k < 8; ++k) {
+      const u32 i = threadIdx.x + kRecCta * k;
+      u32 v = __shfl_sync(0xFFFFFFFFu, first, k);
+      const u32 head = s_head[i];
+      const u32 heads = __ballot_sync(0xFFFFFFFFu, head != 0) & (0xFFFFFFFFu >> (31 - lane));  // up to this lane
+      const u32 mark = __shfl_sync(0xFFFFFFFFu, head, heads ? 31 - __clz((int)heads) : 0);
+      if (heads) v = mark - 1;
+      if (i < here) {
+        if (!staged) v = last_vertex_at_or_before(xadj, v0, v1, (u32)e0 + i) - v0;
+        const u32 off = staged ? s_x[v] : __ldg(xadj + v0 + v);
+        const u32 deg = (staged ? s_x[v + 1] : __ldg(xadj + v0 + v + 1)) - off;
+        u32 alias = sl[k].alias;
+        if (alias >= deg) {  // a table that does not belong to this graph: keep the read inside the list
+          dev_fail(err, DEV_ERR_INDEX, (u32)e0 + i, alias, 22);
+          alias = 0;
         }
-        off = s_x[lo];
-        deg = s_x[lo + 1] - off;
-      } else {
-        const u32 v = last_vertex_at_or_before(xadj, v0, v1, (u32)e);
-        off = __ldg(xadj + v);
-        deg = __ldg(xadj + v + 1) - off;
+        const u32 at = off + alias - (u32)e0;  // (wraps around below the tile)
+        u32 n_alias;
+        uint2 i_alias;
+        if (at < here) {
+          n_alias = s_nbr[at];
+          i_alias = s_info[at];
+        } else {
+          n_alias = __ldg(adjncy + (u64)off + alias);
+          i_alias = n_alias < V ? __ldg(vinfo + n_alias) : make_uint2(0u, 0u);
+        }
+        asm volatile("st.global.v8.u32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(rec + e0 + i), "r"(__float_as_uint(sl[k].prob)),
+                     "r"(nbr[k]), "r"(info[k].x), "r"(info[k].y), "r"(n_alias), "r"(i_alias.x), "r"(i_alias.y), "r"(alias)
+                     : "memory");
       }
-      Slot s = load_slot(slots + e);
-      if (s.alias >= deg) {  // a table that does not belong to this graph: keep the read inside the list
-        dev_fail(err, DEV_ERR_INDEX, (u32)e, s.alias, 22);
-        s.alias = 0;
-      }
-      const u32 n_self = __ldg(adjncy + e);
-      const u32 n_alias = __ldg(adjncy + (u64)off + s.alias);
-      uint2 i_self = make_uint2(0u, 0u), i_alias = make_uint2(0u, 0u);
-      if (n_self < V && n_alias < V) {
-        i_self = __ldg(vinfo + n_self);
-        i_alias = __ldg(vinfo + n_alias);
-      } else {
-        dev_fail(err, DEV_ERR_INDEX, (u32)e, n_self, n_alias);
-      }
-      uint4 a, b;
-      a.x = __float_as_uint(s.prob);
-      a.y = n_self;
-      a.z = i_self.x;
-      a.w = i_self.y;
-      b.x = n_alias;
-      b.y = i_alias.x;
-      b.z = i_alias.y;
-      b.w = s.alias;
-      uint4* out = reinterpret_cast<uint4*>(rec + e);
-      out[0] = a;
-      out[1] = b;
     }
     __syncthreads();
   }
@@ -769,7 +803,10 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
   auto body = [&]() -> int {
     if (!ctx->records) SKW_CUDA(ctx, cudaMalloc(&ctx->records, sizeof(WalkRecord) * (ctx->E ? ctx->E : 1)));
     if (!ctx->vinfo) SKW_CUDA(ctx, cudaMalloc(&ctx->vinfo, sizeof(uint2) * ((size_t)ctx->V + 1)));
-    if (!ctx->vbits) SKW_CUDA(ctx, cudaMalloc(&ctx->vbits, sizeof(u32) * ((size_t)ctx->V / 32 + 1)));
+    // the bitmap, and behind it the first vertex of every tile of the records build
+    const u64 tiles = (ctx->E + kRecTile - 1) / kRecTile;
+    if (!ctx->vbits) SKW_CUDA(ctx, cudaMalloc(&ctx->vbits, sizeof(u32) * ((size_t)ctx->V / 32 + 1 + tiles)));
+    u32* tile_first = static_cast<u32*>(ctx->vbits) + (size_t)ctx->V / 32 + 1;
     int rc = err_reset(ctx);
     if (rc != SKW_OK) return rc;
     cudaStream_t st = ctx->stream;
@@ -777,14 +814,13 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
     if (ctx->V) {
       vertex_info_kernel<<<ctx->sm_count * 16, 256, 0, st>>>(ctx->xadj, ctx->slots, ctx->V,
                                                               static_cast<uint2*>(ctx->vinfo), static_cast<u32*>(ctx->vbits),
-                                                              reinterpret_cast<u32*>(ctx->d_sum + 3));
+                                                              reinterpret_cast<u32*>(ctx->d_sum + 3), tile_first);
       SKW_LAUNCHED(ctx);
     }
     if (ctx->E && ctx->V) {
-      const u64 tiles = (ctx->E + kRecTile - 1) / kRecTile;
       const u64 cap = (u64)ctx->sm_count * 32;
-      walk_records_kernel<<<(unsigned)(tiles < cap ? tiles : cap), 256, 0, st>>>(
-          ctx->xadj, ctx->adjncy, ctx->slots, static_cast<const uint2*>(ctx->vinfo), ctx->V, ctx->E,
+      walk_records_kernel<<<(unsigned)(tiles < cap ? tiles : cap), kRecCta, 0, st>>>(
+          ctx->xadj, ctx->adjncy, ctx->slots, static_cast<const uint2*>(ctx->vinfo), tile_first, ctx->V, ctx->E,
           static_cast<WalkRecord*>(ctx->records), ctx->d_err);
       SKW_LAUNCHED(ctx);
     }
@@ -922,7 +958,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   const bool build_tables = online && (prm->flags & (SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES)) != 0;
   if (build_tables) {
     drop_records(ctx);  // online builds overwrite table slots
-    if ((rc = alloc_table(ctx)) != SKW_OK) return rc;
+    if ((rc = alloc_table(ctx, TableUse::kFrontier)) != SKW_OK) return rc;
   }
   if (!n) return SKW_OK;
   WalkArgs a;
@@ -1011,9 +1047,10 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   return SKW_OK;
 }
 
-// A synchronous walk over device buffers; with h_lengths the lengths come home as well.
+// A synchronous walk over device buffers; with h_lengths the lengths, with h_paths the whole matrix comes home as well.
 static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n, uint32_t* d_paths,
-                         uint32_t* d_lengths, uint32_t* h_lengths, float* ms, uint64_t* sampled_edges) {
+                         uint32_t* d_lengths, uint32_t* h_lengths, uint32_t* h_paths, float* ms,
+                         uint64_t* sampled_edges) {
   cudaStream_t st = ctx->stream;
   int rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
@@ -1022,6 +1059,8 @@ static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_
     return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   if (h_lengths && n) SKW_CUDA(ctx, cudaMemcpyAsync(h_lengths, d_lengths, sizeof(u32) * (size_t)n, cudaMemcpyDeviceToHost, st));
+  if (h_paths && n)
+    SKW_CUDA(ctx, cudaMemcpyAsync(h_paths, d_paths, sizeof(u32) * (size_t)n * prm->hop_num, cudaMemcpyDeviceToHost, st));
   if ((rc = err_check(ctx, "skw_walk")) != SKW_OK) return rc;
   if (ms) SKW_CUDA(ctx, cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1));
   if (sampled_edges) *sampled_edges = *ctx->h_sum;
@@ -1041,7 +1080,7 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
   // recorded until skw_ctx_take_sampled_edges() (or a later synchronous call) looks at it.
   if (!ms && !sampled_edges)
     return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1);
-  return walk_and_wait(ctx, prm, d_starts, n, d_paths, d_lengths, nullptr, ms, sampled_edges);
+  return walk_and_wait(ctx, prm, d_starts, n, d_paths, d_lengths, nullptr, nullptr, ms, sampled_edges);
 }
 
 // Large batches into the caller's n x hop_num host matrix: the walks come home packed (contiguous
@@ -1132,16 +1171,16 @@ int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts,
   if (n && fill) SKW_CUDA(ctx, cudaMemsetAsync(ctx->stage[1], 0xFF, nb * prm->hop_num, ctx->stream));
   uint64_t edges = 0;
   rc = walk_and_wait(ctx, prm, static_cast<uint32_t*>(ctx->stage[0]), n, static_cast<uint32_t*>(ctx->stage[1]),
-                     static_cast<uint32_t*>(ctx->stage[2]), h_lengths, ms, &edges);
+                     static_cast<uint32_t*>(ctx->stage[2]), h_lengths, fill ? h_paths : nullptr, ms, &edges);
   if (rc != SKW_OK) return rc;
   if (sampled_edges) *sampled_edges = edges;
-  if (n) {
+  if (n && !fill) {
     // Pinned host memory is addressable by the GPU: write only the cells each walk produced, unless that is all of
     // them.  Pageable memory gets the whole matrix (cells past a walk's end then hold stale values).
     cudaPointerAttributes at;
     u32* mapped = nullptr;
-    if (fill || edges == n * (prm->hop_num - 1ull)) {
-      // every cell is written: one copy (4096 rows of 81: 31 us against 65 for the kernel)
+    if (edges == n * (prm->hop_num - 1ull)) {
+      // every cell was written: one copy (4096 rows of 81: 31 us against 65 for the kernel)
     } else if (cudaPointerGetAttributes(&at, h_paths) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer) {
       mapped = static_cast<u32*>(at.devicePointer);
     } else {
