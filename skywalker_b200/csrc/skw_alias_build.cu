@@ -33,6 +33,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "skw_alias_f64.cuh"
 #include "skw_alias_long.cuh"
@@ -187,81 +188,90 @@ struct ClassItems {
   }
 };
 
-// Up to G * EPT weights: one group of G lanes per vertex, 32 / G vertices per warp side by side.
+// Shared memory of one vertex, and of a warp that has 32 / G of them side by side.
 template <int G, int EPT>
 struct GroupShared {
   // an odd number of words a group; the slots also hold the staged weights (G >= 8: n + n / EPT words of 4 bytes)
   static constexpr u32 kWords = (G * EPT + 1) | 1;
   uint2 lists[32 / G][kWords], slots[32 / G][kWords];
 };
-constexpr int kGroupWarps = 4, kGroupCtas = 6;  // warps a CTA, CTAs an SM: what registers and shared memory allow
-// bytes of shared memory a warp has, whatever class it is at
-constexpr size_t kGroupBytes =
-    std::max({sizeof(GroupShared<32, 16>), sizeof(GroupShared<16, 16>), sizeof(GroupShared<8, 16>),
-              sizeof(GroupShared<4, 16>), sizeof(GroupShared<2, 16>), sizeof(GroupShared<1, 16>)});
-template <int G, int EPT>
-__device__ __forceinline__ void build_groups(unsigned char* smem, const u32* list, u32 count, const u32* xadj,
-                                             const float* wgt, Slot* slots, uint8_t* valid, u32* err) {
-  GroupShared<G, EPT>* sh = reinterpret_cast<GroupShared<G, EPT>*>(smem);  // this warp's
-  const u32 in_warp = (threadIdx.x & 31) / G;
-  const GroupCoop<G> co;
-  for (ClassItems c(list, count, xadj, (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / G,
-                    gridDim.x * (kGroupWarps * 32 / G)); c.more();) {
-    const ClassItems::After after = c.look_ahead(wgt, co.t, G >= 8 ? 32 : EPT);
-    const u32 n = c.end - c.off;
-    if (n > G * EPT || n == 0) {  // classification and kernel disagree: record and skip
-      if (co.t == 0) dev_fail(err, DEV_ERR_INTERNAL, c.v, n, G);
-    } else {
-      build_list_f64<GroupCoop<G>, EPT>(co, c.v, c.off, n, wgt + c.off, slots, valid, sh->lists[in_warp],
-                                        sh->slots[in_warp], err);
-    }
-    co.sync();  // the group's words are reused by its next vertex
-    c.advance(after);
-  }
-  __syncwarp();
-}
-// All group classes in one launch, every warp taking its share of one class after the other: nothing orders them,
-// and as launches of their own they cost a small graph 9 us each.
-__global__ void __launch_bounds__(kGroupWarps * 32, kGroupCtas)
-    build_groups_kernel(const ClassLists lists, const u32* __restrict__ cls, const u32* __restrict__ xadj,
-                        const float* __restrict__ wgt, Slot* __restrict__ slots, uint8_t* __restrict__ valid,
-                        u32* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char cta_smem[];
-  unsigned char* smem = cta_smem + (threadIdx.x >> 5) * kGroupBytes;
-  build_groups<32, 16>(smem, lists.list[K_32], cls[K_32], xadj, wgt, slots, valid, err);
-  build_groups<16, 16>(smem, lists.list[K_16], cls[K_16], xadj, wgt, slots, valid, err);
-  build_groups<8, 16>(smem, lists.list[K_8], cls[K_8], xadj, wgt, slots, valid, err);
-  build_groups<4, 16>(smem, lists.list[K_4], cls[K_4], xadj, wgt, slots, valid, err);
-  build_groups<2, 16>(smem, lists.list[K_2], cls[K_2], xadj, wgt, slots, valid, err);
-  build_groups<1, 16>(smem, lists.list[K_1B], cls[K_1B], xadj, wgt, slots, valid, err);
-  build_groups<1, 8>(smem, lists.list[K_1A], cls[K_1A], xadj, wgt, slots, valid, err);
-}
-
-// 513 .. 4096 weights: one CTA of NT = 64, 128 or 256 threads per vertex.
 template <int NT>
 struct ListShared {
-  static constexpr u32 kMost = NT * kListEpt;
-  uint2 list[kMost + 2], slots[kMost];
+  uint2 list[NT * kListEpt + 2], slots[NT * kListEpt];
   typename CtaCoop<NT>::Words words;
 };
-template <int NT>
-__global__ void __launch_bounds__(NT, 768 / NT) build_cta_kernel(const u32* __restrict__ list, const u32* __restrict__ count,
-                                                       const u32* __restrict__ xadj,
-                                                       const float* __restrict__ wgt, Slot* __restrict__ slots,
-                                                       uint8_t* __restrict__ valid, u32* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  ListShared<NT>* sh = reinterpret_cast<ListShared<NT>*>(smem);
-  const CtaCoop<NT> co(&sh->words);
-  for (ClassItems c(list, *count, xadj, blockIdx.x, gridDim.x); c.more();) {
-    const ClassItems::After after = c.look_ahead(wgt, co.t, 32);
-    const u32 n = c.end - c.off;
-    if (n > ListShared<NT>::kMost || n == 0) {
-      if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, c.v, n, ListShared<NT>::kMost);
-    } else {
-      build_list_f64<CtaCoop<NT>, (int)kListEpt>(co, c.v, c.off, n, wgt + c.off, slots, valid, sh->list, sh->slots, err);
+// bytes a warp has, whatever class it is at
+constexpr size_t kWarpBytes =
+    (std::max({sizeof(GroupShared<32, 16>), sizeof(GroupShared<16, 16>), sizeof(GroupShared<8, 16>),
+               sizeof(GroupShared<4, 16>), sizeof(GroupShared<2, 16>), sizeof(GroupShared<1, 16>),
+               (sizeof(ListShared<64>) + 1) / 2, (sizeof(ListShared<128>) + 3) / 4, (sizeof(ListShared<256>) + 7) / 8}) + 15) / 16 * 16;
+constexpr u32 kListWarps = 8, kListCtas = 3;  // warps a CTA, CTAs an SM: what registers and shared memory allow
+
+struct ListBuild {
+  const u32* xadj;
+  const float* wgt;
+  Slot* slots;
+  uint8_t* valid;
+  u32* err;
+};
+
+// The lists of one class, NT threads each with up to EPT weights a thread.  `turn` is where in the row of all warps the
+// class starts: classes are dealt out one behind the other, so that the few lists of a small graph go to different warps.
+// Moved on to the end of this class.
+template <int NT, int EPT>
+__device__ __forceinline__ void build_class(const ListBuild& b, unsigned char* smem, const u32* list, u32 count, u32& turn) {
+  const u32 warps = gridDim.x * kListWarps;
+  const u32 workers = NT >= 32 ? warps / (NT / 32) : warps * (32 / NT);
+  const u32 me = (blockIdx.x * (kListWarps * 32) + threadIdx.x) / NT;
+  const u32 start = NT >= 32 ? turn / (NT / 32) : turn * (32 / NT);
+  const u32 first = me >= start ? me - start : me + workers - start;
+  turn = (u32)((turn + ((u64)count * NT + 31) / 32) % warps);
+  auto build = [&](const auto& co, uint2* A, uint2* out) {
+    for (ClassItems c(list, count, b.xadj, first, workers); c.more();) {
+      const ClassItems::After after = c.look_ahead(b.wgt, co.t, NT >= 8 ? 32 : EPT);
+      const u32 n = c.end - c.off;
+      if (n > NT * EPT || n == 0) {  // classification and kernel disagree: record and skip
+        if (co.t == 0) dev_fail(b.err, DEV_ERR_INTERNAL, c.v, n, NT);
+      } else {
+        build_list_f64<std::decay_t<decltype(co)>, EPT>(co, c.v, c.off, n, b.wgt + c.off, b.slots, b.valid, A, out, b.err);
+      }
+      co.sync();  // the words are reused by the next vertex
+      c.advance(after);
     }
-    __syncthreads();
-    c.advance(after);
+  };
+  if constexpr (NT <= 32) {
+    GroupShared<NT, EPT>* sh = reinterpret_cast<GroupShared<NT, EPT>*>(smem + (threadIdx.x >> 5) * kWarpBytes);
+    const u32 in_warp = (threadIdx.x & 31) / NT;
+    if (first < count) build(GroupCoop<NT>(), sh->lists[in_warp], sh->slots[in_warp]);
+    __syncwarp();
+  } else {
+    const u32 part = threadIdx.x / NT;
+    ListShared<NT>* sh = reinterpret_cast<ListShared<NT>*>(smem + part * (NT / 32) * kWarpBytes);
+    if (first < count) build(CtaCoop<NT>(&sh->words, part), sh->list, sh->slots);
+  }
+}
+
+// Lists of up to 4096 weights: a CTA's warps work together or in parts on those of more than 512 (LONGER), alone or with
+// several lists side by side on the others.  Nothing orders the classes.  As launches of their own they cost a small graph
+// 9 us each, with every warp going through all of them in turn 53 us (1 M edges); dealt out one behind the other 24 us.
+// All in one kernel cost more registers than there are: 7 % slower on large graphs.
+template <bool LONGER>
+__global__ void __launch_bounds__(kListWarps * 32, kListCtas)
+    build_lists_kernel(const ClassLists lists, const u32* __restrict__ cls, const __grid_constant__ ListBuild b) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  u32 turn = 0;
+  if constexpr (LONGER) {
+    build_class<256, 16>(b, smem, lists.list[K_C256], cls[K_C256], turn);
+    build_class<128, 16>(b, smem, lists.list[K_C128], cls[K_C128], turn);
+    build_class<64, 16>(b, smem, lists.list[K_C64], cls[K_C64], turn);
+  } else {
+    build_class<32, 16>(b, smem, lists.list[K_32], cls[K_32], turn);
+    build_class<16, 16>(b, smem, lists.list[K_16], cls[K_16], turn);
+    build_class<8, 16>(b, smem, lists.list[K_8], cls[K_8], turn);
+    build_class<4, 16>(b, smem, lists.list[K_4], cls[K_4], turn);
+    build_class<2, 16>(b, smem, lists.list[K_2], cls[K_2], turn);
+    build_class<1, 16>(b, smem, lists.list[K_1B], cls[K_1B], turn);
+    build_class<1, 8>(b, smem, lists.list[K_1A], cls[K_1A], turn);
   }
 }
 
@@ -474,7 +484,8 @@ __device__ void build_vertex_cta(u32 v, u32 off, u32 n, const float* __restrict_
 // Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`.
 static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot* slots, uint8_t* valid) {
   cudaStream_t st = ctx->stream;
-  constexpr size_t kGroupSmem = kGroupWarps * kGroupBytes;
+  constexpr size_t kListSmem = kListWarps * kWarpBytes;
+  static_assert(kListCtas * (kListSmem + 1024) <= 228 * 1024, "shared memory of an SM");
   constexpr size_t kLongA = sizeof(LongShared<512, kMidSmemMax>), kLongB = sizeof(LongShared<1024, kHugeSmemMax>),
                    kLongC = sizeof(LongShared<1024, 8192>);
   static_assert(2 * (kLongA + 1024) <= 228 * 1024, "two CTAs an SM");
@@ -482,9 +493,8 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   if (!attr_set[ctx->device & 63]) {
 #define SMEM(BYTES, ...) \
   SKW_CUDA(ctx, cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)))
-    SMEM(sizeof(ListShared<256>), build_cta_kernel<256>);
-    SMEM(sizeof(ListShared<128>), build_cta_kernel<128>);
-    SMEM(kGroupSmem, build_groups_kernel);
+    SMEM(kListSmem, build_lists_kernel<true>);
+    SMEM(kListSmem, build_lists_kernel<false>);
     SMEM(kLongA, (build_long_kernel<512, kMidSmemMax, false>));
     SMEM(kLongB, (build_long_kernel<1024, kHugeSmemMax, false>));
     SMEM(kLongC, (build_long_kernel<1024, 8192, true>));
@@ -507,20 +517,13 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
     int rc = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, slab_bytes * gmem_ctas);
     if (rc != SKW_OK) return rc;
   }
-  // The classes are independent and each kernel drains its own work list through an atomic cursor,
-  // so they run side by side: the large classes (few, long-running CTAs, whose last vertices would
-  // otherwise leave most SMs idle) start first on streams of their own, the small classes fill in
-  // on the caller's stream.
-  const bool fork = ctx->max_degree > kGroupMax;
-  cudaStream_t s_h = st, s_a = st, s_b = st, s_c = st;
-  if (fork) {
-    SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
-    for (int i = 0; i < skw_ctx::kBuilderStreams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
-    s_h = ctx->bstream[0];
-    s_a = ctx->bstream[1];
-    s_b = ctx->bstream[2];
-    s_c = ctx->bstream[3];
-  }
+  // The classes are independent.  The long lists take few CTAs for long, so their kernels start first, on streams of their
+  // own, and the many short ones fill in on the caller's.
+  const int streams = ctx->max_degree > kHugeSmemMax ? 4 : ctx->max_degree > kMidSmemMax ? 3 : ctx->max_degree > kF64Max ? 2
+                      : ctx->max_degree > 32 * kListEpt ? 1 : 0;
+  cudaStream_t s_h = ctx->bstream[3], s_a = ctx->bstream[2], s_b = ctx->bstream[1], s_c = ctx->bstream[0];
+  if (streams) SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
+  for (int i = 0; i < streams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
 #define LONG(MORE_THAN, KCLS, NT, CAP, GLOBAL, CTAS, BYTES, SCRATCH, MOST, STREAM)                                       \
   if (ctx->max_degree > (MORE_THAN)) {                                                                                 \
     build_long_kernel<NT, CAP, GLOBAL><<<CTAS, NT, BYTES, STREAM>>>(lists.list[KCLS], cls, KCLS, ctx->xadj,            \
@@ -531,26 +534,17 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   LONG(kMidSmemMax, K_C2, 1024, kHugeSmemMax, false, ctx->sm_count, kLongB, nullptr, kHugeSmemMax, s_a)
   LONG(kF64Max, K_C2A, 512, kMidSmemMax, false, ctx->sm_count * 2, kLongA, nullptr, kMidSmemMax, s_b)
 #undef LONG
-  // 24 warps an SM: what the registers and the shared memory of these kernels allow, all of them resident at once
-  // (the vertices are dealt out by a stride over the grid: a second wave of CTAs would start when the first is done)
-#define LISTS(MORE_THAN, KCLS, NT, STREAM)                                                                      \
-  if (ctx->max_degree > (MORE_THAN)) {                                                                          \
-    build_cta_kernel<NT><<<ctx->sm_count * (768 / (NT)), NT, sizeof(ListShared<NT>), STREAM>>>(                 \
-        lists.list[KCLS], cls + KCLS, ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err);                       \
-    SKW_LAUNCHED(ctx);                                                                                          \
+  const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err};
+  const unsigned grid = ctx->sm_count * kListCtas;
+  if (streams) {
+    build_lists_kernel<true><<<grid, kListWarps * 32, kListSmem, s_c>>>(lists, cls, b);
+    SKW_LAUNCHED(ctx);
   }
-  LISTS(2048, K_C256, 256, s_c)
-  LISTS(1024, K_C128, 128, s_a)
-  LISTS(512, K_C64, 64, s_b)
-#undef LISTS
-  build_groups_kernel<<<ctx->sm_count * kGroupCtas, kGroupWarps * 32, kGroupSmem, st>>>(
-      lists, cls, ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err);
+  build_lists_kernel<false><<<grid, kListWarps * 32, kListSmem, st>>>(lists, cls, b);
   SKW_LAUNCHED(ctx);
-  if (fork) {
-    for (int i = 0; i < skw_ctx::kBuilderStreams; ++i) {
-      SKW_CUDA(ctx, cudaEventRecord(ctx->bjoin[i], ctx->bstream[i]));
-      SKW_CUDA(ctx, cudaStreamWaitEvent(st, ctx->bjoin[i], 0));
-    }
+  for (int i = 0; i < streams; ++i) {
+    SKW_CUDA(ctx, cudaEventRecord(ctx->bjoin[i], ctx->bstream[i]));
+    SKW_CUDA(ctx, cudaStreamWaitEvent(st, ctx->bjoin[i], 0));
   }
   return SKW_OK;
 }
@@ -561,42 +555,62 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
 // units still running.  A vertex is claimed by the first unit that stamps it in the current collection.
 constexpr u32 kAliveMark = 0xFFFFFFFFu;
 
+// A tile of 1024 units is claimed and binned at a time, like the vertices of classify_kernel: one atomic a class and tile on
+// the counters instead of one a class and warp, which all warps queued up for (hop 2 of 65,536 x 25, 10: 79 -> 28 us).
+constexpr u32 kFrontierUnits = 4;  // per thread
 __global__ void __launch_bounds__(256) frontier_collect_kernel(
     const u32* __restrict__ verts, u64 units, u32 width, u32 cells, u32 offs,
     const u32* __restrict__ alive, const u32* __restrict__ xadj, u32 V, u32* __restrict__ stamp,
     u32 round, u32* __restrict__ cls, const ClassLists lists, u32 cap, u32* __restrict__ err) {
+  __shared__ u32 s_cnt[K_CLASSES], s_base[K_CLASSES];
   const u32 lane = threadIdx.x & 31;
-  const u64 T = (u64)gridDim.x * blockDim.x;
-  for (u64 u0 = (u64)blockIdx.x * blockDim.x; u0 < units; u0 += T) {
-    const u64 u = u0 + threadIdx.x;
-    int c = -1;
-    u32 v = 0;
-    if (u < units && (!alive || alive[u / width] == kAliveMark)) {
-      v = verts[(u / width) * cells + offs + u % width];
-      if (v != 0xFFFFFFFFu) {
-        if (v >= V) {
-          dev_fail(err, DEV_ERR_INDEX, v, (u32)u, 10);
-        } else {
-          const u32 deg = xadj[v + 1] - xadj[v];
-          // a hub stands in thousands of cells of one frontier: look before claiming, so that only the
-          // first few of them queue up at its stamp word with an atomic
-          if (deg && __ldcg(stamp + v) != round && atomicExch(&stamp[v], round) != round) c = degree_class(deg);
-        }
+  constexpr u32 kTile = 256 * kFrontierUnits;
+  for (u64 u0 = (u64)blockIdx.x * kTile; u0 < units; u0 += (u64)gridDim.x * kTile) {
+    if (threadIdx.x < K_CLASSES) s_cnt[threadIdx.x] = 0;
+    u32 v[kFrontierUnits], rank[kFrontierUnits];
+    int c[kFrontierUnits];
+#pragma unroll
+    for (u32 j = 0; j < kFrontierUnits; ++j) {
+      const u64 u = u0 + j * 256 + threadIdx.x;
+      v[j] = 0xFFFFFFFFu;
+      if (u < units && (!alive || alive[u / width] == kAliveMark)) v[j] = verts[(u / width) * cells + offs + u % width];
+    }
+    // a hub stands in thousands of cells of one frontier: look before claiming, so that only the first few of them queue
+    // up at its stamp word with an atomic
+#pragma unroll
+    for (u32 j = 0; j < kFrontierUnits; ++j) {
+      c[j] = -1;
+      if (v[j] == 0xFFFFFFFFu) continue;
+      if (v[j] >= V) {
+        dev_fail(err, DEV_ERR_INDEX, v[j], 0, 10);
+        continue;
       }
+      const u32 deg = __ldg(xadj + v[j] + 1) - __ldg(xadj + v[j]);
+      if (deg && __ldcg(stamp + v[j]) != round) c[j] = degree_class(deg);
     }
 #pragma unroll
-    for (int k = 0; k < K_CLASSES; ++k) {
-      const u32 m = __ballot_sync(0xFFFFFFFFu, c == k);
-      if (!m) continue;
-      u32 base = 0;
-      if (lane == (u32)(__ffs(m) - 1)) base = atomicAdd(&cls[k], __popc(m));
-      base = __shfl_sync(0xFFFFFFFFu, base, __ffs(m) - 1);
-      if (c == k) {
-        const u32 idx = base + __popc(m & ((1u << lane) - 1u));
-        if (idx < cap) lists.list[k][idx] = v;
-        else dev_fail(err, DEV_ERR_CAPACITY, idx, cap, 11);
-      }
+    for (u32 j = 0; j < kFrontierUnits; ++j)
+      if (c[j] >= 0 && atomicExch(&stamp[v[j]], round) == round) c[j] = -1;
+    __syncthreads();
+#pragma unroll
+    for (u32 j = 0; j < kFrontierUnits; ++j) {
+      const u32 same = __match_any_sync(0xFFFFFFFFu, c[j]);
+      const int first = __ffs(same) - 1;
+      u32 at = 0;
+      if (c[j] >= 0 && lane == (u32)first) at = atomicAdd(&s_cnt[c[j]], (u32)__popc(same));
+      rank[j] = __shfl_sync(0xFFFFFFFFu, at, first) + __popc(same & ((1u << lane) - 1u));
     }
+    __syncthreads();
+    if (threadIdx.x < K_CLASSES && s_cnt[threadIdx.x]) s_base[threadIdx.x] = atomicAdd(&cls[threadIdx.x], s_cnt[threadIdx.x]);
+    __syncthreads();
+#pragma unroll
+    for (u32 j = 0; j < kFrontierUnits; ++j) {
+      if (c[j] < 0) continue;
+      const u32 idx = s_base[c[j]] + rank[j];
+      if (idx < cap) lists.list[c[j]][idx] = v[j];
+      else dev_fail(err, DEV_ERR_CAPACITY, idx, cap, 11);
+    }
+    __syncthreads();
   }
 }
 
@@ -624,8 +638,8 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
   SKW_CUDA(ctx, cudaMemsetAsync(ctx->frontier_cls, 0, 2 * K_CLASSES * sizeof(u32), st));
   if (units) {
     // the claim is a chain of dependent accesses (vertex, offsets, stamp): fill every thread slot of the GPU
-    const u64 want = (units + 255) / 256;
-    const int grid = (int)(want < (u64)ctx->sm_count * 16 ? want : (u64)ctx->sm_count * 16);
+    const u64 want = (units + 256 * kFrontierUnits - 1) / (256 * kFrontierUnits);
+    const int grid = (int)(want < (u64)ctx->sm_count * 8 ? want : (u64)ctx->sm_count * 8);
     ClassLists lists;
     for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->frontier_lists + (size_t)k * cap;
     frontier_collect_kernel<<<grid, 256, 0, st>>>(verts, units, width, cells, offs, alive_lengths,

@@ -78,8 +78,9 @@ struct GroupCoop {
   }
 };
 
-// Cooperation inside a CTA of NTHREADS threads.  Every reduction has its own words of shared memory, so each takes
-// one barrier; the warps all scan the (at most 32) warp totals themselves instead of waiting for one that does.
+// Cooperation inside NTHREADS threads of a CTA of 256, the part-th such part of it.  Every reduction has its own words of
+// shared memory, so each takes one barrier; the warps all scan the (at most 32) warp totals themselves instead of waiting
+// for one that does.
 template <int NTHREADS>
 struct CtaCoop {
   static constexpr int NT = NTHREADS, NW = NTHREADS / 32;
@@ -90,13 +91,17 @@ struct CtaCoop {
   };
   u32 t;
   Words* sh;
-  __device__ __forceinline__ explicit CtaCoop(Words* words) : t(threadIdx.x), sh(words) {}
-  __device__ __forceinline__ void sync() const { __syncthreads(); }
+  // Barrier of this part (0 is the CTA's own).  Parts of different sizes have different ones: while one part is still at a
+  // list, another may have gone on to smaller parts, and a barrier has one thread count at a time.
+  u32 bar;
+  __device__ __forceinline__ CtaCoop(Words* words, u32 part)
+      : t(threadIdx.x % NTHREADS), sh(words), bar(256 / NTHREADS + part) {}
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NTHREADS) : "memory"); }
   template <int USE>
   __device__ __forceinline__ int max(int v) const {
     v = __reduce_max_sync(0xFFFFFFFFu, v);
     if ((t & 31) == 0) sh->m[USE][t >> 5] = v;
-    __syncthreads();
+    sync();
     return __reduce_max_sync(0xFFFFFFFFu, sh->m[USE][(t & 31) < NW ? (t & 31) : 0]);
   }
   __device__ __forceinline__ void scan(double& v, double& total) const {
@@ -104,7 +109,7 @@ struct CtaCoop {
     double part = v, sum;
     w.scan(part, sum);
     if ((t & 31) == 0) sh->q[t >> 5] = sum;
-    __syncthreads();
+    sync();
     double before = (t & 31) < NW ? sh->q[t & 31] : 0.0;
     w.scan(before, total);
     v = part + __shfl_sync(0xFFFFFFFFu, before, t >> 5);
@@ -118,7 +123,7 @@ struct CtaCoop {
       sh->d[t >> 5] = sum;
       sh->s[t >> 5] = sc;
     }
-    __syncthreads();
+    sync();
     double before = (t & 31) < NW ? sh->d[t & 31] : 0.0;
     u32 bc = (t & 31) < NW ? sh->s[t & 31] : 0u;
     w.scan(before, bc, total, count);
