@@ -537,7 +537,12 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err};
   const unsigned grid = ctx->sm_count * kListCtas;
   if (streams) {
-    build_lists_kernel<true><<<grid, kListWarps * 32, kListSmem, s_c>>>(lists, cls, b);
+    // The lists of a CTA are dealt out beforehand, so one that starts late, behind a long list, ends late.  They start when
+    // the CTAs of 4097 to 8192 weights run out, and with 64 K edges or more for each there are up to four for every one that
+    // fits (457 M edges: 4.69 -> 4.42 ms; 65 M: 1.73 -> 1.72; fewer edges would pay for the start of each instead).  More
+    // CTAs for the short lists cost more in starts, seven classes each, than they gave (2.50 -> 2.55 ms at 226 M edges).
+    const u64 waves = std::clamp<u64>((u64)ctx->E / ((u64)grid << 16), 1, 4);
+    build_lists_kernel<true><<<(unsigned)(grid * waves), kListWarps * 32, kListSmem, streams > 1 ? s_b : s_c>>>(lists, cls, b);
     SKW_LAUNCHED(ctx);
   }
   build_lists_kernel<false><<<grid, kListWarps * 32, kListSmem, st>>>(lists, cls, b);

@@ -60,3 +60,24 @@ def test_alias_class_edges(ctx, oracle, kind, shift):
     usable = np.repeat(want_valid.astype(bool), sizes)
     bad = np.flatnonzero(usable & ((prob != want_prob) | (alias != want_alias)))
     assert bad.size == 0, "list lengths that differ: %s" % sorted({sizes[np.searchsorted(x, b, "right") - 1] for b in bad})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("least, most, lists", [(513, 1024, 3000), (1025, 2048, 1500), (2049, 4096, 700), (1, 40, 200000), (3, 4500, 1500)])
+def test_alias_several_lists_a_worker(ctx, oracle, least, most, lists):
+    """More lists of a class than there are lanes, warps or parts of a CTA to take one each, next to few of the others."""
+    import torch
+    rng = np.random.default_rng(most)
+    sizes = np.concatenate([rng.integers(least, most + 1, lists), [0, 7, 20, 90, 700, 1300, 3000, 9000, 17000]])
+    rng.shuffle(sizes)
+    x = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    E, V = int(x[-1]), len(sizes)
+    w = rng.lognormal(0, 1, E).astype(np.float32)
+    d_x, d_a = torch.from_numpy(x.view(np.int32)).cuda(), torch.zeros(E, dtype=torch.int32, device="cuda")
+    d_w = torch.from_numpy(w).cuda()
+    torch.cuda.synchronize()
+    ctx.adopt_device(V, E, d_x, d_a, d_w)
+    ctx.alias_build_offline()
+    prob, alias, valid = ctx.alias_export()
+    want_prob, want_alias, want_valid = oracle.alias_build(x, w)
+    assert np.array_equal(valid, want_valid) and np.array_equal(prob, want_prob) and np.array_equal(alias, want_alias)
