@@ -26,7 +26,7 @@
 // Work distribution: vertices are binned by degree with warp ballots and shared-memory prefix sums (classify_*
 // kernels), one work list per class.  Lists of up to 4096 weights are built in double precision by a lane, a group of
 // lanes, a warp or a CTA that holds the whole list in registers (skw_alias_f64.cuh); longer ones by CTAs that work
-// through it in tiles of 64-bit integers (build_vertex_merge).
+// through it in tiles (skw_alias_long.cuh), a few giant ones by clusters of CTAs (skw_alias_cluster.cuh).
 #include <math_constants.h>
 
 #include <algorithm>
@@ -35,6 +35,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "skw_alias_cluster.cuh"
 #include "skw_alias_f64.cuh"
 #include "skw_alias_long.cuh"
 #include "skw_alias_math.cuh"
@@ -52,7 +53,7 @@ enum { K_1A = 0, K_1B, K_2, K_4, K_8, K_16, K_32, K_C64, K_C128, K_C256, K_C2A, 
 constexpr u32 kListEpt = 16;
 constexpr u32 kGroupMax = 32 * kListEpt;      // 512: the longest list of a group of lanes
 constexpr u32 kMidSmemMax = 8192;             // two 512-thread CTAs per SM with 96 KB of lists each
-constexpr u32 kHugeSmemMax = 16384;           // one 1024-thread CTA per SM with 192 KB of lists
+constexpr u32 kHugeSmemMax = 16384;           // one 1024-thread CTA per SM with 192 KB of lists; longer ones have them in global memory
 static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
 static_assert(2 * K_CLASSES <= 64, "class counters");
 
@@ -276,19 +277,21 @@ __global__ void __launch_bounds__(kListWarps * 32, kListCtas)
 }
 
 // More than 4096 weights: one CTA per vertex, handed out by the class's cursor (degrees, hence costs, vary widely).
-// GLOBAL: lists in this CTA's slab of global scratch (cap + 2 entries of 12 bytes), else in shared memory.
+// GLOBAL: lists in this CTA's slab of global scratch (cap + 2 entries of 12 bytes), else in shared memory.  A class of at
+// most `others` lists is left to build_cluster_kernel.
 template <int NT, int CAP, bool GLOBAL>
 __global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __restrict__ list, u32* __restrict__ cls, int k,
                                                                    const u32* __restrict__ xadj,
                                                                    const float* __restrict__ wgt, Slot* __restrict__ slots,
                                                                    uint8_t* __restrict__ valid,
                                                                    unsigned char* __restrict__ scratch, u64 cap,
-                                                                   u32* __restrict__ err) {
+                                                                   u32 others, u32* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem[];
   LongShared<NT, CAP>* sh = reinterpret_cast<LongShared<NT, CAP>*>(smem);
   u64* A = GLOBAL ? reinterpret_cast<u64*>(scratch + (u64)blockIdx.x * (cap + 2) * 12ull) : nullptr;
   u32* P = GLOBAL ? reinterpret_cast<u32*>(A + cap + 2) : nullptr;
   const u32 count = cls[k];
+  if (count <= others) return;
   __shared__ u32 s_it;
   for (;;) {
     if (threadIdx.x == 0) s_it = atomicAdd(cls + K_CLASSES + k, 1u);
@@ -305,6 +308,26 @@ __global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __
     build_list_long<NT, CAP, GLOBAL>(v, off, n, wgt + off, slots, valid, sh, A, P, err);
     __syncthreads();
   }
+}
+
+// As many lists of class k as there are clusters, or fewer: one for each, with a slab of scratch of its own for up to cap
+// weights (cap even), 12 bytes each.
+__global__ void __launch_bounds__(kClusterThreads, 3) __cluster_dims__(kClusterCtas, 1, 1)
+    build_cluster_kernel(const u32* __restrict__ list, const u32* __restrict__ cls, int k, const __grid_constant__ ListBuild b,
+                         unsigned char* __restrict__ scratch, u64 cap) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const u32 rank = blockIdx.x % kClusterCtas, it = blockIdx.x / kClusterCtas, count = cls[k];
+  if (it >= count || count > gridDim.x / kClusterCtas) return;  // (the whole cluster)
+  const u32 v = list[it];
+  const u32 off = b.xadj[v], n = b.xadj[v + 1] - off;
+  if (n > cap || n == 0) {
+    if (rank == 0 && threadIdx.x == 0) dev_fail(b.err, DEV_ERR_CAPACITY, v, n, (u32)cap);
+    return;
+  }
+  u64* A = reinterpret_cast<u64*>(scratch + it * cap * 12);
+  build_list_cluster(rank, v, off, n, b.wgt + off, b.slots, b.valid, reinterpret_cast<ClusterShared*>(smem), A,
+                     reinterpret_cast<u32*>(A + cap), b.err);
+  cluster_sync();  // the CTAs read one another's shared memory
 }
 
 // ------------------------------------------------------------------ one CTA per vertex -----
@@ -489,12 +512,14 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   constexpr size_t kLongA = sizeof(LongShared<512, kMidSmemMax>), kLongB = sizeof(LongShared<1024, kHugeSmemMax>),
                    kLongC = sizeof(LongShared<1024, 8192>);
   static_assert(2 * (kLongA + 1024) <= 228 * 1024, "two CTAs an SM");
+  static_assert(3 * (sizeof(ClusterShared) + 1024) <= 228 * 1024, "three CTAs an SM");
   static bool attr_set[64] = {false};
   if (!attr_set[ctx->device & 63]) {
 #define SMEM(BYTES, ...) \
   SKW_CUDA(ctx, cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)))
     SMEM(kListSmem, build_lists_kernel<true>);
     SMEM(kListSmem, build_lists_kernel<false>);
+    SMEM(sizeof(ClusterShared), build_cluster_kernel);
     SMEM(kLongA, (build_long_kernel<512, kMidSmemMax, false>));
     SMEM(kLongB, (build_long_kernel<1024, kHugeSmemMax, false>));
     SMEM(kLongC, (build_long_kernel<1024, 8192, true>));
@@ -502,10 +527,7 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
     attr_set[ctx->device & 63] = true;
   }
   // one slab per CTA of the scratch class, sized by the largest degree; fewer CTAs when a giant hub
-  // would make the slabs exceed 4 GB in total.  (Two 512-thread CTAs per SM instead of one of 1024 were
-  // measured: 4.61 against 4.70 ms for this class at scale 26, where thousands of such vertices keep
-  // every SM busy either way, but 0.23 ms instead of about 0.15 ms for the largest vertex of an online
-  // frontier, which a hop has to wait for; so one vertex gets the 1024 threads.)
+  // would make the slabs exceed 4 GB in total.
   const uint64_t slab_elems = ctx->max_degree > kHugeSmemMax ? (((uint64_t)ctx->max_degree + 1) & ~1ull) : 0;
   const uint64_t slab_bytes = (slab_elems + 2) * 12ull;
   int gmem_ctas = ctx->sm_count;
@@ -520,21 +542,30 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   // The classes are independent.  The long lists take few CTAs for long, so their kernels start first, on streams of their
   // own, and the many short ones fill in on the caller's.
   const int streams = ctx->max_degree > kHugeSmemMax ? 4 : ctx->max_degree > kMidSmemMax ? 3 : ctx->max_degree > kF64Max ? 2
-                      : ctx->max_degree > 32 * kListEpt ? 1 : 0;
+                      : ctx->max_degree > kGroupMax ? 1 : 0;
   cudaStream_t s_h = ctx->bstream[3], s_a = ctx->bstream[2], s_b = ctx->bstream[1], s_c = ctx->bstream[0];
   if (streams) SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
   for (int i = 0; i < streams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
-#define LONG(MORE_THAN, KCLS, NT, CAP, GLOBAL, CTAS, BYTES, SCRATCH, MOST, STREAM)                                       \
+  const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err};
+  // The lists beyond 16384 weights: one of these two kernels finds that they are its own, by their number, and both use the
+  // same scratch.
+  unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
+  const unsigned clusters = slab_elems ? std::min<unsigned>(ctx->sm_count * 3 / kClusterCtas, gmem_ctas) : 0;
+  if (clusters) {
+    build_cluster_kernel<<<clusters * kClusterCtas, kClusterThreads, sizeof(ClusterShared), s_h>>>(lists.list[K_H], cls, K_H, b,
+                                                                                                  scratch, slab_elems);
+    SKW_LAUNCHED(ctx);
+  }
+#define LONG(MORE_THAN, KCLS, NT, CAP, GLOBAL, CTAS, BYTES, SCRATCH, MOST, OTHERS, STREAM)                                     \
   if (ctx->max_degree > (MORE_THAN)) {                                                                                 \
     build_long_kernel<NT, CAP, GLOBAL><<<CTAS, NT, BYTES, STREAM>>>(lists.list[KCLS], cls, KCLS, ctx->xadj,            \
-                                                                   ctx->adjwgt, slots, valid, SCRATCH, MOST, ctx->d_err); \
+                                                                   ctx->adjwgt, slots, valid, SCRATCH, MOST, OTHERS, ctx->d_err); \
     SKW_LAUNCHED(ctx);                                                                                                 \
   }
-  LONG(kHugeSmemMax, K_H, 1024, 8192, true, gmem_ctas, kLongC, static_cast<unsigned char*>(ctx->cta_scratch), slab_elems, s_h)
-  LONG(kMidSmemMax, K_C2, 1024, kHugeSmemMax, false, ctx->sm_count, kLongB, nullptr, kHugeSmemMax, s_a)
-  LONG(kF64Max, K_C2A, 512, kMidSmemMax, false, ctx->sm_count * 2, kLongA, nullptr, kMidSmemMax, s_b)
+  LONG(kHugeSmemMax, K_H, 1024, 8192, true, gmem_ctas, kLongC, scratch, slab_elems, clusters, s_h)
+  LONG(kMidSmemMax, K_C2, 1024, kHugeSmemMax, false, ctx->sm_count, kLongB, nullptr, kHugeSmemMax, 0, s_a)
+  LONG(kF64Max, K_C2A, 512, kMidSmemMax, false, ctx->sm_count * 2, kLongA, nullptr, kMidSmemMax, 0, s_b)
 #undef LONG
-  const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err};
   const unsigned grid = ctx->sm_count * kListCtas;
   if (streams) {
     // The lists of a CTA are dealt out beforehand, so one that starts late, behind a long list, ends late.  They start when
