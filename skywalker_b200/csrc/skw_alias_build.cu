@@ -660,7 +660,7 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
   ctx->frontier_lists = static_cast<u32*>(p);
   if (rc != SKW_OK) return rc;
   if (!ctx->stamp) {
-    SKW_CUDA(ctx, dev_malloc(ctx, reinterpret_cast<void**>(&ctx->stamp), sizeof(u32) * ((size_t)ctx->V + 1)));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->stamp, sizeof(u32) * ((size_t)ctx->V + 1)));
     SKW_CUDA(ctx, cudaMemsetAsync(ctx->stamp, 0, sizeof(u32) * ((size_t)ctx->V + 1), ctx->stream));
     ctx->stamp_round = 0;
   }

@@ -4,7 +4,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <unordered_map>
 #include <vector>
 
 #include "skw_ctx.h"
@@ -39,21 +41,119 @@ int fail_cuda(skw_ctx* ctx, cudaError_t e, const char* what, const char* file, i
 
 int ensure_bytes(skw_ctx* ctx, void** p, size_t* cap, size_t want) {
   if (*cap >= want && *p) return SKW_OK;
-  if (*p) SKW_CUDA(ctx, cudaFree(*p));
+  dev_free(*p);
   *p = nullptr;
   *cap = 0;
   if (want == 0) want = 256;
-  SKW_CUDA(ctx, dev_malloc(ctx, p, want));
+  SKW_CUDA(ctx, dev_malloc_bytes(ctx, p, want));
   *cap = want;
   return SKW_OK;
 }
 
-cudaError_t dev_malloc(skw_ctx* ctx, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
+// Device memory of all contexts.  Freed blocks wait here for the next graph or context: a program that goes from batch
+// graph to batch graph allocates the same few sizes over and over, and a cudaMalloc with its cudaFree costs 1 to 10 ms a
+// gigabyte, several times the kernels that fill it.  At most a 16th of a GPU's memory waits; it is given back when an
+// allocation would fail otherwise, by the calls that free memory on request, and with the last context of the GPU.  A block is only reused once the GPU is idle, as
+// cudaFree would have waited for too, so streams and threads do not matter.
+struct DeviceMemory {
+  struct Block {
+    size_t bytes;
+    int device;
+  };
+  std::mutex mu;
+  std::unordered_map<void*, Block> live;
+  struct Spare {
+    std::multimap<size_t, void*> blocks;
+    size_t bytes = 0, most = 0;
+    int contexts = 0;
+  } spare[64];
+  static DeviceMemory& get() {
+    static DeviceMemory* m = new DeviceMemory;  // outlives every context, whenever that is destroyed
+    return *m;
+  }
+  // small blocks in powers of two, large ones in the 2 MB pages that the driver hands out anyway
+  static size_t rounded(size_t bytes) {
+    size_t r = 512;
+    while (r < bytes && r < ((size_t)1 << 20)) r *= 2;
+    return r >= bytes ? r : (bytes + ((size_t)2 << 20) - 1) & ~(((size_t)2 << 20) - 1);
+  }
+  void give_back(int device) {
+    Spare& s = spare[device & 63];
+    for (const auto& b : s.blocks) cudaFree(b.second);
+    s.blocks.clear();
+    s.bytes = 0;
+  }
+  cudaError_t alloc(void** p, size_t bytes) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const size_t size = rounded(bytes);
+    std::lock_guard<std::mutex> lk(mu);
+    Spare& s = spare[device & 63];
+    const auto it = s.blocks.lower_bound(size);
+    if (it != s.blocks.end() && it->first <= size + size / 4) {
+      *p = it->second;
+      live[*p] = Block{it->first, device};
+      s.bytes -= it->first;
+      s.blocks.erase(it);
+      return cudaSuccess;
+    }
+    e = cudaMalloc(p, size);
+    if (e == cudaErrorMemoryAllocation && !s.blocks.empty()) {
+      cudaGetLastError();
+      give_back(device);
+      e = cudaMalloc(p, size);
+    }
+    if (e == cudaSuccess) live[*p] = Block{size, device};
+    return e;
+  }
+  void free(void* p) {
+    if (!p) return;
+    std::unique_lock<std::mutex> lk(mu);
+    const auto it = live.find(p);
+    if (it == live.end()) {
+      cudaFree(p);
+      return;
+    }
+    const Block b = it->second;
+    live.erase(it);
+    lk.unlock();
+    DeviceGuard g(b.device);
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    lk.lock();
+    Spare& s = spare[b.device & 63];
+    if (!idle || s.contexts == 0 || b.bytes > s.most - s.bytes) {
+      cudaFree(p);
+      return;
+    }
+    s.blocks.emplace(b.bytes, p);
+    s.bytes += b.bytes;
+  }
+  void context_made(int device) {
+    std::lock_guard<std::mutex> lk(mu);
+    Spare& s = spare[device & 63];
+    size_t unused = 0, total = 0;
+    if (s.contexts++ == 0 && cudaMemGetInfo(&unused, &total) == cudaSuccess) s.most = total / 16;
+  }
+  void context_gone(int device) {
+    std::lock_guard<std::mutex> lk(mu);
+    if (--spare[device & 63].contexts == 0) give_back(device);
+  }
+};
+
+void dev_free(void* p) { DeviceMemory::get().free(p); }
+void dev_give_back(int device) {
+  DeviceMemory& m = DeviceMemory::get();
+  std::lock_guard<std::mutex> lk(m.mu);
+  m.give_back(device);
+}
+
+cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes) {
+  cudaError_t e = DeviceMemory::get().alloc(p, bytes);
   if (e == cudaErrorMemoryAllocation && ctx->records && !ctx->records_ready) {
     cudaGetLastError();
     drop_records(ctx);
-    e = cudaMalloc(p, bytes);
+    e = DeviceMemory::get().alloc(p, bytes);
   }
   return e;
 }
@@ -95,28 +195,28 @@ int err_check(skw_ctx* ctx, const char* where, uint32_t sums_to_clear) {
 
 static void free_graph(skw_ctx* ctx) {
   if (ctx->owns_graph) {
-    cudaFree(ctx->xadj);
-    cudaFree(ctx->adjncy);
+    dev_free(ctx->xadj);
+    dev_free(ctx->adjncy);
   }
-  if (ctx->owns_weights) cudaFree(ctx->adjwgt);
+  if (ctx->owns_weights) dev_free(ctx->adjwgt);
   ctx->xadj = ctx->adjncy = nullptr;
   ctx->adjwgt = nullptr;
   ctx->owns_graph = ctx->owns_weights = false;
-  cudaFree(ctx->slots);
-  cudaFree(ctx->valid);
-  cudaFree(ctx->online_slots);
-  cudaFree(ctx->online_valid);
+  dev_free(ctx->slots);
+  dev_free(ctx->valid);
+  dev_free(ctx->online_slots);
+  dev_free(ctx->online_valid);
   ctx->online_slots = nullptr;
   ctx->online_valid = nullptr;
-  cudaFree(ctx->stamp);
-  cudaFree(ctx->prep_memo);
-  cudaFree(ctx->prep_ckpt);
+  dev_free(ctx->stamp);
+  dev_free(ctx->prep_memo);
+  dev_free(ctx->prep_ckpt);
   ctx->prep_ckpt = nullptr;
   ctx->prep_memo = nullptr;
   ctx->prep_stamp = 0;
-  cudaFree(ctx->records);
-  cudaFree(ctx->vinfo);
-  cudaFree(ctx->vbits);
+  dev_free(ctx->records);
+  dev_free(ctx->vinfo);
+  dev_free(ctx->vbits);
   ctx->records = nullptr;
   ctx->vinfo = nullptr;
   ctx->vbits = nullptr;
@@ -294,9 +394,9 @@ int finish_graph(skw_ctx* ctx) {
 void drop_records(skw_ctx* ctx) {
   ctx->records_ready = false;
   if (ctx->records || ctx->vinfo) cudaStreamSynchronize(ctx->stream);
-  cudaFree(ctx->records);
-  cudaFree(ctx->vinfo);
-  cudaFree(ctx->vbits);
+  dev_free(ctx->records);
+  dev_free(ctx->vinfo);
+  dev_free(ctx->vbits);
   ctx->records = nullptr;
   ctx->vinfo = nullptr;
   ctx->vbits = nullptr;
@@ -306,7 +406,7 @@ int alloc_table(skw_ctx* ctx, TableUse use) {
   // kSlotSlack spare entries let a multi-GPU caller all-gather the table in equal chunks in place
   const size_t n = (size_t)ctx->E + kSlotSlack;
   if (!ctx->slots) {
-    SKW_CUDA(ctx, dev_malloc(ctx, reinterpret_cast<void**>(&ctx->slots), sizeof(Slot) * n));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->slots, sizeof(Slot) * n));
     ctx->slots_marked = false;
   }
   if (!ctx->slots_marked && use != TableUse::kFrontier) {
@@ -317,7 +417,7 @@ int alloc_table(skw_ctx* ctx, TableUse use) {
     ctx->slots_marked = true;
   }
   if (!ctx->valid) {
-    SKW_CUDA(ctx, cudaMalloc(&ctx->valid, ctx->V ? ctx->V : 1));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->valid, ctx->V ? ctx->V : 1));
     SKW_CUDA(ctx, cudaMemsetAsync(ctx->valid, 0, ctx->V ? ctx->V : 1, ctx->stream));
   }
   return SKW_OK;
@@ -362,6 +462,8 @@ int skw_ctx_create(int device, skw_ctx** out) {
     }                                                                            \
   } while (0)
   CK(cudaSetDevice(device));
+  DeviceMemory::get().context_made(device);
+  ctx->counted = true;
   CK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
   CK(cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking));
@@ -374,7 +476,7 @@ int skw_ctx_create(int device, skw_ctx** out) {
   CK(cudaEventCreateWithFlags(&ctx->bfork, cudaEventDisableTiming));
   CK(cudaEventCreate(&ctx->ev0));
   CK(cudaEventCreate(&ctx->ev1));
-  CK(cudaMalloc(&ctx->d_err, 64));
+  CK(dev_malloc(ctx, &ctx->d_err, 64));
   CK(cudaMemset(ctx->d_err, 0, 64));
   CK(cudaMallocHost(&ctx->h_err, 64));
   ctx->d_sum = reinterpret_cast<uint64_t*>(ctx->d_err + 8);
@@ -386,8 +488,8 @@ int skw_ctx_create(int device, skw_ctx** out) {
     CK(cudaEventCreate(&ctx->pk_t1[i]));
   }
   CK(cudaMallocHost(&ctx->h_tot, skw_ctx::kPackSlices * sizeof(uint64_t)));
-  CK(cudaMalloc(&ctx->cls_counts, 64 * sizeof(uint32_t)));
-  CK(cudaMalloc(&ctx->frontier_cls, 64 * sizeof(uint32_t)));
+  CK(dev_malloc(ctx, &ctx->cls_counts, 64 * sizeof(uint32_t)));
+  CK(dev_malloc(ctx, &ctx->frontier_cls, 64 * sizeof(uint32_t)));
 #undef CK
   *out = ctx;
   return SKW_OK;
@@ -398,14 +500,14 @@ void skw_ctx_destroy(skw_ctx* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->own_stream) cudaStreamSynchronize(ctx->own_stream);
   free_graph(ctx);
-  cudaFree(ctx->d_err);
+  dev_free(ctx->d_err);
   cudaFreeHost(ctx->h_err);
-  cudaFree(ctx->worklist);
-  cudaFree(ctx->cls_counts);
-  cudaFree(ctx->cta_scratch);
-  cudaFree(ctx->frontier_lists);
-  cudaFree(ctx->frontier_cls);
-  for (int i = 0; i < skw_ctx::kStages; ++i) cudaFree(ctx->stage[i]);
+  dev_free(ctx->worklist);
+  dev_free(ctx->cls_counts);
+  dev_free(ctx->cta_scratch);
+  dev_free(ctx->frontier_lists);
+  dev_free(ctx->frontier_cls);
+  for (int i = 0; i < skw_ctx::kStages; ++i) dev_free(ctx->stage[i]);
   if (ctx->h_pack) cudaFreeHost(ctx->h_pack);
   delete static_cast<skw::HostPool*>(ctx->host_pool);
   cudaFreeHost(ctx->h_tot);
@@ -425,6 +527,7 @@ void skw_ctx_destroy(skw_ctx* ctx) {
     if (ctx->pk_t0[i]) cudaEventDestroy(ctx->pk_t0[i]);
     if (ctx->pk_t1[i]) cudaEventDestroy(ctx->pk_t1[i]);
   }
+  if (ctx->counted) DeviceMemory::get().context_gone(ctx->device);
   delete ctx;
 }
 
@@ -453,9 +556,9 @@ int skw_graph_upload(skw_ctx* ctx, uint32_t V, uint64_t E, const uint32_t* h_xad
     return fail(ctx, SKW_ERR_ARG, "skw_graph_upload: xadj[0] must be 0 and xadj[V] must equal E");
   DeviceGuard g(ctx->device);
   free_graph(ctx);
-  SKW_CUDA(ctx, cudaMalloc(&ctx->xadj, sizeof(uint32_t) * ((size_t)V + 1)));
-  SKW_CUDA(ctx, cudaMalloc(&ctx->adjncy, sizeof(uint32_t) * (E ? E : 1)));
-  SKW_CUDA(ctx, cudaMalloc(&ctx->adjwgt, sizeof(float) * (E ? E : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &ctx->xadj, sizeof(uint32_t) * ((size_t)V + 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &ctx->adjncy, sizeof(uint32_t) * (E ? E : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &ctx->adjwgt, sizeof(float) * (E ? E : 1)));
   ctx->owns_graph = ctx->owns_weights = true;
   ctx->V = V;
   ctx->E = E;
@@ -491,7 +594,7 @@ int skw_graph_adopt_device(skw_ctx* ctx, uint32_t V, uint64_t E, const uint32_t*
   ctx->V = V;
   ctx->E = E;
   if (!d_adjwgt) {
-    SKW_CUDA(ctx, cudaMalloc(&ctx->adjwgt, sizeof(float) * (E ? E : 1)));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->adjwgt, sizeof(float) * (E ? E : 1)));
     ctx->owns_weights = true;
     fill_ones_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(ctx->adjwgt, E);
     SKW_LAUNCHED(ctx);
@@ -541,7 +644,9 @@ int skw_graph_free_weights(skw_ctx* ctx) {
   if (!ctx) return SKW_ERR_ARG;
   DeviceGuard g(ctx->device);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (ctx->owns_weights) SKW_CUDA(ctx, cudaFree(ctx->adjwgt));
+  if (ctx->owns_weights) dev_free(ctx->adjwgt);
+  dev_give_back(ctx->device);
+  dev_give_back(ctx->device);
   ctx->adjwgt = nullptr;
   ctx->owns_weights = false;
   return SKW_OK;
@@ -585,14 +690,14 @@ struct GrPipe {
     cudaStreamSynchronize(ctx->stream);
     for (int i = 0; i < 2; ++i) {
       if (h[i]) cudaFreeHost(h[i]);
-      if (d[i]) cudaFree(d[i]);
+      if (d[i]) dev_free(d[i]);
       if (done[i]) cudaEventDestroy(done[i]);
     }
   }
   int init() {
     for (int i = 0; i < 2; ++i) {
       SKW_CUDA(ctx, cudaMallocHost(&h[i], kPiece));
-      SKW_CUDA(ctx, cudaMalloc(&d[i], kPiece));
+      SKW_CUDA(ctx, dev_malloc(ctx, &d[i], kPiece));
       SKW_CUDA(ctx, cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
     }
     return SKW_OK;
@@ -641,9 +746,9 @@ int skw_graph_load_gr(skw_ctx* ctx, const char* path, int weight_mode, uint32_t 
   const uint64_t E = num_edge;
   // on any failure below the half-filled arrays are released again
   auto body = [&]() -> int {
-    SKW_CUDA(ctx, cudaMalloc(&ctx->xadj, sizeof(uint32_t) * ((size_t)V + 1)));
-    SKW_CUDA(ctx, cudaMalloc(&ctx->adjncy, sizeof(uint32_t) * (E ? E : 1)));
-    SKW_CUDA(ctx, cudaMalloc(&ctx->adjwgt, sizeof(float) * (E ? E : 1)));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->xadj, sizeof(uint32_t) * ((size_t)V + 1)));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->adjncy, sizeof(uint32_t) * (E ? E : 1)));
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->adjwgt, sizeof(float) * (E ? E : 1)));
     ctx->owns_graph = ctx->owns_weights = true;
     ctx->V = V;
     ctx->E = E;

@@ -98,6 +98,7 @@ struct skw_ctx {
   uint32_t* h_pack = nullptr;
   size_t h_pack_cells = 0;
   void* host_pool = nullptr;  // skw::HostPool
+  bool counted = false;       // among the contexts for which freed device memory is kept
 
   // staging buffers of the host-pointer entry points, grown on demand
   static constexpr int kStages = 13;
@@ -121,8 +122,18 @@ int alloc_table(skw_ctx* ctx, TableUse use);
 int enqueue_tables(skw_ctx* ctx, uint32_t v_begin, uint32_t v_end, Slot* slots, uint8_t* valid);
 // forget the fused walk records (they are derived from the table and die with it) and free their memory
 void drop_records(skw_ctx* ctx);
-// cudaMalloc that gives up the memory of records that are no longer valid before it fails
-cudaError_t dev_malloc(skw_ctx* ctx, void** p, size_t bytes);
+// Device memory, from blocks freed earlier where one fits; gives up the memory of records that are no longer valid before
+// it fails.  dev_free waits for the GPU.
+cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(skw_ctx* ctx, T** p, size_t bytes) {
+  void* q = nullptr;
+  const cudaError_t e = dev_malloc_bytes(ctx, &q, bytes);
+  if (e == cudaSuccess) *p = static_cast<T*>(q);
+  return e;
+}
+void dev_free(void* p);
+void dev_give_back(int device);  // what dev_free kept
 int fail_cuda(skw_ctx* ctx, cudaError_t e, const char* what, const char* file, int line);
 void set_global_error(const char* msg);
 

@@ -110,12 +110,12 @@ static int keys_to_graph(skw_ctx* ctx, u64* keys, u64* alt, u64 count, u32 V, in
   size_t need2 = 0;
   cub::DeviceSelect::Unique(nullptr, need2, keys, alt, d_num, (long long)count, st);
   if (need2 > tmp_bytes) tmp_bytes = need2;
-  SKW_CUDA(ctx, cudaMalloc(&tmp, tmp_bytes + 16));
+  SKW_CUDA(ctx, dev_malloc(ctx, &tmp, tmp_bytes + 16));
   struct Free {
     void* p;
-    ~Free() { cudaFree(p); }
+    ~Free() { dev_free(p); }
   } f1{tmp};
-  SKW_CUDA(ctx, cudaMalloc(&d_num, sizeof(u64)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &d_num, sizeof(u64)));
   Free f2{d_num};
   need = tmp_bytes;
   SKW_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, need, buf, (long long)count, 0, key_bits, st));
@@ -137,9 +137,9 @@ static int keys_to_graph(skw_ctx* ctx, u64* keys, u64* alt, u64 count, u32 V, in
                                      (unsigned long long)E);
   u32 *xadj = nullptr, *adjncy = nullptr;
   float* wgt = nullptr;
-  SKW_CUDA(ctx, cudaMalloc(&xadj, sizeof(u32) * ((size_t)V + 1)));
-  SKW_CUDA(ctx, cudaMalloc(&adjncy, sizeof(u32) * (E ? E : 1)));
-  SKW_CUDA(ctx, cudaMalloc(&wgt, sizeof(float) * (E ? E : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &xadj, sizeof(u32) * ((size_t)V + 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &adjncy, sizeof(u32) * (E ? E : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &wgt, sizeof(float) * (E ? E : 1)));
   const int grid = ctx->sm_count * 8;
   csr_from_keys_kernel<<<grid, 256, 0, st>>>(out, E, V, xadj, adjncy);
   SKW_LAUNCHED(ctx);
@@ -148,9 +148,9 @@ static int keys_to_graph(skw_ctx* ctx, u64* keys, u64* alt, u64 count, u32 V, in
   SKW_CUDA(ctx, cudaStreamSynchronize(st));
   int rc = skw_graph_adopt_device(ctx, V, E, xadj, adjncy, wgt);
   if (rc != SKW_OK) {
-    cudaFree(xadj);
-    cudaFree(adjncy);
-    cudaFree(wgt);
+    dev_free(xadj);
+    dev_free(adjncy);
+    dev_free(wgt);
     return rc;
   }
   ctx->owns_graph = true;
@@ -181,16 +181,16 @@ int skw_graph_generate_rmat(skw_ctx* ctx, uint32_t scale, uint32_t num_vertices,
   const u64 count = raw_edges * (symmetric ? 2 : 1);
   const u64 sentinel = (u64)1 << (32 + scale);  // a source id one past the last vertex
   u64 *keys = nullptr, *alt = nullptr;
-  SKW_CUDA(ctx, cudaMalloc(&keys, sizeof(u64) * (count ? count : 1)));
-  SKW_CUDA(ctx, cudaMalloc(&alt, sizeof(u64) * (count ? count : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &keys, sizeof(u64) * (count ? count : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &alt, sizeof(u64) * (count ? count : 1)));
   if (raw_edges) {
     rmat_keys_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(keys, raw_edges, scale, ta, tab, tabc,
                                                                  symmetric, graph_seed, sentinel, fold);
     ctx->launches++;
   }
   int rc = keys_to_graph(ctx, keys, alt, count, fold ? fold : 1u << scale, 33 + (int)scale, sentinel, weight_seed);
-  cudaFree(keys);
-  cudaFree(alt);
+  dev_free(keys);
+  dev_free(alt);
   return rc;
 }
 
@@ -222,23 +222,23 @@ int skw_graph_generate_powerlaw(skw_ctx* ctx, uint32_t V, uint64_t raw_edges, do
     cum[v + 1] = cum[v] + (u64)d;
   }
   u64* d_cum = nullptr;
-  SKW_CUDA(ctx, cudaMalloc(&d_cum, sizeof(u64) * ((size_t)V + 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &d_cum, sizeof(u64) * ((size_t)V + 1)));
   SKW_CUDA(ctx, cudaMemcpyAsync(d_cum, cum.data(), sizeof(u64) * ((size_t)V + 1), cudaMemcpyHostToDevice, ctx->stream));
   const u64 count = raw_edges * 2;
   int bits = 0;
   while (((u64)1 << bits) <= V) ++bits;  // bits of the largest id, and of V itself for the sentinel
   const u64 sentinel = (u64)V << 32;
   u64 *keys = nullptr, *alt = nullptr;
-  SKW_CUDA(ctx, cudaMalloc(&keys, sizeof(u64) * (count ? count : 1)));
-  SKW_CUDA(ctx, cudaMalloc(&alt, sizeof(u64) * (count ? count : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &keys, sizeof(u64) * (count ? count : 1)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &alt, sizeof(u64) * (count ? count : 1)));
   if (raw_edges) {
     powerlaw_keys_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(keys, raw_edges, d_cum, V, graph_seed, sentinel);
     ctx->launches++;
   }
   int rc = keys_to_graph(ctx, keys, alt, count, V, 32 + bits, sentinel, weight_seed);
-  cudaFree(keys);
-  cudaFree(alt);
-  cudaFree(d_cum);
+  dev_free(keys);
+  dev_free(alt);
+  dev_free(d_cum);
   return rc;
 }
 

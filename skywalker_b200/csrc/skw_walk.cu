@@ -801,11 +801,11 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
   ctx->records_ready = false;
   // any failure below leaves no half-built records behind
   auto body = [&]() -> int {
-    if (!ctx->records) SKW_CUDA(ctx, cudaMalloc(&ctx->records, sizeof(WalkRecord) * (ctx->E ? ctx->E : 1)));
-    if (!ctx->vinfo) SKW_CUDA(ctx, cudaMalloc(&ctx->vinfo, sizeof(uint2) * ((size_t)ctx->V + 1)));
+    if (!ctx->records) SKW_CUDA(ctx, dev_malloc(ctx, &ctx->records, sizeof(WalkRecord) * (ctx->E ? ctx->E : 1)));
+    if (!ctx->vinfo) SKW_CUDA(ctx, dev_malloc(ctx, &ctx->vinfo, sizeof(uint2) * ((size_t)ctx->V + 1)));
     // the bitmap, and behind it the first vertex of every tile of the records build
     const u64 tiles = (ctx->E + kRecTile - 1) / kRecTile;
-    if (!ctx->vbits) SKW_CUDA(ctx, cudaMalloc(&ctx->vbits, sizeof(u32) * ((size_t)ctx->V / 32 + 1 + tiles)));
+    if (!ctx->vbits) SKW_CUDA(ctx, dev_malloc(ctx, &ctx->vbits, sizeof(u32) * ((size_t)ctx->V / 32 + 1 + tiles)));
     u32* tile_first = static_cast<u32*>(ctx->vbits) + (size_t)ctx->V / 32 + 1;
     int rc = err_reset(ctx);
     if (rc != SKW_OK) return rc;
@@ -861,7 +861,7 @@ int skw_probe_random_gather(skw_ctx* ctx, uint64_t footprint_bytes, uint32_t ite
   DeviceGuard g(ctx->device);
   const u64 nrec = footprint_bytes / sizeof(WalkRecord);
   WalkRecord* buf = nullptr;
-  SKW_CUDA(ctx, cudaMalloc(&buf, nrec * sizeof(WalkRecord)));
+  SKW_CUDA(ctx, dev_malloc(ctx, &buf, nrec * sizeof(WalkRecord)));
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaMemsetAsync(buf, 1, nrec * sizeof(WalkRecord), st);
   const int grid = ctx->sm_count * 8;
@@ -876,7 +876,7 @@ int skw_probe_random_gather(skw_ctx* ctx, uint64_t footprint_bytes, uint32_t ite
     e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   }
-  cudaFree(buf);
+  dev_free(buf);
   if (e != cudaSuccess) return fail_cuda(ctx, e, "skw_probe_random_gather", __FILE__, __LINE__);
   *gaccesses_per_s = (double)grid * 256.0 * iters / (ms * 1e-3) / 1e9;
   return SKW_OK;
@@ -886,9 +886,10 @@ int skw_walk_records_free(skw_ctx* ctx) {
   if (!ctx) return SKW_ERR_ARG;
   DeviceGuard g(ctx->device);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  cudaFree(ctx->records);
-  cudaFree(ctx->vinfo);
-  cudaFree(ctx->vbits);
+  dev_free(ctx->records);
+  dev_free(ctx->vinfo);
+  dev_free(ctx->vbits);
+  dev_give_back(ctx->device);
   ctx->records = nullptr;
   ctx->vinfo = nullptr;
   ctx->vbits = nullptr;
@@ -937,11 +938,11 @@ static bool tables_pay(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t 
 // Memory for such tables: 8 bytes an edge, kept until the graph changes.  False when there is none to be had.
 static bool online_table_memory(skw_ctx* ctx) {
   if (ctx->online_slots) return true;
-  if (dev_malloc(ctx, reinterpret_cast<void**>(&ctx->online_slots), sizeof(Slot) * (ctx->E ? ctx->E : 1)) == cudaSuccess &&
-      dev_malloc(ctx, reinterpret_cast<void**>(&ctx->online_valid), ctx->V ? ctx->V : 1) == cudaSuccess)
+  if (dev_malloc(ctx, &ctx->online_slots, sizeof(Slot) * (ctx->E ? ctx->E : 1)) == cudaSuccess &&
+      dev_malloc(ctx, &ctx->online_valid, ctx->V ? ctx->V : 1) == cudaSuccess)
     return true;
   cudaGetLastError();
-  cudaFree(ctx->online_slots);
+  dev_free(ctx->online_slots);
   ctx->online_slots = nullptr;
   return false;
 }
