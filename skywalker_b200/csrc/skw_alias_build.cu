@@ -541,18 +541,18 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   }
   // The classes are independent.  The long lists take few CTAs for long, so their kernels start first, on streams of their
   // own, and the many short ones fill in on the caller's.
-  const int streams = ctx->max_degree > kHugeSmemMax ? 4 : ctx->max_degree > kMidSmemMax ? 3 : ctx->max_degree > kF64Max ? 2
+  const int streams = ctx->max_degree > kHugeSmemMax ? 5 : ctx->max_degree > kMidSmemMax ? 3 : ctx->max_degree > kF64Max ? 2
                       : ctx->max_degree > kGroupMax ? 1 : 0;
   cudaStream_t s_h = ctx->bstream[3], s_a = ctx->bstream[2], s_b = ctx->bstream[1], s_c = ctx->bstream[0];
   if (streams) SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
   for (int i = 0; i < streams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
   const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err};
   // The lists beyond 16384 weights: one of these two kernels finds that they are its own, by their number, and both use the
-  // same scratch.
+  // same scratch.  On streams of their own: behind the other, the one with the work would start after everybody else.
   unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
   const unsigned clusters = slab_elems ? std::min<unsigned>(ctx->sm_count * 3 / kClusterCtas, gmem_ctas) : 0;
   if (clusters) {
-    build_cluster_kernel<<<clusters * kClusterCtas, kClusterThreads, sizeof(ClusterShared), s_h>>>(lists.list[K_H], cls, K_H, b,
+    build_cluster_kernel<<<clusters * kClusterCtas, kClusterThreads, sizeof(ClusterShared), ctx->bstream[4]>>>(lists.list[K_H], cls, K_H, b,
                                                                                                   scratch, slab_elems);
     SKW_LAUNCHED(ctx);
   }
@@ -568,12 +568,13 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
 #undef LONG
   const unsigned grid = ctx->sm_count * kListCtas;
   if (streams) {
-    // The lists of a CTA are dealt out beforehand, so one that starts late, behind a long list, ends late.  They start when
-    // the CTAs of 4097 to 8192 weights run out, and with 64 K edges or more for each there are up to four for every one that
-    // fits (457 M edges: 4.69 -> 4.42 ms; 65 M: 1.73 -> 1.72; fewer edges would pay for the start of each instead).  More
-    // CTAs for the short lists cost more in starts, seven classes each, than they gave (2.50 -> 2.55 ms at 226 M edges).
+    // The lists of a CTA are dealt out beforehand, so one that starts late, behind a long list, ends late.  With 64 K edges
+    // or more for each there are up to four CTAs for every one that fits, and they start when those of 4097 to 8192 weights
+    // run out (457 M edges: 4.69 -> 4.42 ms; 65 M: 1.73 -> 1.72).  With fewer edges they would pay for the start of each, and
+    // for the wait (1 M edges: 49 -> 61 us).  More CTAs for the short lists cost more in starts, seven classes each, than
+    // they gave (2.50 -> 2.55 ms at 226 M edges).
     const u64 waves = std::clamp<u64>((u64)ctx->E / ((u64)grid << 16), 1, 4);
-    build_lists_kernel<true><<<(unsigned)(grid * waves), kListWarps * 32, kListSmem, streams > 1 ? s_b : s_c>>>(lists, cls, b);
+    build_lists_kernel<true><<<(unsigned)(grid * waves), kListWarps * 32, kListSmem, waves > 1 && streams > 1 ? s_b : s_c>>>(lists, cls, b);
     SKW_LAUNCHED(ctx);
   }
   build_lists_kernel<false><<<grid, kListWarps * 32, kListSmem, st>>>(lists, cls, b);
