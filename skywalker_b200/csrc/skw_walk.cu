@@ -93,14 +93,34 @@ __device__ __forceinline__ bool walk_step_n2v(const WalkArgs& a, u32 step, u64 g
   }
 }
 
-// All steps of all walkers in one launch.  Each lane owns walkers tid, tid + T, tid + 2T ...;
+// Launch of the all-steps walk kernels.  A walk is a chain of dependent accesses and a warp goes on when the last of its
+// lanes has its data, so a batch that leaves the GPU room takes fewer walkers a warp: as few as give `warps` warps an SM
+// (what is resident: with more, the second wave costs the gain many times over).  Slots, three accesses a step, R-MAT 22,
+// 80 steps: 4,096 walkers 164 -> 110 us with one walker a warp, 16,384 150 -> 127 with four, 40,000 160 -> 141 with
+// eight; records, one access a step: 4,096 43 -> 38 with eight, and fewer gain no more.
+// CTAs of two warps: a CTA lives as long as its unluckiest lane, and small ones keep the SMs evenly loaded to the end (slots,
+// 300,000 walkers: 714 -> 668 us).  For the same reason a lane takes one walker (PPR over slots with three a thread: 1,000
+// walkers 45 -> 31 us, 100,000 122 -> 100, 1 M 338 -> 309, 2 M 558 -> 532), but for PPR of many more, where a third of the
+// threads starts a third of the warps (8 M walkers: 1.35 -> 1.19 ms).
+struct WalkGrid {
+  u32 ctas, lanes;  // walkers a warp takes at a time
+};
+constexpr u32 kWalkCta = 64;
+static WalkGrid walk_grid(const skw_ctx* ctx, uint32_t app, u64 n, u32 warps, u32 least) {
+  u32 lanes = least;
+  while (lanes < 32 && n > (u64)lanes * warps * ctx->sm_count) lanes *= 2;
+  const u64 per_cta = (u64)lanes * (kWalkCta / 32) * (app == SKW_APP_PPR && n > (2u << 20) ? 3 : 1);
+  return WalkGrid{(u32)std::clamp<u64>((n + per_cta - 1) / per_cta, 1, 0x7FFFFFFF), lanes};
+}
+
+// All steps of all walkers in one launch.  The first `lanes` lanes of each warp own walkers w, w + T, w + 2T ...;
 // the loop body is one step, so lanes of a warp stay converged although their walkers differ.
 template <int APP>
-__global__ void __launch_bounds__(256) walk_offline_kernel(const WalkArgs a) {
-  const u64 T = (u64)gridDim.x * blockDim.x;
-  u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kWalkCta) walk_offline_kernel(const WalkArgs a, u32 lanes) {
+  const u64 T = (u64)gridDim.x * (kWalkCta / 32) * lanes;
+  u64 w = ((u64)blockIdx.x * (kWalkCta / 32) + threadIdx.x / 32) * lanes + (threadIdx.x & 31);
   u64 edges = 0;
-  bool have = w < a.n;
+  bool have = (threadIdx.x & 31) < lanes && w < a.n;
   u32 cur = 0, step = 0;
   u32* row = nullptr;
   Rand4 r{0, 0, 0, 0};  // random words of the walker's current step
@@ -506,11 +526,11 @@ struct RecordWalkArgs {
 
 // Same lane-owns-a-stride loop as walk_offline_kernel; a step is one record load.
 template <int APP>
-__global__ void __launch_bounds__(256) walk_records_walk_kernel(const RecordWalkArgs a) {
-  const u64 T = (u64)gridDim.x * blockDim.x;
-  u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kWalkCta) walk_records_walk_kernel(const RecordWalkArgs a, u32 lanes) {
+  const u64 T = (u64)gridDim.x * (kWalkCta / 32) * lanes;
+  u64 w = ((u64)blockIdx.x * (kWalkCta / 32) + threadIdx.x / 32) * lanes + (threadIdx.x & 31);
   u64 edges = 0;
-  bool have = w < a.n;
+  bool have = (threadIdx.x & 31) < lanes && w < a.n;
   u32 off = 0, deg = 0, step = 0;
   u32* row = nullptr;
   Rand4 r{0, 0, 0, 0};  // random words of the walker's current step
@@ -734,19 +754,6 @@ __global__ void __launch_bounds__(256) generate_starts_kernel(u32* __restrict__ 
     const Rand4 r = philox_tagged(seed, TAG_STRT, id_base + i, 0, 0);
     starts[i] = __umulhi(r.x, V);
   }
-}
-
-// Grid of the all-steps walk kernels.  A lane walks its walkers one after another, so a CTA lives
-// as long as its unluckiest lane; many short CTAs (about 5 are resident per SM at a time) keep the
-// SMs evenly loaded to the end.  Measured on B200 for 1, 2, 4 and 8 M walkers alike: fixed-length
-// walks are fastest with one walker per thread (8 M walkers, scale-26 DeepWalk: 6.8 ms against
-// 7.4 at three per thread and 10.3 at 8 CTAs per SM); PPR, where most walkers stop after a few
-// steps, with three walkers per thread (1.19 ms against 1.35 at one per thread and 1.46 at 8 CTAs
-// per SM; PPR over walk records has its own chunked kernel, walk_records_ppr_kernel).
-static int walk_grid(uint32_t app, u64 n) {
-  const u64 per_cta = 256ull * (app == SKW_APP_PPR ? 3 : 1);
-  const u64 b = (n + per_cta - 1) / per_cta;
-  return (int)(b ? (b < 0x7FFFFFFFull ? b : 0x7FFFFFFFull) : 1);
 }
 
 // Measurement aid: a dependent chain of random 32-byte record loads, the memory behaviour of a walk
@@ -1010,19 +1017,19 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     ra.V = a.V;
     ra.hop_num = a.hop_num;
     ra.tp = a.tp;
-    const int grid = walk_grid(prm->app, n);
+    const WalkGrid g = walk_grid(ctx, prm->app, n, 17, 8);
     // (the chunked kernel stages lengths as 16-bit values and has no grid-stride loop)
     const u64 ctas = (n + 8 * kChunk - 1) / (8 * kChunk);
     if (prm->app == SKW_APP_PPR && prm->hop_num <= 65535 && ctas <= 0x7FFFFFFFull) {
       walk_records_ppr_kernel<8, kChunk, kStage><<<(unsigned)ctas, 256, 0, st>>>(ra);
-    } else if (prm->app == SKW_APP_PPR) walk_records_walk_kernel<SKW_APP_PPR><<<grid, 256, 0, st>>>(ra);
-    else walk_records_walk_kernel<SKW_APP_DEEPWALK><<<grid, 256, 0, st>>>(ra);
+    } else if (prm->app == SKW_APP_PPR) walk_records_walk_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);
+    else walk_records_walk_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);
     SKW_LAUNCHED(ctx);
   } else if (!online || whole_table) {
-    const int grid = walk_grid(prm->app, n);
+    const WalkGrid g = walk_grid(ctx, prm->app, n, 34, 1);
     switch (prm->app) {
-      case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<grid, 256, 0, st>>>(a); break;
-      case SKW_APP_PPR: walk_offline_kernel<SKW_APP_PPR><<<grid, 256, 0, st>>>(a); break;
+      case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
+      case SKW_APP_PPR: walk_offline_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
       default:
         walk_n2v_kernel<<<(unsigned)std::min<u64>((n + kN2vCta - 1) / kN2vCta, 0x7FFFFFFFull), kN2vCta, 0, st>>>(a);
         break;

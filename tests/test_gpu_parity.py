@@ -1004,3 +1004,21 @@ def test_walk_host_rows_large_batch_scatter(ctx, oracle, rmat16, app, kw):
                          fill=0xABABABAB, **kw)
     assert np.array_equal(lens, ol) and edges == int(ol.sum())
     assert np.array_equal(paths, op)
+
+
+@pytest.mark.parametrize("app,kw", [(APP_DEEPWALK, {}), (APP_PPR, {"tp": 0.15})])
+@pytest.mark.parametrize("n", [1, 3, 5033, 10065, 20129, 40257, 161025])
+def test_walks_with_fewer_walkers_a_warp(ctx, oracle, rmat12, app, kw, n):
+    """Batch sizes around which the number of walkers a warp changes, over slots and over records."""
+    g = rmat12
+    _upload(ctx, g)
+    ctx.alias_build_offline()
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    starts = oracle.gen_starts(n, g.V, 5)
+    want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, 12, app=app, seed=8, **kw)
+    for records in (False, True):
+        if records:
+            ctx.walk_records_build()
+        paths, lens, _, edges = ctx.walk(starts, 12, app=app, seed=8, **kw)
+        _cmp_walks(paths, lens, want, want_len)
+        assert edges == int(want_len.sum())
