@@ -1020,7 +1020,9 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     const WalkGrid g = walk_grid(ctx, prm->app, n, 17, 8);
     // (the chunked kernel stages lengths as 16-bit values and has no grid-stride loop)
     const u64 ctas = (n + 8 * kChunk - 1) / (8 * kChunk);
-    if (prm->app == SKW_APP_PPR && prm->hop_num <= 65535 && ctas <= 0x7FFFFFFFull) {
+    // It hands a lane its next walker cheaply; a batch with a lane for every walker, resident at once, does not need that
+    // (4,096 walkers: 29 -> 26 us, 100,000: 40 -> 38, equal at 200,000, 81 -> 89 at 400,000).
+    if (prm->app == SKW_APP_PPR && prm->hop_num <= 65535 && ctas <= 0x7FFFFFFFull && n > 700ull * ctx->sm_count) {
       walk_records_ppr_kernel<8, kChunk, kStage><<<(unsigned)ctas, 256, 0, st>>>(ra);
     } else if (prm->app == SKW_APP_PPR) walk_records_walk_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);
     else walk_records_walk_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);

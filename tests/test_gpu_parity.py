@@ -1007,7 +1007,7 @@ def test_walk_host_rows_large_batch_scatter(ctx, oracle, rmat16, app, kw):
 
 
 @pytest.mark.parametrize("app,kw", [(APP_DEEPWALK, {}), (APP_PPR, {"tp": 0.15})])
-@pytest.mark.parametrize("n", [1, 3, 5033, 10065, 20129, 40257, 161025])
+@pytest.mark.parametrize("n", [1, 3, 5033, 10065, 20129, 40257, 103600, 103663, 161025])
 def test_walks_with_fewer_walkers_a_warp(ctx, oracle, rmat12, app, kw, n):
     """Batch sizes around which the number of walkers a warp changes, over slots and over records."""
     g = rmat12
