@@ -150,7 +150,7 @@ void dev_give_back(int device) {
 
 cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes) {
   cudaError_t e = DeviceMemory::get().alloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && ctx->records && !ctx->records_ready) {
+  if (e == cudaErrorMemoryAllocation && ctx->records && !ctx->records_ready && !ctx->records_building) {
     cudaGetLastError();
     drop_records(ctx);
     e = DeviceMemory::get().alloc(p, bytes);

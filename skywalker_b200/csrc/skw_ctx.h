@@ -64,6 +64,7 @@ struct skw_ctx {
   void* vinfo = nullptr;
   void* vbits = nullptr;  // one bit per vertex: usable degree != 0
   bool records_ready = false;  // set once records, vinfo and vbits were all written
+  bool records_building = false;  // between their allocation and that: not to be given up
   bool records_all_usable = false;  // ... and no vertex with out-edges lacks a usable table
 
   // status words on the device and in mapped host memory: the error record (4 words, 4 spare) and four 64-bit sums

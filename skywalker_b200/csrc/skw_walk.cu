@@ -806,6 +806,7 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
   if (!ctx->table_ready) return fail(ctx, SKW_ERR_STATE, "skw_walk_records_build: build or import the alias table first");
   DeviceGuard g(ctx->device);
   ctx->records_ready = false;
+  ctx->records_building = true;
   // any failure below leaves no half-built records behind
   auto body = [&]() -> int {
     if (!ctx->records) SKW_CUDA(ctx, dev_malloc(ctx, &ctx->records, sizeof(WalkRecord) * (ctx->E ? ctx->E : 1)));
@@ -837,6 +838,7 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
     return SKW_OK;
   };
   const int rc = body();
+  ctx->records_building = false;
   if (rc != SKW_OK) {
     const std::string why = ctx->err;
     cudaGetLastError();

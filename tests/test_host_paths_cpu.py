@@ -1,0 +1,97 @@
+"""Host paths that a GPU takes only when memory is short or streams change, run on the CPU: the library in a child
+process whose CUDA runtime is tests/fake_cudart.cpp (no kernel runs; allocations fail on request)."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PRELUDE = """
+import ctypes as C
+import numpy as np
+from skywalker_b200 import _capi
+from skywalker_b200.api import Context, SkwError
+fake = C.CDLL(%r)
+fake.fake_log.restype = C.c_char_p
+fake.fake_used.restype = C.c_size_t
+fake.fake_memory.argtypes = [C.c_size_t]
+def calls(clear=True):
+    lines = [x.split() for x in fake.fake_log().decode().splitlines()]
+    if clear:
+        fake.fake_clear_log()
+    return lines
+def launches(lines, kernel):
+    return [x for x in lines if x[0] == "launch" and kernel in x[2]]
+class Device:   # stands for a tensor on the device
+    is_cuda = True
+    def __init__(self, *shape):
+        self.a = np.zeros(shape, np.uint32)
+    def data_ptr(self):
+        return self.a.ctypes.data
+    def numel(self):
+        return self.a.size
+def ring(V=1000, deg=12):   # a graph to be resident
+    x = np.arange(V + 1, dtype=np.uint32) * deg
+    a = (np.arange(V * deg, dtype=np.uint32) // deg + 1) %% V
+    return x, a, np.ones(V * deg, np.float32)
+"""
+
+
+@pytest.fixture(scope="session")
+def fake_cudart(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I/usr/local/cuda/include",
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), "-o", out], check=True, timeout=300)
+    return out
+
+
+def _run(fake_cudart, body):
+    env = dict(os.environ, LD_PRELOAD=fake_cudart, PYTHONPATH=ROOT)
+    p = subprocess.run([sys.executable, "-c", PRELUDE % fake_cudart + body], capture_output=True, text=True, timeout=300,
+                       env=env, cwd=ROOT)
+    assert p.returncode == 0, p.stdout + p.stderr
+
+
+@pytest.mark.parametrize("nth", [0, 1, 2])
+@pytest.mark.parametrize("times", [1, 2])
+def test_records_build_without_memory(fake_cudart, nth, times):
+    """The build of the walk records runs out of memory at any of its three allocations, for good or with one success
+    before the next try: an error, no kernel that would write records, and a context that goes on."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring())
+ctx.alias_build_offline()
+calls()
+fake.fake_fail_malloc(%d, %d)
+try:
+    ctx.walk_records_build()
+    assert False, "built"
+except SkwError as e:
+    assert "out of memory" in str(e), e
+assert not [x for x in calls() if x[0] == "launch"]
+fake.fake_fail_malloc(-1, 0)
+ctx.walk_records_build()
+assert launches(calls(), "walk_records_kernel")
+ctx.walk_records_build()
+log = calls()
+assert launches(log, "walk_records_kernel") and not [x for x in log if x[0] == "malloc"]
+""" % (nth, times))
+
+
+def test_records_that_wait_for_a_rebuild_make_room(fake_cudart):
+    """Records of a table that was built anew are given up when another allocation fails."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring())
+ctx.alias_build_offline()
+ctx.walk_records_build()
+ctx.alias_build_offline()
+calls()
+fake.fake_fail_malloc(0, 1)
+ctx.walk(np.zeros(5000, np.uint32), 50)      # its staging buffers are new
+log = calls()
+assert sum(x[0] == "malloc" and x[2] == "fail" for x in log) == 1
+assert sum(x[0] == "device_sync" for x in log) >= 3    # three blocks returned
+""")
