@@ -182,7 +182,7 @@ int err_check(skw_ctx* ctx, const char* where, uint32_t sums_to_clear) {
   report_status_kernel<<<1, 16, 0, ctx->stream>>>(ctx->d_err, ctx->h_err, sums_to_clear);
   SKW_LAUNCHED(ctx);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->status_clean = true;
+  if ((sums_to_clear & 9u) == 9u) ctx->status_clean = true;  // else the sums of the calls before are still there
   if (ctx->h_err[0] != DEV_OK) {
     static const char* names[] = {"ok", "index out of range", "bounded wait ran out",
                                   "capacity exceeded", "construction invariant broken"};

@@ -856,7 +856,7 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
 int skw_ctx_take_sampled_edges(skw_ctx* ctx, uint64_t* out) {
   if (!ctx) return SKW_ERR_ARG;
   DeviceGuard g(ctx->device);
-  const int rc = err_check(ctx, "enqueued walks", 2u);  // synchronises the stream
+  const int rc = err_check(ctx, "enqueued walks", 1u | 2u | 8u);  // synchronises the stream
   if (rc != SKW_OK) return rc;
   const uint64_t v = ctx->h_sum[1];
   if (out) *out = v;
