@@ -759,13 +759,9 @@ extern "C" int skw_alias_build_offline(skw_ctx* ctx, uint32_t v_begin, uint32_t 
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
   if ((rc = enqueue_tables(ctx, v_begin, v_end, ctx->slots, ctx->valid)) != SKW_OK) return rc;
   SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
-  rc = err_check(ctx, "skw_alias_build_offline");
-  if (rc != SKW_OK) {
-    if (whole && !ctx->table_ready) ctx->slots_marked = false;
-    return rc;
-  }
+  if ((rc = err_check(ctx, "skw_alias_build_offline")) != SKW_OK) return rc;
   if (ms) SKW_CUDA(ctx, cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1));
-  ctx->table_ready = true;
+  ctx->table_ready = ctx->slots_marked = true;
   return SKW_OK;
 }
 

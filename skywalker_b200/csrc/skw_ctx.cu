@@ -410,11 +410,12 @@ int alloc_table(skw_ctx* ctx, TableUse use) {
     ctx->slots_marked = false;
   }
   if (!ctx->slots_marked && use != TableUse::kFrontier) {
-    // what this call leaves out must read as "no usable table here"
+    // what this call leaves out must read as "no usable table here"; one that is to write all of it has the slots marked
+    // when it has succeeded
     const size_t from = use == TableUse::kAll ? (size_t)ctx->E : 0;
     fill_unbuilt_slots_kernel<<<from ? 4 : ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->slots + from, n - from);
     SKW_LAUNCHED(ctx);
-    ctx->slots_marked = true;
+    ctx->slots_marked = use == TableUse::kSome;
   }
   if (!ctx->valid) {
     SKW_CUDA(ctx, dev_malloc(ctx, &ctx->valid, ctx->V ? ctx->V : 1));
@@ -886,15 +887,15 @@ int skw_alias_import(skw_ctx* ctx, const float* h_prob, const uint32_t* h_alias,
       if (!h_valid[v])
         for (uint32_t i = xadj[v]; i < xadj[v + 1]; ++i) tmp[i].prob = -1.0f;
   }
+  ctx->table_ready = ctx->slots_marked = false;
   if (ctx->E)
     SKW_CUDA(ctx, cudaMemcpyAsync(ctx->slots, tmp.data(), sizeof(Slot) * ctx->E,
                                   cudaMemcpyHostToDevice, ctx->stream));
   if (ctx->V)
     SKW_CUDA(ctx, cudaMemcpyAsync(ctx->valid, h_valid, ctx->V, cudaMemcpyHostToDevice, ctx->stream));
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->table_ready = false;
   if ((rc = validate_table(ctx, "skw_alias_import")) != SKW_OK) return rc;
-  ctx->table_ready = true;
+  ctx->table_ready = ctx->slots_marked = true;
   return SKW_OK;
 }
 
@@ -964,7 +965,7 @@ int skw_alias_load(skw_ctx* ctx, const char* path) {
   ctx->records_ready = false;  // derived from the old table
   rc = alloc_table(ctx, TableUse::kAll);
   if (rc != SKW_OK) return rc;
-  ctx->table_ready = false;
+  ctx->table_ready = ctx->slots_marked = false;
   const size_t chunk = 64u << 20;
   std::vector<unsigned char> buf(chunk);
   auto fill = [&](void* dptr, size_t bytes) -> int {
@@ -980,7 +981,7 @@ int skw_alias_load(skw_ctx* ctx, const char* path) {
   if ((rc = fill(ctx->slots, sizeof(Slot) * ctx->E)) != SKW_OK) return rc;
   if ((rc = fill(ctx->valid, ctx->V)) != SKW_OK) return rc;
   if ((rc = validate_table(ctx, "skw_alias_load")) != SKW_OK) return rc;
-  ctx->table_ready = true;
+  ctx->table_ready = ctx->slots_marked = true;
   return SKW_OK;
 }
 

@@ -33,3 +33,40 @@ def test_queued_walks_leave_no_edges_to_the_next_call(ctx, oracle, rmat12, tmp_p
     assert edges == int(lens.sum()) == queued
     _, sl, _, edges = ctx.sample_khop(starts[:100], [5, 3], mode=MODE_ONLINE)
     assert edges == int(sl.sum())
+
+
+def _slots(ctx):
+    """prob and alias of every slot as they are on the device."""
+    import torch
+    s = torch.as_tensor(ctx.alias_device_arrays()[0], device="cuda").cpu().numpy().view(np.uint32).reshape(-1, 2)
+    return s[:, 0].copy().view(np.float32), s[:, 1].copy()
+
+
+@pytest.mark.parametrize("first", ["truncated", "refused"])
+def test_partial_build_after_a_table_that_failed(ctx, oracle, rmat12, tmp_path, first):
+    """A checkpoint that ends too soon or an import that is refused leaves no slots that a build of a range would let
+    pass as built: outside the range they say "no table"."""
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    path = str(tmp_path / "t.skw")
+    ctx.alias_save(path)
+    prob, alias, valid = ctx.alias_export()
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)          # new slots, in memory that held the table before
+    with pytest.raises(SkwError):
+        if first == "truncated":
+            with open(path, "r+b") as f:
+                f.truncate(48 + 8 * 100)
+            ctx.alias_load(path)
+        else:
+            alias[-1] = 1 << 30
+            ctx.alias_import(prob, alias, valid)
+    half = g.V // 2
+    ctx.alias_build_offline(0, half)
+    got, _ = _slots(ctx)
+    want, _, want_valid = oracle.alias_build(g.xadj, g.adjwgt)
+    cut = int(g.xadj[half])
+    assert (got[cut:] == -1.0).all()
+    deg = np.diff(g.xadj.astype(np.int64))
+    usable = np.repeat(want_valid.astype(bool), deg)[:cut]
+    assert np.array_equal(got[:cut][usable], want[:cut][usable])
