@@ -404,22 +404,23 @@ void drop_records(skw_ctx* ctx) {
 
 int alloc_table(skw_ctx* ctx, TableUse use) {
   // kSlotSlack spare entries let a multi-GPU caller all-gather the table in equal chunks in place
-  const size_t n = (size_t)ctx->E + kSlotSlack;
+  const size_t n = (size_t)ctx->E + kSlotSlack, flags = ctx->V ? ctx->V : 1;
   if (!ctx->slots) {
     SKW_CUDA(ctx, dev_malloc(ctx, &ctx->slots, sizeof(Slot) * n));
     ctx->slots_marked = false;
   }
+  if (!ctx->valid) {
+    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->valid, flags));
+    SKW_CUDA(ctx, cudaMemsetAsync(ctx->valid, 0, flags, ctx->stream));
+  }
   if (!ctx->slots_marked && use != TableUse::kFrontier) {
-    // what this call leaves out must read as "no usable table here"; one that is to write all of it has the slots marked
-    // when it has succeeded
+    // what this call leaves out must read as "no usable table here", in the slots and in the flags of tables that an
+    // online call or a failed one has left; a call that is to write all of it has them marked when it has succeeded
     const size_t from = use == TableUse::kAll ? (size_t)ctx->E : 0;
     fill_unbuilt_slots_kernel<<<from ? 4 : ctx->sm_count * 8, 256, 0, ctx->stream>>>(ctx->slots + from, n - from);
     SKW_LAUNCHED(ctx);
+    if (use == TableUse::kSome) SKW_CUDA(ctx, cudaMemsetAsync(ctx->valid, 0, flags, ctx->stream));
     ctx->slots_marked = use == TableUse::kSome;
-  }
-  if (!ctx->valid) {
-    SKW_CUDA(ctx, dev_malloc(ctx, &ctx->valid, ctx->V ? ctx->V : 1));
-    SKW_CUDA(ctx, cudaMemsetAsync(ctx->valid, 0, ctx->V ? ctx->V : 1, ctx->stream));
   }
   return SKW_OK;
 }

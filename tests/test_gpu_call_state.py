@@ -70,3 +70,19 @@ def test_partial_build_after_a_table_that_failed(ctx, oracle, rmat12, tmp_path, 
     deg = np.diff(g.xadj.astype(np.int64))
     usable = np.repeat(want_valid.astype(bool), deg)[:cut]
     assert np.array_equal(got[:cut][usable], want[:cut][usable])
+    assert not ctx.alias_export()[2][half:].any()
+
+
+def test_partial_build_after_online_sampling(ctx, oracle, rmat12):
+    """Online sampling leaves tables of the vertices it met; a build of a range starts from "no table" everywhere, in
+    the flags as in the slots."""
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.sample_khop(oracle.gen_starts(500, g.V, 3), [5, 3], mode=MODE_ONLINE)
+    half = g.V // 2
+    ctx.alias_build_offline(0, half)
+    prob, alias, valid = ctx.alias_export()
+    want_prob, want_alias, want_valid = oracle.alias_build(g.xadj, g.adjwgt)
+    assert np.array_equal(valid[:half], want_valid[:half])
+    usable = np.repeat(valid.astype(bool), np.diff(g.xadj.astype(np.int64)))
+    assert np.array_equal(prob[usable], want_prob[usable]) and np.array_equal(alias[usable], want_alias[usable])
