@@ -258,7 +258,7 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
  * the kernels are queued on the context's stream (no synchronisation, no readback), so back to
  * back calls leave no host gap between kernels.  The sampled edges of such calls add up in the
  * context; skw_ctx_take_sampled_edges() waits for the stream, reports a device error of any of
- * them, returns the sum and clears it. */
+ * them (synchronous calls in between do not), returns the sum and clears it. */
 int skw_ctx_take_sampled_edges(skw_ctx* ctx, uint64_t* out);
 /* Same with host buffers: copies starts in, runs, copies paths and lengths out.  When h_paths is
  * pinned memory (skw_host_alloc, cudaHostAlloc, cudaHostRegister) only the cells each walk wrote

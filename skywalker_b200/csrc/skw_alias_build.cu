@@ -546,7 +546,7 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   cudaStream_t s_h = ctx->bstream[3], s_a = ctx->bstream[2], s_b = ctx->bstream[1], s_c = ctx->bstream[0];
   if (streams) SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
   for (int i = 0; i < streams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
-  const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->d_err};
+  const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->launch_err};
   // The lists beyond 16384 weights: one of these two kernels finds that they are its own, by their number, and both use the
   // same scratch.  On streams of their own: behind the other, the one with the work would start after everybody else.
   unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
@@ -559,7 +559,7 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
 #define LONG(MORE_THAN, KCLS, NT, CAP, GLOBAL, CTAS, BYTES, SCRATCH, MOST, OTHERS, STREAM)                                     \
   if (ctx->max_degree > (MORE_THAN)) {                                                                                 \
     build_long_kernel<NT, CAP, GLOBAL><<<CTAS, NT, BYTES, STREAM>>>(lists.list[KCLS], cls, KCLS, ctx->xadj,            \
-                                                                   ctx->adjwgt, slots, valid, SCRATCH, MOST, OTHERS, ctx->d_err); \
+                                                                   ctx->adjwgt, slots, valid, SCRATCH, MOST, OTHERS, ctx->launch_err); \
     SKW_LAUNCHED(ctx);                                                                                                 \
   }
   LONG(kHugeSmemMax, K_H, 1024, 8192, true, gmem_ctas, kLongC, scratch, slab_elems, clusters, s_h)
@@ -681,7 +681,7 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
     for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->frontier_lists + (size_t)k * cap;
     frontier_collect_kernel<<<grid, 256, 0, st>>>(verts, units, width, cells, offs, alive_lengths,
                                                   ctx->xadj, ctx->V, ctx->stamp, ctx->stamp_round,
-                                                  ctx->frontier_cls, lists, cap, ctx->d_err);
+                                                  ctx->frontier_cls, lists, cap, ctx->launch_err);
     SKW_LAUNCHED(ctx);
     rc = launch_builders(ctx, lists, ctx->frontier_cls, ctx->slots, ctx->valid);
     if (rc != SKW_OK) return rc;

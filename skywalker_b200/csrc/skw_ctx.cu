@@ -160,12 +160,12 @@ cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes) {
 
 // The status words of a context: 16 x u32 on the device (error records, then the four 64-bit sums at word 8) and the
 // same 16 words in mapped host memory.  A synchronous call ends with this kernel, which hands them to the host and
-// leaves them cleared for the next call: one small launch where two memsets before a call and two copies after it
-// took about 14 us of a call of 65.
-__global__ void report_status_kernel(uint32_t* __restrict__ d, uint32_t* __restrict__ h, uint32_t sums_to_clear) {
+// leaves those of `clear` (a bit a word) cleared for the next call: one small launch where two memsets before a call and
+// two copies after it took about 14 us of a call of 65.
+__global__ void report_status_kernel(uint32_t* __restrict__ d, uint32_t* __restrict__ h, uint32_t clear) {
   const uint32_t t = threadIdx.x;
   h[t] = d[t];
-  if (t < 4 || (t >= 8 && ((sums_to_clear >> ((t - 8) >> 1)) & 1u))) d[t] = 0;
+  if ((clear >> t) & 1u) d[t] = 0;
 }
 
 int err_reset(skw_ctx* ctx) {
@@ -178,17 +178,19 @@ int err_reset(skw_ctx* ctx) {
   return SKW_OK;
 }
 
-int err_check(skw_ctx* ctx, const char* where, uint32_t sums_to_clear) {
-  report_status_kernel<<<1, 16, 0, ctx->stream>>>(ctx->d_err, ctx->h_err, sums_to_clear);
+int err_check(skw_ctx* ctx, const char* where, bool queued) {
+  // words 0-3 and 4-7: the error records; 8-9, 14-15: sums 0 and 3; 10-11: sum 1
+  report_status_kernel<<<1, 16, 0, ctx->stream>>>(ctx->d_err, ctx->h_err, queued ? 0xCFFFu : 0xC30Fu);
   SKW_LAUNCHED(ctx);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if ((sums_to_clear & 9u) == 9u) ctx->status_clean = true;  // else the sums of the calls before are still there
-  if (ctx->h_err[0] != DEV_OK) {
+  ctx->status_clean = true;
+  const uint32_t* rec = ctx->h_err + (queued ? 4 : 0);
+  if (rec[0] != DEV_OK) {
     static const char* names[] = {"ok", "index out of range", "bounded wait ran out",
                                   "capacity exceeded", "construction invariant broken"};
-    const uint32_t c = ctx->h_err[0];
+    const uint32_t c = rec[0];
     return fail(ctx, SKW_ERR_DEVICE, "%s: device error %u (%s), detail %u %u %u", where, c,
-                c < 5 ? names[c] : "?", ctx->h_err[1], ctx->h_err[2], ctx->h_err[3]);
+                c < 5 ? names[c] : "?", rec[1], rec[2], rec[3]);
   }
   return SKW_OK;
 }
@@ -481,6 +483,7 @@ int skw_ctx_create(int device, skw_ctx** out) {
   CK(dev_malloc(ctx, &ctx->d_err, 64));
   CK(cudaMemset(ctx->d_err, 0, 64));
   CK(cudaMallocHost(&ctx->h_err, 64));
+  ctx->launch_err = ctx->d_err;
   ctx->d_sum = reinterpret_cast<uint64_t*>(ctx->d_err + 8);
   ctx->h_sum = reinterpret_cast<uint64_t*>(ctx->h_err + 8);
   for (int i = 0; i < skw_ctx::kPackSlices; ++i) {

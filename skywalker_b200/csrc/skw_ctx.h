@@ -67,13 +67,14 @@ struct skw_ctx {
   bool records_building = false;  // between their allocation and that: not to be given up
   bool records_all_usable = false;  // ... and no vertex with out-edges lacks a usable table
 
-  // status words on the device and in mapped host memory: the error record (4 words, 4 spare) and four 64-bit sums
-  // (edges of a synchronous call, of enqueued calls, of packed calls; vertices without a usable table)
+  // status words on the device and in mapped host memory: the error records of synchronous and of queued calls (4 words
+  // each) and four 64-bit sums (edges of a synchronous call, of queued calls, of packed calls; vertices without a usable table)
   uint32_t* d_err = nullptr;
+  uint32_t* launch_err = nullptr;  // the record that the kernels of the current call write
   uint32_t* h_err = nullptr;
   uint64_t* d_sum = nullptr;
   uint64_t* h_sum = nullptr;
-  bool status_clean = true;  // error record and sums 0 and 3 are zero
+  bool status_clean = true;  // the record of synchronous calls and sums 0 and 3 are zero
 
   // builder scratch, grown on demand
   uint32_t* worklist = nullptr;      // vertices by degree class, one list per class
@@ -140,10 +141,17 @@ void set_global_error(const char* msg);
 
 // Grow-only device buffer.
 int ensure_bytes(skw_ctx* ctx, void** p, size_t* cap, size_t want);
-// Bracket of a synchronous call: the error record and sums 0 and 3 are zero after err_reset; err_check brings all
-// status words to the host, waits for the stream, clears the record and the given sums and reports an error.
+// Bracket of a synchronous call: its error record and sums 0 and 3 are zero after err_reset; err_check brings all
+// status words to the host, waits for the stream, clears them but for those of queued calls and reports an error.
+// queued: what queued calls reported, cleared as well.
 int err_reset(skw_ctx* ctx);
-int err_check(skw_ctx* ctx, const char* where, uint32_t sums_to_clear = 1u | 8u);
+int err_check(skw_ctx* ctx, const char* where, bool queued = false);
+// Kernels launched while this lives write the record of queued calls.
+struct QueuedErrors {
+  skw_ctx* ctx;
+  explicit QueuedErrors(skw_ctx* c) : ctx(c) { ctx->launch_err = ctx->d_err + 4; }
+  ~QueuedErrors() { ctx->launch_err = ctx->d_err; }
+};
 
 struct DeviceGuard {
   int prev = -1;

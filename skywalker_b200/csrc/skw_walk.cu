@@ -856,7 +856,7 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
 int skw_ctx_take_sampled_edges(skw_ctx* ctx, uint64_t* out) {
   if (!ctx) return SKW_ERR_ARG;
   DeviceGuard g(ctx->device);
-  const int rc = err_check(ctx, "enqueued walks", 1u | 2u | 8u);  // synchronises the stream
+  const int rc = err_check(ctx, "enqueued walks", true);  // synchronises the stream
   if (rc != SKW_OK) return rc;
   const uint64_t v = ctx->h_sum[1];
   if (out) *out = v;
@@ -979,7 +979,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   a.paths = d_paths;
   a.lengths = d_lengths;
   a.sum = sum;
-  a.err = ctx->d_err;
+  a.err = ctx->launch_err;
   a.n = n;
   a.seed = prm->seed;
   a.walker_base = prm->walker_base;
@@ -1089,9 +1089,11 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
   DeviceGuard g(ctx->device);
   // With both result pointers null the call only enqueues work: no reset, no readback, no
   // synchronisation.  Sampled edges then add up in a second counter and a device error stays
-  // recorded until skw_ctx_take_sampled_edges() (or a later synchronous call) looks at it.
-  if (!ms && !sampled_edges)
+  // in a second record until skw_ctx_take_sampled_edges() looks at them.
+  if (!ms && !sampled_edges) {
+    QueuedErrors q(ctx);
     return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1);
+  }
   return walk_and_wait(ctx, prm, d_starts, n, d_paths, d_lengths, nullptr, nullptr, ms, sampled_edges);
 }
 

@@ -86,3 +86,26 @@ def test_partial_build_after_online_sampling(ctx, oracle, rmat12):
     assert np.array_equal(valid[:half], want_valid[:half])
     usable = np.repeat(valid.astype(bool), np.diff(g.xadj.astype(np.int64)))
     assert np.array_equal(prob[usable], want_prob[usable]) and np.array_equal(alias[usable], want_alias[usable])
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(mode=MODE_ONLINE), dict(mode=MODE_ONLINE, flags=4)])
+def test_error_of_a_queued_walk_waits_for_its_own_report(ctx, oracle, rmat12, kw):
+    """A synchronous call neither reports nor loses what a queued walk before it did wrong."""
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(300, g.V, 3)
+    want, want_len, _, want_edges = ctx.walk(starts, 11, seed=5)
+    bad = starts.copy()
+    bad[7] = g.V + 7
+    d_s, d_p, d_l = _device_batch(bad, 11)
+    ctx.walk(d_s, 11, seed=5, paths=d_p, lengths=d_l, enqueue_only=True, **kw)
+    paths, lens, _, edges = ctx.walk(starts, 11, seed=5, **kw)
+    assert np.array_equal(paths, want) and np.array_equal(lens, want_len) and edges == want_edges
+    with pytest.raises(SkwError) as e:
+        ctx.take_sampled_edges()
+    assert "index out of range" in str(e.value)
+    with pytest.raises(SkwError):                   # the synchronous call's own errors are its own
+        ctx.walk(bad, 11, seed=5, **kw)
+    ctx.walk(starts, 11, seed=5, **kw)
+    assert ctx.take_sampled_edges() == 0
