@@ -956,10 +956,23 @@ static bool online_table_memory(skw_ctx* ctx) {
   return false;
 }
 
+// Queue the tables of the whole graph for the n walkers of an online call, where they pay: *slots, else null.
+static int online_tables(skw_ctx* ctx, const skw_walk_params* prm, uint64_t n, const Slot** slots) {
+  *slots = nullptr;
+  if (prm->mode != SKW_MODE_ONLINE || !n ||
+      (prm->flags & (SKW_WALK_UNBIASED | SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES | SKW_WALK_DIRECT_SLOTS)))
+    return SKW_OK;
+  if (!tables_pay(ctx, prm, n) || !online_table_memory(ctx)) return SKW_OK;
+  const int rc = enqueue_tables(ctx, 0, ctx->V, ctx->online_slots, ctx->online_valid);
+  if (rc == SKW_OK) *slots = ctx->online_slots;
+  return rc;
+}
+
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
-// No reset, no readback, no synchronisation (the online paths allocate on first use).
+// No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: what online_tables
+// gave for the call.
 static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n,
-                       uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum) {
+                       uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum, const Slot* whole_table) {
   const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
   const bool online = prm->mode == SKW_MODE_ONLINE && !unbiased;
   int rc;
@@ -992,12 +1005,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   a.inv_q = prm->app == SKW_APP_NODE2VEC ? 1.0f / prm->q : 1.0f;
   a.fmax = fmaxf(1.0f, fmaxf(a.inv_p, a.inv_q));
   cudaStream_t st = ctx->stream;
-  const bool whole_table = online && !build_tables && !(prm->flags & SKW_WALK_DIRECT_SLOTS) && tables_pay(ctx, prm, n) &&
-                           online_table_memory(ctx);
-  if (whole_table) {
-    if ((rc = enqueue_tables(ctx, 0, ctx->V, ctx->online_slots, ctx->online_valid)) != SKW_OK) return rc;
-    a.slots = ctx->online_slots;
-  }
+  if (whole_table) a.slots = whole_table;
   // Walk records serve unbiased walks as well (the record of column c names the c-th neighbour with its
   // offset and degree: one access per step instead of two), as long as every vertex with out-edges has
   // a usable table, i.e. the degrees in the records are the graph's own.
@@ -1067,7 +1075,10 @@ static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_
   int rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
-  if ((rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum))) != SKW_OK)
+  const Slot* tables;
+  if ((rc = online_tables(ctx, prm, n, &tables)) != SKW_OK) return rc;
+  if ((rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum), tables)) !=
+      SKW_OK)
     return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   if (h_lengths && n) SKW_CUDA(ctx, cudaMemcpyAsync(h_lengths, d_lengths, sizeof(u32) * (size_t)n, cudaMemcpyDeviceToHost, st));
@@ -1092,7 +1103,9 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
   // in a second record until skw_ctx_take_sampled_edges() looks at them.
   if (!ms && !sampled_edges) {
     QueuedErrors q(ctx);
-    return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1);
+    const Slot* tables;
+    if ((rc = online_tables(ctx, prm, n, &tables)) != SKW_OK) return rc;
+    return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1, tables);
   }
   return walk_and_wait(ctx, prm, d_starts, n, d_paths, d_lengths, nullptr, nullptr, ms, sampled_edges);
 }
@@ -1316,6 +1329,7 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
     SKW_CUDA(ctx, cudaStreamWaitEvent(side, ctx->pk_ready[c], 0));
     return SKW_OK;
   };
+  const Slot* tables = nullptr;
   auto body = [&]() -> int {
     // the start vertices come in slice by slice on the side stream, ahead of everything else it will
     // carry: a walk waits for its own slice only, and no walk waits behind a copy of a later slice
@@ -1330,7 +1344,9 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
       skw_walk_params p = *prm;
       p.walker_base = prm->walker_base + base * stride;
       SKW_CUDA(ctx, cudaEventRecord(ctx->pk_t0[c], st));
-      int r = walk_launch(ctx, &p, d_starts + base, nc, d_rows + base * prm->hop_num, d_len + base, scratch_sum);
+      int r = c == 0 ? online_tables(ctx, prm, n, &tables) : SKW_OK;  // for all slices
+      if (r != SKW_OK) return r;
+      r = walk_launch(ctx, &p, d_starts + base, nc, d_rows + base * prm->hop_num, d_len + base, scratch_sum, tables);
       if (r != SKW_OK) return r;
       SKW_CUDA(ctx, cudaEventRecord(ctx->pk_t1[c], st));
       if ((r = scan_and_pack(c)) != SKW_OK) return r;

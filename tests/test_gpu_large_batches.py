@@ -1,0 +1,28 @@
+"""Batches that are large enough for slices, host threads or tables of the whole graph."""
+import numpy as np
+import pytest
+
+from skywalker_b200 import APP_DEEPWALK, APP_NODE2VEC, APP_PPR, MODE_OFFLINE, MODE_ONLINE
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("app,kw", [(APP_DEEPWALK, {}), (APP_PPR, {"tp": 0.3}), (APP_NODE2VEC, {"p": 2.0, "q": 0.5})])
+@pytest.mark.parametrize("n", [(1 << 18) + 3, (1 << 20) + 12345])      # one slice, two slices
+def test_online_host_batches(ctx, oracle, plaw, app, kw, n):
+    """Online walks with host results, packed and as rows, are the offline walks of the same seed."""
+    g = plaw
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, g.V, 5)
+    want, want_len, want_cells, _, want_edges = ctx.walk_packed(starts, 6, app=app, seed=8, mode=MODE_OFFLINE, **kw)
+    out, lens, cells, ms, edges = ctx.walk_packed(starts, 6, app=app, seed=8, mode=MODE_ONLINE, **kw)
+    assert (cells, edges) == (want_cells, want_edges) and ms > 0
+    assert np.array_equal(lens, want_len) and np.array_equal(out[:cells], want[:cells])
+    rows, lens, _, edges = ctx.walk(starts, 6, app=app, seed=8, mode=MODE_ONLINE, **kw)
+    live = np.arange(6)[None, :] <= lens[:, None]
+    assert np.array_equal(lens, want_len) and edges == want_edges and np.array_equal(rows[live], want[:cells])
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    for w in range(0, n, n // 50):
+        op, ol = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts[w:w + 1], 6, app=app, seed=8, walker_base=int(w), **kw)
+        assert ol[0] == lens[w] and np.array_equal(op[0, :ol[0] + 1], rows[w, :ol[0] + 1])

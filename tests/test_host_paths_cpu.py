@@ -95,3 +95,22 @@ log = calls()
 assert sum(x[0] == "malloc" and x[2] == "fail" for x in log) == 1
 assert sum(x[0] == "device_sync" for x in log) >= 3    # three blocks returned
 """)
+
+
+@pytest.mark.parametrize("call", ["walk", "walk_packed"])
+def test_online_tables_are_built_once_a_call(fake_cudart, call):
+    """Large batches with host results run in slices; the tables of the whole graph serve all of them."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring())
+calls()
+n = (1 << 21) + 5          # four slices
+starts = np.zeros(n, np.uint32)
+try:
+    ctx.%s(starts, 3, mode=1)
+except SkwError as e:      # (no kernel ran, so the rows do not add up)
+    assert "lengths add up" in str(e), e
+log = calls()
+assert len(launches(log, "walk_offline_kernel")) == 4 and not launches(log, "direct")
+assert len(launches(log, "classify_kernel")) == 1
+""" % call)
