@@ -504,6 +504,20 @@ __device__ void build_vertex_cta(u32 v, u32 off, u32 n, const float* __restrict_
   if (tid == 0) valid[v] = 1;
 }
 
+// Scratch of the lists beyond 16384 weights: one slab a CTA, sized by the largest degree; fewer CTAs when a giant hub
+// would make the slabs exceed 4 GB in total.
+static uint64_t scratch_slab(const skw_ctx* ctx) {
+  return ctx->max_degree > kHugeSmemMax ? ((uint64_t)ctx->max_degree + 1) & ~1ull : 0;
+}
+static uint64_t scratch_slab_bytes(const skw_ctx* ctx) { return (scratch_slab(ctx) + 2) * 12ull; }
+static int scratch_slabs(const skw_ctx* ctx) {
+  return (int)std::min<uint64_t>(ctx->sm_count, std::max<uint64_t>((4ull << 30) / scratch_slab_bytes(ctx), 8));
+}
+static int reserve_scratch(skw_ctx* ctx) {
+  if (!scratch_slab(ctx)) return SKW_OK;
+  return ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, scratch_slab_bytes(ctx) * scratch_slabs(ctx));
+}
+
 // Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`.
 static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot* slots, uint8_t* valid) {
   cudaStream_t st = ctx->stream;
@@ -526,19 +540,9 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
 #undef SMEM
     attr_set[ctx->device & 63] = true;
   }
-  // one slab per CTA of the scratch class, sized by the largest degree; fewer CTAs when a giant hub
-  // would make the slabs exceed 4 GB in total.
-  const uint64_t slab_elems = ctx->max_degree > kHugeSmemMax ? (((uint64_t)ctx->max_degree + 1) & ~1ull) : 0;
-  const uint64_t slab_bytes = (slab_elems + 2) * 12ull;
-  int gmem_ctas = ctx->sm_count;
-  if (slab_elems) {
-    const uint64_t fit = (4ull << 30) / slab_bytes;
-    if (fit < (uint64_t)gmem_ctas) gmem_ctas = (int)(fit < 8 ? 8 : fit);
-  }
-  if (slab_elems) {
-    int rc = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, slab_bytes * gmem_ctas);
-    if (rc != SKW_OK) return rc;
-  }
+  if (const int rc = reserve_scratch(ctx); rc != SKW_OK) return rc;
+  const uint64_t slab_elems = scratch_slab(ctx);
+  const int gmem_ctas = scratch_slabs(ctx);
   // The classes are independent.  The long lists take few CTAs for long, so their kernels start first, on streams of their
   // own, and the many short ones fill in on the caller's.
   const int streams = ctx->max_degree > kHugeSmemMax ? 5 : ctx->max_degree > kMidSmemMax ? 3 : ctx->max_degree > kF64Max ? 2
@@ -714,18 +718,30 @@ extern "C" int skw_selftest_bounded_wait(skw_ctx* ctx) {
 }
 
 namespace skw {
+// Words of the work lists of `vertices` vertices; at: where the list of each class starts.
+static u64 worklist_words(const skw_ctx* ctx, u32 vertices, u64* at) {
+  u64 words = 0;
+  for (int k = 0; k < K_CLASSES; ++k) {
+    at[k] = words;
+    words += class_room(k, vertices, ctx->E);
+  }
+  return words;
+}
+
+int reserve_builders(skw_ctx* ctx, u32 vertices) {
+  u64 at[K_CLASSES];
+  void* wl = ctx->worklist;
+  const int rc = ensure_bytes(ctx, &wl, &ctx->worklist_cap, sizeof(u32) * worklist_words(ctx, vertices, at));
+  ctx->worklist = static_cast<u32*>(wl);
+  return rc != SKW_OK ? rc : reserve_scratch(ctx);
+}
+
 // Queue the construction of the tables of vertices [v_begin, v_end) into `slots` and `valid`.
 int enqueue_tables(skw_ctx* ctx, u32 v_begin, u32 v_end, Slot* slots, uint8_t* valid) {
   if (v_end <= v_begin) return SKW_OK;
-  u64 words = 0, at[K_CLASSES];
-  for (int k = 0; k < K_CLASSES; ++k) {
-    at[k] = words;
-    words += class_room(k, v_end - v_begin, ctx->E);
-  }
-  void* wl = ctx->worklist;
-  int rc = ensure_bytes(ctx, &wl, &ctx->worklist_cap, sizeof(u32) * words);
-  ctx->worklist = static_cast<u32*>(wl);
-  if (rc != SKW_OK) return rc;
+  if (const int rc = reserve_builders(ctx, v_end - v_begin); rc != SKW_OK) return rc;
+  u64 at[K_CLASSES];
+  worklist_words(ctx, v_end - v_begin, at);
   ClassLists lists;
   for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->worklist + at[k];
   SKW_CUDA(ctx, cudaMemsetAsync(ctx->cls_counts, 0, 2 * K_CLASSES * sizeof(u32), ctx->stream));

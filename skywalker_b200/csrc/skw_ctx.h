@@ -120,6 +120,8 @@ enum class TableUse {
   kFrontier  // draws only from the slots that it writes
 };
 int alloc_table(skw_ctx* ctx, TableUse use);
+// memory that the builders of the tables of so many vertices need besides the tables
+int reserve_builders(skw_ctx* ctx, uint32_t vertices);
 // queue the construction of the tables of vertices [v_begin, v_end)
 int enqueue_tables(skw_ctx* ctx, uint32_t v_begin, uint32_t v_end, Slot* slots, uint8_t* valid);
 // forget the fused walk records (they are derived from the table and die with it) and free their memory

@@ -963,6 +963,10 @@ static int online_tables(skw_ctx* ctx, const skw_walk_params* prm, uint64_t n, c
       (prm->flags & (SKW_WALK_UNBIASED | SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES | SKW_WALK_DIRECT_SLOTS)))
     return SKW_OK;
   if (!tables_pay(ctx, prm, n) || !online_table_memory(ctx)) return SKW_OK;
+  if (reserve_builders(ctx, ctx->V) != SKW_OK) {
+    cudaGetLastError();
+    return SKW_OK;
+  }
   const int rc = enqueue_tables(ctx, 0, ctx->V, ctx->online_slots, ctx->online_valid);
   if (rc == SKW_OK) *slots = ctx->online_slots;
   return rc;

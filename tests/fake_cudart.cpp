@@ -1,6 +1,6 @@
 // A CUDA runtime without a GPU, for tests of the library's host paths: preloaded into a child process it answers the
 // runtime calls that the library makes.  Device memory is host memory, copies and memsets take place at once, kernels
-// are noted down and not run.  Allocations fail on request, and fake_log() tells what was called, one call a line:
+// are noted down and (but for the one that finds the largest degree) not run.  Allocations fail on request, and fake_log() tells what was called, one call a line:
 //   malloc <bytes> <ok|fail>    free    host_malloc <ok|fail>    device_sync    launch <stream> <kernel>
 //   record <event> <stream>     wait <stream> <event>            sync <stream>  memset <stream>    copy <stream>
 #include <cuda_runtime.h>
@@ -87,9 +87,15 @@ cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, vo
   *static_cast<cudaStream_t*>(stream) = config.stream;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t, cudaStream_t s) {
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t s) {
   std::lock_guard<std::recursive_mutex> l(mu);
   note("launch " + hex(s) + " " + kernels[f]);
+  if (kernels[f].find("max_degree_kernel") != std::string::npos) {  // the one whose result decides on host paths
+    const unsigned* xadj = *static_cast<const unsigned**>(args[0]);
+    const unsigned V = *static_cast<unsigned*>(args[1]);
+    unsigned* out = *static_cast<unsigned**>(args[2]);
+    for (unsigned v = 0; v < V; ++v) *out = xadj[v + 1] - xadj[v] > *out ? xadj[v + 1] - xadj[v] : *out;
+  }
   return cudaSuccess;
 }
 

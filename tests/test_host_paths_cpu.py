@@ -32,10 +32,11 @@ class Device:   # stands for a tensor on the device
         return self.a.ctypes.data
     def numel(self):
         return self.a.size
-def ring(V=1000, deg=12):   # a graph to be resident
-    x = np.arange(V + 1, dtype=np.uint32) * deg
-    a = (np.arange(V * deg, dtype=np.uint32) // deg + 1) %% V
-    return x, a, np.ones(V * deg, np.float32)
+def ring(V=1000, deg=12, hub=0):   # a graph to be resident
+    d = np.full(V, deg)
+    d[0] += hub
+    x = np.concatenate([[0], np.cumsum(d)]).astype(np.uint32)
+    return x, np.arange(x[-1], dtype=np.uint32) %% V, np.ones(x[-1], np.float32)
 """
 
 
@@ -114,3 +115,24 @@ log = calls()
 assert len(launches(log, "walk_offline_kernel")) == 4 and not launches(log, "direct")
 assert len(launches(log, "classify_kernel")) == 1
 """ % call)
+
+
+@pytest.mark.parametrize("nth,times,hub", [(0, 1, 0), (1, 1, 0), (2, 1, 0), (0, 1000, 0), (2, 1000, 0), (3, 1, 20000)])
+def test_online_walk_without_memory_for_tables(fake_cudart, nth, times, hub):
+    """Tables of the whole graph are a choice of the library: where their memory (slots, flags, work lists, scratch of
+    the longest lists) is not to be had, the walk computes its slots one by one."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring(hub=%d))
+s, p, l = Device(1 << 18), Device(1 << 18, 20), Device(1 << 18)
+calls()
+fake.fake_fail_malloc(%d, %d)
+ctx.walk(s, 20, mode=1, paths=p, lengths=l)
+log = calls()
+assert sum(x[0] == "malloc" and x[2] == "fail" for x in log)
+assert len(launches(log, "walk_online_direct_kernel")) == 1 and not launches(log, "classify")
+fake.fake_fail_malloc(-1, 0)
+ctx.walk(s, 20, mode=1, paths=p, lengths=l)
+log = calls()
+assert len(launches(log, "classify")) == 1 and len(launches(log, "walk_offline_kernel")) == 1
+""" % (hub, nth, times))
