@@ -225,9 +225,10 @@ typedef struct skw_walk_params {
  * in one launch; for the duration of a call it memoises, per vertex, the largest weight, the total and
  * prefix sums at every 64th list position -- never a table entry).  With neither flag the library
  * takes the cheaper of DIRECT_SLOTS and, for batches that are large for the graph, the tables of the
- * whole graph built for the call, in memory of their own (8 bytes an edge, kept until the graph
- * changes): the table of skw_alias_build_offline and its walk records stay as they are.  All ways give
- * identical walks.  SKW_WALK_CACHE_TABLES implies BUILD_TABLES. */
+ * whole graph built for the call, in memory of their own: the table of skw_alias_build_offline and its
+ * walk records stay as they are.  That memory (8 bytes an edge) is kept for the next such call until the
+ * graph changes, skw_graph_free_weights is called or another allocation of the context would fail; where
+ * it is not to be had, slots are computed.  All ways give identical walks.  SKW_WALK_CACHE_TABLES implies BUILD_TABLES. */
 #define SKW_WALK_BUILD_TABLES 4u
 #define SKW_WALK_DIRECT_SLOTS 8u
 /* skw_walk only: the whole h_paths matrix is written, cells past a walk's end with SKW_INVALID_VERTEX. */

@@ -155,6 +155,11 @@ cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes) {
     drop_records(ctx);
     e = DeviceMemory::get().alloc(p, bytes);
   }
+  if (e == cudaErrorMemoryAllocation && ctx->online_slots && !ctx->online_in_use) {
+    cudaGetLastError();
+    drop_online_tables(ctx);
+    e = DeviceMemory::get().alloc(p, bytes);
+  }
   return e;
 }
 
@@ -195,6 +200,13 @@ int err_check(skw_ctx* ctx, const char* where, bool queued) {
   return SKW_OK;
 }
 
+void drop_online_tables(skw_ctx* ctx) {
+  dev_free(ctx->online_slots);
+  dev_free(ctx->online_valid);
+  ctx->online_slots = nullptr;
+  ctx->online_valid = nullptr;
+}
+
 static void free_graph(skw_ctx* ctx) {
   if (ctx->owns_graph) {
     dev_free(ctx->xadj);
@@ -206,10 +218,7 @@ static void free_graph(skw_ctx* ctx) {
   ctx->owns_graph = ctx->owns_weights = false;
   dev_free(ctx->slots);
   dev_free(ctx->valid);
-  dev_free(ctx->online_slots);
-  dev_free(ctx->online_valid);
-  ctx->online_slots = nullptr;
-  ctx->online_valid = nullptr;
+  drop_online_tables(ctx);
   dev_free(ctx->stamp);
   dev_free(ctx->prep_memo);
   dev_free(ctx->prep_ckpt);
@@ -650,7 +659,7 @@ int skw_graph_free_weights(skw_ctx* ctx) {
   DeviceGuard g(ctx->device);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (ctx->owns_weights) dev_free(ctx->adjwgt);
-  dev_give_back(ctx->device);
+  drop_online_tables(ctx);  // there are no online calls without weights
   dev_give_back(ctx->device);
   ctx->adjwgt = nullptr;
   ctx->owns_weights = false;

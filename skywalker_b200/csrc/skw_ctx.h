@@ -56,9 +56,10 @@ struct skw_ctx {
   uint8_t* valid = nullptr;
   bool slots_marked = false;  // slots that no build has reached hold prob = -1
   bool table_ready = false;
-  // tables of one online call (the table above stays as it is)
+  // tables of one online call (the table above stays as it is); their memory is kept for the next
   skw::Slot* online_slots = nullptr;
   uint8_t* online_valid = nullptr;
+  bool online_in_use = false;  // by the call that is being made: not to be given up
   // optional fused walk records (32 B per edge slot) and per-vertex {offset, usable degree}
   void* records = nullptr;
   void* vinfo = nullptr;
@@ -124,10 +125,12 @@ int alloc_table(skw_ctx* ctx, TableUse use);
 int reserve_builders(skw_ctx* ctx, uint32_t vertices);
 // queue the construction of the tables of vertices [v_begin, v_end)
 int enqueue_tables(skw_ctx* ctx, uint32_t v_begin, uint32_t v_end, Slot* slots, uint8_t* valid);
+// free the memory of an online call's tables
+void drop_online_tables(skw_ctx* ctx);
 // forget the fused walk records (they are derived from the table and die with it) and free their memory
 void drop_records(skw_ctx* ctx);
-// Device memory, from blocks freed earlier where one fits; gives up the memory of records that are no longer valid before
-// it fails.  dev_free waits for the GPU.
+// Device memory, from blocks freed earlier where one fits; gives up the memory of records that are no longer valid, then
+// that of an online call's tables, before it fails.  dev_free waits for the GPU.
 cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes);
 template <class T>
 cudaError_t dev_malloc(skw_ctx* ctx, T** p, size_t bytes) {

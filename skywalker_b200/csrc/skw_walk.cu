@@ -944,37 +944,44 @@ static bool tables_pay(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t 
   return tables < computed;
 }
 
-// Memory for such tables: 8 bytes an edge, kept until the graph changes.  False when there is none to be had.
+// Memory for such tables: 8 bytes an edge, and what the builders need.  False when there is none to be had.
 static bool online_table_memory(skw_ctx* ctx) {
-  if (ctx->online_slots) return true;
-  if (dev_malloc(ctx, &ctx->online_slots, sizeof(Slot) * (ctx->E ? ctx->E : 1)) == cudaSuccess &&
-      dev_malloc(ctx, &ctx->online_valid, ctx->V ? ctx->V : 1) == cudaSuccess)
+  if ((ctx->online_slots || dev_malloc(ctx, &ctx->online_slots, sizeof(Slot) * (ctx->E ? ctx->E : 1)) == cudaSuccess) &&
+      (ctx->online_valid || dev_malloc(ctx, &ctx->online_valid, ctx->V ? ctx->V : 1) == cudaSuccess) &&
+      reserve_builders(ctx, ctx->V) == SKW_OK)
     return true;
   cudaGetLastError();
-  dev_free(ctx->online_slots);
-  ctx->online_slots = nullptr;
   return false;
 }
 
-// Queue the tables of the whole graph for the n walkers of an online call, where they pay: *slots, else null.
-static int online_tables(skw_ctx* ctx, const skw_walk_params* prm, uint64_t n, const Slot** slots) {
-  *slots = nullptr;
+// Tables of the whole graph for one online call; slots is null if it does without.
+struct OnlineTables {
+  skw_ctx* ctx;
+  const Slot* slots = nullptr;
+  explicit OnlineTables(skw_ctx* c) : ctx(c) {}
+  ~OnlineTables() { ctx->online_in_use = false; }
+};
+
+// Queue such tables for the n walkers of a call, where they pay.
+static int online_tables(const skw_walk_params* prm, uint64_t n, OnlineTables& t) {
+  skw_ctx* ctx = t.ctx;
   if (prm->mode != SKW_MODE_ONLINE || !n ||
       (prm->flags & (SKW_WALK_UNBIASED | SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES | SKW_WALK_DIRECT_SLOTS)))
     return SKW_OK;
-  if (!tables_pay(ctx, prm, n) || !online_table_memory(ctx)) return SKW_OK;
-  if (reserve_builders(ctx, ctx->V) != SKW_OK) {
-    cudaGetLastError();
+  if (!tables_pay(ctx, prm, n)) return SKW_OK;
+  ctx->online_in_use = true;
+  if (!online_table_memory(ctx)) {
+    ctx->online_in_use = false;  // computing slots takes memory as well
     return SKW_OK;
   }
   const int rc = enqueue_tables(ctx, 0, ctx->V, ctx->online_slots, ctx->online_valid);
-  if (rc == SKW_OK) *slots = ctx->online_slots;
+  if (rc == SKW_OK) t.slots = ctx->online_slots;
   return rc;
 }
 
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
-// No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: what online_tables
-// gave for the call.
+// No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: the
+// slots that online_tables gave for the call.
 static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n,
                        uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum, const Slot* whole_table) {
   const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
@@ -1079,10 +1086,10 @@ static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_
   int rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
-  const Slot* tables;
-  if ((rc = online_tables(ctx, prm, n, &tables)) != SKW_OK) return rc;
-  if ((rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum), tables)) !=
-      SKW_OK)
+  OnlineTables tables(ctx);
+  if ((rc = online_tables(prm, n, tables)) != SKW_OK) return rc;
+  if ((rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum),
+                        tables.slots)) != SKW_OK)
     return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   if (h_lengths && n) SKW_CUDA(ctx, cudaMemcpyAsync(h_lengths, d_lengths, sizeof(u32) * (size_t)n, cudaMemcpyDeviceToHost, st));
@@ -1107,9 +1114,10 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
   // in a second record until skw_ctx_take_sampled_edges() looks at them.
   if (!ms && !sampled_edges) {
     QueuedErrors q(ctx);
-    const Slot* tables;
-    if ((rc = online_tables(ctx, prm, n, &tables)) != SKW_OK) return rc;
-    return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1, tables);
+    OnlineTables tables(ctx);
+    if ((rc = online_tables(prm, n, tables)) != SKW_OK) return rc;
+    return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1,
+                       tables.slots);
   }
   return walk_and_wait(ctx, prm, d_starts, n, d_paths, d_lengths, nullptr, nullptr, ms, sampled_edges);
 }
@@ -1333,7 +1341,7 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
     SKW_CUDA(ctx, cudaStreamWaitEvent(side, ctx->pk_ready[c], 0));
     return SKW_OK;
   };
-  const Slot* tables = nullptr;
+  OnlineTables tables(ctx);
   auto body = [&]() -> int {
     // the start vertices come in slice by slice on the side stream, ahead of everything else it will
     // carry: a walk waits for its own slice only, and no walk waits behind a copy of a later slice
@@ -1348,9 +1356,9 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
       skw_walk_params p = *prm;
       p.walker_base = prm->walker_base + base * stride;
       SKW_CUDA(ctx, cudaEventRecord(ctx->pk_t0[c], st));
-      int r = c == 0 ? online_tables(ctx, prm, n, &tables) : SKW_OK;  // for all slices
+      int r = c == 0 ? online_tables(prm, n, tables) : SKW_OK;  // for all slices
       if (r != SKW_OK) return r;
-      r = walk_launch(ctx, &p, d_starts + base, nc, d_rows + base * prm->hop_num, d_len + base, scratch_sum, tables);
+      r = walk_launch(ctx, &p, d_starts + base, nc, d_rows + base * prm->hop_num, d_len + base, scratch_sum, tables.slots);
       if (r != SKW_OK) return r;
       SKW_CUDA(ctx, cudaEventRecord(ctx->pk_t1[c], st));
       if ((r = scan_and_pack(c)) != SKW_OK) return r;
@@ -1359,6 +1367,7 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
       else
         SKW_CUDA(ctx, cudaMemcpyAsync(h_lengths + base, d_len + base, sizeof(u32) * (size_t)nc, cudaMemcpyDeviceToHost, side));
     }
+    ctx->online_in_use = false;  // every walk is queued, and freeing waits for the GPU
     // the host follows the device slice by slice: learn the size, start the copy
     uint64_t total_cells = 0;
     bool fits = h_packed != nullptr;

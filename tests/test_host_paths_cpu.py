@@ -136,3 +136,27 @@ ctx.walk(s, 20, mode=1, paths=p, lengths=l)
 log = calls()
 assert len(launches(log, "classify")) == 1 and len(launches(log, "walk_offline_kernel")) == 1
 """ % (hub, nth, times))
+
+
+def test_tables_of_an_online_call_make_room(fake_cudart):
+    """The memory of an online call's tables is kept for the next one, but given up when an allocation fails without it,
+    and returned with the weights."""
+    _run(fake_cudart, """
+ctx = Context(0)
+V, E = 40000, 480000
+ctx.upload(*ring(V))
+s, p, l = Device(1 << 18), Device(1 << 18, 20), Device(1 << 18)
+ctx.walk(s, 20, mode=1, paths=p, lengths=l)
+calls()
+fake.fake_memory(fake.fake_used() + 8 * E - 1)      # room for nearly the table
+ctx.alias_build_offline()
+ctx.walk(s, 20, mode=1, paths=p, lengths=l)         # nothing left for tables of its own
+log = calls()
+assert len(launches(log, "walk_online_direct_kernel")) == 1
+fake.fake_memory(64 << 30)
+ctx.walk(s, 20, mode=1, paths=p, lengths=l)
+assert len(launches(calls(), "walk_offline_kernel")) == 1
+used = fake.fake_used()
+ctx.free_weights()
+assert used - fake.fake_used() >= 4 * E + 8 * E
+""")
