@@ -163,6 +163,13 @@ cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes) {
   return e;
 }
 
+bool capturing(const skw_ctx* ctx) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 // The status words of a context: 16 x u32 on the device (error records, then the four 64-bit sums at word 8) and the
 // same 16 words in mapped host memory.  A synchronous call ends with this kernel, which hands them to the host and
 // leaves those of `clear` (a bit a word) cleared for the next call: one small launch where two memsets before a call and

@@ -144,6 +144,8 @@ void dev_give_back(int device);  // what dev_free kept
 int fail_cuda(skw_ctx* ctx, cudaError_t e, const char* what, const char* file, int line);
 void set_global_error(const char* msg);
 
+// Whether the context's stream is being captured into a graph: no allocation then, and no memory that may change later.
+bool capturing(const skw_ctx* ctx);
 // Grow-only device buffer.
 int ensure_bytes(skw_ctx* ctx, void** p, size_t* cap, size_t want);
 // Bracket of a synchronous call: its error record and sums 0 and 3 are zero after err_reset; err_check brings all

@@ -968,7 +968,8 @@ static int online_tables(const skw_walk_params* prm, uint64_t n, OnlineTables& t
   if (prm->mode != SKW_MODE_ONLINE || !n ||
       (prm->flags & (SKW_WALK_UNBIASED | SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES | SKW_WALK_DIRECT_SLOTS)))
     return SKW_OK;
-  if (!tables_pay(ctx, prm, n)) return SKW_OK;
+  // A graph would keep the addresses of this memory, which can be given up or grow once the call is over.
+  if (!tables_pay(ctx, prm, n) || capturing(ctx)) return SKW_OK;
   ctx->online_in_use = true;
   if (!online_table_memory(ctx)) {
     ctx->online_in_use = false;  // computing slots takes memory as well

@@ -463,9 +463,11 @@ int launch_walk_online_direct(skw_ctx* ctx, const WalkArgs& a, uint32_t app) {
   const int grid = (int)std::min<u64>(std::max<u64>(want, 1), (u64)ctx->sm_count * 32);
   cudaStream_t st = ctx->stream;
   // the per-vertex memo of (largest weight, total): allocated on first use when the graph has lists long
-  // enough to use it, valid for one call (a new stamp per call; zero never names a call)
+  // enough to use it, valid for one call (a new stamp per call; zero never names a call).  A call that is captured
+  // before there is one goes without.
   PrepMemo* memo = nullptr;
-  if (ctx->max_degree >= kMemoMinDegree) {
+  const bool may_allocate = !capturing(ctx);
+  if (ctx->max_degree >= kMemoMinDegree && (ctx->prep_memo || may_allocate)) {
     if (!ctx->prep_memo) {
       SKW_CUDA(ctx, dev_malloc(ctx, &ctx->prep_memo, sizeof(PrepMemo) * ((size_t)ctx->V + 1)));
       SKW_CUDA(ctx, cudaMemsetAsync(ctx->prep_memo, 0, sizeof(PrepMemo) * ((size_t)ctx->V + 1), st));
@@ -478,7 +480,7 @@ int launch_walk_online_direct(skw_ctx* ctx, const WalkArgs& a, uint32_t app) {
     memo = static_cast<PrepMemo*>(ctx->prep_memo);
   }
   Ckpt* ck_all = nullptr;
-  if (memo != nullptr && ctx->max_degree >= kCkMinDegree) {
+  if (memo != nullptr && ctx->max_degree >= kCkMinDegree && (ctx->prep_ckpt || may_allocate)) {
     if (!ctx->prep_ckpt) SKW_CUDA(ctx, dev_malloc(ctx, &ctx->prep_ckpt, sizeof(Ckpt) * ((size_t)(ctx->E / kCkChunk) + 2)));
     ck_all = static_cast<Ckpt*>(ctx->prep_ckpt);  // validated by the memo's stamp: no clearing needed
   }

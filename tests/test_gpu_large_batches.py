@@ -26,3 +26,42 @@ def test_online_host_batches(ctx, oracle, plaw, app, kw, n):
     for w in range(0, n, n // 50):
         op, ol = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts[w:w + 1], 6, app=app, seed=8, walker_base=int(w), **kw)
         assert ol[0] == lens[w] and np.array_equal(op[0, :ol[0] + 1], rows[w, :ol[0] + 1])
+
+
+@pytest.mark.parametrize("warm", [0, 300, 40000])      # walkers of the call before: none, slots computed, tables
+def test_captured_online_walk(oracle, plaw, warm):
+    """A queued online walk captured into a graph and replayed, before and after calls that take tables."""
+    import torch
+    from skywalker_b200.api import Context
+    g = plaw
+    n, hop = 40000, 21
+    c = Context(0)
+    c.upload(g.xadj, g.adjncy, g.adjwgt)
+    starts = oracle.gen_starts(n, g.V, 5)
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, hop, seed=8)
+    live = np.arange(hop)[None, :] <= want_len[:, None]
+    s = torch.from_numpy(starts.view(np.int32)).cuda()
+    p = torch.zeros((n, hop), dtype=torch.int32, device="cuda")
+    l = torch.zeros(n, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    c.set_stream(stream.cuda_stream)
+    kw = dict(mode=MODE_ONLINE, seed=8, paths=p, lengths=l, enqueue_only=True)
+    if warm:
+        c.walk(s, hop, n=warm, **kw)
+        c.take_sampled_edges()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        c.walk(s, hop, **kw)
+    for _ in range(2):
+        p.zero_(), l.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        assert c.take_sampled_edges() == int(want_len.sum())
+        assert np.array_equal(l.cpu().numpy(), want_len)
+        assert np.array_equal(p.cpu().numpy().view(np.uint32)[live], want[live])
+        c.walk(starts, hop, mode=MODE_ONLINE, seed=9)
+    del graph
+    c.close()

@@ -160,3 +160,25 @@ used = fake.fake_used()
 ctx.free_weights()
 assert used - fake.fake_used() >= 4 * E + 8 * E
 """)
+
+
+@pytest.mark.parametrize("warm", [None, 256, 1 << 18])
+@pytest.mark.parametrize("hub", [0, 20000])
+def test_online_walk_under_capture_allocates_nothing(fake_cudart, warm, hub):
+    """A queued online walk can be captured into a graph, whatever ran before it: one kernel, and no memory that the
+    library may later take away from the graph."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring(hub=%d))
+s, p, l = Device(1 << 18), Device(1 << 18, 20), Device(1 << 18)
+if %r:
+    ctx.walk(s, 20, mode=1, paths=p, lengths=l, n=%r)
+calls()
+fake.fake_capture(1)
+ctx.walk(s, 20, mode=1, paths=p, lengths=l, enqueue_only=True)
+log = calls()
+assert len(log) == 1 and launches(log, "walk_online_direct_kernel"), log
+fake.fake_capture(0)
+ctx.walk(s, 20, mode=1, paths=p, lengths=l, enqueue_only=True)
+assert launches(calls(), "walk_offline_kernel")
+""" % (hub, warm, warm))
