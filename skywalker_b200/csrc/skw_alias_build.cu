@@ -504,6 +504,18 @@ __device__ void build_vertex_cta(u32 v, u32 off, u32 n, const float* __restrict_
   if (tid == 0) valid[v] = 1;
 }
 
+// (A capture holds neither: an event from outside may not be waited for in it, nor one of its own outside.)
+int builders_begin(skw_ctx* ctx) {
+  if (ctx->tables_queued && !capturing(ctx)) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->tables_used, 0));
+  return SKW_OK;
+}
+int builders_queued(skw_ctx* ctx) {
+  if (capturing(ctx)) return SKW_OK;
+  SKW_CUDA(ctx, cudaEventRecord(ctx->tables_used, ctx->stream));
+  ctx->tables_queued = true;
+  return SKW_OK;
+}
+
 // Scratch of the lists beyond 16384 weights: one slab a CTA, sized by the largest degree; fewer CTAs when a giant hub
 // would make the slabs exceed 4 GB in total.
 static uint64_t scratch_slab(const skw_ctx* ctx) {
@@ -663,7 +675,7 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
   void* p = ctx->frontier_lists;
   int rc = ensure_bytes(ctx, &p, &ctx->frontier_lists_bytes, sizeof(u32) * (size_t)K_CLASSES * (cap ? cap : 1));
   ctx->frontier_lists = static_cast<u32*>(p);
-  if (rc != SKW_OK) return rc;
+  if (rc != SKW_OK || (rc = builders_begin(ctx)) != SKW_OK) return rc;
   if (!ctx->stamp) {
     SKW_CUDA(ctx, dev_malloc(ctx, &ctx->stamp, sizeof(u32) * ((size_t)ctx->V + 1)));
     SKW_CUDA(ctx, cudaMemsetAsync(ctx->stamp, 0, sizeof(u32) * ((size_t)ctx->V + 1), ctx->stream));
@@ -739,7 +751,8 @@ int reserve_builders(skw_ctx* ctx, u32 vertices) {
 // Queue the construction of the tables of vertices [v_begin, v_end) into `slots` and `valid`.
 int enqueue_tables(skw_ctx* ctx, u32 v_begin, u32 v_end, Slot* slots, uint8_t* valid) {
   if (v_end <= v_begin) return SKW_OK;
-  if (const int rc = reserve_builders(ctx, v_end - v_begin); rc != SKW_OK) return rc;
+  int rc = reserve_builders(ctx, v_end - v_begin);
+  if (rc != SKW_OK || (rc = builders_begin(ctx)) != SKW_OK) return rc;
   u64 at[K_CLASSES];
   worklist_words(ctx, v_end - v_begin, at);
   ClassLists lists;

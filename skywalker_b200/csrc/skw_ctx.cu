@@ -494,6 +494,7 @@ int skw_ctx_create(int device, skw_ctx** out) {
     CK(cudaEventCreateWithFlags(&ctx->bjoin[i], cudaEventDisableTiming));
   }
   CK(cudaEventCreateWithFlags(&ctx->bfork, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&ctx->tables_used, cudaEventDisableTiming));
   CK(cudaEventCreate(&ctx->ev0));
   CK(cudaEventCreate(&ctx->ev1));
   CK(dev_malloc(ctx, &ctx->d_err, 64));
@@ -542,6 +543,7 @@ void skw_ctx_destroy(skw_ctx* ctx) {
     if (ctx->bjoin[i]) cudaEventDestroy(ctx->bjoin[i]);
   }
   if (ctx->bfork) cudaEventDestroy(ctx->bfork);
+  if (ctx->tables_used) cudaEventDestroy(ctx->tables_used);
   for (int i = 0; i < skw_ctx::kPackSlices; ++i) {
     if (ctx->pk_ready[i]) cudaEventDestroy(ctx->pk_ready[i]);
     if (ctx->pk_in[i]) cudaEventDestroy(ctx->pk_in[i]);

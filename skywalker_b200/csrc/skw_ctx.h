@@ -38,6 +38,10 @@ struct skw_ctx {
   static constexpr int kBuilderStreams = 5;
   cudaStream_t bstream[kBuilderStreams] = {};
   cudaEvent_t bfork = nullptr, bjoin[kBuilderStreams] = {};
+  // behind the last queued call that builds tables, whatever stream it went to: the builders' work lists and scratch and
+  // the tables of an online call are the context's
+  cudaEvent_t tables_used = nullptr;
+  bool tables_queued = false;
   std::string err;
   uint64_t launches = 0;
 
@@ -121,6 +125,9 @@ enum class TableUse {
   kFrontier  // draws only from the slots that it writes
 };
 int alloc_table(skw_ctx* ctx, TableUse use);
+// the calls that queue builders wait on the GPU for the last queued call that did, if it was on another stream
+int builders_begin(skw_ctx* ctx);
+int builders_queued(skw_ctx* ctx);
 // memory that the builders of the tables of so many vertices need besides the tables
 int reserve_builders(skw_ctx* ctx, uint32_t vertices);
 // queue the construction of the tables of vertices [v_begin, v_end)

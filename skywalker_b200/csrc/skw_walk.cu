@@ -980,6 +980,12 @@ static int online_tables(const skw_walk_params* prm, uint64_t n, OnlineTables& t
   return rc;
 }
 
+// Whether a call builds the tables of its walkers' vertices at every step.
+static bool builds_frontiers(const skw_walk_params* prm) {
+  return prm->mode == SKW_MODE_ONLINE && !(prm->flags & SKW_WALK_UNBIASED) &&
+         (prm->flags & (SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES)) != 0;
+}
+
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
 // No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: the
 // slots that online_tables gave for the call.
@@ -990,7 +996,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   int rc;
   // Online walks make one launch over tables of the whole graph or one that computes every slot it draws, whichever
   // pays; on request they build the tables of the frontier at every step (same walks).
-  const bool build_tables = online && (prm->flags & (SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES)) != 0;
+  const bool build_tables = builds_frontiers(prm);
   if (build_tables) {
     drop_records(ctx);  // online builds overwrite table slots
     if ((rc = alloc_table(ctx, TableUse::kFrontier)) != SKW_OK) return rc;
@@ -1117,8 +1123,10 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
     QueuedErrors q(ctx);
     OnlineTables tables(ctx);
     if ((rc = online_tables(prm, n, tables)) != SKW_OK) return rc;
-    return walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1,
-                       tables.slots);
+    rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1,
+                     tables.slots);
+    const int after = tables.slots || builds_frontiers(prm) ? builders_queued(ctx) : SKW_OK;
+    return rc != SKW_OK ? rc : after;
   }
   return walk_and_wait(ctx, prm, d_starts, n, d_paths, d_lengths, nullptr, nullptr, ms, sampled_edges);
 }

@@ -65,3 +65,38 @@ def test_captured_online_walk(oracle, plaw, warm):
         c.walk(starts, hop, mode=MODE_ONLINE, seed=9)
     del graph
     c.close()
+
+
+@pytest.mark.parametrize("flags", [0, 4])
+def test_queued_online_walks_on_two_streams(oracle, plaw, flags):
+    """Queued walks that build tables, one behind the other on different streams, and a table built meanwhile."""
+    import torch
+    from skywalker_b200.api import Context
+    g = plaw
+    n, hop = 40000, 11
+    c = Context(0)
+    c.upload(g.xadj, g.adjncy, g.adjwgt)
+    starts = oracle.gen_starts(n, g.V, 5)
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    s = torch.from_numpy(starts.view(np.int32)).cuda()
+    outs = [(torch.zeros((n, hop), dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda"))
+            for _ in range(6)]
+    torch.cuda.synchronize()
+    for i, (p, l) in enumerate(outs):
+        c.set_stream(streams[i % 2].cuda_stream)
+        c.walk(s, hop, mode=MODE_ONLINE, flags=flags, seed=i, paths=p, lengths=l, enqueue_only=True)
+    c.set_stream(0)
+    c.alias_build_offline()
+    prob, alias, valid = c.alias_export()
+    assert np.array_equal(valid, table[2]) and np.array_equal(prob, table[0]) and np.array_equal(alias, table[1])
+    torch.cuda.synchronize()
+    total = 0
+    for i, (p, l) in enumerate(outs):
+        want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, hop, seed=i)
+        live = np.arange(hop)[None, :] <= want_len[:, None]
+        assert np.array_equal(l.cpu().numpy(), want_len)
+        assert np.array_equal(p.cpu().numpy().view(np.uint32)[live], want[live])
+        total += int(want_len.sum())
+    assert c.take_sampled_edges() == total
+    c.close()

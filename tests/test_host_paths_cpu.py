@@ -182,3 +182,45 @@ fake.fake_capture(0)
 ctx.walk(s, 20, mode=1, paths=p, lengths=l, enqueue_only=True)
 assert launches(calls(), "walk_offline_kernel")
 """ % (hub, warm, warm))
+
+
+@pytest.mark.parametrize("flags", [0, 4])       # tables of the whole graph, of every step's vertices
+@pytest.mark.parametrize("then", ["build", "queued", "khop"])
+def test_builders_wait_for_queued_tables_on_another_stream(fake_cudart, flags, then):
+    """Work lists, scratch and online tables belong to the context: after a change of stream a call that builds tables
+    waits for queued walks that still use them."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring(hub=20000))
+ctx.alias_build_offline()
+s, p, l = Device(1 << 18), Device(1 << 18, 20), Device(1 << 18)
+one, two = C.create_string_buffer(8), C.create_string_buffer(8)
+ctx.set_stream(C.addressof(one))
+calls()
+ctx.walk(s, 20, mode=1, paths=p, lengths=l, flags=%d, enqueue_only=True)
+first = calls()
+ctx.set_stream(C.addressof(two))
+if %r == "build":
+    ctx.alias_build_offline()
+elif %r == "khop":
+    ctx.sample_khop(np.zeros(100, np.uint32), [5, 3], mode=1)
+else:
+    ctx.walk(s, 20, mode=1, paths=p, lengths=l, enqueue_only=True)
+second = calls()
+# what the last kernel of the first call happens before, through stream order and events
+a, b = hex(C.addressof(one)), hex(C.addressof(two))
+last = max(i for i, x in enumerate(first) if x[0] == "launch" and x[1] == a)
+reached, events = {a}, set()
+builders = 0
+for x in first[last + 1:] + second:
+    if x[0] == "record":
+        (events.add if x[2] in reached else events.discard)(x[1])
+    elif x[0] == "wait" and x[2] in events:
+        reached.add(x[1])
+    elif x[0] == "device_sync":
+        reached.update((a, b))
+    elif x[0] in ("launch", "memset") and (x[0] == "memset" or any(k in x[2] for k in ("classify", "collect", "build_"))):
+        builders += 1
+        assert x[1] in reached, (x, reached)
+assert builders > 3
+""" % (flags, then, then))
