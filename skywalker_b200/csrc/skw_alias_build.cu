@@ -780,8 +780,9 @@ extern "C" int skw_alias_build_offline(skw_ctx* ctx, uint32_t v_begin, uint32_t 
   // returns the memory, and so does any allocation of the context that would fail without it (dev_malloc).
   ctx->records_ready = false;
   const bool whole = v_begin == 0 && v_end == ctx->V;
-  int rc = alloc_table(ctx, whole ? TableUse::kAll : TableUse::kSome);
+  int rc = settle_queued(ctx);
   if (rc != SKW_OK) return rc;
+  if ((rc = alloc_table(ctx, whole ? TableUse::kAll : TableUse::kSome)) != SKW_OK) return rc;
   rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
   cudaStream_t st = ctx->stream;

@@ -196,6 +196,7 @@ int err_check(skw_ctx* ctx, const char* where, bool queued) {
   SKW_LAUNCHED(ctx);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->status_clean = true;
+  ctx->queued = false;
   const uint32_t* rec = ctx->h_err + (queued ? 4 : 0);
   if (rec[0] != DEV_OK) {
     static const char* names[] = {"ok", "index out of range", "bounded wait ran out",
@@ -212,6 +213,13 @@ void drop_online_tables(skw_ctx* ctx) {
   dev_free(ctx->online_valid);
   ctx->online_slots = nullptr;
   ctx->online_valid = nullptr;
+}
+
+int settle_queued(skw_ctx* ctx) {
+  if (!ctx->queued_before) return SKW_OK;
+  SKW_CUDA(ctx, cudaDeviceSynchronize());
+  ctx->queued = ctx->queued_before = false;
+  return SKW_OK;
 }
 
 static void free_graph(skw_ctx* ctx) {
@@ -556,6 +564,8 @@ void skw_ctx_destroy(skw_ctx* ctx) {
 
 int skw_ctx_set_stream(skw_ctx* ctx, void* cuda_stream) {
   if (!ctx) return SKW_ERR_ARG;
+  if (ctx->queued) ctx->queued_before = true;
+  ctx->queued = false;
   ctx->stream = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : ctx->own_stream;
   return SKW_OK;
 }
@@ -892,9 +902,10 @@ int skw_alias_import(skw_ctx* ctx, const float* h_prob, const uint32_t* h_alias,
   if (!ctx->xadj) return fail(ctx, SKW_ERR_STATE, "skw_alias_import: no graph resident");
   if (!h_prob || !h_alias || !h_valid) return fail(ctx, SKW_ERR_ARG, "skw_alias_import: null array");
   DeviceGuard g(ctx->device);
-  ctx->records_ready = false;  // derived from the old table
-  int rc = alloc_table(ctx, TableUse::kAll);
+  int rc = settle_queued(ctx);
   if (rc != SKW_OK) return rc;
+  ctx->records_ready = false;  // derived from the old table
+  if ((rc = alloc_table(ctx, TableUse::kAll)) != SKW_OK) return rc;
   std::vector<Slot> tmp(ctx->E ? ctx->E : 1);
   for (uint64_t i = 0; i < ctx->E; ++i) {
     tmp[i].prob = h_prob[i];
@@ -980,8 +991,8 @@ int skw_alias_load(skw_ctx* ctx, const char* path) {
     return fail(ctx, SKW_ERR_IO, "skw_alias_load: %s holds a table for V=%llu E=%llu, the resident graph has V=%u E=%llu",
                 path, (unsigned long long)hdr[1], (unsigned long long)hdr[2], ctx->V, (unsigned long long)ctx->E);
   uint64_t fp = 0;
-  int rc = xadj_fingerprint(ctx, &fp);
-  if (rc != SKW_OK) return rc;
+  int rc = settle_queued(ctx);
+  if (rc != SKW_OK || (rc = xadj_fingerprint(ctx, &fp)) != SKW_OK) return rc;
   if (hdr[4] != fp)
     return fail(ctx, SKW_ERR_IO, "skw_alias_load: %s was written for another graph (same V and E, different offsets)", path);
   ctx->records_ready = false;  // derived from the old table

@@ -38,6 +38,8 @@ struct skw_ctx {
   static constexpr int kBuilderStreams = 5;
   cudaStream_t bstream[kBuilderStreams] = {};
   cudaEvent_t bfork = nullptr, bjoin[kBuilderStreams] = {};
+  bool queued = false;          // walks on the current stream that no call has waited for
+  bool queued_before = false;   // ... and on the stream before it
   // behind the last queued call that builds tables, whatever stream it went to: the builders' work lists and scratch and
   // the tables of an online call are the context's
   cudaEvent_t tables_used = nullptr;
@@ -125,6 +127,8 @@ enum class TableUse {
   kFrontier  // draws only from the slots that it writes
 };
 int alloc_table(skw_ctx* ctx, TableUse use);
+// the calls that write a table or its records in place wait for walks that were queued on other streams
+int settle_queued(skw_ctx* ctx);
 // the calls that queue builders wait on the GPU for the last queued call that did, if it was on another stream
 int builders_begin(skw_ctx* ctx);
 int builders_queued(skw_ctx* ctx);

@@ -805,6 +805,7 @@ int skw_walk_records_build(skw_ctx* ctx, float* ms) {
   if (!ctx) return SKW_ERR_ARG;
   if (!ctx->table_ready) return fail(ctx, SKW_ERR_STATE, "skw_walk_records_build: build or import the alias table first");
   DeviceGuard g(ctx->device);
+  if (const int rc = settle_queued(ctx); rc != SKW_OK) return rc;
   ctx->records_ready = false;
   ctx->records_building = true;
   // any failure below leaves no half-built records behind
@@ -1121,6 +1122,7 @@ int skw_walk_device(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_
   // in a second record until skw_ctx_take_sampled_edges() looks at them.
   if (!ms && !sampled_edges) {
     QueuedErrors q(ctx);
+    ctx->queued = true;
     OnlineTables tables(ctx);
     if ((rc = online_tables(prm, n, tables)) != SKW_OK) return rc;
     rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum) + 1,

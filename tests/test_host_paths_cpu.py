@@ -224,3 +224,31 @@ for x in first[last + 1:] + second:
         assert x[1] in reached, (x, reached)
 assert builders > 3
 """ % (flags, then, then))
+
+
+@pytest.mark.parametrize("writer", ["alias_build_offline()", "alias_build_offline(0, 10)", "walk_records_build()", "alias_load(path)",
+                                    "alias_import(*table)"])
+def test_table_writers_wait_for_queued_walks_on_another_stream(fake_cudart, tmp_path, writer):
+    """A table or its records are written in place; walks that were queued on another stream may still read them."""
+    _run(fake_cudart, """
+path = %r
+ctx = Context(0)
+ctx.upload(*ring())
+ctx.alias_build_offline()
+ctx.alias_save(path)
+table = ctx.alias_export()
+ctx.walk_records_build()
+s, p, l = Device(1 << 10), Device(1 << 10, 20), Device(1 << 10)
+one, two = C.create_string_buffer(8), C.create_string_buffer(8)
+ctx.set_stream(C.addressof(one))
+ctx.walk(s, 20, paths=p, lengths=l, enqueue_only=True)
+ctx.set_stream(C.addressof(two))
+calls()
+ctx.%s
+assert calls()[0] == ["device_sync"]
+ctx.%s
+assert ["device_sync"] not in calls()       # once
+ctx.walk(s, 20, paths=p, lengths=l, enqueue_only=True)
+ctx.%s                                      # the same stream: its order is enough
+assert ["device_sync"] not in calls()
+""" % (str(tmp_path / "t.skw"), writer, writer, writer))
