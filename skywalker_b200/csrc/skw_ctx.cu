@@ -1029,6 +1029,7 @@ int skw_host_alloc(size_t bytes, void** out) {
   if (!out) return SKW_ERR_ARG;
   cudaError_t e = cudaMallocHost(out, bytes ? bytes : 1);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next launch
     *out = nullptr;
     return fail(nullptr, SKW_ERR_NOMEM, "skw_host_alloc(%zu): %s", bytes, cudaGetErrorString(e));
   }

@@ -252,3 +252,19 @@ ctx.walk(s, 20, paths=p, lengths=l, enqueue_only=True)
 ctx.%s                                      # the same stream: its order is enough
 assert ["device_sync"] not in calls()
 """ % (str(tmp_path / "t.skw"), writer, writer, writer))
+
+
+@pytest.mark.parametrize("times", [1, 1000])
+def test_results_without_pinned_memory(fake_cudart, times):
+    """Result arrays come from pinned memory where there is some, else from pageable memory."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring())
+ctx.alias_build_offline()
+calls()
+fake.fake_fail_host_malloc(0, %d)
+for _ in range(3):
+    paths, lengths, _, _ = ctx.walk(np.zeros(100, np.uint32), 5)
+    assert paths.shape == (100, 5) and lengths.shape == (100,)
+assert sum(x[0] == "host_malloc" and x[1] == "fail" for x in calls()) >= 1
+""" % times)
