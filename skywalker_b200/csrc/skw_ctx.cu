@@ -35,6 +35,7 @@ int fail(skw_ctx* ctx, int code, const char* fmt, ...) {
 
 int fail_cuda(skw_ctx* ctx, cudaError_t e, const char* what, const char* file, int line) {
   const char* base = strrchr(file, '/');
+  cudaGetLastError();  // reported here, not by the next launch
   return fail(ctx, SKW_ERR_CUDA, "%s: %s (%s:%d)", what, cudaGetErrorString(e),
               base ? base + 1 : file, line);
 }

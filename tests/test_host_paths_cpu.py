@@ -268,3 +268,22 @@ for _ in range(3):
     assert paths.shape == (100, 5) and lengths.shape == (100,)
 assert sum(x[0] == "host_malloc" and x[1] == "fail" for x in calls()) >= 1
 """ % times)
+
+
+@pytest.mark.parametrize("call", ["alias_build_offline()", "sample_khop(np.zeros(10, np.uint32), [3], mode=1)",
+                                  "walk(np.zeros(5000, np.uint32), 100, flags=2)"])
+@pytest.mark.parametrize("after", [0, 2])
+def test_call_after_one_that_ran_out_of_memory(fake_cudart, call, after):
+    """An error that a call has reported is not met again by the next one."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring())
+fake.fake_fail_malloc(%d, 1000)
+try:
+    ctx.%s
+    assert False
+except SkwError as e:
+    assert "out of memory" in str(e) and "dev_malloc" in str(e), e
+fake.fake_fail_malloc(-1, 0)
+ctx.%s
+""" % (after, call, call))
