@@ -53,9 +53,9 @@ def _host_u32(x):
     """x as contiguous 32-bit words on the host: itself where it already is (a numpy array or a CPU tensor of
     32-bit integers, pinned ones included), else a converted copy."""
     if isinstance(x, np.ndarray):
-        if x.flags.c_contiguous and x.dtype.kind in "iu" and x.dtype.itemsize == 4 and x.dtype.isnative:
+        if x.ndim and x.flags.c_contiguous and x.dtype.kind in "iu" and x.dtype.itemsize == 4 and x.dtype.isnative:
             return x
-    elif hasattr(x, "data_ptr") and x.element_size() == 4 and not x.is_floating_point() and x.is_contiguous():
+    elif str(getattr(x, "dtype", "")) in ("torch.int32", "torch.uint32") and x.device.type == "cpu" and x.dim() and x.is_contiguous():
         return x
     return np.ascontiguousarray(x, np.uint32)
 
