@@ -16,6 +16,7 @@ Buffers may be numpy arrays (host entry points; copies happen inside the call) o
 """
 import ctypes as C
 import functools
+import operator
 import threading
 import weakref
 
@@ -330,7 +331,7 @@ class Context:
     # -- k-hop
     @staticmethod
     def khop_layout(fanout):
-        return Context._khop_layout(tuple(fanout))
+        return Context._khop_layout(tuple(operator.index(f) for f in fanout))
 
     @staticmethod
     @functools.lru_cache(maxsize=64)

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from skywalker_b200.api import _host_u32
+from skywalker_b200.api import Context, SkwError, _host_u32
 
 
 @pytest.mark.parametrize("x", [
@@ -37,3 +37,25 @@ def test_what_a_conversion_refuses_is_refused(make):
 def test_no_conversion_where_none_is_needed():
     for x in (np.arange(5, dtype=np.uint32), np.arange(5, dtype=np.int32), torch.arange(5, dtype=torch.int32)):
         assert _host_u32(x) is x
+
+
+class _Count:
+    """A fan-out that is a number to ctypes, equal to none, and may change."""
+
+    def __init__(self, n):
+        self.n = n
+
+    def __index__(self):
+        return self.n
+
+
+def test_khop_layout_goes_by_the_numbers():
+    changing = [_Count(25), _Count(10)]
+    assert Context.khop_layout(changing) == (276, 26)
+    changing[0].n = 2
+    assert Context.khop_layout(changing) == (23, 3)
+    assert Context.khop_layout(np.array([25, 10])) == Context.khop_layout(torch.tensor([25, 10])) == (276, 26)
+    for refused in ([25.0, 10], [], [1] * 5, [0, 3], [1 << 16, 1 << 16]):
+        for _ in range(2):                 # after the same numbers were accepted, and after a refusal
+            with pytest.raises((TypeError, SkwError)):
+                Context.khop_layout(refused)
