@@ -1206,16 +1206,16 @@ int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts,
   if (n && (!h_starts || !h_paths || !h_lengths)) return fail(ctx, SKW_ERR_ARG, "skw_walk: null buffer");
   if (prm->hop_num < 1) return fail(ctx, SKW_ERR_ARG, "skw_walk: hop_num must be >= 1");
   DeviceGuard g(ctx->device);
+  int rc = walk_check(ctx, prm);
+  if (rc != SKW_OK) return rc;
   if (n >= (1u << 18)) {
     if (prm->flags & SKW_WALK_FILL_ROWS) memset(h_paths, 0xFF, sizeof(uint32_t) * (size_t)n * prm->hop_num);
     return walk_rows_by_scatter(ctx, prm, h_starts, n, h_paths, h_lengths, ms, sampled_edges);
   }
-  int rc;
   const size_t nb = sizeof(uint32_t) * (size_t)n;
   if ((rc = ensure_bytes(ctx, &ctx->stage[0], &ctx->stage_bytes[0], nb)) != SKW_OK) return rc;
   if ((rc = ensure_bytes(ctx, &ctx->stage[1], &ctx->stage_bytes[1], nb * prm->hop_num)) != SKW_OK) return rc;
   if ((rc = ensure_bytes(ctx, &ctx->stage[2], &ctx->stage_bytes[2], nb)) != SKW_OK) return rc;
-  if ((rc = walk_check(ctx, prm)) != SKW_OK) return rc;
   if (n) SKW_CUDA(ctx, cudaMemcpyAsync(ctx->stage[0], h_starts, nb, cudaMemcpyHostToDevice, ctx->stream));
   const bool fill = (prm->flags & SKW_WALK_FILL_ROWS) != 0;
   if (n && fill) SKW_CUDA(ctx, cudaMemsetAsync(ctx->stage[1], 0xFF, nb * prm->hop_num, ctx->stream));

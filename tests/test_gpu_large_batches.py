@@ -100,3 +100,20 @@ def test_queued_online_walks_on_two_streams(oracle, plaw, flags):
         total += int(want_len.sum())
     assert c.take_sampled_edges() == total
     c.close()
+
+
+@pytest.mark.parametrize("app,kw", [(APP_DEEPWALK, {}), (APP_PPR, {"tp": 0.15})])
+@pytest.mark.parametrize("n", [5000, (1 << 18) + 777])      # a copy of the matrix, host threads
+def test_rows_made_by_the_library_are_filled(ctx, oracle, rmat12, app, kw, n):
+    """Rows that the caller did not bring: cells past a walk's end hold INVALID_VERTEX, also in memory used before."""
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, g.V, 31)
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    for seed in (8, 9):
+        rows, lens, _, edges = ctx.walk(starts, 21, app=app, seed=seed, **kw)
+        want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, 21, app=app, seed=seed, fill=0xFFFFFFFF, **kw)
+        assert np.array_equal(lens, want_len) and edges == int(want_len.sum()) and np.array_equal(rows, want)
+        rows[:] = 0x5A5A5A5A
+        del rows, lens

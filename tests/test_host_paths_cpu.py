@@ -287,3 +287,18 @@ except SkwError as e:
 fake.fake_fail_malloc(-1, 0)
 ctx.%s
 """ % (after, call, call))
+
+
+@pytest.mark.parametrize("n", [1000, 1 << 18])
+def test_refused_walk_leaves_the_rows_alone(fake_cudart, n):
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring())
+paths, lengths = np.full((%d, 3), 5, np.uint32), np.full(%d, 5, np.uint32)
+try:                                   # 16: fill the rows; there is no table
+    ctx.walk(np.zeros(%d, np.uint32), 3, paths=paths, lengths=lengths, flags=16)
+    assert False
+except SkwError as e:
+    assert e.code == -3
+assert (paths == 5).all() and (lengths == 5).all()
+""" % (n, n, n))
