@@ -81,3 +81,51 @@ def test_alias_several_lists_a_worker(ctx, oracle, least, most, lists):
     prob, alias, valid = ctx.alias_export()
     want_prob, want_alias, want_valid = oracle.alias_build(x, w)
     assert np.array_equal(valid, want_valid) and np.array_equal(prob, want_prob) and np.array_equal(alias, want_alias)
+
+
+KINDS = ["uniform", "equal", "one_heavy", "one_light", "lognormal", "pareto", "tiny", "unusable"]
+
+
+def _check_lists(ctx, oracle, lists):
+    import torch
+    sizes = [len(w) for w in lists]
+    x = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    with np.errstate(over="ignore"):
+        w = np.concatenate(lists).astype(np.float32)
+    d_x, d_a = torch.from_numpy(x.view(np.int32)).cuda(), torch.zeros(len(w), dtype=torch.int32, device="cuda")
+    d_w = torch.from_numpy(w).cuda()
+    torch.cuda.synchronize()
+    ctx.adopt_device(len(sizes), len(w), d_x, d_a, d_w)
+    ctx.alias_build_offline()
+    prob, alias, valid = ctx.alias_export()
+    want_prob, want_alias, want_valid = oracle.alias_build(x, w)
+    assert np.array_equal(valid, want_valid)
+    usable = np.repeat(want_valid.astype(bool), sizes)
+    bad = np.flatnonzero(usable & ((prob != want_prob) | (alias != want_alias)))
+    assert bad.size == 0, "list lengths that differ: %s" % sorted({sizes[np.searchsorted(x, b, "right") - 1] for b in bad})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("more_than_clusters", [-1, 0, 1, 150])
+def test_alias_many_giant_lists(ctx, oracle, kind, more_than_clusters):
+    """Lists of more than 16384 weights by clusters of CTAs, and by one CTA each from one list more than there are
+    clusters on: around the tiles and windows of 8192, of all kinds of weights, and a list without usable weights
+    between others."""
+    import torch
+    rng = np.random.default_rng(len(kind))
+    clusters = torch.cuda.get_device_properties(0).multi_processor_count * 3 // 8
+    sizes = [16385, 16386, 20000, 24575, 24576, 24577, 32768, 32769, 40000, 16384 + 2048, 16384 + 2049]
+    sizes = [sizes[i % len(sizes)] for i in range(clusters + more_than_clusters)]
+    lists = [_weights(kind, n, rng) for n in sizes]
+    lists[len(lists) // 2] = np.zeros(sizes[len(lists) // 2])
+    _check_lists(ctx, oracle, lists)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["lognormal", "one_heavy"])
+@pytest.mark.parametrize("others", [0, 60])
+def test_alias_list_of_many_windows(ctx, oracle, kind, others):
+    """A list that takes more than one round of merge windows, alone (a cluster) and among others (one CTA)."""
+    rng = np.random.default_rng(others)
+    _check_lists(ctx, oracle, [_weights(kind, 20000, rng) for _ in range(others)] + [_weights(kind, 1024 * 8192 + 5, rng)])

@@ -117,3 +117,22 @@ def test_rows_made_by_the_library_are_filled(ctx, oracle, rmat12, app, kw, n):
         assert np.array_equal(lens, want_len) and edges == int(want_len.sum()) and np.array_equal(rows, want)
         rows[:] = 0x5A5A5A5A
         del rows, lens
+
+
+@pytest.mark.parametrize("n", [1, 31, 63, 64, 65, 511, 512, 513])
+def test_ppr_records_chunk_edges(ctx, oracle, rmat12, n):
+    """The chunked kernel of PPR over records, which takes batches of more walkers than fit the GPU at a lane each: the
+    walkers of the last chunk and CTA, paths that leave the staged cells, rows of several lines."""
+    import torch
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    ctx.walk_records_build()
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    least = 700 * torch.cuda.get_device_properties(0).multi_processor_count
+    n += (least + 511) // 512 * 512
+    starts = oracle.gen_starts(n, g.V, n)
+    paths, lens, _, edges = ctx.walk(starts, 40, app=APP_PPR, tp=0.02, seed=n, walker_base=7)
+    want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, 40, app=APP_PPR, tp=0.02, seed=n, walker_base=7)
+    live = np.arange(40)[None, :] <= want_len[:, None]
+    assert np.array_equal(lens, want_len) and edges == int(want_len.sum()) and np.array_equal(paths[live], want[live])
