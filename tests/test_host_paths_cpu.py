@@ -302,3 +302,88 @@ except SkwError as e:
     assert e.code == -3
 assert (paths == 5).all() and (lengths == 5).all()
 """ % (n, n, n))
+
+
+def test_freed_device_memory_waits_within_bounds(fake_cudart):
+    """Freed blocks serve the next graph, up to a sixteenth of the memory, and are returned when an allocation fails
+    without them, on request, and with the last context."""
+    _run(fake_cudart, """
+G = 1 << 30
+fake.fake_memory(16 * G)
+idle = fake.fake_used()
+a, b = Context(0), Context(0)
+a.upload(*ring(100000))
+a.alias_build_offline()
+calls()
+a.upload(*ring(100000))
+a.alias_build_offline()
+log = calls()
+assert not [x for x in log if x[0] == "malloc"]            # the same sizes again
+free = [i for i, x in enumerate(log) if x[0] == "device_sync"]
+assert free and free[0] < min(i for i, x in enumerate(log) if x[0] in ("copy", "launch"))   # idle before it is used again
+for v in (300000, 500000, 700000, 900000, 1100000, 1500000, 2000000):
+    a.upload(*ring(v))
+    a.alias_build_offline()
+    a.walk_records_build()
+    live = v * 12 * (8 + 8 + 32) + v * 24
+    assert fake.fake_used() - live < G + (64 << 20) + v * 300, (v, fake.fake_used() >> 20)   # a sixteenth, and the work lists
+held = fake.fake_used()
+a.walk_records_free()
+assert fake.fake_used() <= held - 2000000 * 12 * 32
+a.upload(*ring(1000))
+waiting = fake.fake_used()
+fake.fake_memory(waiting + (1 << 20))                      # an allocation of more than is unused
+a.upload(*ring(300000))
+fake.fake_memory(16 * G)
+a.close()
+b.close()
+assert fake.fake_used() == idle
+""")
+
+
+def test_result_pool_lends_within_bounds(fake_cudart):
+    """Pinned result arrays: a block serves again when the last view of it is gone, so many bytes are out or wait at a
+    time, and large results are pageable."""
+    _run(fake_cudart, """
+import gc, threading
+from skywalker_b200 import api
+pool = api._results
+def pinned(n):
+    return sum(x[0] == "host_malloc" for x in calls()) == n
+calls()
+x = pool.array((1000, 10))
+at = x.ctypes.data
+view = x[3:7].T
+assert pinned(1)
+del x
+y = pool.array((1000, 10))                 # the first block is still seen through a view
+assert pinned(1) and y.ctypes.data != at
+del view
+gc.collect()
+z = pool.array((500, 17))                  # the same size class
+assert pinned(0) and z.ctypes.data == at
+big = pool.array((pool.LARGEST // 4 + 1,))
+assert pinned(0) and big.flags.owndata
+out = [pool.array((pool.LARGEST // 4,)) for _ in range(8)]
+assert sum(not a.flags.owndata for a in out) == 3 and pool.out <= pool.OUT     # beside y and z
+del out, y, z
+gc.collect()
+assert pool.out == 0 and pool.kept <= pool.KEEP
+assert sum(len(v) * k for k, v in pool.waiting.items()) == pool.kept
+# threads: no block is lent twice
+seen, bad = set(), []
+lock = threading.Lock()
+def work():
+    for _ in range(300):
+        a = pool.array((700,))
+        with lock:
+            (bad.append if a.ctypes.data in seen else seen.add)(a.ctypes.data)
+        a[:] = 1
+        with lock:
+            seen.discard(a.ctypes.data)
+        del a
+ts = [threading.Thread(target=work) for _ in range(8)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+assert not bad and pool.out == 0 and pool.kept <= pool.KEEP
+""")
