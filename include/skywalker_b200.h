@@ -326,7 +326,8 @@ int skw_sample_khop(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t* h_
  * the result needs; when capacity_cells is smaller (or h_packed is NULL) the call fills
  * h_sample_lengths and *cells, leaves h_packed unspecified (never written past capacity_cells) and
  * returns SKW_ERR_ARG.  The tree of a power-law graph is sparse (vertices without out-edges have no
- * children), and the host result is bound by the bus: BASELINE config 4 sends 47 MB instead of 79. */
+ * children), and the host result is bound by the bus: 65,536 seeds with fan-outs 25 and 10 on an R-MAT-like
+ * graph of 4.85 M vertices send 47 MB instead of 79. */
 int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t* h_seeds, uint64_t n,
                            uint32_t* h_packed, uint64_t capacity_cells, uint32_t* h_sample_lengths,
                            uint64_t* cells, float* ms, uint64_t* sampled_edges);
@@ -339,10 +340,11 @@ int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint3
 int skw_probe_random_gather(skw_ctx* ctx, uint64_t footprint_bytes, uint32_t iters,
                             double* gaccesses_per_s);
 
-/* Self-test of the kernels' bounded waits, no counterpart in the reference (whose block-level
- * constructor can spin forever, include/alias_table_new.cuh:637-708): launches a kernel that waits
- * on a barrier nothing signals; the wait must run out after its poll limit (about a millisecond)
- * and the call must return SKW_ERR_DEVICE ("bounded wait ran out") with the context still usable. */
+/* Self-test of a wait that runs out, no counterpart in the reference (whose block-level constructor
+ * can spin forever, include/alias_table_new.cuh:637-708): launches a kernel that polls a barrier
+ * nothing signals; it must give up after its poll limit (about a millisecond) and the call must
+ * return SKW_ERR_DEVICE ("bounded wait ran out") with the context still usable.  No other kernel of
+ * the library polls memory; they meet at hardware barriers that every thread reaches. */
 int skw_selftest_bounded_wait(skw_ctx* ctx);
 
 /* ---------------------------------------------------------------- host helpers ----------- */

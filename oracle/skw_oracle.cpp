@@ -1,7 +1,7 @@
 // CPU oracle for the alias-method sampling / random-walk path.  TEST INFRASTRUCTURE ONLY.
 //
 // Nothing in the shipped library includes, links or calls this file; it is loaded by the tests,
-// by the smoke check and by the benchmark's cpu-baseline / reference legs, as the checker and
+// by the smoke check and by the benchmark's cpu-baseline / reference legs, to compare with and
 // as the timed CPU implementation.
 //
 // Parity status: PARITY UNPINNED at the bit level.  wpybtw/Skywalker is CUDA-only (no CPU code

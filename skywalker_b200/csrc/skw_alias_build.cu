@@ -122,6 +122,7 @@ static u64 class_room(int k, u64 V, u64 E) {
 }
 
 // ------------------------------------------------------------------ bounded wait ----------
+// (of the self-test; the builders wait for nothing)
 __device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(u64* bar, u32 arrivals) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");

@@ -75,7 +75,6 @@ struct ClusterShared {
   int chunk_top;
   u64 chunk_q, chunk_d;
   u32 chunk_s;
-  u32 item;                        // the list the cluster is at
   u64 before_d[kClusterCtas + 1];  // deficit and smalls before each chunk
   u32 before_s[kClusterCtas + 1];
   u32 bound[32];                   // smalls before the start of each window of a round

@@ -54,8 +54,8 @@ int ensure_bytes(skw_ctx* ctx, void** p, size_t* cap, size_t want) {
 // Device memory of all contexts.  Freed blocks wait here for the next graph or context: a program that goes from batch
 // graph to batch graph allocates the same few sizes over and over, and a cudaMalloc with its cudaFree costs 1 to 10 ms a
 // gigabyte, several times the kernels that fill it.  At most a 16th of a GPU's memory waits; it is given back when an
-// allocation would fail otherwise, by the calls that free memory on request, and with the last context of the GPU.  A block is only reused once the GPU is idle, as
-// cudaFree would have waited for too, so streams and threads do not matter.
+// allocation would fail otherwise, by the calls that free memory on request, and with the last context of the GPU.  A
+// block is only reused once the GPU is idle, as cudaFree would have waited for too, so streams and threads do not matter.
 struct DeviceMemory {
   struct Block {
     size_t bytes;

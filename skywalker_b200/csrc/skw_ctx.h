@@ -15,9 +15,6 @@ namespace skw {
 // all-gather over up to 1024 ranks).
 constexpr uint32_t kSlotSlack = 1024;
 
-// Largest degree the shared-memory CTA builder takes (12 bytes of list state per edge).
-constexpr uint32_t kCtaSmemMaxDegree = 4096;
-
 }  // namespace skw
 
 struct skw_ctx {
@@ -33,7 +30,7 @@ struct skw_ctx {
               pk_in[kPackSlices] = {};
   uint64_t* h_tot = nullptr;  // cells each slice's packed result needs: mapped, written by the packing kernel
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  // the degree-class builders of one build run side by side: classes 257+ on streams of their own,
+  // the builders of one build run side by side: those of lists of more than 512 weights on streams of their own,
   // forked from and joined back into `stream` by events
   static constexpr int kBuilderStreams = 5;
   cudaStream_t bstream[kBuilderStreams] = {};

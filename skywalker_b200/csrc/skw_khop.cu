@@ -8,8 +8,9 @@
 // frontier vertex.  Here one thread works on an OUTPUT cell: thread
 // (seed s, parent idx, child j) reads the parent vertex, makes its own Philox draw keyed by
 // (seed id, child cell, hop) and stores one coalesced word; no queues and no atomics on the data
-// path.  Offline a CTA makes the whole trees of a few seeds; online mode goes hop by hop, and first builds the tables of the distinct vertices of the hop's frontier with
-// the degree-bucketed builders, then runs the same draw kernel.
+// path.  Offline a CTA makes the whole trees of a few seeds; online mode goes hop by hop, and first
+// builds the tables of the distinct vertices of the hop's frontier with the degree-bucketed builders,
+// then runs the same draw kernel.
 #include <algorithm>
 #include <string>
 
@@ -546,7 +547,7 @@ int skw_sample_khop_packed(skw_ctx* ctx, const skw_khop_params* prm, const uint3
     return SKW_OK;
   };
   auto body = [&]() -> int {
-      SKW_CUDA(ctx, cudaMemcpyAsync(d_seeds, h_seeds, nb, cudaMemcpyHostToDevice, st));
+    SKW_CUDA(ctx, cudaMemcpyAsync(d_seeds, h_seeds, nb, cudaMemcpyHostToDevice, st));
     SKW_CUDA(ctx, cudaEventRecord(ctx->ev0, st));
     for (uint32_t c = 0; c < slices && nc_of[c]; ++c) {
       const uint64_t base = (uint64_t)c * per, nc = nc_of[c];

@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kRecCta, 1024 / kRecCta) walk_records_kernel(c
     for (u32 k = 0; k < 8; ++k) {
       info[k] = make_uint2(0u, 0u);
       if (nbr[k] < V) info[k] = __ldg(vinfo + nbr[k]);
-      else dev_fail(err, DEV_ERR_INDEX, (u32)e0 + k, nbr[k], 22);
+      else dev_fail(err, DEV_ERR_INDEX, (u32)e0 + min(threadIdx.x + kRecCta * k, here - 1), nbr[k], 22);
     }
 #pragma unroll
     for (u32 k = 0; k < 8; ++k) {

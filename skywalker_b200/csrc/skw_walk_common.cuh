@@ -69,7 +69,8 @@ struct ListSearch {
     return lo >= hi || vlo > dst || vhi <= dst;
   }
 };
-// The sector of eight entries from s on; `wide`: the array starts on a 32-byte boundary.
+// The sector of eight entries from s on; `wide`: the array starts on a 32-byte boundary, so that a sector with an entry of
+// the list in it lies in one page with that entry, also where the array ends inside it.
 __device__ __forceinline__ void load_sector(const u32* __restrict__ adjncy, u32 s, u32 lo, u32 hi, bool wide, u32 (&x)[8]) {
   if (wide) {
     asm volatile("ld.global.nc.L1::no_allocate.L2::64B.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
