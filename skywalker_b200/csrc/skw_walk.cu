@@ -98,6 +98,9 @@ __device__ __forceinline__ bool walk_step_n2v(const WalkArgs& a, u32 step, u64 g
 // (what is resident: with more, the second wave costs the gain many times over).  Slots, three accesses a step, R-MAT 22,
 // 80 steps: 4,096 walkers 164 -> 110 us with one walker a warp, 16,384 150 -> 127 with four, 40,000 160 -> 141 with
 // eight; records, one access a step: 4,096 43 -> 38 with eight, and fewer gain no more.
+// Where tables and lists take up to 8 MB the accesses are short and the warps share the issue slots: half as many warps an
+// SM then (DeepWalk with uniform draws, R-MAT 14 to 16, 4,000 to 30,000 walkers: 85 -> 68 us, which 32 walkers a warp take
+// 70 for; with tables 93 -> 84 us up to R-MAT 14; from 16 MB on fewer walkers a warp win again, 151 against 157 us).
 // CTAs of two warps: a CTA lives as long as its unluckiest lane, and small ones keep the SMs evenly loaded to the end (slots,
 // 300,000 walkers: 714 -> 668 us).  For the same reason a lane takes one walker (PPR over slots with three a thread: 1,000
 // walkers 45 -> 31 us, 100,000 122 -> 100, 1 M 338 -> 309, 2 M 558 -> 532), but for PPR of many more, where a third of the
@@ -1057,7 +1060,8 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     else walk_records_walk_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);
     SKW_LAUNCHED(ctx);
   } else if (!online || whole_table) {
-    const WalkGrid g = walk_grid(ctx, prm->app, n, 34, 1);
+    const u64 read = ctx->E * (unbiased ? 4u : 12u);  // lists, and slots if they are drawn from
+    const WalkGrid g = walk_grid(ctx, prm->app, n, prm->app == SKW_APP_DEEPWALK && read <= (8u << 20) ? 17 : 34, 1);
     switch (prm->app) {
       case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
       case SKW_APP_PPR: walk_offline_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;

@@ -136,3 +136,19 @@ def test_ppr_records_chunk_edges(ctx, oracle, rmat12, n):
     want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, 40, app=APP_PPR, tp=0.02, seed=n, walker_base=7)
     live = np.arange(40)[None, :] <= want_len[:, None]
     assert np.array_equal(lens, want_len) and edges == int(want_len.sum()) and np.array_equal(paths[live], want[live])
+
+
+@pytest.mark.parametrize("flags", [0, 2])
+@pytest.mark.parametrize("n", [2516, 2517, 5032, 5033, 10064, 10065, 20129, 40257])
+def test_deepwalk_walkers_a_warp_on_a_small_graph(ctx, oracle, rmat12, n, flags):
+    """Batch sizes around which the number of walkers a warp changes on a graph whose tables are small."""
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, g.V, 5)
+    paths, lens, _, edges = ctx.walk(starts, 12, seed=8, flags=flags)
+    table = oracle.alias_build(g.xadj, g.adjwgt) if flags == 0 else None
+    want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt if flags == 0 else None, table, starts, 12, seed=8,
+                                 **({} if flags == 0 else {"unbiased": True}))
+    live = np.arange(12)[None, :] <= want_len[:, None]
+    assert np.array_equal(lens, want_len) and edges == int(want_len.sum()) and np.array_equal(paths[live], want[live])
