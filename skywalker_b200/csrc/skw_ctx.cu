@@ -256,16 +256,25 @@ static void free_graph(skw_ctx* ctx) {
   ctx->V = 0;
   ctx->E = 0;
   ctx->max_degree = 0;
+  ctx->empty_lists = 0;
 }
 
+// out[0]: the largest degree, out[1]: the number of vertices of degree 0
 __global__ void max_degree_kernel(const uint32_t* __restrict__ xadj, uint32_t V,
                                   uint32_t* __restrict__ out) {
-  uint32_t m = 0;
+  uint32_t m = 0, empty = 0;
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < V;
-       v += (size_t)gridDim.x * blockDim.x)
-    m = max(m, xadj[v + 1] - xadj[v]);
-  for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+       v += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t d = xadj[v + 1] - xadj[v];
+    m = max(m, d);
+    empty += d == 0 ? 1u : 0u;
+  }
+  for (int o = 16; o; o >>= 1) {
+    m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+    empty += __shfl_xor_sync(0xFFFFFFFFu, empty, o);
+  }
   if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+  if ((threadIdx.x & 31) == 0 && empty) atomicAdd(out + 1, empty);
 }
 
 __global__ void fill_ones_kernel(float* __restrict__ w, size_t n) {
@@ -414,6 +423,7 @@ int finish_graph(skw_ctx* ctx) {
                                 ctx->stream));
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->max_degree = (uint32_t)*ctx->h_sum;
+  ctx->empty_lists = (uint32_t)(*ctx->h_sum >> 32);
   ctx->status_clean = false;
   return SKW_OK;
 }

@@ -48,6 +48,7 @@ struct skw_ctx {
   uint32_t V = 0;
   uint64_t E = 0;
   uint32_t max_degree = 0;
+  uint32_t empty_lists = 0;  // vertices without out-edges
   uint32_t* xadj = nullptr;
   uint32_t* adjncy = nullptr;
   float* adjwgt = nullptr;
@@ -115,7 +116,7 @@ struct skw_ctx {
 namespace skw {
 
 int fail(skw_ctx* ctx, int code, const char* fmt, ...);
-// after the CSR pointers are set: compute max_degree
+// after the CSR pointers are set: compute max_degree and empty_lists
 int finish_graph(skw_ctx* ctx);
 // allocate slots[E] / valid[V] if absent; a call that writes only a part of the table has the rest marked unusable
 enum class TableUse {

@@ -75,6 +75,7 @@ __device__ __forceinline__ bool walk_step(const WalkArgs& a, u32 step, u64 gw, u
 // step).  A step is a chain of dependent accesses -- slot, neighbour, search of that list -- so the list of
 // the proposed vertex is fetched beside the search instead of at the start of the next step, and the list
 // of the vertex that is left is handed on.
+template <bool HALVING>
 __device__ __forceinline__ bool walk_step_n2v(const WalkArgs& a, u32 step, u64 gw, u32 cur, u32 prev, EdgeList here,
                                               EdgeList there, u32& next, EdgeList& next_list, Rand4 r) {
   if (here.deg == 0) return false;
@@ -86,7 +87,10 @@ __device__ __forceinline__ bool walk_step_n2v(const WalkArgs& a, u32 step, u64 g
     }
     next_list = edge_list(a, next);
     if (prev == kNoVertex || n2v_keep(__fmul_rn(u01(r.w), a.fmax), next == prev, a.inv_p, a.inv_q,
-                                      [&] { return connected(a.adjncy, there.off, there.off + there.deg, next, a.V); }))
+                                      [&] {
+                                        return HALVING ? connected_by_halving(a.adjncy, there.off, there.off + there.deg, next)
+                                                       : connected(a.adjncy, there.off, there.off + there.deg, next, a.V);
+                                      }))
       return true;
     if (++trial == kN2vMaxTrials) return true;  // keep the last proposal
     r = philox_tagged(a.seed, TAG_WALK, gw, step, trial);
@@ -301,6 +305,75 @@ __global__ void __launch_bounds__(kN2vCta) walk_n2v_kernel(const WalkArgs a) {
   add_edges(a.sum, edges);
 }
 
+// node2vec over the table with a step an iteration: a third of the instructions of a walker's step, and a warp waits for
+// the lane with the most rejections and the longest search.
+template <bool HALVING>
+__global__ void __launch_bounds__(kN2vCta) walk_n2v_steps_kernel(const WalkArgs a) {
+  const u64 T = (u64)gridDim.x * blockDim.x;
+  u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+  u64 edges = 0;
+  bool have = w < a.n;
+  u32 cur = 0, prev = kNoVertex, step = 0;
+  EdgeList here{0, 0}, there{0, 0};  // of the vertex stood on, and of the one before
+  u32* row = nullptr;
+  Rand4 r{0, 0, 0, 0};  // random words of the walker's current step
+  auto begin = [&]() {
+    cur = __ldg(a.starts + w);
+    row = a.paths + w * a.hop_num;
+    row[0] = cur;
+    prev = kNoVertex;
+    step = 0;
+    here = EdgeList{0, 0};
+    if (cur < a.V) here = edge_list(a, cur);
+    else dev_fail(a.err, DEV_ERR_INDEX, cur, 0, (u32)w);
+    r = philox_tagged(a.seed, TAG_WALK, a.walker_base + w * a.walker_stride, 0, 0);
+  };
+  if (have) begin();
+  while (have) {
+    u32 next = 0;
+    EdgeList next_list{0, 0};
+    const u64 gw = a.walker_base + w * a.walker_stride;
+    const Rand4 rn = philox_tagged(a.seed, TAG_WALK, gw, step + 1, 0);
+    if (step + 1 < a.hop_num && walk_step_n2v<HALVING>(a, step, gw, cur, prev, here, there, next, next_list, r)) {
+      ++step;
+      row[step] = next;
+      prev = cur;
+      cur = next;
+      there = here;
+      here = next_list;
+      r = rn;
+    } else {
+      a.lengths[w] = step;
+      edges += step;
+      w += T;
+      have = w < a.n;
+      if (have) begin();
+    }
+  }
+  add_edges(a.sum, edges);
+}
+
+// Which of them: an access an iteration where walkers wait for memory, a step an iteration where the warps wait for issue
+// slots, i.e. where more walkers run than the GPU holds at a time and their accesses are short or few; with the list halved
+// where several rounds of walkers follow one another over lists in cache.  An access / a step / a step and halving, us:
+//   lists in cache, many walkers       power law of 0.5 M edges, 300,000 x 40: 720 / 692 / 669; R-MAT 14 of 0.23 M, 1 M x 10: 578 / 411 / 354
+//   mostly dead ends, short lists      R-MAT 14 of 62,000 edges, 1,000 x 80: 197 / 156 / 175
+//   uniform draws, lists in cache      R-MAT 16 of 0.96 M edges, 100,000 x 40: 254 / 195 / 220; power law of 3.5 M, 70,000: 212 / 204 / 272
+//   walks of a few steps               R-MAT 20 of 16 M edges, 1 M x 10: 521 / 440 / 450; power law of 226 M, 3 M x 5: 1,289 / 981
+//   few vertices                       power law of 4,000 vertices, 111,000 edges, 100,000 x 40: 415 / 290
+//   some dead ends, lists in cache     R-MAT 14 to 18 of 0.2 to 4 M edges, 100,000 x 40: 285 to 303 / 226 to 245 / 235 to 274
+//   none of these                      power law of 11 M edges, 100,000 x 40: 301 / 314 / 397; 10,000 x 80: 367 / 524 / 738
+enum class N2vWay { kAccess, kStep, kStepHalving };
+static N2vWay n2v_way(const skw_ctx* ctx, const skw_walk_params* prm, u64 n, bool unbiased) {
+  const u64 sms = ctx->sm_count, V = ctx->V, ends = ctx->empty_lists;
+  const bool cached = ctx->E <= (unbiased ? 8u << 20 : 4u << 20);
+  if (cached && n > 1500 * sms) return N2vWay::kStepHalving;
+  if (ends * 2 > V && ctx->E < V * 8) return N2vWay::kStep;
+  const bool many = n > 600 * sms;
+  if (cached && n > 400 * sms && (unbiased || (ends * 5 > V * 2) || (many && ends * 5 > V))) return N2vWay::kStep;
+  return many && (V <= 8192 || (prm->hop_num <= 17 && n > 1000 * sms)) ? N2vWay::kStep : N2vWay::kAccess;
+}
+
 // Online mode: start of a run (row[0] = start, length = "alive").
 __global__ void __launch_bounds__(256) walk_online_init_kernel(const WalkArgs a) {
   for (u64 w = (u64)blockIdx.x * blockDim.x + threadIdx.x; w < a.n; w += (u64)gridDim.x * blockDim.x) {
@@ -324,7 +397,7 @@ __global__ void __launch_bounds__(256) walk_online_step_kernel(const WalkArgs a,
     if (APP == SKW_APP_NODE2VEC && cur < a.V) {
       const u32 prev = step ? row[step - 1] : kNoVertex;
       EdgeList next_list;
-      go = walk_step_n2v(a, step, gw, cur, prev, edge_list(a, cur), step ? edge_list(a, prev) : EdgeList{0, 0}, next,
+      go = walk_step_n2v<false>(a, step, gw, cur, prev, edge_list(a, cur), step ? edge_list(a, prev) : EdgeList{0, 0}, next,
                          next_list, r);
     } else {
       go = walk_step<APP>(a, step, gw, cur, next, r);
@@ -1065,9 +1138,15 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     switch (prm->app) {
       case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
       case SKW_APP_PPR: walk_offline_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
-      default:
-        walk_n2v_kernel<<<(unsigned)std::min<u64>((n + kN2vCta - 1) / kN2vCta, 0x7FFFFFFFull), kN2vCta, 0, st>>>(a);
+      default: {
+        const unsigned ctas = (unsigned)std::min<u64>((n + kN2vCta - 1) / kN2vCta, 0x7FFFFFFFull);
+        switch (n2v_way(ctx, prm, n, unbiased)) {
+          case N2vWay::kAccess: walk_n2v_kernel<<<ctas, kN2vCta, 0, st>>>(a); break;
+          case N2vWay::kStep: walk_n2v_steps_kernel<false><<<ctas, kN2vCta, 0, st>>>(a); break;
+          case N2vWay::kStepHalving: walk_n2v_steps_kernel<true><<<ctas, kN2vCta, 0, st>>>(a); break;
+        }
         break;
+      }
     }
     SKW_LAUNCHED(ctx);
   } else if (!build_tables) {

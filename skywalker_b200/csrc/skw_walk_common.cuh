@@ -94,6 +94,18 @@ __device__ __forceinline__ bool connected(const u32* __restrict__ adjncy, u32 lo
   return hit;
 }
 
+// The same by halving the list: more accesses, a third of the instructions of a round each.
+__device__ __forceinline__ bool connected_by_halving(const u32* __restrict__ adjncy, u32 lo, u32 hi, u32 dst) {
+  while (lo < hi) {
+    const u32 mid = lo + ((hi - lo) >> 1);
+    const u32 x = __ldg(adjncy + mid);
+    if (x == dst) return true;
+    if (x < dst) lo = mid + 1;
+    else hi = mid;
+  }
+  return false;
+}
+
 // Whether node2vec keeps a proposal: x = u * max(1/p, 1, 1/q) lies below f, where f is 1/p for the vertex
 // the walk came from, 1 for a neighbour of that vertex and 1/q for any other.  The list of that vertex is
 // searched (linked()) only when the answer depends on it: below both 1 and 1/q the proposal is kept, at

@@ -50,3 +50,41 @@ def test_node2vec_search_shapes(ctx, oracle, shift, p, q):
         paths, lens, _, edges = ctx.walk(starts, 31, app=APP_NODE2VEC, p=p, q=q, seed=5, mode=mode, flags=flags)
         assert np.array_equal(lens, want_len) and edges == int(want_len.sum())
         assert np.array_equal(paths[live], want[live])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [0, 3])
+@pytest.mark.parametrize("unbiased", [False, True])
+@pytest.mark.parametrize("V,share,n,hop", [
+    (3001, 1.0, 65, 31), (3001, 1.0, 95000, 31), (3001, 1.0, 222000, 11), (3001, 1.0, 222001, 11),
+    (9001, 1.0, 59201, 21), (9001, 1.0, 150000, 17), (9001, 1.0, 150000, 18),
+    (9001, 0.7, 88800, 30), (9001, 0.7, 88801, 30), (9001, 0.55, 59201, 20),      # dead ends
+    (9001, 0.3, 1, 31), (9001, 0.3, 3000, 31), (9001, 0.3, 3000, 1)])              # ... mostly, short lists
+def test_node2vec_kernels(ctx, oracle, shift, unbiased, V, share, n, hop):
+    """The node2vec kernels around the sizes that choose between them, with vertices without out-edges."""
+    import torch
+    x, a, w = _clustered_graph(V, 11)
+    deg = np.diff(x.astype(np.int64))
+    deg[np.random.default_rng(V).random(V) >= share] = 0
+    if share < 0.5:
+        deg = np.minimum(deg, 9)
+    a = np.concatenate([a[x[v]:x[v] + deg[v]] for v in range(V)])
+    w = np.concatenate([w[x[v]:x[v] + deg[v]] for v in range(V)])
+    x = np.concatenate([[0], np.cumsum(deg)]).astype(np.uint32)
+    E = len(a)
+    d_a = torch.zeros(E + 8, dtype=torch.int32, device="cuda")[shift:shift + E]   # borrowed, not on a sector boundary
+    d_a.copy_(torch.from_numpy(a.view(np.int32)))
+    d_x, d_w = torch.from_numpy(x.view(np.int32)).cuda(), torch.from_numpy(w).cuda()
+    torch.cuda.synchronize()
+    ctx.adopt_device(V, E, d_x, d_a, d_w)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, V, 3)
+    table = None if unbiased else oracle.alias_build(x, w)
+    want, want_len = oracle.walk(x, a, None if unbiased else w, table, starts, hop, app=APP_NODE2VEC, p=0.5, q=2.0, seed=5,
+                                 walker_base=9, unbiased=unbiased)
+    live = np.arange(hop)[None, :] <= want_len[:, None]
+    for mode in (MODE_OFFLINE, MODE_ONLINE):
+        paths, lens, _, edges = ctx.walk(starts, hop, app=APP_NODE2VEC, p=0.5, q=2.0, seed=5, walker_base=9, mode=mode,
+                                         flags=2 if unbiased else 0)
+        assert np.array_equal(lens, want_len) and edges == int(want_len.sum())
+        assert np.array_equal(paths[live], want[live])
