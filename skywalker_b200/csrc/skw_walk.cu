@@ -476,9 +476,10 @@ __global__ void __launch_bounds__(256) vertex_info_kernel(const u32* __restrict_
 // first of its 32 slots and goes by the marks from there.  A tile that spans more vertices (long runs of empty ones)
 // bisects the global array for every slot.  A neighbour's {offset, degree} is a random access; the one reached through the
 // alias mostly belongs to a slot of the same tile, whose thread has fetched it already.
-// Bound by the wavefronts of the L1 cache: a random access takes one, and so would every record if its thread's
-// records lay side by side (a warp's records side by side take a quarter), and by L2 traffic.  R-MAT 22, 65 M slots: 1.10 ms
-// with two random lookups a slot and every tile's vertices bisected from the whole offset array, 1.09 with eight
+// No unit is at its limit: 112.7 M slots in 1.38 ms are 4.15 TB/s of DRAM (63 % of a copy), the L1 pipe is busy 58 % (a
+// record a thread takes a wavefront where a warp's records side by side take a quarter), L2 46 %, and a warp waits for
+// global memory, shared memory and the barriers between the phases of a tile in about equal parts.  R-MAT 22, 65 M slots:
+// 1.10 ms with two random lookups a slot and every tile's vertices bisected from the whole offset array, 1.09 with eight
 // neighbouring slots a thread, 0.91 with a bisection per slot, 0.84 here; R-MAT 24, 457 M slots: 9.0 -> 7.5 ms.
 __device__ __forceinline__ u32 last_vertex_at_or_before(const u32* __restrict__ xadj, u32 lo, u32 hi, u32 e) {
   while (lo < hi) {  // last v in [lo, hi] with xadj[v] <= e
