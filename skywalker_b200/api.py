@@ -331,7 +331,7 @@ class Context:
     # -- k-hop
     @staticmethod
     def khop_layout(fanout):
-        return Context._khop_layout(tuple(operator.index(f) for f in fanout))
+        return Context._khop_layout(tuple(map(operator.index, fanout)))
 
     @staticmethod
     @functools.lru_cache(maxsize=64)
