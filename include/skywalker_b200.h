@@ -20,6 +20,10 @@
  *   - all randomness is Philox4x32-10, counter = (unit id low, unit id high, step, trial),
  *     key = 64-bit seed xor a per-purpose tag.  Results therefore do not depend on launch
  *     shape, on the number of GPUs, or on how units are split between calls.
+ *   - device memory that the library frees waits in the process for the next graph or context: at
+ *     most a sixteenth of a GPU's memory, out of reach of other allocators meanwhile.  It is returned
+ *     when an allocation of the library would fail without it, by skw_walk_records_free() and
+ *     skw_graph_free_weights(), and with the last context of the GPU.
  *   - there is no CPU fallback: without a CUDA device every compute entry point fails with
  *     SKW_ERR_CUDA.
  */
