@@ -736,8 +736,8 @@ def test_online_direct_slots_every_degree_class(ctx, oracle):
 
 
 def test_ppr_records_chunk_edges_and_long_rows(ctx, oracle, rmat12):
-    """The chunked PPR kernel: walker counts around its chunk size, paths longer than its staging
-    rows, and rows too long for it (hop_num > 65535 takes the lane-per-walker kernel)."""
+    """PPR over records in small batches (a lane a walker; tests/test_gpu_large_batches.py has the chunked
+    kernel's edges): long walks, and rows of more than 65535 cells."""
     g = rmat12
     _upload(ctx, g)
     ctx.alias_build_offline()
