@@ -187,7 +187,7 @@ def host_memory_available():
 
 
 def host_copy_bytes(V, E, online):
-    """Host bytes of the CPU checker's inputs: offsets, neighbours, and weights (online) or the
+    """Host bytes of the CPU oracle's inputs: offsets, neighbours, and weights (online) or the
     exported table (offline), plus staging."""
     return 4 * (V + 1) + 4 * E + (4 * E if online else 8 * E + V) + (1 << 30)
 
@@ -775,7 +775,7 @@ def main():
         parity = {"units": 0, "equal": None, "ranks": world, "skipped": "--no-parity"}
     elif at_once < 1:
         parity = {"units": 0, "equal": None, "ranks": world,
-                  "skipped": "host memory: %.1f GB free, the checker's inputs need %.1f GB" % ((avail or 0) / 1e9, need / 1e9)}
+                  "skipped": "host memory: %.1f GB free, the oracle's inputs need %.1f GB" % ((avail or 0) / 1e9, need / 1e9)}
     else:
         units, equal = 0, True
         for wave in range(0, world, at_once):
