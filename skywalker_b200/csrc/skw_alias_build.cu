@@ -39,6 +39,7 @@
 #include "skw_alias_f64.cuh"
 #include "skw_alias_long.cuh"
 #include "skw_alias_math.cuh"
+#include "skw_alias_wide.cuh"
 #include "skw_ctx.h"
 
 namespace skw {
@@ -46,14 +47,14 @@ namespace skw {
 // Degree classes.  Up to 4096 weights a list is one tile in the registers of NT threads, EPT weights each
 // (skw_alias_f64.cuh): one lane with 8 or 16; groups of 2 to 32 lanes and CTAs of 64 to 256 threads with 16.  What a
 // thread spends on scans, the division and its way into the merge (some 300 instructions) is shared by its weights,
-// so few threads with many weights beat many with few.  Longer lists are worked through in tiles: CTAs with the two
-// prefix lists in shared memory up to 16384, one CTA of 1024 threads with the lists in a global scratch slab, merged
-// through shared-memory windows, beyond.
+// so few threads with many weights beat many with few.  Up to 16384 a list is still one tile, of a CTA of 512 or 1024 threads
+// (skw_alias_wide.cuh).  Longer ones are worked through in tiles: one CTA of 1024 threads with the lists in a global scratch
+// slab, merged through shared-memory windows.
 enum { K_1A = 0, K_1B, K_2, K_4, K_8, K_16, K_32, K_C64, K_C128, K_C256, K_C2A, K_C2, K_H, K_CLASSES };
 constexpr u32 kListEpt = 16;
 constexpr u32 kGroupMax = 32 * kListEpt;      // 512: the longest list of a group of lanes
-constexpr u32 kMidSmemMax = 8192;             // two 512-thread CTAs per SM with 96 KB of lists each
-constexpr u32 kHugeSmemMax = 16384;           // one 1024-thread CTA per SM with 192 KB of lists; longer ones have them in global memory
+constexpr u32 kMidSmemMax = 512 * kWideEpt;   // 8192: two CTAs of 512 threads an SM, 84 KB of lists each
+constexpr u32 kHugeSmemMax = 1024 * kWideEpt;  // 16384: one of 1024 threads; longer lists are in global memory
 static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
 static_assert(2 * K_CLASSES <= 64, "class counters");
 
@@ -277,10 +278,45 @@ __global__ void __launch_bounds__(kListWarps * 32, kListCtas)
   }
 }
 
-// More than 4096 weights: one CTA per vertex, handed out by the class's cursor (degrees, hence costs, vary widely).
-// GLOBAL: lists in this CTA's slab of global scratch (cap + 2 entries of 12 bytes), else in shared memory.  A class of at
-// most `others` lists is left to build_cluster_kernel.
-template <int NT, int CAP, bool GLOBAL>
+// 4097 to 16384 weights: a CTA a list.
+template <u32 NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) build_wide_kernel(const u32* __restrict__ list, u32* __restrict__ cls, int k,
+                                                                   const __grid_constant__ ListBuild b) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ u32 s_next;
+  WideItems items{list, b.xadj, b.wgt, cls + K_CLASSES + k, cls[k], &s_next};
+  if (items.count == 0) return;
+  items.ask();
+  items.tell();
+  __syncthreads();
+  items.vertex();
+  if (!items.more) return;
+  items.offsets();
+  items.advance();
+  for (;;) {
+    items.ask();
+    const u32 n = items.end - items.off;
+    if (n > NT * kWideEpt || n == 0) {  // classification and kernel disagree: record and skip
+      if (threadIdx.x == 0) dev_fail(b.err, DEV_ERR_INTERNAL, items.v, n, NT);
+      __syncthreads();
+      items.tell();
+      __syncthreads();
+      items.vertex();
+      items.offsets();
+    } else {
+      build_list_wide<NT>(items.v, items.off, n, b.wgt + items.off, b.slots, b.valid, reinterpret_cast<WideShared<NT>*>(smem), b.err,
+                          items);
+    }
+    if (!items.more) return;
+    __syncthreads();  // the words are reused by the next list
+    items.advance();
+  }
+}
+
+// More than 16384 weights: one CTA per vertex, handed out by the class's cursor (degrees, hence costs, vary widely).
+// Its entries are in this CTA's slab of global scratch (cap + 2 of 12 bytes).  A class of at most `others` lists is left to
+// build_cluster_kernel.
+template <int NT, int CAP>
 __global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __restrict__ list, u32* __restrict__ cls, int k,
                                                                    const u32* __restrict__ xadj,
                                                                    const float* __restrict__ wgt, Slot* __restrict__ slots,
@@ -289,8 +325,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __
                                                                    u32 others, u32* __restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem[];
   LongShared<NT, CAP>* sh = reinterpret_cast<LongShared<NT, CAP>*>(smem);
-  u64* A = GLOBAL ? reinterpret_cast<u64*>(scratch + (u64)blockIdx.x * (cap + 2) * 12ull) : nullptr;
-  u32* P = GLOBAL ? reinterpret_cast<u32*>(A + cap + 2) : nullptr;
+  u64* A = reinterpret_cast<u64*>(scratch + (u64)blockIdx.x * (cap + 2) * 12ull);
+  u32* P = reinterpret_cast<u32*>(A + cap + 2);
   const u32 count = cls[k];
   if (count <= others) return;
   __shared__ u32 s_it;
@@ -306,7 +342,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __
       if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, (u32)cap);
       continue;
     }
-    build_list_long<NT, CAP, GLOBAL>(v, off, n, wgt + off, slots, valid, sh, A, P, err);
+    build_list_long<NT, CAP>(v, off, n, wgt + off, slots, valid, sh, A, P, err);
     __syncthreads();
   }
 }
@@ -536,9 +572,8 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   cudaStream_t st = ctx->stream;
   constexpr size_t kListSmem = kListWarps * kWarpBytes;
   static_assert(kListCtas * (kListSmem + 1024) <= 228 * 1024, "shared memory of an SM");
-  constexpr size_t kLongA = sizeof(LongShared<512, kMidSmemMax>), kLongB = sizeof(LongShared<1024, kHugeSmemMax>),
-                   kLongC = sizeof(LongShared<1024, 8192>);
-  static_assert(2 * (kLongA + 1024) <= 228 * 1024, "two CTAs an SM");
+  constexpr size_t kWideA = sizeof(WideShared<512>), kWideB = sizeof(WideShared<1024>), kLongSmem = sizeof(LongShared<1024, 8192>);
+  static_assert(2 * (kWideA + 1024) <= 228 * 1024, "two CTAs an SM");
   static_assert(3 * (sizeof(ClusterShared) + 1024) <= 228 * 1024, "three CTAs an SM");
   static bool attr_set[64] = {false};
   if (!attr_set[ctx->device & 63]) {
@@ -547,9 +582,9 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
     SMEM(kListSmem, build_lists_kernel<true>);
     SMEM(kListSmem, build_lists_kernel<false>);
     SMEM(sizeof(ClusterShared), build_cluster_kernel);
-    SMEM(kLongA, (build_long_kernel<512, kMidSmemMax, false>));
-    SMEM(kLongB, (build_long_kernel<1024, kHugeSmemMax, false>));
-    SMEM(kLongC, (build_long_kernel<1024, 8192, true>));
+    SMEM(kLongSmem, (build_long_kernel<1024, 8192>));
+    SMEM(kWideA, build_wide_kernel<512>);
+    SMEM(kWideB, build_wide_kernel<1024>);
 #undef SMEM
     attr_set[ctx->device & 63] = true;
   }
@@ -573,16 +608,19 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
                                                                                                   scratch, slab_elems);
     SKW_LAUNCHED(ctx);
   }
-#define LONG(MORE_THAN, KCLS, NT, CAP, GLOBAL, CTAS, BYTES, SCRATCH, MOST, OTHERS, STREAM)                                     \
-  if (ctx->max_degree > (MORE_THAN)) {                                                                                 \
-    build_long_kernel<NT, CAP, GLOBAL><<<CTAS, NT, BYTES, STREAM>>>(lists.list[KCLS], cls, KCLS, ctx->xadj,            \
-                                                                   ctx->adjwgt, slots, valid, SCRATCH, MOST, OTHERS, ctx->launch_err); \
-    SKW_LAUNCHED(ctx);                                                                                                 \
+  if (ctx->max_degree > kHugeSmemMax) {
+    build_long_kernel<1024, 8192><<<gmem_ctas, 1024, kLongSmem, s_h>>>(lists.list[K_H], cls, K_H, ctx->xadj, ctx->adjwgt, slots, valid,
+                                                                       scratch, slab_elems, clusters, ctx->launch_err);
+    SKW_LAUNCHED(ctx);
   }
-  LONG(kHugeSmemMax, K_H, 1024, 8192, true, gmem_ctas, kLongC, scratch, slab_elems, clusters, s_h)
-  LONG(kMidSmemMax, K_C2, 1024, kHugeSmemMax, false, ctx->sm_count, kLongB, nullptr, kHugeSmemMax, 0, s_a)
-  LONG(kF64Max, K_C2A, 512, kMidSmemMax, false, ctx->sm_count * 2, kLongA, nullptr, kMidSmemMax, 0, s_b)
-#undef LONG
+  if (ctx->max_degree > kMidSmemMax) {
+    build_wide_kernel<1024><<<ctx->sm_count, 1024, kWideB, s_a>>>(lists.list[K_C2], cls, K_C2, b);
+    SKW_LAUNCHED(ctx);
+  }
+  if (ctx->max_degree > kF64Max) {
+    build_wide_kernel<512><<<ctx->sm_count * 2, 512, kWideA, s_b>>>(lists.list[K_C2A], cls, K_C2A, b);
+    SKW_LAUNCHED(ctx);
+  }
   const unsigned grid = ctx->sm_count * kListCtas;
   if (streams) {
     // The lists of a CTA are dealt out beforehand, so one that starts late, behind a long list, ends late.  With 64 K edges

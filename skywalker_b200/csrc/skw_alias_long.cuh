@@ -5,8 +5,8 @@
 // where the sums are exact; what crosses a warp, masses and prefixes are 64-bit integers, since a prefix has up to 62
 // bits here.  The running weight of a thread is a double relative to its warp's base, and one addition to the base's
 // multiple of 2^32 rounds it as the conversion of the 64-bit sum would be rounded.
-// Bound by instruction issue and, in the merge, by the latency of shared memory: 6.8 to 8.5 warp instructions an edge at
-// 43 to 49 % of the issue slots.  R-MAT 22, 1,530 lists of 8,000 weights: 180 -> 161 us, 254 of 26,500: 367 -> 340 us.
+// Bound by instruction issue and, in the merge, by the latency of shared memory: 8.2 warp instructions an edge at 43 % of the
+// issue slots; 254 lists of 26,500 weights 340 us.
 #pragma once
 #include "skw_alias_f64.cuh"
 
@@ -111,8 +111,7 @@ __device__ __forceinline__ void merge_long(u32 t, u32 nl, u32 Sl, u32 A, u32 P, 
   }
 }
 
-// Shared memory of build_list_long: lists of CAP + 2 entries (or, for lists in global memory, one merge window of CAP),
-// then the tile's weights, transposed so that neither writing nor reading them meets the same bank twice.
+// Shared memory of build_list_long: a merge window of CAP entries, then the tile's weights, transposed so that neither writing nor reading them meets the same bank twice.
 template <int NT, int CAP>
 struct LongShared {
   u64 key[CAP + 2];
@@ -121,10 +120,10 @@ struct LongShared {
   LongWords<NT> words;
 };
 
-// GLOBAL: the lists (n + 2 entries) are in global memory at gA, gP and are merged through windows of CAP entries.
-template <int NT, int CAP, bool GLOBAL>
+// The lists (n + 2 entries) are in global memory at A, P and are merged through windows of CAP entries.
+template <int NT, int CAP>
 __device__ __forceinline__ void build_list_long(u32 v, u32 off, u32 n, const float* __restrict__ w, Slot* __restrict__ slots,
-                                                uint8_t* __restrict__ valid, LongShared<NT, CAP>* sh, u64* gA, u32* gP,
+                                                uint8_t* __restrict__ valid, LongShared<NT, CAP>* sh, u64* A, u32* P,
                                                 u32* err) {
   constexpr u32 NW = NT / 32, kTile = NT * 8;
   const u32 t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -183,8 +182,6 @@ __device__ __forceinline__ void build_list_long(u32 v, u32 off, u32 n, const flo
   // ---- lists
   u64 Qc = 0, Dc = 0;  // before the tile: quantised weight, deficit, smalls
   u32 Sc = 0;
-  u64* A = GLOBAL ? gA : sh->key;
-  u32* P = GLOBAL ? gP : sh->pos;
   for (u32 base = 0;; base += kTile) {
     const u32 here = min(kTile, n - base);
     const u32 ept = (here + NT - 1) / NT;
@@ -268,11 +265,11 @@ __device__ __forceinline__ void build_list_long(u32 v, u32 off, u32 n, const flo
       Dc += tile_d;
       inc = __shfl_sync(0xFFFFFFFFu, (u64)s_incl, 31);
     }
-    // Next entries of this thread in the two lists.  Lists in global memory are laid out in shared memory first (the
-    // tile's smalls from the front, its larges from the back) and copied out in order: a thread's entries alone would
-    // go out as scattered 8-byte stores.
-    static_assert(!GLOBAL || CAP >= (int)kTile, "the merge window doubles as the tile's staging area");
-    u32 is = GLOBAL ? s - Sc : s, il = GLOBAL ? here - 1 - (p0 - is) : n + 1 - (base + p0 - s);
+    // Next entries of this thread in the two lists.  They are laid out in shared memory first (the tile's smalls from the
+    // front, its larges from the back) and copied out in order: a thread's entries alone would go out as scattered 8-byte
+    // stores.
+    static_assert(CAP >= (int)kTile, "the merge window doubles as the tile's staging area");
+    u32 is = s - Sc, il = here - 1 - (p0 - is);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       if ((u32)k < cnt) {
@@ -288,16 +285,14 @@ __device__ __forceinline__ void build_list_long(u32 v, u32 off, u32 n, const flo
         il -= small ? 0u : 1u;
       }
     }
-    if constexpr (GLOBAL) {
-      __syncthreads();
-      const u32 ts = (u32)inc;  // smalls of this tile; the larges before it are base - Sc
-      for (u32 y = t; y < here; y += NT) {
-        const u64 to = y < ts ? (u64)Sc + y : (u64)n + 1 - (base - Sc) - (here - 1 - y);
-        A[to] = sh->key[y];
-        P[to] = sh->pos[y];
-      }
-      // (the next tile's entries are three barriers away)
+    __syncthreads();
+    const u32 ts = (u32)inc;  // smalls of this tile; the larges before it are base - Sc
+    for (u32 y = t; y < here; y += NT) {
+      const u64 to = y < ts ? (u64)Sc + y : (u64)n + 1 - (base - Sc) - (here - 1 - y);
+      A[to] = sh->key[y];
+      P[to] = sh->pos[y];
     }
+    // (the next tile's entries are three barriers away)
     Sc += (u32)inc;
     if (n - base <= kTile) break;
   }
@@ -316,44 +311,40 @@ __device__ __forceinline__ void build_list_long(u32 v, u32 off, u32 n, const flo
     return;
   }
   const u32 sA = (u32)__cvta_generic_to_shared(sh->key), sP = (u32)__cvta_generic_to_shared(sh->pos);
-  if constexpr (!GLOBAL) {
-    merge_long<NT>(t, n, S, sA, sP, C, B, slots + off);
-  } else {
-    // the merged order in windows of CAP: each window's slices of the two lists (and the entry after either) come into
-    // shared memory with coalesced copies
-    u32* bnd = reinterpret_cast<u32*>(sh->stage);  // smalls before the start of each window of a round
-    const u32 nwin = (n + CAP - 1) / CAP;
-    for (u32 w0 = 0; w0 < nwin; w0 += NT - 1) {  // a round of cnt windows needs cnt + 1 boundaries
-      const u32 cnt = min((u32)NT - 1, nwin - w0);
-      __syncthreads();
-      if (t <= cnt) {  // one bisection per window boundary, all in parallel
-        const u32 k0 = (u32)min((u64)(w0 + t) * CAP, (u64)n);
-        u32 lo = k0 > L ? k0 - L : 0, hi = min(k0, S);
-        while (lo < hi) {
-          const u32 mid = lo + ((hi - lo) >> 1);
-          const bool before = A[mid] <= A[n + 2 - k0 + mid];
-          lo = before ? mid + 1 : lo;
-          hi = before ? hi : mid;
-        }
-        bnd[t] = lo;
+  // the merged order in windows of CAP: each window's slices of the two lists (and the entry after either) come into
+  // shared memory with coalesced copies
+  u32* bnd = reinterpret_cast<u32*>(sh->stage);  // smalls before the start of each window of a round
+  const u32 nwin = (n + CAP - 1) / CAP;
+  for (u32 w0 = 0; w0 < nwin; w0 += NT - 1) {  // a round of cnt windows needs cnt + 1 boundaries
+    const u32 cnt = min((u32)NT - 1, nwin - w0);
+    __syncthreads();
+    if (t <= cnt) {  // one bisection per window boundary, all in parallel
+      const u32 k0 = (u32)min((u64)(w0 + t) * CAP, (u64)n);
+      u32 lo = k0 > L ? k0 - L : 0, hi = min(k0, S);
+      while (lo < hi) {
+        const u32 mid = lo + ((hi - lo) >> 1);
+        const bool before = A[mid] <= A[n + 2 - k0 + mid];
+        lo = before ? mid + 1 : lo;
+        hi = before ? hi : mid;
+      }
+      bnd[t] = lo;
+    }
+    __syncthreads();
+    for (u32 wi = 0; wi < cnt; ++wi) {
+      const u32 k0 = (w0 + wi) * (u32)CAP, k1 = (u32)min((u64)k0 + CAP, (u64)n);
+      const u32 i0 = bnd[wi], i1 = bnd[wi + 1], j0 = k0 - i0, j1 = k1 - i1;
+      const u32 Sl = i1 - i0, Ll = j1 - j0, nl = Sl + Ll;
+      for (u32 y = t; y <= Sl; y += NT) {
+        sh->key[y] = A[i0 + y];
+        sh->pos[y] = P[i0 + y];
+      }
+      for (u32 y = t; y <= Ll; y += NT) {  // large j0 + y
+        sh->key[nl + 1 - y] = A[n + 1 - j0 - y];
+        sh->pos[nl + 1 - y] = P[n + 1 - j0 - y];
       }
       __syncthreads();
-      for (u32 wi = 0; wi < cnt; ++wi) {
-        const u32 k0 = (w0 + wi) * (u32)CAP, k1 = (u32)min((u64)k0 + CAP, (u64)n);
-        const u32 i0 = bnd[wi], i1 = bnd[wi + 1], j0 = k0 - i0, j1 = k1 - i1;
-        const u32 Sl = i1 - i0, Ll = j1 - j0, nl = Sl + Ll;
-        for (u32 y = t; y <= Sl; y += NT) {
-          sh->key[y] = A[i0 + y];
-          sh->pos[y] = P[i0 + y];
-        }
-        for (u32 y = t; y <= Ll; y += NT) {  // large j0 + y
-          sh->key[nl + 1 - y] = A[n + 1 - j0 - y];
-          sh->pos[nl + 1 - y] = P[n + 1 - j0 - y];
-        }
-        __syncthreads();
-        merge_long<NT>(t, nl, Sl, sA, sP, C, B, slots + off);
-        __syncthreads();
-      }
+      merge_long<NT>(t, nl, Sl, sA, sP, C, B, slots + off);
+      __syncthreads();
     }
   }
   if (t == 0) valid[v] = 1;

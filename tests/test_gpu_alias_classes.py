@@ -129,3 +129,20 @@ def test_alias_list_of_many_windows(ctx, oracle, kind, others):
     """A list that takes more than one round of merge windows, alone (a cluster) and among others (one CTA)."""
     rng = np.random.default_rng(others)
     _check_lists(ctx, oracle, [_weights(kind, 20000, rng) for _ in range(others)] + [_weights(kind, 1024 * 8192 + 5, rng)])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["uniform", "one_heavy", "unusable"])
+def test_alias_many_lists_of_one_tile(ctx, oracle, kind):
+    """Lists of 4097 to 16384 weights, more of them than CTAs take at a time, around whole numbers of weights a thread; a
+    list without usable weights is the last, the first and one between."""
+    import torch
+    rng = np.random.default_rng(len(kind))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    edges = [4097, 4608, 4609, 5000, 7680, 7681, 8191, 8192, 8193, 9216, 9217, 12000, 15360, 15361, 16383, 16384]
+    sizes = edges + list(rng.integers(4097, 8193, 2 * sms)) + list(rng.integers(8193, 16385, sms))
+    rng.shuffle(sizes)
+    lists = [_weights(kind, n, rng) for n in sizes]
+    for i in (0, len(sizes) // 2, len(sizes) - 1):
+        lists[i] = np.zeros(sizes[i])
+    _check_lists(ctx, oracle, lists)
