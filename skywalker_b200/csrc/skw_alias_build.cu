@@ -25,8 +25,9 @@
 //
 // Work distribution: vertices are binned by degree with warp ballots and shared-memory prefix sums (classify_*
 // kernels), one work list per class.  Lists of up to 4096 weights are built in double precision by a lane, a group of
-// lanes, a warp or a CTA that holds the whole list in registers (skw_alias_f64.cuh); longer ones by CTAs that work
-// through it in tiles (skw_alias_long.cuh), a few giant ones by clusters of CTAs (skw_alias_cluster.cuh).
+// lanes, a warp or a CTA that holds the whole list in registers (skw_alias_f64.cuh), up to 16384 by a CTA alike
+// (skw_alias_wide.cuh); longer ones by CTAs that work
+// through it in tiles (skw_alias_long.cuh), the few giant ones by clusters of CTAs.
 #include <math_constants.h>
 
 #include <algorithm>
@@ -35,7 +36,6 @@
 #include <mutex>
 #include <type_traits>
 
-#include "skw_alias_cluster.cuh"
 #include "skw_alias_f64.cuh"
 #include "skw_alias_long.cuh"
 #include "skw_alias_math.cuh"
@@ -48,13 +48,13 @@ namespace skw {
 // (skw_alias_f64.cuh): one lane with 8 or 16; groups of 2 to 32 lanes and CTAs of 64 to 256 threads with 16.  What a
 // thread spends on scans, the division and its way into the merge (some 300 instructions) is shared by its weights,
 // so few threads with many weights beat many with few.  Up to 16384 a list is still one tile, of a CTA of 512 or 1024 threads
-// (skw_alias_wide.cuh).  Longer ones are worked through in tiles: one CTA of 1024 threads with the lists in a global scratch
-// slab, merged through shared-memory windows.
-enum { K_1A = 0, K_1B, K_2, K_4, K_8, K_16, K_32, K_C64, K_C128, K_C256, K_C2A, K_C2, K_H, K_CLASSES };
+// (skw_alias_wide.cuh).  Longer ones are worked through in tiles, with the entries in global scratch (skw_alias_long.cuh).
+enum { K_1A = 0, K_1B, K_2, K_4, K_8, K_16, K_32, K_C64, K_C128, K_C256, K_C2A, K_C2, K_H, K_G, K_CLASSES };
 constexpr u32 kListEpt = 16;
 constexpr u32 kGroupMax = 32 * kListEpt;      // 512: the longest list of a group of lanes
 constexpr u32 kMidSmemMax = 512 * kWideEpt;   // 8192: two CTAs of 512 threads an SM, 84 KB of lists each
 constexpr u32 kHugeSmemMax = 1024 * kWideEpt;  // 16384: one of 1024 threads; longer lists are in global memory
+constexpr u32 kAloneMax = 65536;              // longer ones are always built by clusters
 static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
 static_assert(2 * K_CLASSES <= 64, "class counters");
 
@@ -63,7 +63,7 @@ __device__ __forceinline__ int degree_class(u32 deg) {
   if (deg <= kF64Max) return deg <= kListEpt ? K_1B : K_1B + (32 - __clz((int)((deg - 1) / kListEpt)));
   if (deg <= kMidSmemMax) return K_C2A;
   if (deg <= kHugeSmemMax) return K_C2;
-  return K_H;
+  return deg <= kAloneMax ? K_H : K_G;
 }
 
 // The work list of every class: vertices of that class in no particular order, cls[k] of them; cls[K + k] is the
@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(256) classify_kernel(const u32* __restrict__ x
 
 // Vertices that class k can have at most, with E edges on V vertices.
 static u64 class_room(int k, u64 V, u64 E) {
-  static const u32 least[K_CLASSES] = {1, 9, 17, 33, 65, 129, 257, 513, 1025, 2049, kF64Max + 1, kMidSmemMax + 1, kHugeSmemMax + 1};
+  static const u32 least[K_CLASSES] = {1, 9, 17, 33, 65, 129, 257, 513, 1025, 2049, kF64Max + 1, kMidSmemMax + 1, kHugeSmemMax + 1,
+                                       kAloneMax + 1};
   return std::min<u64>(V, E / least[k]) + 1;
 }
 
@@ -304,7 +305,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) build_wide_kernel(const u32* __
       items.vertex();
       items.offsets();
     } else {
-      build_list_wide<NT>(items.v, items.off, n, b.wgt + items.off, b.slots, b.valid, reinterpret_cast<WideShared<NT>*>(smem), b.err,
+      u32 at = 0;
+      asm volatile("" : "+r"(at));
+      build_list_wide<NT>(items.v, items.off, n, b.wgt + items.off, b.slots, b.valid, reinterpret_cast<WideShared<NT>*>(smem + at), b.err,
                           items);
     }
     if (!items.more) return;
@@ -313,58 +316,48 @@ __global__ void __launch_bounds__(NT, 1024 / NT) build_wide_kernel(const u32* __
   }
 }
 
-// More than 16384 weights: one CTA per vertex, handed out by the class's cursor (degrees, hence costs, vary widely).
-// Its entries are in this CTA's slab of global scratch (cap + 2 of 12 bytes).  A class of at most `others` lists is left to
-// build_cluster_kernel.
-template <int NT, int CAP>
-__global__ void __launch_bounds__(NT, 1024 / NT) build_long_kernel(const u32* __restrict__ list, u32* __restrict__ cls, int k,
-                                                                   const u32* __restrict__ xadj,
-                                                                   const float* __restrict__ wgt, Slot* __restrict__ slots,
-                                                                   uint8_t* __restrict__ valid,
-                                                                   unsigned char* __restrict__ scratch, u64 cap,
-                                                                   u32 others, u32* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  LongShared<NT, CAP>* sh = reinterpret_cast<LongShared<NT, CAP>*>(smem);
-  u64* A = reinterpret_cast<u64*>(scratch + (u64)blockIdx.x * (cap + 2) * 12ull);
-  u32* P = reinterpret_cast<u32*>(A + cap + 2);
-  const u32 count = cls[k];
-  if (count <= others) return;
-  __shared__ u32 s_it;
-  for (;;) {
-    if (threadIdx.x == 0) s_it = atomicAdd(cls + K_CLASSES + k, 1u);
-    __syncthreads();
-    const u32 it = s_it;
-    __syncthreads();
-    if (it >= count) break;
-    const u32 v = list[it];
-    const u32 off = xadj[v], n = xadj[v + 1] - off;
-    if (n > cap) {
-      if (threadIdx.x == 0) dev_fail(err, DEV_ERR_CAPACITY, v, n, (u32)cap);
-      continue;
-    }
-    build_list_long<NT, CAP>(v, off, n, wgt + off, slots, valid, sh, A, P, err);
-    __syncthreads();
-  }
+// How many CTAs build a list of 16385 to 65536 weights together: as many as there are for each of `count` lists, three an SM.
+// Builds of so many lists of 20,000 / 50,000 weights, us, with one CTA of 1024 threads a list beyond 55 of them before:
+//   60 (fours)    72 / 142 -> 44 / 73; by eights, most of which have one list and some two, 55 / 81
+//   180 (pairs)   121 / 275 -> 71 / 176; by eights 129 / 235
+//   222 (pairs)   123 / 279 -> 77 / 186; by single CTAs 131 / 323
+//   300 (single)  173 / 416 -> 131 / 314
+__host__ __device__ __forceinline__ u32 long_team(u32 count, u32 ctas) {
+  u32 team = kLongTeam;
+  while (team > 1 && count > ctas / team) team /= 2;
+  return team;
 }
-
-// As many lists of class k as there are clusters, or fewer: one for each, with a slab of scratch of its own for up to cap
-// weights (cap even), 12 bytes each.
-__global__ void __launch_bounds__(kClusterThreads, 3) __cluster_dims__(kClusterCtas, 1, 1)
-    build_cluster_kernel(const u32* __restrict__ list, const u32* __restrict__ cls, int k, const __grid_constant__ ListBuild b,
-                         unsigned char* __restrict__ scratch, u64 cap) {
+// More than 16384 weights, by teams of CL CTAs: those of up to 65536 (class h) if they are for teams of this size, the longer
+// ones (class g) if there are eight.  Each team has a slab of scratch for up to cap weights (cap even), 12 bytes each.
+template <u32 CL>
+__global__ void __launch_bounds__(kLongThreads, 3) __cluster_dims__(CL, 1, 1)
+    build_long_kernel(const u32* __restrict__ list_g, const u32* __restrict__ list_h, u32* __restrict__ cls, int g, int h,
+                      const __grid_constant__ ListBuild b, unsigned char* __restrict__ scratch, u64 cap, u32 ctas) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const u32 rank = blockIdx.x % kClusterCtas, it = blockIdx.x / kClusterCtas, count = cls[k];
-  if (it >= count || count > gridDim.x / kClusterCtas) return;  // (the whole cluster)
-  const u32 v = list[it];
-  const u32 off = b.xadj[v], n = b.xadj[v + 1] - off;
-  if (n > cap || n == 0) {
-    if (rank == 0 && threadIdx.x == 0) dev_fail(b.err, DEV_ERR_CAPACITY, v, n, (u32)cap);
-    return;
+  __shared__ u32 s_it;
+  const u32 rank = blockIdx.x % CL, team = blockIdx.x / CL;
+  u64* A = reinterpret_cast<u64*>(scratch + team * cap * 12);
+  const u32 count_g = CL == kLongTeam ? cls[g] : 0u, count_h = long_team(cls[h], ctas) == CL ? cls[h] : 0u;
+  // Teams of several have a list each, or little more; single CTAs many, and they start when there is room.
+  for (u32 it = team;; it += gridDim.x / CL) {
+    if constexpr (CL == 1) {
+      if (count_h == 0) break;
+      if (threadIdx.x == 0) s_it = atomicAdd(cls + K_CLASSES + h, 1u);
+      __syncthreads();
+      it = s_it;
+      __syncthreads();
+    }
+    if (it >= count_g + count_h) break;
+    const u32 v = it < count_g ? list_g[it] : list_h[it - count_g];
+    const u32 off = b.xadj[v], n = b.xadj[v + 1] - off;
+    if (n > cap || n == 0) {
+      if (rank == 0 && threadIdx.x == 0) dev_fail(b.err, DEV_ERR_CAPACITY, v, n, (u32)cap);
+    } else {
+      build_list_long<CL>(rank, v, off, n, b.wgt + off, b.slots, b.valid, reinterpret_cast<LongShared*>(smem), A,
+                          reinterpret_cast<u32*>(A + cap), b.err);
+    }
+    cluster_sync<CL>();  // the CTAs read one another's shared memory
   }
-  u64* A = reinterpret_cast<u64*>(scratch + it * cap * 12);
-  build_list_cluster(rank, v, off, n, b.wgt + off, b.slots, b.valid, reinterpret_cast<ClusterShared*>(smem), A,
-                     reinterpret_cast<u32*>(A + cap), b.err);
-  cluster_sync();  // the CTAs read one another's shared memory
 }
 
 // ------------------------------------------------------------------ one CTA per vertex -----
@@ -553,44 +546,53 @@ int builders_queued(skw_ctx* ctx) {
   return SKW_OK;
 }
 
-// Scratch of the lists beyond 16384 weights: one slab a CTA, sized by the largest degree; fewer CTAs when a giant hub
-// would make the slabs exceed 4 GB in total.
-static uint64_t scratch_slab(const skw_ctx* ctx) {
-  return ctx->max_degree > kHugeSmemMax ? ((uint64_t)ctx->max_degree + 1) & ~1ull : 0;
-}
-static uint64_t scratch_slab_bytes(const skw_ctx* ctx) { return (scratch_slab(ctx) + 2) * 12ull; }
-static int scratch_slabs(const skw_ctx* ctx) {
-  return (int)std::min<uint64_t>(ctx->sm_count, std::max<uint64_t>((4ull << 30) / scratch_slab_bytes(ctx), 8));
+// Scratch of the lists beyond 16384 weights: a slab with room for the longest for each team of eight, fewer of them when a
+// giant hub would make the slabs exceed 4 GB in total; then, if smaller teams may be used, as much as the smallest need.
+struct LongScratch {
+  uint64_t cap = 0, cap_small = 0;  // entries of 12 bytes
+  unsigned teams = 0, small = 0;
+  uint64_t bytes() const { return (cap * teams + cap_small * small) * 12; }
+};
+static LongScratch long_scratch(const skw_ctx* ctx) {
+  LongScratch s;
+  if (ctx->max_degree > kHugeSmemMax) {
+    s.cap = ((uint64_t)ctx->max_degree + 1) & ~1ull;
+    s.teams = (unsigned)std::min<uint64_t>(ctx->sm_count * 3 / kLongTeam, std::max<uint64_t>((4ull << 30) / (s.cap * 12), 8));
+    s.cap_small = std::min<uint64_t>(s.cap, kAloneMax);
+    s.small = long_team(ctx->long_lists, ctx->sm_count * 3) < kLongTeam ? ctx->sm_count * 3 : 0;
+  }
+  return s;
 }
 static int reserve_scratch(skw_ctx* ctx) {
-  if (!scratch_slab(ctx)) return SKW_OK;
-  return ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, scratch_slab_bytes(ctx) * scratch_slabs(ctx));
+  const uint64_t bytes = long_scratch(ctx).bytes();
+  return bytes ? ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, bytes) : SKW_OK;
 }
 
-// Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`.
-static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot* slots, uint8_t* valid) {
+// Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`; whole: all vertices of the
+// graph are in them.
+static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot* slots, uint8_t* valid, bool whole) {
   cudaStream_t st = ctx->stream;
   constexpr size_t kListSmem = kListWarps * kWarpBytes;
   static_assert(kListCtas * (kListSmem + 1024) <= 228 * 1024, "shared memory of an SM");
-  constexpr size_t kWideA = sizeof(WideShared<512>), kWideB = sizeof(WideShared<1024>), kLongSmem = sizeof(LongShared<1024, 8192>);
+  constexpr size_t kWideA = sizeof(WideShared<512>), kWideB = sizeof(WideShared<1024>);
   static_assert(2 * (kWideA + 1024) <= 228 * 1024, "two CTAs an SM");
-  static_assert(3 * (sizeof(ClusterShared) + 1024) <= 228 * 1024, "three CTAs an SM");
+  static_assert(3 * (sizeof(LongShared) + 1024) <= 228 * 1024, "three CTAs an SM");
   static bool attr_set[64] = {false};
   if (!attr_set[ctx->device & 63]) {
 #define SMEM(BYTES, ...) \
   SKW_CUDA(ctx, cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)))
     SMEM(kListSmem, build_lists_kernel<true>);
     SMEM(kListSmem, build_lists_kernel<false>);
-    SMEM(sizeof(ClusterShared), build_cluster_kernel);
-    SMEM(kLongSmem, (build_long_kernel<1024, 8192>));
+    SMEM(sizeof(LongShared), build_long_kernel<8>);
+    SMEM(sizeof(LongShared), build_long_kernel<4>);
+    SMEM(sizeof(LongShared), build_long_kernel<2>);
+    SMEM(sizeof(LongShared), build_long_kernel<1>);
     SMEM(kWideA, build_wide_kernel<512>);
     SMEM(kWideB, build_wide_kernel<1024>);
 #undef SMEM
     attr_set[ctx->device & 63] = true;
   }
   if (const int rc = reserve_scratch(ctx); rc != SKW_OK) return rc;
-  const uint64_t slab_elems = scratch_slab(ctx);
-  const int gmem_ctas = scratch_slabs(ctx);
   // The classes are independent.  The long lists take few CTAs for long, so their kernels start first, on streams of their
   // own, and the many short ones fill in on the caller's.
   const int streams = ctx->max_degree > kHugeSmemMax ? 5 : ctx->max_degree > kMidSmemMax ? 3 : ctx->max_degree > kF64Max ? 2
@@ -599,19 +601,30 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   if (streams) SKW_CUDA(ctx, cudaEventRecord(ctx->bfork, st));
   for (int i = 0; i < streams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
   const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->launch_err};
-  // The lists beyond 16384 weights: one of these two kernels finds that they are its own, by their number, and both use the
-  // same scratch.  On streams of their own: behind the other, the one with the work would start after everybody else.
-  unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
-  const unsigned clusters = slab_elems ? std::min<unsigned>(ctx->sm_count * 3 / kClusterCtas, gmem_ctas) : 0;
-  if (clusters) {
-    build_cluster_kernel<<<clusters * kClusterCtas, kClusterThreads, sizeof(ClusterShared), ctx->bstream[4]>>>(lists.list[K_H], cls, K_H, b,
-                                                                                                  scratch, slab_elems);
-    SKW_LAUNCHED(ctx);
-  }
   if (ctx->max_degree > kHugeSmemMax) {
-    build_long_kernel<1024, 8192><<<gmem_ctas, 1024, kLongSmem, s_h>>>(lists.list[K_H], cls, K_H, ctx->xadj, ctx->adjwgt, slots, valid,
-                                                                       scratch, slab_elems, clusters, ctx->launch_err);
-    SKW_LAUNCHED(ctx);
+    // The size of the teams follows from the number of lists, which for all vertices is known here; for others it is at most
+    // that, and the kernels of teams that are not the ones find so.
+    const LongScratch sc = long_scratch(ctx);
+    const u32 ctas = ctx->sm_count * 3, team = long_team(ctx->long_lists, ctas);
+    unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
+    unsigned char* small = scratch + sc.cap * sc.teams * 12;
+#define LONG(CL, CTAS, SCRATCH, CAP, STREAM)                                                                                    \
+  build_long_kernel<CL><<<CTAS, kLongThreads, sizeof(LongShared), STREAM>>>(lists.list[K_G], lists.list[K_H], cls, K_G, K_H, b, \
+                                                                            SCRATCH, CAP, ctas);                                \
+  SKW_LAUNCHED(ctx)
+    if (!whole || team == kLongTeam || ctx->max_degree > kAloneMax) {
+      LONG(8, sc.teams * 8, scratch, sc.cap, ctx->bstream[4]);
+    }
+    if (team == 4 || (!whole && team < 4)) {
+      LONG(4, ctas / 4 * 4, small, sc.cap_small, s_h);
+    }
+    if (team == 2 || (!whole && team < 2)) {
+      LONG(2, ctas / 2 * 2, small, sc.cap_small, s_h);
+    }
+    if (team == 1) {
+      LONG(1, ctas, small, sc.cap_small, s_h);
+    }
+#undef LONG
   }
   if (ctx->max_degree > kMidSmemMax) {
     build_wide_kernel<1024><<<ctx->sm_count, 1024, kWideB, s_a>>>(lists.list[K_C2], cls, K_C2, b);
@@ -738,7 +751,7 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
                                                   ctx->xadj, ctx->V, ctx->stamp, ctx->stamp_round,
                                                   ctx->frontier_cls, lists, cap, ctx->launch_err);
     SKW_LAUNCHED(ctx);
-    rc = launch_builders(ctx, lists, ctx->frontier_cls, ctx->slots, ctx->valid);
+    rc = launch_builders(ctx, lists, ctx->frontier_cls, ctx->slots, ctx->valid, false);
     if (rc != SKW_OK) return rc;
   }
   return SKW_OK;
@@ -801,7 +814,7 @@ int enqueue_tables(skw_ctx* ctx, u32 v_begin, u32 v_end, Slot* slots, uint8_t* v
   classify_kernel<<<(unsigned)std::min<u64>(tiles, (u64)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
       ctx->xadj, v_begin, v_end, ctx->cls_counts, lists, valid);
   SKW_LAUNCHED(ctx);
-  return launch_builders(ctx, lists, ctx->cls_counts, slots, valid);
+  return launch_builders(ctx, lists, ctx->cls_counts, slots, valid, v_begin == 0 && v_end == ctx->V);
 }
 }  // namespace skw
 

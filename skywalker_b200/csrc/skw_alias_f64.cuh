@@ -25,6 +25,7 @@ constexpr double kTwo52 = 4503599627370496.0;  // 2^52
 constexpr double kBucket = 1099511627776.0;    // 2^40, the bucket of every list of up to 2^22 weights
 constexpr u32 kBiasHi = 0x43300000u;           // high word of 2^52
 
+__device__ __forceinline__ double u32_to_double(u32 x) { return __dsub_rn(__hiloint2double((int)kBiasHi, (int)x), kTwo52); }
 __device__ __forceinline__ uint2 list_entry(double key, u32 pos) {
   return make_uint2((u32)__double2loint(key), (u32)__double2hiint(key) + ((pos << 20) - kBiasHi));
 }

@@ -19,12 +19,30 @@
 // to 290 / 262 to 269.
 #pragma once
 #include "skw_alias_f64.cuh"
-#include "skw_alias_long.cuh"
 
 namespace skw {
 
 constexpr u32 kWideEpt = 16;
 constexpr double kTwo53 = 2.0 * kTwo52;
+
+// Cross-thread words of a CTA of NT threads.
+template <int NT>
+struct WideWords {
+  static constexpr int NW = NT / 32;
+  u64 q[NW], d[NW];
+  u32 s[NW];
+};
+
+__device__ __forceinline__ u64 warp_scan_u64(u64 v, u32 lane, u64& total) {
+  u64 inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u64 x = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+    if (lane >= (u32)o) inc += x;
+  }
+  total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+  return inc - v;
+}
 
 // Shared memory of a CTA: the staged weights, then the two lists.
 template <u32 NT>
@@ -37,7 +55,7 @@ struct WideShared {
     };
     int stage[kMost + NT];  // an even number a thread is spread by one word a thread
   };
-  LongWords<(int)NT> words;
+  WideWords<(int)NT> words;
   u64 first_q[NT / 32], total;  // running weight before each warp, and of the list
   u32 top[2][NT / 32];
 };
@@ -175,7 +193,7 @@ __device__ __forceinline__ void build_list_wide(u32 v, u32 off, u32 n, const flo
   constexpr bool kBig = NT * kWideEpt > 8192;
   const u32 t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const GroupCoop<32> wc;
-  LongWords<(int)NT>& words = sh->words;
+  WideWords<(int)NT>& words = sh->words;
   const u32 ept = (n + NT - 1) / NT;
   const u32 p0 = min(t * ept, n), cnt = min(ept, n - p0);
   const u32 over = min((ept + CH - 1) / CH * CH, (u32)EPT) - cnt;

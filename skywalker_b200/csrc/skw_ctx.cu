@@ -257,17 +257,19 @@ static void free_graph(skw_ctx* ctx) {
   ctx->E = 0;
   ctx->max_degree = 0;
   ctx->empty_lists = 0;
+  ctx->long_lists = 0;
 }
 
-// out[0]: the largest degree, out[1]: the number of vertices of degree 0
+// out[0]: the largest degree, out[1]: the number of vertices of degree 0, longs: of those of degree 16385 to 65536
 __global__ void max_degree_kernel(const uint32_t* __restrict__ xadj, uint32_t V,
-                                  uint32_t* __restrict__ out) {
+                                  uint32_t* __restrict__ out, uint32_t* __restrict__ longs) {
   uint32_t m = 0, empty = 0;
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < V;
        v += (size_t)gridDim.x * blockDim.x) {
     const uint32_t d = xadj[v + 1] - xadj[v];
     m = max(m, d);
     empty += d == 0 ? 1u : 0u;
+    if (d > 16384u && d <= 65536u) atomicAdd(longs, 1u);  // (rare)
   }
   for (int o = 16; o; o >>= 1) {
     m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
@@ -414,15 +416,18 @@ static int xadj_fingerprint(skw_ctx* ctx, uint64_t* out) {
 
 int finish_graph(skw_ctx* ctx) {
   SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum, 0, sizeof(uint64_t), ctx->stream));
+  SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum + 2, 0, sizeof(uint64_t), ctx->stream));
   if (ctx->V) {
     max_degree_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(
-        ctx->xadj, ctx->V, reinterpret_cast<uint32_t*>(ctx->d_sum));
+        ctx->xadj, ctx->V, reinterpret_cast<uint32_t*>(ctx->d_sum), reinterpret_cast<uint32_t*>(ctx->d_sum + 2));
     SKW_LAUNCHED(ctx);
   }
   SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum, ctx->d_sum, sizeof(uint64_t), cudaMemcpyDeviceToHost,
                                 ctx->stream));
+  SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum + 2, ctx->d_sum + 2, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->max_degree = (uint32_t)*ctx->h_sum;
+  ctx->long_lists = (uint32_t)ctx->h_sum[2];
   ctx->empty_lists = (uint32_t)(*ctx->h_sum >> 32);
   ctx->status_clean = false;
   return SKW_OK;

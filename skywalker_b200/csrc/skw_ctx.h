@@ -49,6 +49,7 @@ struct skw_ctx {
   uint64_t E = 0;
   uint32_t max_degree = 0;
   uint32_t empty_lists = 0;  // vertices without out-edges
+  uint32_t long_lists = 0;   // vertices of degree 16385 to 65536
   uint32_t* xadj = nullptr;
   uint32_t* adjncy = nullptr;
   float* adjwgt = nullptr;

@@ -146,3 +146,24 @@ def test_alias_many_lists_of_one_tile(ctx, oracle, kind):
     for i in (0, len(sizes) // 2, len(sizes) - 1):
         lists[i] = np.zeros(sizes[i])
     _check_lists(ctx, oracle, lists)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["uniform", "one_heavy"])
+@pytest.mark.parametrize("quarters", [1, 2])
+@pytest.mark.parametrize("more", [0, 1])
+def test_alias_teams_of_long_lists(ctx, oracle, kind, quarters, more):
+    """Lists of 16385 to 65536 weights by fours, pairs and single CTAs, at the counts where the teams change, next to longer
+    ones; all vertices at once, and in two ranges, whose kernels find the number of lists for themselves."""
+    import torch
+    rng = np.random.default_rng(quarters)
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count * 3
+    sizes = [16385 + (i * 977) % 3000 for i in range(ctas * quarters // 4 + more - 2)] + [65535, 65536] + [65537, 100001]
+    lists = [_weights(kind, n, rng) for n in sizes]
+    lists[len(lists) // 2] = np.zeros(sizes[len(lists) // 2])
+    _check_lists(ctx, oracle, lists)
+    whole = ctx.alias_export()
+    cut = len(lists) // 3
+    ctx.alias_build_offline(0, cut)
+    ctx.alias_build_offline(cut, len(lists))
+    assert all(np.array_equal(a, b) for a, b in zip(whole, ctx.alias_export()))
