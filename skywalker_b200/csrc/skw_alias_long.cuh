@@ -2,7 +2,7 @@
 // which share it out in chunks: two passes for the largest weight and the total, one in tiles of up to 4096 weights that
 // writes the two lists to global memory, and the merge in windows of up to 4096 entries.
 // Bound by the latencies of its phases: 221 warp instructions per 32 edges by single CTAs, three an SM, at 41 % of the issue
-// slots (297 by clusters of eight).  A CTA alone is the whole latency of a list, 0.13 ms for 20,000 weights and 0.5 for 92,000,
+// slots (some 300 by clusters of eight).  A CTA alone is the whole latency of a list, 0.13 ms for 20,000 weights and 0.5 for 92,000,
 // so there is a cluster for each while lists are few (long_team).  16.7 M edges in lists of one length, by one CTA of 1024
 // threads and tiles of eight weights a thread before: 16,385 weights 338 -> 265 us, 19,900 341 -> 253, 24,300 330 -> 264,
 // 33,000 370 -> 326, 100,000 515 -> 410.

@@ -439,8 +439,8 @@ __device__ __forceinline__ void load_record(const WalkRecord* p, u32 (&w)[8]) {
                : "l"(p));
 }
 
-constexpr u32 kRecTile = 2048, kRecSpan = 2048;  // slots of a tile of the records build, offsets it keeps at hand
-constexpr u32 kRecCta = kRecTile / 8;
+constexpr u32 kRecTile = 1024, kRecSpan = 1024;  // slots of a tile of the records build, offsets it keeps at hand
+constexpr u32 kRecPer = 4, kRecCta = kRecTile / kRecPer;  // slots a thread
 
 // vinfo[v] = {first-edge offset, usable degree}; vbits = one bit per vertex, set when the usable
 // degree is not zero.  The bitmap is V/8 bytes and stays in L2, so a walker that starts on a dead
@@ -476,11 +476,13 @@ __global__ void __launch_bounds__(256) vertex_info_kernel(const u32* __restrict_
 // first of its 32 slots and goes by the marks from there.  A tile that spans more vertices (long runs of empty ones)
 // bisects the global array for every slot.  A neighbour's {offset, degree} is a random access; the one reached through the
 // alias mostly belongs to a slot of the same tile, whose thread has fetched it already.
-// No unit is at its limit: 112.7 M slots in 1.38 ms are 4.15 TB/s of DRAM (63 % of a copy), the L1 pipe is busy 58 % (a
-// record a thread takes a wavefront where a warp's records side by side take a quarter), L2 46 %, and a warp waits for
-// global memory, shared memory and the barriers between the phases of a tile in about equal parts.  R-MAT 22, 65 M slots:
-// 1.10 ms with two random lookups a slot and every tile's vertices bisected from the whole offset array, 1.09 with eight
-// neighbouring slots a thread, 0.91 with a bisection per slot, 0.84 here; R-MAT 24, 457 M slots: 9.0 -> 7.5 ms.
+// Bound by the pipe of L1 and shared memory (a random lookup a slot, and a record a thread takes a wavefront where a warp's
+// records side by side take a quarter) and by waiting in the phases of a tile, so four slots a thread in 38 registers and 48
+// warps an SM beat eight in 60 and 32: R-MAT 22, 65 M slots 845 -> 754 us, R-MAT 24, 457 M slots 7.49 -> 6.67 ms (4.1 ->
+// 4.6 TB/s of DRAM).  Before: 1.10 ms with two random lookups a slot and every tile's vertices bisected from the whole offset
+// array, 0.91 with a bisection per slot.  Two slots a thread and 64 warps: 755 us / 6.64 ms.  Slower: two 16-byte stores a
+// record 834, halves exchanged between neighbours so that 16 records fill a store 919, records laid out in shared memory and
+// copied out by the bulk engine, a tile or 32 at a time, 1569 and 1680; the next tile fetched to L2 ahead 884.
 __device__ __forceinline__ u32 last_vertex_at_or_before(const u32* __restrict__ xadj, u32 lo, u32 hi, u32 e) {
   while (lo < hi) {  // last v in [lo, hi] with xadj[v] <= e
     const u32 mid = lo + ((hi - lo + 1) >> 1);
@@ -489,7 +491,7 @@ __device__ __forceinline__ u32 last_vertex_at_or_before(const u32* __restrict__ 
   }
   return lo;
 }
-__global__ void __launch_bounds__(kRecCta, 1024 / kRecCta) walk_records_kernel(const u32* __restrict__ xadj,
+__global__ void __launch_bounds__(kRecCta, 6) walk_records_kernel(const u32* __restrict__ xadj,
                                                               const u32* __restrict__ adjncy,
                                                               const Slot* __restrict__ slots,
                                                               const uint2* __restrict__ vinfo,
@@ -504,16 +506,17 @@ __global__ void __launch_bounds__(kRecCta, 1024 / kRecCta) walk_records_kernel(c
     const u64 e0 = tile * kRecTile;
     const u32 here = (u32)min((u64)kRecTile, E - e0);
     const u32 v0 = __ldg(tile_first + tile), v1 = tile + 1 < tiles ? __ldg(tile_first + tile + 1) : V - 1;
-    u32 nbr[8];
-    Slot sl[8];
+    u32 nbr[kRecPer];
+    Slot sl[kRecPer];
 #pragma unroll
-    for (u32 k = 0; k < 8; ++k) {  // (past the end: the last slot again)
+    for (u32 k = 0; k < kRecPer; ++k) {  // (past the end: the last slot again)
       const u32 e = (u32)e0 + min(threadIdx.x + kRecCta * k, here - 1);
       sl[k] = load_slot(slots + e);
       nbr[k] = __ldg(adjncy + e);
     }
     const bool staged = v1 - v0 < kRecSpan;
-    *reinterpret_cast<uint4*>(s_head + threadIdx.x * 8) = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint2*>(s_head + threadIdx.x * kRecPer) = make_uint2(0u, 0u);
+    static_assert(kRecPer == 4, "four half-words a thread are cleared");
     __syncthreads();
     if (staged) {
       for (u32 i = threadIdx.x; i <= v1 - v0 + 1; i += kRecCta) {
@@ -522,23 +525,23 @@ __global__ void __launch_bounds__(kRecCta, 1024 / kRecCta) walk_records_kernel(c
         if (i <= v1 - v0 && x - (u32)e0 < here && __ldg(xadj + v0 + i + 1) != x) s_head[x - (u32)e0] = (uint16_t)(i + 1);
       }
     }
-    uint2 info[8];
+    uint2 info[kRecPer];
 #pragma unroll
-    for (u32 k = 0; k < 8; ++k) {
+    for (u32 k = 0; k < kRecPer; ++k) {
       info[k] = make_uint2(0u, 0u);
       if (nbr[k] < V) info[k] = __ldg(vinfo + nbr[k]);
       else dev_fail(err, DEV_ERR_INDEX, (u32)e0 + min(threadIdx.x + kRecCta * k, here - 1), nbr[k], 22);
     }
 #pragma unroll
-    for (u32 k = 0; k < 8; ++k) {
+    for (u32 k = 0; k < kRecPer; ++k) {
       s_nbr[threadIdx.x + kRecCta * k] = nbr[k];
       s_info[threadIdx.x + kRecCta * k] = info[k];
     }
     __syncthreads();
-    // the vertex (relative to v0) of the first slot of each of the warp's eight runs of 32, by one lane each
+    // the vertex (relative to v0) of the first slot of each of the warp's runs of 32, by one lane each
     const u32 lane = threadIdx.x & 31;
     u32 first = 0;
-    if (staged && lane < 8) {
+    if (staged && lane < kRecPer) {
       const u32 e = (u32)e0 + min(threadIdx.x - lane + kRecCta * lane, here - 1);
       for (u32 hi = v1 - v0; first < hi;) {
         const u32 mid = (first + hi + 1) >> 1;
@@ -547,7 +550,7 @@ __global__ void __launch_bounds__(kRecCta, 1024 / kRecCta) walk_records_kernel(c
       }
     }
 #pragma unroll
-    for (u32 k = 0; k < 8; ++k) {
+    for (u32 k = 0; k < kRecPer; ++k) {
       const u32 i = threadIdx.x + kRecCta * k;
       u32 v = __shfl_sync(0xFFFFFFFFu, first, k);
       const u32 head = s_head[i];
