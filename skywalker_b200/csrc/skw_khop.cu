@@ -144,7 +144,7 @@ __device__ __forceinline__ void khop_add(unsigned long long* sum, u64 mine) {
 // 159 us, the parents being in cache and the cell numbers 32-bit.  A
 // hop's parents were written by this CTA, so they are read with plain loads.
 template <bool DISTINCT>
-__global__ void __launch_bounds__(256) khop_tree_kernel(const KhopArgs a, u32 per_cta) {
+__device__ __forceinline__ void khop_trees(const KhopArgs& a, u32 per_cta) {
   __shared__ u32 s_seen[DISTINCT ? 8 : 1][DISTINCT ? kDistinctMaxFanout : 1];
   const u64 s0 = (u64)blockIdx.x * per_cta;
   const u32 ns = (u32)min((u64)per_cta, a.n - s0);
@@ -182,14 +182,30 @@ __global__ void __launch_bounds__(256) khop_tree_kernel(const KhopArgs a, u32 pe
   khop_add(a.sum, got_sum);
 }
 
-// One hop of every tree (online mode, whose tables are built hop by hop, and trees that are too large for a CTA).
+// A draw is a chain of dependent random accesses (parent, offsets, slot, neighbour), so the kernels that follow tables have as
+// many warps an SM as fit, 64 with 32 registers each: 65,536 x 25, 10 with the take-all rule 165 -> 153 us, with replacement 202
+// -> 195, 16,384 x 15, 10, 5 on a power-law graph 324 -> 291.  Uniform draws have an access less and are bound by the rate of
+// random accesses, and draws of distinct neighbours by their instructions: 152 -> 157 and 340 -> 356 us, so they keep 40
+// registers and 48 warps.
+template <bool DISTINCT>
+__global__ void __launch_bounds__(256) khop_tree_kernel(const KhopArgs a, u32 per_cta) {
+  khop_trees<DISTINCT>(a, per_cta);
+}
+__global__ void __launch_bounds__(256, 8) khop_weighted_tree_kernel(const KhopArgs a, u32 per_cta) {
+  khop_trees<false>(a, per_cta);
+}
+
+// One hop of every tree (online mode, whose tables are built hop by hop, and trees that are too large for a CTA).  64 warps an SM,
+// as above: hop 2 of 65,536 x 25, 10 (16.4 M cells, 9 M draws) waited for memory 18 of every 25 cycles with 40 warps; the
+// whole batch 672 -> 640 us, by distinct draws 834 -> 813.  (A warp that takes 32 parents, reads their offsets once and deals
+// out the children of those that have any: 677.)
 __global__ void __launch_bounds__(256) khop_init_kernel(const u32* __restrict__ seeds, u64 n,
                                                         u32 cells, u32* __restrict__ data) {
   for (u64 s = (u64)blockIdx.x * blockDim.x + threadIdx.x; s < n; s += (u64)gridDim.x * blockDim.x)
     data[s * cells] = seeds[s];
 }
 
-__global__ void __launch_bounds__(256) khop_hop_kernel(const KhopArgs a, u32 h) {
+__global__ void __launch_bounds__(256, 8) khop_hop_kernel(const KhopArgs a, u32 h) {
   const u32 per_seed = a.width[h + 1], f = a.fanout[h];
   const u64 total = a.n * per_seed, T = (u64)gridDim.x * blockDim.x;
   u64 got_sum = 0;
@@ -215,7 +231,7 @@ __global__ void __launch_bounds__(256) khop_hop_kernel(const KhopArgs a, u32 h) 
   khop_add(a.sum, got_sum);
 }
 
-__global__ void __launch_bounds__(256) khop_distinct_kernel(const KhopArgs a, u32 h) {
+__global__ void __launch_bounds__(256, 8) khop_distinct_kernel(const KhopArgs a, u32 h) {
   __shared__ u32 s_seen[8][kDistinctMaxFanout];
   const u32 wp = a.width[h];
   const u64 nwarps = ((u64)gridDim.x * blockDim.x) >> 5, parents = a.n * wp;
@@ -374,7 +390,8 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
     const uint64_t ctas = (n + per_cta - 1) / per_cta;
     if (ctas <= 0x7FFFFFFFull) {
       if (distinct) khop_tree_kernel<true><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
-      else khop_tree_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
+      else if (a.flags & SKW_KHOP_UNBIASED) khop_tree_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
+      else khop_weighted_tree_kernel<<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
       SKW_LAUNCHED(ctx);
       return SKW_OK;
     }
