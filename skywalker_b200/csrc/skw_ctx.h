@@ -109,7 +109,7 @@ struct skw_ctx {
   bool counted = false;       // among the contexts for which freed device memory is kept
 
   // staging buffers of the host-pointer entry points, grown on demand
-  static constexpr int kStages = 13;
+  static constexpr int kStages = 14;
   void* stage[kStages] = {};
   size_t stage_bytes[kStages] = {};
 };

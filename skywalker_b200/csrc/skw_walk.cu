@@ -591,6 +591,7 @@ struct RecordWalkArgs {
   const u32* vbits;
   const u32* starts;
   u32* paths;
+  u32* heads;  // walk_records_ppr_kernel: the first cells of the rows go here, back to back, or (null) to the rows
   u32* lengths;
   unsigned long long* sum;
   u32* err;
@@ -775,10 +776,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2048 / (WARPS * 32)) walk_records_
   }
   __syncwarp();
   // write-out: 8 lanes per row, four neighbouring rows per pass; then the lengths, coalesced
+  static_assert(STAGE == 8, "a lane a cell");
   for (u32 r = lane >> 3; r < cnt; r += 4) {
     const u32 c = lane & 7;
     const u32 cells = min((u32)len[r] + 1u, (u32)STAGE);
-    if (c < cells) a.paths[(w_begin + r) * a.hop_num + c] = buf[r * kPitch + c];
+    if (a.heads) a.heads[(w_begin + r) * STAGE + c] = buf[r * kPitch + c];  // (whole sectors)
+    else if (c < cells) a.paths[(w_begin + r) * a.hop_num + c] = buf[r * kPitch + c];
   }
   for (u32 i = lane; i < cnt; i += 32) a.lengths[w_begin + i] = len[i];
   add_edges(a.sum, edges);
@@ -825,6 +828,66 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const u32* __restrict__ 
     if (o + cells > capacity) continue;
     const u32* s = src + w * hop_num;
     for (u32 c = sub; c < cells; c += 8) packed[o + c] = ldg_once(s + c);
+  }
+}
+
+// The same where the first kStage cells of the rows are in `heads`, back to back.  A warp takes 32 rows: lengths, places and
+// then the heads of all of them are fetched with independent loads, eight lanes a row; longer rows go on with eight lanes each,
+// or the whole warp where most are long.  A row at a time, each group of eight lanes waits for two dependent accesses a row:
+// 667,000 PPR walks of at most 100 steps, 2.7 M cells, 46 us.
+__global__ void __launch_bounds__(256) pack_heads_kernel(const u32* __restrict__ src, const u32* __restrict__ heads,
+                                                        u32* __restrict__ packed, const u32* __restrict__ lengths,
+                                                        const u64* __restrict__ offs, u64 n, u32 hop_num,
+                                                        u64 capacity, u64* __restrict__ total,
+                                                        uint8_t* __restrict__ lengths8) {
+  static_assert(kStage == 8, "a lane a cell");
+  const u32 lane = threadIdx.x & 31, sub = lane & 7, group = lane >> 3;
+  const u64 stride = ((u64)gridDim.x * blockDim.x >> 5) * 32;
+  for (u64 w0 = (((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; w0 < n; w0 += stride) {
+    const u64 w = w0 + lane;
+    u32 cells = 0;
+    u64 o = 0;
+    if (w < n) {
+      const u32 len = __ldg(lengths + w);
+      cells = min(len + 1u, hop_num);
+      o = __ldg(offs + w);
+      if (lengths8) lengths8[w] = (uint8_t)len;  // the caller asked for one byte per walk
+      if (w == n - 1) *total = o + cells;        // cells the whole batch needs
+      // rows that do not fit are left out: the host compares *total with the capacity and packs again
+      // into a larger buffer
+      if (o + cells > capacity) cells = 0;
+    }
+    u32 first[8];
+#pragma unroll
+    for (u32 r = 0; r < 8; ++r) {
+      const u32 row = r * 4 + group;
+      const u32 have = __shfl_sync(0xFFFFFFFFu, cells, row);
+      first[r] = 0;
+      if (sub < have) first[r] = __ldg(heads + (w0 + row) * kStage + sub);
+    }
+#pragma unroll
+    for (u32 r = 0; r < 8; ++r) {
+      const u32 row = r * 4 + group;
+      const u32 have = __shfl_sync(0xFFFFFFFFu, cells, row);
+      const u64 to = __shfl_sync(0xFFFFFFFFu, o, row);
+      if (sub < have) packed[to + sub] = first[r];
+    }
+    u32 more = __ballot_sync(0xFFFFFFFFu, cells > 8);
+    const u32 lanes = __popc(more) > 16 ? 32 : 8;  // a row
+    while (more) {
+      // the next row, or the next four
+      u32 row = 32;
+      for (u32 g = 0; more && g < 32 / lanes; ++g) {
+        if (lane / lanes == g) row = __ffs(more) - 1;
+        more &= more - 1;
+      }
+      const u32 have = __shfl_sync(0xFFFFFFFFu, cells, row & 31);
+      const u64 to = __shfl_sync(0xFFFFFFFFu, o, row & 31);
+      if (row < 32) {
+        const u32* from = src + (w0 + row) * hop_num;
+        for (u32 c = 8 + lane % lanes; c < have; c += lanes) packed[to + c] = ldg_once(from + c);
+      }
+    }
   }
 }
 
@@ -1067,11 +1130,29 @@ static bool builds_frontiers(const skw_walk_params* prm) {
          (prm->flags & (SKW_WALK_CACHE_TABLES | SKW_WALK_BUILD_TABLES)) != 0;
 }
 
+// Walk records serve unbiased walks as well (the record of column c names the c-th neighbour with its offset and degree: one
+// access per step instead of two), as long as every vertex with out-edges has a usable table, i.e. the degrees in the records
+// are the graph's own.
+static bool follows_records(const skw_ctx* ctx, const skw_walk_params* prm) {
+  const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
+  return (prm->mode != SKW_MODE_ONLINE || unbiased) && ctx->records_ready && prm->app != SKW_APP_NODE2VEC &&
+         (!unbiased || ctx->records_all_usable);
+}
+// PPR over the records by chunks.  The kernel hands a lane its next walker cheaply; a batch with a lane for every walker,
+// resident at once, does not need that (4,096 walkers: 29 -> 26 us, 100,000: 40 -> 38, equal at 200,000, 81 -> 89 at
+// 400,000).  It stages lengths as 16-bit values and has no grid-stride loop.
+static u64 ppr_chunk_ctas(u64 n) { return (n + 8 * kChunk - 1) / (8 * kChunk); }
+static bool ppr_by_chunks(const skw_ctx* ctx, const skw_walk_params* prm, u64 n) {
+  return follows_records(ctx, prm) && prm->app == SKW_APP_PPR && prm->hop_num <= 65535 && ppr_chunk_ctas(n) <= 0x7FFFFFFFull &&
+         n > 700ull * ctx->sm_count;
+}
+
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
 // No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: the
-// slots that online_tables gave for the call.
+// slots that online_tables gave for the call.  d_heads: where ppr_by_chunks may leave the first cells of the rows instead.
 static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n,
-                       uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum, const Slot* whole_table) {
+                       uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum, const Slot* whole_table,
+                       uint32_t* d_heads = nullptr) {
   const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
   const bool online = prm->mode == SKW_MODE_ONLINE && !unbiased;
   int rc;
@@ -1105,10 +1186,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   a.fmax = fmaxf(1.0f, fmaxf(a.inv_p, a.inv_q));
   cudaStream_t st = ctx->stream;
   if (whole_table) a.slots = whole_table;
-  // Walk records serve unbiased walks as well (the record of column c names the c-th neighbour with its
-  // offset and degree: one access per step instead of two), as long as every vertex with out-edges has
-  // a usable table, i.e. the degrees in the records are the graph's own.
-  if (!online && ctx->records_ready && prm->app != SKW_APP_NODE2VEC && (!unbiased || ctx->records_all_usable)) {
+  if (follows_records(ctx, prm)) {
     RecordWalkArgs ra;
     ra.unbiased = unbiased ? 1u : 0u;
     ra.rec = static_cast<const WalkRecord*>(ctx->records);
@@ -1116,6 +1194,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     ra.vbits = static_cast<const u32*>(ctx->vbits);
     ra.starts = d_starts;
     ra.paths = d_paths;
+    ra.heads = d_heads;
     ra.lengths = d_lengths;
     ra.sum = a.sum;
     ra.err = a.err;
@@ -1127,12 +1206,8 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     ra.hop_num = a.hop_num;
     ra.tp = a.tp;
     const WalkGrid g = walk_grid(ctx, prm->app, n, 17, 8);
-    // (the chunked kernel stages lengths as 16-bit values and has no grid-stride loop)
-    const u64 ctas = (n + 8 * kChunk - 1) / (8 * kChunk);
-    // It hands a lane its next walker cheaply; a batch with a lane for every walker, resident at once, does not need that
-    // (4,096 walkers: 29 -> 26 us, 100,000: 40 -> 38, equal at 200,000, 81 -> 89 at 400,000).
-    if (prm->app == SKW_APP_PPR && prm->hop_num <= 65535 && ctas <= 0x7FFFFFFFull && n > 700ull * ctx->sm_count) {
-      walk_records_ppr_kernel<8, kChunk, kStage><<<(unsigned)ctas, 256, 0, st>>>(ra);
+    if (ppr_by_chunks(ctx, prm, n)) {
+      walk_records_ppr_kernel<8, kChunk, kStage><<<(unsigned)ppr_chunk_ctas(n), 256, 0, st>>>(ra);
     } else if (prm->app == SKW_APP_PPR) walk_records_walk_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);
     else walk_records_walk_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(ra, g.lanes);
     SKW_LAUNCHED(ctx);
@@ -1361,19 +1436,19 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
   // the context's stream is already walking the next slice (the bus carries both directions at once).
   // Walker ids, hence walks, do not depend on the slicing.
   const uint64_t kSliceMin = 1u << 19;
-  const uint32_t slices = n >= 8 * kSliceMin ? 8 : (n >= 4 * kSliceMin ? 4 : (n >= 2 * kSliceMin ? 2 : 1));
+  const uint32_t slices = n >= 8 * kSliceMin ? 8 : (n >= 4 * kSliceMin ? 4 : (n >= 2 * kSliceMin ? 3 : 1));
   static_assert(skw_ctx::kPackSlices >= 8 && skw_ctx::kStages >= 4 + 8, "one event set and one packing buffer per slice");
-  // Slice sizes in the ratio 1 : 2 : 4 : 4 ...: the first results are on the bus early (the call is
+  // Slice sizes in the ratio 1 : 2 : 4 : 4 ... (three: 1 : 2 : 2): the first results are on the bus early (the call is
   // as long as the time to the first packed slice plus the copy of everything), the later slices are
-  // large enough to walk efficiently.
+  // large enough to walk efficiently.  2 M PPR walks: 926 us in two slices of 1 : 2, 880 in these three, 893 in four.
   uint64_t base_of[skw_ctx::kPackSlices + 1] = {};
   uint64_t per = n;  // the largest slice
   if (slices > 1) {
-    const uint64_t parts = 3 + 4ull * (slices - 2);
+    const uint64_t last = slices == 3 ? 2 : 4, parts = 3 + last * (slices - 2);
     const uint64_t unit = ((n + parts - 1) / parts + 1023) & ~1023ull;
-    per = (slices == 2 ? 2 : 4) * unit;
+    per = last * unit;
     for (uint32_t c = 0; c <= slices; ++c) {
-      const uint64_t b = c == 0 ? 0 : (c == 1 ? unit : (3 + 4ull * (c - 2)) * unit);
+      const uint64_t b = c == 0 ? 0 : (c == 1 ? unit : (3 + last * (c - 2)) * unit);
       base_of[c] = std::min<uint64_t>(b, n);
     }
   } else {
@@ -1392,10 +1467,17 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
   if ((rc = ensure_bytes(ctx, &ctx->stage[2], &ctx->stage_bytes[2], sizeof(u32) * (size_t)n)) != SKW_OK) return rc;
   if ((rc = ensure_bytes(ctx, &ctx->stage[3], &ctx->stage_bytes[3], offs_bytes + tmp_bytes)) != SKW_OK) return rc;
   constexpr int kLen8Stage = 4 + skw_ctx::kPackSlices;
-  static_assert(skw_ctx::kStages > kLen8Stage, "one more staging buffer for byte lengths");
+  constexpr int kHeadStage = kLen8Stage + 1;
+  static_assert(skw_ctx::kStages > kHeadStage, "two more staging buffers for byte lengths and heads of rows");
   if (h_lengths8 && (rc = ensure_bytes(ctx, &ctx->stage[kLen8Stage], &ctx->stage_bytes[kLen8Stage], (size_t)n)) != SKW_OK)
     return rc;
   uint8_t* d_len8 = h_lengths8 ? static_cast<uint8_t*>(ctx->stage[kLen8Stage]) : nullptr;
+  // PPR walks mostly end within the first cells of their rows.  Written to the rows, 404 bytes apart for 100 steps, these are
+  // isolated sectors, a third of the walk's time, and read back as such; side by side both are streams.
+  // (Without memory for them the rows will do.)
+  const bool heads = ppr_by_chunks(ctx, prm, n) && ensure_bytes(ctx, &ctx->stage[kHeadStage], &ctx->stage_bytes[kHeadStage],
+                                                                sizeof(u32) * kStage * (size_t)n) == SKW_OK;
+  if (!heads) cudaGetLastError();
   u32* d_starts = static_cast<u32*>(ctx->stage[0]);
   u32* d_rows = static_cast<u32*>(ctx->stage[1]);
   u32* d_len = static_cast<u32*>(ctx->stage[2]);
@@ -1420,6 +1502,9 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
   }
   if ((rc = err_reset(ctx)) != SKW_OK) return rc;
   unsigned long long* scratch_sum = reinterpret_cast<unsigned long long*>(ctx->d_sum) + 2;
+  auto heads_of = [&](uint32_t c) -> u32* {
+    return heads && ppr_by_chunks(ctx, prm, nc_of[c]) ? static_cast<u32*>(ctx->stage[kHeadStage]) + base_of[c] * kStage : nullptr;
+  };
   auto scan_and_pack = [&](uint32_t c) -> int {
     const uint64_t base = base_of[c], nc = nc_of[c];
     cub::TransformInputIterator<u64, CellsOfRow, const u32*> row_cells(d_len + base, CellsOfRow());
@@ -1430,10 +1515,15 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
     // Packed on the device, then one contiguous copy per slice: measured on B200 with 8 M PPR walks,
     // half the time of a pack kernel that writes the pinned host buffer itself (its 4-byte stores
     // per row do not merge into full-size bus writes).
-    pack_rows_kernel<<<grid_for(ctx, nc * 8, 8), 256, 0, st>>>(d_rows + base * prm->hop_num,
-                                                              static_cast<u32*>(ctx->stage[4 + c]), d_len + base, d_offs, nc,
-                                                              prm->hop_num, cap[c], ctx->h_tot + c,
-                                                              d_len8 ? d_len8 + base : nullptr);
+    u32* packed = static_cast<u32*>(ctx->stage[4 + c]);
+    uint8_t* len8 = d_len8 ? d_len8 + base : nullptr;
+    const u32* rows = d_rows + base * prm->hop_num;
+    if (const u32* first = heads_of(c))
+      pack_heads_kernel<<<grid_for(ctx, nc, 8), 256, 0, st>>>(rows, first, packed, d_len + base, d_offs, nc, prm->hop_num, cap[c],
+                                                             ctx->h_tot + c, len8);
+    else
+      pack_rows_kernel<<<grid_for(ctx, nc * 8, 8), 256, 0, st>>>(rows, packed, d_len + base, d_offs, nc, prm->hop_num, cap[c],
+                                                                ctx->h_tot + c, len8);
     SKW_LAUNCHED(ctx);
     SKW_CUDA(ctx, cudaEventRecord(ctx->pk_ready[c], st));
     SKW_CUDA(ctx, cudaStreamWaitEvent(side, ctx->pk_ready[c], 0));
@@ -1456,7 +1546,8 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
       SKW_CUDA(ctx, cudaEventRecord(ctx->pk_t0[c], st));
       int r = c == 0 ? online_tables(prm, n, tables) : SKW_OK;  // for all slices
       if (r != SKW_OK) return r;
-      r = walk_launch(ctx, &p, d_starts + base, nc, d_rows + base * prm->hop_num, d_len + base, scratch_sum, tables.slots);
+      r = walk_launch(ctx, &p, d_starts + base, nc, d_rows + base * prm->hop_num, d_len + base, scratch_sum, tables.slots,
+                      heads_of(c));
       if (r != SKW_OK) return r;
       SKW_CUDA(ctx, cudaEventRecord(ctx->pk_t1[c], st));
       if ((r = scan_and_pack(c)) != SKW_OK) return r;
@@ -1497,9 +1588,9 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
       SKW_CUDA(ctx, cudaEventElapsedTime(&t, ctx->pk_t0[c], ctx->pk_t1[c]));  // the walk is long over
       total_ms += t;
     }
+    int r = err_check(ctx, "skw_walk_packed");  // synchronises the context's stream, while the last copies are under way
     SKW_CUDA(ctx, cudaStreamSynchronize(side));
     SKW_CUDA(ctx, cudaStreamSynchronize(ctx->copy_stream));
-    int r = err_check(ctx, "skw_walk_packed");  // synchronises the context's stream
     if (r != SKW_OK) return r;
     *cells = total_cells;
     if (ms) *ms = total_ms;

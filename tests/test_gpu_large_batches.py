@@ -152,3 +152,37 @@ def test_deepwalk_walkers_a_warp_on_a_small_graph(ctx, oracle, rmat12, n, flags)
                                  **({} if flags == 0 else {"unbiased": True}))
     live = np.arange(12)[None, :] <= want_len[:, None]
     assert np.array_equal(lens, want_len) and edges == int(want_len.sum()) and np.array_equal(paths[live], want[live])
+
+
+@pytest.mark.parametrize("graph", ["rmat16", "plaw"])                  # mostly dead ends, none
+@pytest.mark.parametrize("hop,tp", [(1, 0.15), (2, 0.5), (8, 0.15), (9, 0.1), (10, 0.0), (81, 0.02), (101, 0.15)])
+@pytest.mark.parametrize("n", [104001, (1 << 20) + 33])                # chunked PPR in one slice, in three
+def test_packed_ppr_over_records(ctx, oracle, request, graph, hop, tp, n):
+    """PPR over the records, packed: the first eight cells of the rows travel apart from the rest.  The same cells and
+    lengths as the rows of the same call, at row lengths around eight, and as the oracle's walks."""
+    import torch
+    g = request.getfixturevalue(graph)
+    if n > 1 << 20 and hop > 10:
+        n = (1 << 20) // 8 * 8 + 1 if tp > 0.1 else 104001
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    ctx.walk_records_build()
+    starts = oracle.gen_starts(n, g.V, 5)
+    rows = torch.full((n, hop), -1, dtype=torch.int32, device="cuda")
+    lens = torch.zeros(n, dtype=torch.int32, device="cuda")
+    kw = dict(app=APP_PPR, tp=tp, seed=8, walker_base=3)
+    s = torch.from_numpy(starts.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    _, _, _, edges = ctx.walk(s, hop, paths=rows, lengths=lens, **kw)
+    rows, lens = rows.cpu().numpy().view(np.uint32), lens.cpu().numpy().view(np.uint32)
+    live = np.arange(hop)[None, :] <= lens[:, None]
+    want = rows[live]
+    for u8 in (False, True):
+        out, got, cells, ms, e = ctx.walk_packed(starts, hop, lengths_u8=u8, **kw)
+        assert cells == len(want) and e == edges and ms > 0
+        assert np.array_equal(got, lens) and np.array_equal(out[:cells], want)
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    op, ol = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts[:2000], hop, **kw)
+    assert np.array_equal(ol, lens[:2000])
+    keep = np.arange(hop)[None, :] <= ol[:, None]
+    assert np.array_equal(op[keep], rows[:2000][keep])
