@@ -56,7 +56,7 @@ constexpr u32 kMidSmemMax = 512 * kWideEpt;   // 8192: two CTAs of 512 threads a
 constexpr u32 kHugeSmemMax = 1024 * kWideEpt;  // 16384: one of 1024 threads; longer lists are in global memory
 constexpr u32 kAloneMax = 65536;              // longer ones are always built by clusters
 static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
-static_assert(2 * K_CLASSES <= 64, "class counters");
+static_assert(2 * K_CLASSES <= skw_ctx::kClassWords, "class counters");
 
 __device__ __forceinline__ int degree_class(u32 deg) {
   if (deg <= 8) return K_1A;
@@ -546,6 +546,23 @@ int builders_queued(skw_ctx* ctx) {
   return SKW_OK;
 }
 
+// Zero class counters for one build.  A graph that is being captured brings its own clearing along, and has a set that no
+// other build takes.
+static int class_counters(skw_ctx* ctx, u32** cls) {
+  constexpr unsigned kWords = skw_ctx::kClassWords, kLast = skw_ctx::kClassSets - 1;
+  if (capturing(ctx)) {
+    *cls = ctx->cls_counts + kLast * kWords;
+    SKW_CUDA(ctx, cudaMemsetAsync(*cls, 0, kWords * sizeof(u32), ctx->stream));
+    return SKW_OK;
+  }
+  if (ctx->cls_used == kLast) {
+    SKW_CUDA(ctx, cudaMemsetAsync(ctx->cls_counts, 0, kLast * kWords * sizeof(u32), ctx->stream));
+    ctx->cls_used = 0;
+  }
+  *cls = ctx->cls_counts + kWords * ctx->cls_used++;
+  return SKW_OK;
+}
+
 // Scratch of the lists beyond 16384 weights: a slab with room for the longest for each team of eight, fewer of them when a
 // giant hub would make the slabs exceed 4 GB in total; then, if smaller teams may be used, as much as the smallest need.
 struct LongScratch {
@@ -740,8 +757,9 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
     ctx->stamp_round = 1;
   }
   cudaStream_t st = ctx->stream;
-  SKW_CUDA(ctx, cudaMemsetAsync(ctx->frontier_cls, 0, 2 * K_CLASSES * sizeof(u32), st));
   if (units) {
+    u32* cls = nullptr;
+    if ((rc = class_counters(ctx, &cls)) != SKW_OK) return rc;
     // the claim is a chain of dependent accesses (vertex, offsets, stamp): fill every thread slot of the GPU
     const u64 want = (units + 256 * kFrontierUnits - 1) / (256 * kFrontierUnits);
     const int grid = (int)(want < (u64)ctx->sm_count * 8 ? want : (u64)ctx->sm_count * 8);
@@ -749,9 +767,9 @@ int frontier_collect(skw_ctx* ctx, const u32* verts, u64 units, u32 width, u32 c
     for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->frontier_lists + (size_t)k * cap;
     frontier_collect_kernel<<<grid, 256, 0, st>>>(verts, units, width, cells, offs, alive_lengths,
                                                   ctx->xadj, ctx->V, ctx->stamp, ctx->stamp_round,
-                                                  ctx->frontier_cls, lists, cap, ctx->launch_err);
+                                                  cls, lists, cap, ctx->launch_err);
     SKW_LAUNCHED(ctx);
-    rc = launch_builders(ctx, lists, ctx->frontier_cls, ctx->slots, ctx->valid, false);
+    rc = launch_builders(ctx, lists, cls, ctx->slots, ctx->valid, false);
     if (rc != SKW_OK) return rc;
   }
   return SKW_OK;
@@ -809,12 +827,13 @@ int enqueue_tables(skw_ctx* ctx, u32 v_begin, u32 v_end, Slot* slots, uint8_t* v
   worklist_words(ctx, v_end - v_begin, at);
   ClassLists lists;
   for (int k = 0; k < K_CLASSES; ++k) lists.list[k] = ctx->worklist + at[k];
-  SKW_CUDA(ctx, cudaMemsetAsync(ctx->cls_counts, 0, 2 * K_CLASSES * sizeof(u32), ctx->stream));
+  u32* cls = nullptr;
+  if ((rc = class_counters(ctx, &cls)) != SKW_OK) return rc;
   const u64 tiles = ((u64)(v_end - v_begin) + 256 * kClassifyVertices - 1) / (256 * kClassifyVertices);
   classify_kernel<<<(unsigned)std::min<u64>(tiles, (u64)ctx->sm_count * 8), 256, 0, ctx->stream>>>(
-      ctx->xadj, v_begin, v_end, ctx->cls_counts, lists, valid);
+      ctx->xadj, v_begin, v_end, cls, lists, valid);
   SKW_LAUNCHED(ctx);
-  return launch_builders(ctx, lists, ctx->cls_counts, slots, valid, v_begin == 0 && v_end == ctx->V);
+  return launch_builders(ctx, lists, cls, slots, valid, v_begin == 0 && v_end == ctx->V);
 }
 }  // namespace skw
 

@@ -175,10 +175,16 @@ bool capturing(const skw_ctx* ctx) {
 // same 16 words in mapped host memory.  A synchronous call ends with this kernel, which hands them to the host and
 // leaves those of `clear` (a bit a word) cleared for the next call: one small launch where two memsets before a call and
 // two copies after it took about 14 us of a call of 65.
-__global__ void report_status_kernel(uint32_t* __restrict__ d, uint32_t* __restrict__ h, uint32_t clear) {
+// The class counters of the builders that the call queued are cleared along with them.
+constexpr unsigned kClassCounters = (skw_ctx::kClassSets - 1) * skw_ctx::kClassWords;
+__global__ void report_status_kernel(uint32_t* __restrict__ d, uint32_t* __restrict__ h, uint32_t clear,
+                                     uint32_t* __restrict__ classes) {
   const uint32_t t = threadIdx.x;
-  h[t] = d[t];
-  if ((clear >> t) & 1u) d[t] = 0;
+  if (t < 16) {
+    h[t] = d[t];
+    if ((clear >> t) & 1u) d[t] = 0;
+  }
+  if (classes) classes[t] = 0;
 }
 
 int err_reset(skw_ctx* ctx) {
@@ -193,11 +199,16 @@ int err_reset(skw_ctx* ctx) {
 
 int err_check(skw_ctx* ctx, const char* where, bool queued) {
   // words 0-3 and 4-7: the error records; 8-9, 14-15: sums 0 and 3; 10-11: sum 1
-  report_status_kernel<<<1, 16, 0, ctx->stream>>>(ctx->d_err, ctx->h_err, queued ? 0xCFFFu : 0xC30Fu);
+  // (builders that were queued on another stream may still count)
+  const bool classes = ctx->cls_used != 0 && !ctx->tables_queued;
+  report_status_kernel<<<1, classes ? kClassCounters : 16, 0, ctx->stream>>>(ctx->d_err, ctx->h_err, queued ? 0xCFFFu : 0xC30Fu,
+                                                                             classes ? ctx->cls_counts : nullptr);
   SKW_LAUNCHED(ctx);
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->status_clean = true;
+  if (classes) ctx->cls_used = 0;
   ctx->queued = false;
+  if (!ctx->queued_before) ctx->tables_queued = false;  // whatever was queued has been waited for
   const uint32_t* rec = ctx->h_err + (queued ? 4 : 0);
   if (rec[0] != DEV_OK) {
     static const char* names[] = {"ok", "index out of range", "bounded wait ran out",
@@ -534,8 +545,9 @@ int skw_ctx_create(int device, skw_ctx** out) {
     CK(cudaEventCreate(&ctx->pk_t1[i]));
   }
   CK(cudaMallocHost(&ctx->h_tot, skw_ctx::kPackSlices * sizeof(uint64_t)));
-  CK(dev_malloc(ctx, &ctx->cls_counts, 64 * sizeof(uint32_t)));
-  CK(dev_malloc(ctx, &ctx->frontier_cls, 64 * sizeof(uint32_t)));
+  CK(dev_malloc(ctx, &ctx->cls_counts, skw_ctx::kClassSets * skw_ctx::kClassWords * sizeof(uint32_t)));
+  CK(cudaMemsetAsync(ctx->cls_counts, 0, skw_ctx::kClassSets * skw_ctx::kClassWords * sizeof(uint32_t), ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
 #undef CK
   *out = ctx;
   return SKW_OK;
@@ -552,7 +564,6 @@ void skw_ctx_destroy(skw_ctx* ctx) {
   dev_free(ctx->cls_counts);
   dev_free(ctx->cta_scratch);
   dev_free(ctx->frontier_lists);
-  dev_free(ctx->frontier_cls);
   for (int i = 0; i < skw_ctx::kStages; ++i) dev_free(ctx->stage[i]);
   if (ctx->h_pack) cudaFreeHost(ctx->h_pack);
   delete static_cast<skw::HostPool*>(ctx->host_pool);

@@ -85,7 +85,11 @@ struct skw_ctx {
   // builder scratch, grown on demand
   uint32_t* worklist = nullptr;      // vertices by degree class, one list per class
   size_t worklist_cap = 0;
-  uint32_t* cls_counts = nullptr;    // per degree class: count, then cursor
+  // Counts and cursors of the degree classes, a set of words a build.  A build takes the next set, which is zero; the kernel
+  // that reports a call's status clears them all again, so that a build needs no memset of its own (1 M edges: 50 -> 47 us).
+  static constexpr unsigned kClassSets = 8, kClassWords = 32;
+  uint32_t* cls_counts = nullptr;
+  unsigned cls_used = 0;  // sets that are not zero; the last one belongs to graphs
   void* cta_scratch = nullptr;       // slabs of the global-memory CTA builder
   size_t cta_scratch_bytes = 0;
 
@@ -93,7 +97,6 @@ struct skw_ctx {
   // every distinct frontier vertex be built once per round
   uint32_t* frontier_lists = nullptr;
   size_t frontier_lists_bytes = 0;
-  uint32_t* frontier_cls = nullptr;  // same layout as cls_counts
   uint32_t* stamp = nullptr;         // V entries, last round that claimed the vertex
   uint32_t stamp_round = 0;
   // online direct walks: per-vertex memo of {call stamp, largest weight, total quantised weight}

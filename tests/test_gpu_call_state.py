@@ -109,3 +109,45 @@ def test_error_of_a_queued_walk_waits_for_its_own_report(ctx, oracle, rmat12, kw
         ctx.walk(bad, 11, seed=5, **kw)
     ctx.walk(starts, 11, seed=5, **kw)
     assert ctx.take_sampled_edges() == 0
+
+
+def test_class_counters_across_calls_and_streams(oracle, plaw):
+    """Builds take zeroed counters from a few sets that the status kernel clears: more builds in one call than there are
+    sets, queued builds whose call nothing waits for, and builds on another stream behind them."""
+    import torch
+    from skywalker_b200 import MODE_ONLINE
+    from skywalker_b200.api import Context
+    g = plaw
+    c = Context(0)
+    c.upload(g.xadj, g.adjncy, g.adjwgt)
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    n, hop = 20000, 21                              # 20 frontiers a call
+    starts = oracle.gen_starts(n, g.V, 5)
+    want, want_len = oracle.walk(g.xadj, g.adjncy, g.adjwgt, table, starts, hop, seed=8)
+    s = torch.from_numpy(starts.view(np.int32)).cuda()
+    p = torch.zeros((n, hop), dtype=torch.int32, device="cuda")
+    l = torch.zeros(n, dtype=torch.int32, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    live = np.arange(hop)[None, :] <= want_len[:, None]
+
+    def same():
+        assert np.array_equal(l.cpu().numpy().view(np.uint32), want_len)
+        assert np.array_equal(p.cpu().numpy().view(np.uint32)[live], want[live])
+
+    for turn in range(4):
+        c.set_stream(streams[turn % 2].cuda_stream)
+        for flags in (0, 4, 0, 0):                  # tables of the whole graph, of every step's frontier
+            c.walk(s, hop, seed=8, mode=MODE_ONLINE, paths=p, lengths=l, flags=flags, enqueue_only=True)
+        c.set_stream(streams[1 - turn % 2].cuda_stream)
+        c.alias_build_offline()
+        prob, alias, valid = c.alias_export()
+        assert np.array_equal(prob, table[0]) and np.array_equal(alias, table[1]) and np.array_equal(valid, table[2])
+        torch.cuda.synchronize()
+        same()
+        for flags in (4, 0):
+            p.zero_(), l.zero_()
+            torch.cuda.synchronize()
+            c.walk(s, hop, seed=8, mode=MODE_ONLINE, paths=p, lengths=l, flags=flags)
+            same()
+    c.close()
