@@ -41,10 +41,13 @@ __device__ __forceinline__ EdgeList edge_list(const WalkArgs& a, u32 v) {
   return EdgeList{off, __ldg(a.xadj + v + 1) - off};
 }
 
-// The neighbour that random words r draw from the list of `cur`.  Returns false when there is none.
+// The neighbour that random words r draw from the list of `cur`.  Returns false when there is none.  AHEAD: the neighbour of the
+// drawn column is fetched beside its slot, since the draw mostly keeps it.
+template <bool AHEAD>
 __device__ __forceinline__ bool walk_draw(const WalkArgs& a, u32 cur, EdgeList here, Rand4 r, u32& next) {
   const u32 col = __umulhi(r.x, here.deg);
   u32 cand = col;
+  if (AHEAD) next = ldg_once(a.adjncy + (u64)here.off + col);
   if (!a.unbiased) {
     const Slot s = load_slot(a.slots + (u64)here.off + col);
     if (s.prob < 0.0f) return false;  // vertex without usable weight
@@ -54,13 +57,13 @@ __device__ __forceinline__ bool walk_draw(const WalkArgs& a, u32 cur, EdgeList h
       return false;
     }
   }
-  next = ldg_once(a.adjncy + (u64)here.off + cand);
+  if (!AHEAD || cand != col) next = ldg_once(a.adjncy + (u64)here.off + cand);
   return true;
 }
 
 // One step of one walker standing on `cur`.  Returns false when the walk ends here.
 // r: the random words of (walker, step, trial 0).
-template <int APP>
+template <int APP, bool AHEAD>
 __device__ __forceinline__ bool walk_step(const WalkArgs& a, u32 step, u64 gw, u32 cur, u32& next, Rand4 r) {
   if (APP == SKW_APP_PPR && u01(r.z) < a.tp) return false;
   if (cur >= a.V) {
@@ -68,7 +71,7 @@ __device__ __forceinline__ bool walk_step(const WalkArgs& a, u32 step, u64 gw, u
     return false;
   }
   const EdgeList here = edge_list(a, cur);
-  return here.deg != 0 && walk_draw(a, cur, here, r, next);
+  return here.deg != 0 && walk_draw<AHEAD>(a, cur, here, r, next);
 }
 
 // The same for node2vec, which also needs the list of the vertex it came from (there, deg 0 on the first
@@ -80,7 +83,7 @@ __device__ __forceinline__ bool walk_step_n2v(const WalkArgs& a, u32 step, u64 g
                                               EdgeList there, u32& next, EdgeList& next_list, Rand4 r) {
   if (here.deg == 0) return false;
   for (u32 trial = 0;;) {
-    if (!walk_draw(a, cur, here, r, next)) return false;
+    if (!walk_draw<false>(a, cur, here, r, next)) return false;
     if (next >= a.V) {
       dev_fail(a.err, DEV_ERR_INDEX, next, step, (u32)gw);
       return false;
@@ -120,9 +123,20 @@ static WalkGrid walk_grid(const skw_ctx* ctx, uint32_t app, u64 n, u32 warps, u3
   return WalkGrid{(u32)std::clamp<u64>((n + per_cta - 1) / per_cta, 1, 0x7FFFFFFF), lanes};
 }
 
+// Whether a draw fetches the neighbour of its column beside the slot: an access less in the chain of most steps, and one more
+// where the alias is taken.  It pays while walkers wait for memory and not for its rate.  80 steps, us, without / with:
+//   PPR        4,096 walkers 40 / 39 (R-MAT 22) and 45 / 44 (power law of 226 M edges), 40,000 75 / 68 and 101 / 92;
+//              1 M walkers of 20 steps on the power law 325 / 346
+//   DeepWalk   tables out of cache: 1,000 walkers 96 / 89 and 111 / 98, 16,000 129 / 114 and 132 / 122, 100,000 170 / 190 and
+//              455 / 524; in cache (R-MAT 16, 4,096 walkers) 73 / 77
+static bool walk_ahead(const skw_ctx* ctx, uint32_t app, u64 n, bool unbiased) {
+  if (unbiased) return false;
+  return app == SKW_APP_PPR ? n <= 270ull * ctx->sm_count : n <= 110ull * ctx->sm_count && ctx->E * 12 > (64u << 20);
+}
+
 // All steps of all walkers in one launch.  The first `lanes` lanes of each warp own walkers w, w + T, w + 2T ...;
 // the loop body is one step, so lanes of a warp stay converged although their walkers differ.
-template <int APP>
+template <int APP, bool AHEAD>
 __global__ void __launch_bounds__(kWalkCta) walk_offline_kernel(const WalkArgs a, u32 lanes) {
   const u64 T = (u64)gridDim.x * (kWalkCta / 32) * lanes;
   u64 w = ((u64)blockIdx.x * (kWalkCta / 32) + threadIdx.x / 32) * lanes + (threadIdx.x & 31);
@@ -150,10 +164,10 @@ __global__ void __launch_bounds__(kWalkCta) walk_offline_kernel(const WalkArgs a
     bool go;
     if (APP == SKW_APP_PPR) {
       go = step + 1 < a.hop_num &&
-           walk_step<APP>(a, step, gw, cur, next, philox_tagged(a.seed, TAG_WALK, gw, step, 0));
+           walk_step<APP, AHEAD>(a, step, gw, cur, next, philox_tagged(a.seed, TAG_WALK, gw, step, 0));
     } else {
       rn = philox_tagged(a.seed, TAG_WALK, gw, step + 1, 0);
-      go = step + 1 < a.hop_num && walk_step<APP>(a, step, gw, cur, next, r);
+      go = step + 1 < a.hop_num && walk_step<APP, AHEAD>(a, step, gw, cur, next, r);
     }
     if (go) {
       ++step;
@@ -400,7 +414,7 @@ __global__ void __launch_bounds__(256) walk_online_step_kernel(const WalkArgs a,
       go = walk_step_n2v<false>(a, step, gw, cur, prev, edge_list(a, cur), step ? edge_list(a, prev) : EdgeList{0, 0}, next,
                          next_list, r);
     } else {
-      go = walk_step<APP>(a, step, gw, cur, next, r);
+      go = walk_step<APP, false>(a, step, gw, cur, next, r);
     }
     if (go) {
       row[step + 1] = next;
@@ -1214,9 +1228,16 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   } else if (!online || whole_table) {
     const u64 read = ctx->E * (unbiased ? 4u : 12u);  // lists, and slots if they are drawn from
     const WalkGrid g = walk_grid(ctx, prm->app, n, prm->app == SKW_APP_DEEPWALK && read <= (8u << 20) ? 17 : 34, 1);
+    const bool ahead = walk_ahead(ctx, prm->app, n, unbiased);
     switch (prm->app) {
-      case SKW_APP_DEEPWALK: walk_offline_kernel<SKW_APP_DEEPWALK><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
-      case SKW_APP_PPR: walk_offline_kernel<SKW_APP_PPR><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes); break;
+      case SKW_APP_DEEPWALK:
+        if (ahead) walk_offline_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        else walk_offline_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        break;
+      case SKW_APP_PPR:
+        if (ahead) walk_offline_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        else walk_offline_kernel<SKW_APP_PPR, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        break;
       default: {
         const unsigned ctas = (unsigned)std::min<u64>((n + kN2vCta - 1) / kN2vCta, 0x7FFFFFFFull);
         switch (n2v_way(ctx, prm, n, unbiased)) {
