@@ -170,12 +170,12 @@ __device__ __noinline__ void build_list_long(u32 rank, u32 v, u32 off, u32 n, co
   // ---- largest weight; bits of positive floats are ordered as the floats are, others count as zero
   auto usable = [](int x) { return (u32)(x - 1) < 0x7F7FFFFFu ? x : 0; };
   int top = 0;
-  for (u32 p = cb; p < ce; p += min(8 * NT, ce - p)) {
-    int x[8];
+  for (u32 p = cb; p < ce; p += min(16 * NT, ce - p)) {
+    int x[16];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = t + k * NT < ce - p ? __float_as_int(__ldg(w + p + t + k * NT)) : 0;
+    for (int k = 0; k < 16; ++k) x[k] = t + k * NT < ce - p ? __float_as_int(__ldg(w + p + t + k * NT)) : 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) top = max(top, usable(x[k]));
+    for (int k = 0; k < 16; ++k) top = max(top, usable(x[k]));
   }
   top = co.template max<0>(top);
   if (t == 0) sh->chunk_top = top;
@@ -198,13 +198,13 @@ __device__ __noinline__ void build_list_long(u32 rank, u32 v, u32 off, u32 n, co
   };
   // ---- total, and what is before this chunk
   u64 W = 0, Qc = 0;
-  for (u32 p = cb; p < ce; p += min(8 * NT, ce - p)) {
-    int x[8];
+  for (u32 p = cb; p < ce; p += min(16 * NT, ce - p)) {
+    int x[16];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = t + k * NT < ce - p ? __float_as_int(__ldg(w + p + t + k * NT)) : 0;
+    for (int k = 0; k < 16; ++k) x[k] = t + k * NT < ce - p ? __float_as_int(__ldg(w + p + t + k * NT)) : 0;
     double s = 0.0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s = __dadd_rn(s, quantised(x[k]));
+    for (int k = 0; k < 16; ++k) s = __dadd_rn(s, quantised(x[k]));
     W += (u64)s;
   }
 #pragma unroll
