@@ -185,6 +185,68 @@ __global__ void __launch_bounds__(kWalkCta) walk_offline_kernel(const WalkArgs a
   add_edges(a.sum, edges);
 }
 
+// The same for DeepWalk into a matrix in pinned host memory (a.paths, a.lengths as the GPU sees them): the rows go over the bus
+// while the walks are under way instead of behind them.  The bus carries a write of a sector with about as many bytes of its
+// own, and single cells at a fraction of its rate.  So cells wait in shared memory, two 128-byte lines of the matrix a walker
+// (rows start anywhere in a line), and every 32 steps the warp writes the line that each of its walkers has filled; when in the
+// 32 steps differs from warp to warp.  fill: cells past a walk's end get kNoVertex, otherwise they keep what they held.
+constexpr u32 kLineCells = 32, kLineRing = 2 * kLineCells;
+template <bool AHEAD>
+__global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u32 lanes, u32 fill) {
+  extern __shared__ u32 rings[];  // a ring a walker, an odd number of words apart
+  const u32 lane = threadIdx.x & 31, warp = blockIdx.x * (kWalkCta / 32) + threadIdx.x / 32;
+  u32* const warp_rings = rings + threadIdx.x / 32 * lanes * (kLineRing + 1);
+  u32* const ring = warp_rings + lane * (kLineRing + 1);
+  const u64 first = (u64)warp * lanes, w = first + lane;
+  const u64 gw = a.walker_base + w * a.walker_stride;
+  const bool have = lane < lanes && w < a.n;
+  const u32 walkers = first < a.n ? (u32)min((u64)lanes, a.n - first) : 0;  // of the warp
+  // cell c of a row is place + c words behind the beginning of the line that the row starts in
+  const u32 place = (u32)((((uintptr_t)a.paths >> 2) + w * a.hop_num) & (kLineCells - 1));
+  bool live = have;
+  u32 cur = 0, len = 0;
+  Rand4 r{0, 0, 0, 0};
+  if (have) {
+    cur = __ldg(a.starts + w);
+    r = philox_tagged(a.seed, TAG_WALK, gw, 0, 0);
+  }
+  u32 sent = 0;  // the lines that `sent` cells of a row fill are written
+  for (u32 step = 0; walkers && step < a.hop_num;) {
+    // one step less than a line at first for some warps, then lines
+    const u32 end = min(a.hop_num, step == 0 ? kLineCells - (warp & (kLineCells - 1)) : step + kLineCells);
+    if (have) {
+      for (; step < end; ++step) {
+        ring[(place + step) & (kLineRing - 1)] = live ? cur : kNoVertex;
+        if (live && step + 1 < a.hop_num) {
+          const Rand4 rn = philox_tagged(a.seed, TAG_WALK, gw, step + 1, 0);
+          u32 next = 0;
+          live = walk_step<SKW_APP_DEEPWALK, AHEAD>(a, step, gw, cur, next, r);
+          if (live) {
+            cur = next;
+            ++len;
+            r = rn;
+          }
+        }
+      }
+    }
+    step = end;
+    __syncwarp();
+    for (u32 k = 0; k < walkers; ++k) {
+      const u32 at = __shfl_sync(0xFFFFFFFFu, place, k), wrote = __shfl_sync(0xFFFFFFFFu, len, k);
+      const u32 lines = (at + end + (end == a.hop_num ? kLineCells - 1 : 0)) / kLineCells;
+      for (u32 j = (at + sent) / kLineCells; j < lines; ++j) {
+        const u32 cell = j * kLineCells + lane - at;  // wraps in front of the row's first cell
+        if (cell < end && (fill || cell <= wrote))
+          a.paths[(first + k) * a.hop_num + cell] = warp_rings[k * (kLineRing + 1) + ((j * kLineCells + lane) & (kLineRing - 1))];
+      }
+    }
+    __syncwarp();
+    sent = end;
+  }
+  if (have) a.lengths[w] = len;
+  add_edges(a.sum, len);
+}
+
 // node2vec over the table.  A step is a chain of dependent accesses of varying length: slot and neighbour of
 // every proposal, the list of the proposed vertex, and for about half of the proposals a search of the list the
 // walk came from.  With one STEP per iteration every lane of a warp waits for the one with the most rejections
@@ -1164,9 +1226,10 @@ static bool ppr_by_chunks(const skw_ctx* ctx, const skw_walk_params* prm, u64 n)
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
 // No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: the
 // slots that online_tables gave for the call.  d_heads: where ppr_by_chunks may leave the first cells of the rows instead.
+// home: the rows are written_home's, fill: cells past a walk's end are overwritten there.
 static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n,
                        uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum, const Slot* whole_table,
-                       uint32_t* d_heads = nullptr) {
+                       uint32_t* d_heads = nullptr, bool home = false, bool fill = false) {
   const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
   const bool online = prm->mode == SKW_MODE_ONLINE && !unbiased;
   int rc;
@@ -1231,7 +1294,11 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     const bool ahead = walk_ahead(ctx, prm->app, n, unbiased);
     switch (prm->app) {
       case SKW_APP_DEEPWALK:
-        if (ahead) walk_offline_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        if (home) {
+          const size_t rings = sizeof(u32) * (kWalkCta / 32) * g.lanes * (kLineRing + 1);
+          if (ahead) walk_home_kernel<true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+          else walk_home_kernel<false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        } else if (ahead) walk_offline_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         else walk_offline_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         break;
       case SKW_APP_PPR:
@@ -1272,7 +1339,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
 // A synchronous walk over device buffers; with h_lengths the lengths, with h_paths the whole matrix comes home as well.
 static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n, uint32_t* d_paths,
                          uint32_t* d_lengths, uint32_t* h_lengths, uint32_t* h_paths, float* ms,
-                         uint64_t* sampled_edges) {
+                         uint64_t* sampled_edges, bool home = false, bool fill = false) {
   cudaStream_t st = ctx->stream;
   int rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
@@ -1280,7 +1347,7 @@ static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_
   OnlineTables tables(ctx);
   if ((rc = online_tables(prm, n, tables)) != SKW_OK) return rc;
   if ((rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum),
-                        tables.slots)) != SKW_OK)
+                        tables.slots, nullptr, home, fill)) != SKW_OK)
     return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   if (h_lengths && n) SKW_CUDA(ctx, cudaMemcpyAsync(h_lengths, d_lengths, sizeof(u32) * (size_t)n, cudaMemcpyDeviceToHost, st));
@@ -1383,6 +1450,31 @@ static int walk_rows_by_scatter(skw_ctx* ctx, const skw_walk_params* prm, const 
   return SKW_OK;
 }
 
+// `count` words of host memory as the GPU sees them, or null where it does not (both ends are asked for, a part of an allocation
+// may be registered) or where they are not at a word boundary.
+static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
+  cudaPointerAttributes first, last;
+  if ((reinterpret_cast<uintptr_t>(h) & 3) == 0 && cudaPointerGetAttributes(&first, h) == cudaSuccess &&
+      cudaPointerGetAttributes(&last, h + (count - 1)) == cudaSuccess && first.type == cudaMemoryTypeHost &&
+      last.type == cudaMemoryTypeHost && first.devicePointer &&
+      static_cast<u32*>(last.devicePointer) == static_cast<u32*>(first.devicePointer) + (count - 1))
+    return static_cast<u32*>(first.devicePointer);
+  cudaGetLastError();
+  return nullptr;
+}
+
+// Whether walk_home_kernel takes a batch: as long as the walks, a chain of hop_num dependent steps whatever their number, hide
+// most of the writes, which cross the bus at 36 GB/s where a copy behind the walks takes 52 (a sector a packet against whole
+// lines).  Rows of a line or less are mostly ends of lines; what they gain is the copies and the clearing of the matrix that
+// nobody has to queue, as long as every walker has a warp.  Calls, us, copied / written (R-MAT 16, 18, 20 and 22): 80 steps, 256
+// walkers 163-197 / 135-152, 4,096 177-194 / 140-148, 16,000 274-291 / 202-209, 29,600 359-385 / 295-311, and with the same
+// walks at every call 40,000 424-467 / 369-385, 80,000 642-809 / 681-722; 200 steps, 4,096 305-379 / 245-275, 16,000 539-605 /
+// 356-410; 10 steps, 256 73-77 / 59-60, 5,000 84-88 / 72-74, 10,000 86-90 / 78-89, 20,000 97-102 / 106-115.
+static bool written_home(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
+  return n != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app == SKW_APP_DEEPWALK &&
+         (prm->mode != SKW_MODE_ONLINE || (prm->flags & SKW_WALK_UNBIASED)) && !follows_records(ctx, prm);
+}
+
 int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts, uint64_t n,
              uint32_t* h_paths, uint32_t* h_lengths, float* ms, uint64_t* sampled_edges) {
   if (!ctx || !prm) return SKW_ERR_ARG;
@@ -1397,10 +1489,19 @@ int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts,
   }
   const size_t nb = sizeof(uint32_t) * (size_t)n;
   if ((rc = ensure_bytes(ctx, &ctx->stage[0], &ctx->stage_bytes[0], nb)) != SKW_OK) return rc;
+  const bool fill = (prm->flags & SKW_WALK_FILL_ROWS) != 0;
+  if (written_home(ctx, prm, n)) {
+    u32* const rows = seen_by_gpu(h_paths, n * prm->hop_num);
+    u32* const lengths = rows ? seen_by_gpu(h_lengths, n) : nullptr;
+    if (lengths) {
+      SKW_CUDA(ctx, cudaMemcpyAsync(ctx->stage[0], h_starts, nb, cudaMemcpyHostToDevice, ctx->stream));
+      return walk_and_wait(ctx, prm, static_cast<uint32_t*>(ctx->stage[0]), n, rows, lengths, nullptr, nullptr, ms, sampled_edges,
+                           true, fill);
+    }
+  }
   if ((rc = ensure_bytes(ctx, &ctx->stage[1], &ctx->stage_bytes[1], nb * prm->hop_num)) != SKW_OK) return rc;
   if ((rc = ensure_bytes(ctx, &ctx->stage[2], &ctx->stage_bytes[2], nb)) != SKW_OK) return rc;
   if (n) SKW_CUDA(ctx, cudaMemcpyAsync(ctx->stage[0], h_starts, nb, cudaMemcpyHostToDevice, ctx->stream));
-  const bool fill = (prm->flags & SKW_WALK_FILL_ROWS) != 0;
   if (n && fill) SKW_CUDA(ctx, cudaMemsetAsync(ctx->stage[1], 0xFF, nb * prm->hop_num, ctx->stream));
   uint64_t edges = 0;
   rc = walk_and_wait(ctx, prm, static_cast<uint32_t*>(ctx->stage[0]), n, static_cast<uint32_t*>(ctx->stage[1]),
@@ -1409,16 +1510,9 @@ int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts,
   if (sampled_edges) *sampled_edges = edges;
   if (n && !fill) {
     // Pinned host memory is addressable by the GPU: write only the cells each walk produced, unless that is all of
-    // them.  Pageable memory gets the whole matrix (cells past a walk's end then hold stale values).
-    cudaPointerAttributes at;
-    u32* mapped = nullptr;
-    if (edges == n * (prm->hop_num - 1ull)) {
-      // every cell was written: one copy (4096 rows of 81: 31 us against 65 for the kernel)
-    } else if (cudaPointerGetAttributes(&at, h_paths) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer) {
-      mapped = static_cast<u32*>(at.devicePointer);
-    } else {
-      cudaGetLastError();
-    }
+    // them (4096 rows of 81: one copy takes 31 us, the kernel 65).  Pageable memory gets the whole matrix (cells past a walk's
+    // end then hold stale values).
+    u32* const mapped = edges == n * (prm->hop_num - 1ull) ? nullptr : seen_by_gpu(h_paths, n * prm->hop_num);
     if (mapped) {
       copy_row_prefixes_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(
           static_cast<const u32*>(ctx->stage[1]), mapped, static_cast<const u32*>(ctx->stage[2]), n, prm->hop_num);

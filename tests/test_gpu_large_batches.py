@@ -186,3 +186,33 @@ def test_packed_ppr_over_records(ctx, oracle, request, graph, hop, tp, n):
     assert np.array_equal(ol, lens[:2000])
     keep = np.arange(hop)[None, :] <= ol[:, None]
     assert np.array_equal(op[keep], rows[:2000][keep])
+
+
+@pytest.mark.parametrize("hop", [1, 2, 31, 32, 33, 81])
+@pytest.mark.parametrize("n,off,flags", [(1, 0, 0), (37, 5, 16), (4096, 31, 16), (4097, 2, 0), (9999, 1, 18)])
+def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, hop, n, off, flags):
+    """DeepWalk writes its rows into the caller's pinned matrix a 128-byte line at a time, wherever in a line a row starts (off
+    words).  Cells past a walk's end keep their contents or (16, fill rows) get the invalid vertex, words around the matrix
+    keep theirs, and all of it equals the rows of pageable memory; 2: uniform draws."""
+    import torch
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, g.V, 11)
+    paths = torch.full((n * hop + 64,), 0x5A5A5A5A, dtype=torch.int32).pin_memory()
+    lengths = torch.full((n + 2,), 0x5A5A5A5A, dtype=torch.int32).pin_memory()
+    kw = dict(seed=6, walker_base=9, flags=flags)
+    _, _, ms, edges = ctx.walk(starts, hop, paths=paths[off:off + n * hop], lengths=lengths[1:n + 1], **kw)
+    p, l = paths.numpy().view(np.uint32), lengths.numpy().view(np.uint32)
+    rows, lens = p[off:off + n * hop].reshape(n, hop), l[1:n + 1]
+    assert (p[:off] == 0x5A5A5A5A).all() and (p[off + n * hop:] == 0x5A5A5A5A).all()
+    assert l[0] == l[-1] == 0x5A5A5A5A and ms > 0 and edges == int(lens.sum())
+    live = np.arange(hop)[None, :] <= lens[:, None]
+    assert (rows[~live] == (0xFFFFFFFF if flags & 16 else 0x5A5A5A5A)).all()
+    wp, wl = np.zeros((n, hop), np.uint32), np.zeros(n, np.uint32)
+    _, _, _, e = ctx.walk(starts, hop, paths=wp, lengths=wl, **kw)
+    assert e == edges and np.array_equal(wl, lens) and np.array_equal(wp[live], rows[live])
+    # not at a word boundary: pinned memory as well, but copied
+    odd = torch.zeros(n * hop * 4 + 4, dtype=torch.uint8).pin_memory().numpy()[2:2 + n * hop * 4].view(np.uint32)
+    ctx.walk(starts, hop, paths=odd, lengths=wl, **kw)
+    assert np.array_equal(odd.reshape(n, hop)[live], rows[live])
