@@ -1472,6 +1472,7 @@ static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
 // 356-410; 10 steps, 256 73-77 / 59-60, 5,000 84-88 / 72-74, 10,000 86-90 / 78-89, 20,000 97-102 / 106-115.
 static bool written_home(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
   return n != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app == SKW_APP_DEEPWALK &&
+         prm->hop_num <= (1u << 24) &&  // the kernel counts up to a line past the row's end in 32 bits
          (prm->mode != SKW_MODE_ONLINE || (prm->flags & SKW_WALK_UNBIASED)) && !follows_records(ctx, prm);
 }
 
