@@ -269,7 +269,7 @@ int skw_ctx_take_sampled_edges(skw_ctx* ctx, uint64_t* out);
  * pinned memory (skw_host_alloc, cudaHostAlloc, cudaHostRegister) only the cells each walk wrote
  * (0 .. length) are transferred, by a kernel writing into the mapped host matrix; the other cells
  * keep what the caller had there.  With pageable memory the whole matrix is copied and cells past a
- * walk's end are unspecified.  Into pinned h_paths and h_lengths small DeepWalk batches over the table
+ * walk's end are unspecified.  Into pinned h_paths and h_lengths small DeepWalk and PPR batches over the table
  * are written by the walk kernel itself while they run; *ms then covers these writes. */
 int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts, uint64_t n,
              uint32_t* h_paths, uint32_t* h_lengths, float* ms, uint64_t* sampled_edges);

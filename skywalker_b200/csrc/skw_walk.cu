@@ -185,13 +185,13 @@ __global__ void __launch_bounds__(kWalkCta) walk_offline_kernel(const WalkArgs a
   add_edges(a.sum, edges);
 }
 
-// The same for DeepWalk into a matrix in pinned host memory (a.paths, a.lengths as the GPU sees them): the rows go over the bus
+// The same for DeepWalk and PPR into a matrix in pinned host memory (a.paths, a.lengths as the GPU sees them): the rows go over the bus
 // while the walks are under way instead of behind them.  The bus carries a write of a sector with about as many bytes of its
 // own, and single cells at a fraction of its rate.  So cells wait in shared memory, two 128-byte lines of the matrix a walker
 // (rows start anywhere in a line), and every 32 steps the warp writes the line that each of its walkers has filled; when in the
 // 32 steps differs from warp to warp.  fill: cells past a walk's end get kNoVertex, otherwise they keep what they held.
 constexpr u32 kLineCells = 32, kLineRing = 2 * kLineCells;
-template <bool AHEAD>
+template <int APP, bool AHEAD>
 __global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u32 lanes, u32 fill) {
   extern __shared__ u32 rings[];  // a ring a walker, an odd number of words apart
   const u32 lane = threadIdx.x & 31, warp = blockIdx.x * (kWalkCta / 32) + threadIdx.x / 32;
@@ -208,32 +208,35 @@ __global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u
   Rand4 r{0, 0, 0, 0};
   if (have) {
     cur = __ldg(a.starts + w);
-    r = philox_tagged(a.seed, TAG_WALK, gw, 0, 0);
+    if (APP != SKW_APP_PPR) r = philox_tagged(a.seed, TAG_WALK, gw, 0, 0);
   }
   u32 sent = 0;  // the lines that `sent` cells of a row fill are written
   for (u32 step = 0; walkers && step < a.hop_num;) {
-    // one step less than a line at first for some warps, then lines
+    // a line of steps at a time, but for the first, which is shorter by warp
     const u32 end = min(a.hop_num, step == 0 ? kLineCells - (warp & (kLineCells - 1)) : step + kLineCells);
     if (have) {
       for (; step < end; ++step) {
         ring[(place + step) & (kLineRing - 1)] = live ? cur : kNoVertex;
         if (live && step + 1 < a.hop_num) {
-          const Rand4 rn = philox_tagged(a.seed, TAG_WALK, gw, step + 1, 0);
+          // the words of the next step are computed beside this one's loads, but for PPR, which mostly ends (walk_offline_kernel)
+          Rand4 rn{0, 0, 0, 0};
+          if (APP == SKW_APP_PPR) r = philox_tagged(a.seed, TAG_WALK, gw, step, 0);
+          else rn = philox_tagged(a.seed, TAG_WALK, gw, step + 1, 0);
           u32 next = 0;
-          live = walk_step<SKW_APP_DEEPWALK, AHEAD>(a, step, gw, cur, next, r);
+          live = walk_step<APP, AHEAD>(a, step, gw, cur, next, r);
           if (live) {
             cur = next;
             ++len;
-            r = rn;
+            if (APP != SKW_APP_PPR) r = rn;
           }
         }
       }
     }
     step = end;
-    __syncwarp();
+    const bool last = !__any_sync(0xFFFFFFFFu, live) && !fill || end == a.hop_num;  // nothing follows for any of them
     for (u32 k = 0; k < walkers; ++k) {
       const u32 at = __shfl_sync(0xFFFFFFFFu, place, k), wrote = __shfl_sync(0xFFFFFFFFu, len, k);
-      const u32 lines = (at + end + (end == a.hop_num ? kLineCells - 1 : 0)) / kLineCells;
+      const u32 lines = (at + end + (last ? kLineCells - 1 : 0)) / kLineCells;
       for (u32 j = (at + sent) / kLineCells; j < lines; ++j) {
         const u32 cell = j * kLineCells + lane - at;  // wraps in front of the row's first cell
         if (cell < end && (fill || cell <= wrote))
@@ -241,6 +244,7 @@ __global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u
       }
     }
     __syncwarp();
+    if (last) break;
     sent = end;
   }
   if (have) a.lengths[w] = len;
@@ -1292,17 +1296,18 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     const u64 read = ctx->E * (unbiased ? 4u : 12u);  // lists, and slots if they are drawn from
     const WalkGrid g = walk_grid(ctx, prm->app, n, prm->app == SKW_APP_DEEPWALK && read <= (8u << 20) ? 17 : 34, 1);
     const bool ahead = walk_ahead(ctx, prm->app, n, unbiased);
+    const size_t rings = home ? sizeof(u32) * (kWalkCta / 32) * g.lanes * (kLineRing + 1) : 0;
     switch (prm->app) {
       case SKW_APP_DEEPWALK:
-        if (home) {
-          const size_t rings = sizeof(u32) * (kWalkCta / 32) * g.lanes * (kLineRing + 1);
-          if (ahead) walk_home_kernel<true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
-          else walk_home_kernel<false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
-        } else if (ahead) walk_offline_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        if (home && ahead) walk_home_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        else if (home) walk_home_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        else if (ahead) walk_offline_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         else walk_offline_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         break;
       case SKW_APP_PPR:
-        if (ahead) walk_offline_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
+        if (home && ahead) walk_home_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        else if (home) walk_home_kernel<SKW_APP_PPR, false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        else if (ahead) walk_offline_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         else walk_offline_kernel<SKW_APP_PPR, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         break;
       default: {
@@ -1469,9 +1474,11 @@ static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
 // nobody has to queue, as long as every walker has a warp.  Calls, us, copied / written (R-MAT 16, 18, 20 and 22): 80 steps, 256
 // walkers 163-197 / 135-152, 4,096 177-194 / 140-148, 16,000 274-291 / 202-209, 29,600 359-385 / 295-311, and with the same
 // walks at every call 40,000 424-467 / 369-385, 80,000 642-809 / 681-722; 200 steps, 4,096 305-379 / 245-275, 16,000 539-605 /
-// 356-410; 10 steps, 256 73-77 / 59-60, 5,000 84-88 / 72-74, 10,000 86-90 / 78-89, 20,000 97-102 / 106-115.
+// 356-410; 10 steps, 256 73-77 / 59-60, 5,000 84-88 / 72-74, 10,000 86-90 / 78-89, 20,000 97-102 / 106-115.  PPR of at most
+// 100 steps, tp 0.15: 256 walkers 94-98 / 79-82, 4,096 151-165 / 108-112, 29,600 344-365 / 321-330; without filling the rows
+// 4,096 118-132 / 87-96, 29,600 201-218 / 123-131 (a kernel wrote the rows' cells behind the walks).
 static bool written_home(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
-  return n != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app == SKW_APP_DEEPWALK &&
+  return n != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app != SKW_APP_NODE2VEC &&
          prm->hop_num <= (1u << 24) &&  // the kernel counts up to a line past the row's end in 32 bits
          (prm->mode != SKW_MODE_ONLINE || (prm->flags & SKW_WALK_UNBIASED)) && !follows_records(ctx, prm);
 }

@@ -189,9 +189,10 @@ def test_packed_ppr_over_records(ctx, oracle, request, graph, hop, tp, n):
 
 
 @pytest.mark.parametrize("hop", [1, 2, 31, 32, 33, 81])
+@pytest.mark.parametrize("app", [APP_DEEPWALK, APP_PPR])
 @pytest.mark.parametrize("n,off,flags", [(1, 0, 0), (37, 5, 16), (4096, 31, 16), (4097, 2, 0), (9999, 1, 18)])
-def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, hop, n, off, flags):
-    """DeepWalk writes its rows into the caller's pinned matrix a 128-byte line at a time, wherever in a line a row starts (off
+def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, app, hop, n, off, flags):
+    """DeepWalk and PPR write their rows into the caller's pinned matrix a 128-byte line at a time, wherever in a line a row starts (off
     words).  Cells past a walk's end keep their contents or (16, fill rows) get the invalid vertex, words around the matrix
     keep theirs, and all of it equals the rows of pageable memory; 2: uniform draws."""
     import torch
@@ -201,7 +202,7 @@ def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, hop, n, off, flags
     starts = oracle.gen_starts(n, g.V, 11)
     paths = torch.full((n * hop + 64,), 0x5A5A5A5A, dtype=torch.int32).pin_memory()
     lengths = torch.full((n + 2,), 0x5A5A5A5A, dtype=torch.int32).pin_memory()
-    kw = dict(seed=6, walker_base=9, flags=flags)
+    kw = dict(app=app, tp=0.1, seed=6, walker_base=9, flags=flags)
     _, _, ms, edges = ctx.walk(starts, hop, paths=paths[off:off + n * hop], lengths=lengths[1:n + 1], **kw)
     p, l = paths.numpy().view(np.uint32), lengths.numpy().view(np.uint32)
     rows, lens = p[off:off + n * hop].reshape(n, hop), l[1:n + 1]
