@@ -182,17 +182,26 @@ __device__ __forceinline__ void khop_trees(const KhopArgs& a, u32 per_cta) {
   khop_add(a.sum, got_sum);
 }
 
-// A draw is a chain of dependent random accesses (parent, offsets, slot, neighbour), so the kernels that follow tables have as
-// many warps an SM as fit, 64 with 32 registers each: 65,536 x 25, 10 with the take-all rule 165 -> 153 us, with replacement 202
-// -> 195, 16,384 x 15, 10, 5 on a power-law graph 324 -> 291.  Uniform draws have an access less and are bound by the rate of
-// random accesses, and draws of distinct neighbours by their instructions: 152 -> 157 and 340 -> 356 us, so they keep 40
-// registers and 48 warps.
+// A draw is a chain of dependent random accesses (parent, offsets, slot, neighbour), so hops over tables have as many warps an
+// SM as fit, 64 with 32 registers each: 65,536 x 25, 10 with the take-all rule 165 -> 153 us, with replacement 202 -> 195.
+// Uniform draws have an access less and are bound by the rate of random accesses, and draws of distinct neighbours by their
+// instructions: 152 -> 157 and 340 -> 356 us, so they keep 40 registers and 48 warps (weighted_tree_warps has the rest).
 template <bool DISTINCT>
 __global__ void __launch_bounds__(256) khop_tree_kernel(const KhopArgs a, u32 per_cta) {
   khop_trees<DISTINCT>(a, per_cta);
 }
 __global__ void __launch_bounds__(256, 8) khop_weighted_tree_kernel(const KhopArgs a, u32 per_cta) {
   khop_trees<false>(a, per_cta);
+}
+
+// Whether trees of weighted draws take 64 warps an SM.  Trees of one or two hops do where 48 do not hold all CTAs (40 / 32
+// registers, us: 65,536 x 25, 10 on R-MAT and power-law graphs 126-212 / 117-199, 30,000 x 25, 10 60-98 / 59-89, 65,536 x 40
+// 33-42 / 31-40).  From three hops on the short hops between barriers are bound by instructions, and fewer registers
+// take more of them (65,536 x 5, 5, 3 100-128 / 105-138, 8,191 x 15, 10, 5 114-121 / 120-122), unless the eight CTAs an SM make
+// the difference between one wave and two (1,000 x 15, 10, 5 20-28 / 19-22, x 5, 5, 3 14-18 / 13-14).  Up to 48 warps an SM
+// more registers are never worse (380 x 15, 10, 5 16-18 / 16-18).
+static bool weighted_tree_warps(const skw_ctx* ctx, uint32_t nhops, uint64_t ctas) {
+  return ctas > ctx->sm_count * 6ull && (nhops <= 2 || ctas <= ctx->sm_count * 8ull);
 }
 
 // One hop of every tree (online mode, whose tables are built hop by hop, and trees that are too large for a CTA).  64 warps an SM,
@@ -390,7 +399,8 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
     const uint64_t ctas = (n + per_cta - 1) / per_cta;
     if (ctas <= 0x7FFFFFFFull) {
       if (distinct) khop_tree_kernel<true><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
-      else if (a.flags & SKW_KHOP_UNBIASED) khop_tree_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
+      else if ((a.flags & SKW_KHOP_UNBIASED) || !weighted_tree_warps(ctx, prm->nhops, ctas))
+        khop_tree_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
       else khop_weighted_tree_kernel<<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
       SKW_LAUNCHED(ctx);
       return SKW_OK;

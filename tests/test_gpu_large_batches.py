@@ -217,3 +217,19 @@ def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, app, hop, n, off, 
     odd = torch.zeros(n * hop * 4 + 4, dtype=torch.uint8).pin_memory().numpy()[2:2 + n * hop * 4].view(np.uint32)
     ctx.walk(starts, hop, paths=odd, lengths=wl, **kw)
     assert np.array_equal(odd.reshape(n, hop)[live], rows[live])
+
+
+@pytest.mark.parametrize("fanout", [[4, 3, 2], [5, 3]])
+@pytest.mark.parametrize("per_sm,more", [(6, 0), (6, 1), (8, 0), (8, 1)])
+def test_weighted_trees_around_whole_waves(ctx, oracle, rmat12, fanout, per_sm, more):
+    """Offline trees of weighted draws have two kernels, chosen by hops and by the CTAs an SM that the batch makes."""
+    import torch
+    g = rmat12
+    n = torch.cuda.get_device_properties(0).multi_processor_count * per_sm + more
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    table = oracle.alias_build(g.xadj, g.adjwgt)
+    seeds = oracle.gen_starts(n, g.V, 4)
+    data, sl, _, e = ctx.sample_khop(seeds, fanout, mode=MODE_OFFLINE, seed=5)
+    odata, osl = oracle.khop(g.xadj, g.adjncy, g.adjwgt, table, seeds, fanout, seed=5)
+    assert np.array_equal(data, odata) and np.array_equal(sl, osl) and e == int(osl.sum())
