@@ -233,6 +233,7 @@ __global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u
       }
     }
     step = end;
+    __syncwarp();  // every lane's cells are in its ring before other lanes read them: votes and shuffles do not order memory
     const bool last = !__any_sync(0xFFFFFFFFu, live) && !fill || end == a.hop_num;  // nothing follows for any of them
     for (u32 k = 0; k < walkers; ++k) {
       const u32 at = __shfl_sync(0xFFFFFFFFu, place, k), wrote = __shfl_sync(0xFFFFFFFFu, len, k);
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u
           a.paths[(first + k) * a.hop_num + cell] = warp_rings[k * (kLineRing + 1) + ((j * kLineCells + lane) & (kLineRing - 1))];
       }
     }
-    __syncwarp();
+    __syncwarp();  // and they are read before the next ones take their places
     if (last) break;
     sent = end;
   }
