@@ -269,8 +269,9 @@ int skw_ctx_take_sampled_edges(skw_ctx* ctx, uint64_t* out);
  * pinned memory (skw_host_alloc, cudaHostAlloc, cudaHostRegister) only the cells each walk wrote
  * (0 .. length) are transferred, by a kernel writing into the mapped host matrix; the other cells
  * keep what the caller had there.  With pageable memory the whole matrix is copied and cells past a
- * walk's end are unspecified.  Into pinned h_paths and h_lengths small DeepWalk and PPR batches over the table
- * are written by the walk kernel itself while they run; *ms then covers these writes. */
+ * walk's end are unspecified.  A call that a device error refuses has copied no row then.  With SKW_WALK_FILL_ROWS
+ * into pinned h_paths and h_lengths small DeepWalk and PPR batches over the table are written by the walk kernel itself
+ * while they run; *ms then covers these writes. */
 int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts, uint64_t n,
              uint32_t* h_paths, uint32_t* h_lengths, float* ms, uint64_t* sampled_edges);
 /* Host buffers, packed result.  No counterpart in the reference, which leaves results on the

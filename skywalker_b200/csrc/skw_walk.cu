@@ -189,10 +189,10 @@ __global__ void __launch_bounds__(kWalkCta) walk_offline_kernel(const WalkArgs a
 // while the walks are under way instead of behind them.  The bus carries a write of a sector with about as many bytes of its
 // own, and single cells at a fraction of its rate.  So cells wait in shared memory, two 128-byte lines of the matrix a walker
 // (rows start anywhere in a line), and every 32 steps the warp writes the line that each of its walkers has filled; when in the
-// 32 steps differs from warp to warp.  fill: cells past a walk's end get kNoVertex, otherwise they keep what they held.
+// 32 steps differs from warp to warp.  Cells past a walk's end get kNoVertex.
 constexpr u32 kLineCells = 32, kLineRing = 2 * kLineCells;
 template <int APP, bool AHEAD>
-__global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u32 lanes, u32 fill) {
+__global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u32 lanes) {
   extern __shared__ u32 rings[];  // a ring a walker, an odd number of words apart
   const u32 lane = threadIdx.x & 31, warp = blockIdx.x * (kWalkCta / 32) + threadIdx.x / 32;
   u32* const warp_rings = rings + threadIdx.x / 32 * lanes * (kLineRing + 1);
@@ -233,19 +233,17 @@ __global__ void __launch_bounds__(kWalkCta) walk_home_kernel(const WalkArgs a, u
       }
     }
     step = end;
-    __syncwarp();  // every lane's cells are in its ring before other lanes read them: votes and shuffles do not order memory
-    const bool last = !__any_sync(0xFFFFFFFFu, live) && !fill || end == a.hop_num;  // nothing follows for any of them
+    __syncwarp();  // every lane's cells are in its ring before other lanes read them: shuffles do not order memory
     for (u32 k = 0; k < walkers; ++k) {
-      const u32 at = __shfl_sync(0xFFFFFFFFu, place, k), wrote = __shfl_sync(0xFFFFFFFFu, len, k);
-      const u32 lines = (at + end + (last ? kLineCells - 1 : 0)) / kLineCells;
+      const u32 at = __shfl_sync(0xFFFFFFFFu, place, k);
+      const u32 lines = (at + end + (end == a.hop_num ? kLineCells - 1 : 0)) / kLineCells;
       for (u32 j = (at + sent) / kLineCells; j < lines; ++j) {
         const u32 cell = j * kLineCells + lane - at;  // wraps in front of the row's first cell
-        if (cell < end && (fill || cell <= wrote))
+        if (cell < end)
           a.paths[(first + k) * a.hop_num + cell] = warp_rings[k * (kLineRing + 1) + ((j * kLineCells + lane) & (kLineRing - 1))];
       }
     }
     __syncwarp();  // and they are read before the next ones take their places
-    if (last) break;
     sent = end;
   }
   if (have) a.lengths[w] = len;
@@ -1231,10 +1229,10 @@ static bool ppr_by_chunks(const skw_ctx* ctx, const skw_walk_params* prm, u64 n)
 // Queue the kernels of one batch of walkers on the context's stream; sampled edges are added to *sum.
 // No reset, no readback, no synchronisation (the online paths allocate on first use).  whole_table: the
 // slots that online_tables gave for the call.  d_heads: where ppr_by_chunks may leave the first cells of the rows instead.
-// home: the rows are written_home's, fill: cells past a walk's end are overwritten there.
+// home: the rows are written_home's.
 static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n,
                        uint32_t* d_paths, uint32_t* d_lengths, unsigned long long* sum, const Slot* whole_table,
-                       uint32_t* d_heads = nullptr, bool home = false, bool fill = false) {
+                       uint32_t* d_heads = nullptr, bool home = false) {
   const bool unbiased = (prm->flags & SKW_WALK_UNBIASED) != 0;
   const bool online = prm->mode == SKW_MODE_ONLINE && !unbiased;
   int rc;
@@ -1300,14 +1298,14 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
     const size_t rings = home ? sizeof(u32) * (kWalkCta / 32) * g.lanes * (kLineRing + 1) : 0;
     switch (prm->app) {
       case SKW_APP_DEEPWALK:
-        if (home && ahead) walk_home_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
-        else if (home) walk_home_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        if (home && ahead) walk_home_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes);
+        else if (home) walk_home_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes);
         else if (ahead) walk_offline_kernel<SKW_APP_DEEPWALK, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         else walk_offline_kernel<SKW_APP_DEEPWALK, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         break;
       case SKW_APP_PPR:
-        if (home && ahead) walk_home_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
-        else if (home) walk_home_kernel<SKW_APP_PPR, false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes, fill);
+        if (home && ahead) walk_home_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes);
+        else if (home) walk_home_kernel<SKW_APP_PPR, false><<<g.ctas, kWalkCta, rings, st>>>(a, g.lanes);
         else if (ahead) walk_offline_kernel<SKW_APP_PPR, true><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         else walk_offline_kernel<SKW_APP_PPR, false><<<g.ctas, kWalkCta, 0, st>>>(a, g.lanes);
         break;
@@ -1345,7 +1343,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
 // A synchronous walk over device buffers; with h_lengths the lengths, with h_paths the whole matrix comes home as well.
 static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* d_starts, uint64_t n, uint32_t* d_paths,
                          uint32_t* d_lengths, uint32_t* h_lengths, uint32_t* h_paths, float* ms,
-                         uint64_t* sampled_edges, bool home = false, bool fill = false) {
+                         uint64_t* sampled_edges, bool home = false) {
   cudaStream_t st = ctx->stream;
   int rc = err_reset(ctx);
   if (rc != SKW_OK) return rc;
@@ -1353,7 +1351,7 @@ static int walk_and_wait(skw_ctx* ctx, const skw_walk_params* prm, const uint32_
   OnlineTables tables(ctx);
   if ((rc = online_tables(prm, n, tables)) != SKW_OK) return rc;
   if ((rc = walk_launch(ctx, prm, d_starts, n, d_paths, d_lengths, reinterpret_cast<unsigned long long*>(ctx->d_sum),
-                        tables.slots, nullptr, home, fill)) != SKW_OK)
+                        tables.slots, nullptr, home)) != SKW_OK)
     return rc;
   if (ms) SKW_CUDA(ctx, cudaEventRecord(ctx->ev1, st));
   if (h_lengths && n) SKW_CUDA(ctx, cudaMemcpyAsync(h_lengths, d_lengths, sizeof(u32) * (size_t)n, cudaMemcpyDeviceToHost, st));
@@ -1476,10 +1474,12 @@ static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
 // walkers 163-197 / 135-152, 4,096 177-194 / 140-148, 16,000 274-291 / 202-209, 29,600 359-385 / 295-311, and with the same
 // walks at every call 40,000 424-467 / 369-385, 80,000 642-809 / 681-722; 200 steps, 4,096 305-379 / 245-275, 16,000 539-605 /
 // 356-410; 10 steps, 256 73-77 / 59-60, 5,000 84-88 / 72-74, 10,000 86-90 / 78-89, 20,000 97-102 / 106-115.  PPR of at most
-// 100 steps, tp 0.15: 256 walkers 94-98 / 79-82, 4,096 151-165 / 108-112, 29,600 344-365 / 321-330; without filling the rows
-// 4,096 118-132 / 87-96, 29,600 201-218 / 123-131 (a kernel wrote the rows' cells behind the walks).
+// 100 steps, tp 0.15: 256 walkers 94-98 / 79-82, 4,096 151-165 / 108-112, 29,600 344-365 / 321-330.
+// Only where the whole matrix comes home whatever happens, as it does where rows are filled.  Where they are not, cells past
+// a walk's end keep what the caller had there, and so do all of them when a walk meets a vertex that does not exist: rows are
+// not written before the whole batch is known to be good.
 static bool written_home(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
-  return n != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app != SKW_APP_NODE2VEC &&
+  return n != 0 && (prm->flags & SKW_WALK_FILL_ROWS) != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app != SKW_APP_NODE2VEC &&
          prm->hop_num <= (1u << 24) &&  // the kernel counts up to a line past the row's end in 32 bits
          (prm->mode != SKW_MODE_ONLINE || (prm->flags & SKW_WALK_UNBIASED)) && !follows_records(ctx, prm);
 }
@@ -1498,19 +1498,19 @@ int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts,
   }
   const size_t nb = sizeof(uint32_t) * (size_t)n;
   if ((rc = ensure_bytes(ctx, &ctx->stage[0], &ctx->stage_bytes[0], nb)) != SKW_OK) return rc;
-  const bool fill = (prm->flags & SKW_WALK_FILL_ROWS) != 0;
   if (written_home(ctx, prm, n)) {
     u32* const rows = seen_by_gpu(h_paths, n * prm->hop_num);
     u32* const lengths = rows ? seen_by_gpu(h_lengths, n) : nullptr;
     if (lengths) {
       SKW_CUDA(ctx, cudaMemcpyAsync(ctx->stage[0], h_starts, nb, cudaMemcpyHostToDevice, ctx->stream));
       return walk_and_wait(ctx, prm, static_cast<uint32_t*>(ctx->stage[0]), n, rows, lengths, nullptr, nullptr, ms, sampled_edges,
-                           true, fill);
+                           true);
     }
   }
   if ((rc = ensure_bytes(ctx, &ctx->stage[1], &ctx->stage_bytes[1], nb * prm->hop_num)) != SKW_OK) return rc;
   if ((rc = ensure_bytes(ctx, &ctx->stage[2], &ctx->stage_bytes[2], nb)) != SKW_OK) return rc;
   if (n) SKW_CUDA(ctx, cudaMemcpyAsync(ctx->stage[0], h_starts, nb, cudaMemcpyHostToDevice, ctx->stream));
+  const bool fill = (prm->flags & SKW_WALK_FILL_ROWS) != 0;
   if (n && fill) SKW_CUDA(ctx, cudaMemsetAsync(ctx->stage[1], 0xFF, nb * prm->hop_num, ctx->stream));
   uint64_t edges = 0;
   rc = walk_and_wait(ctx, prm, static_cast<uint32_t*>(ctx->stage[0]), n, static_cast<uint32_t*>(ctx->stage[1]),

@@ -18,6 +18,8 @@ std::recursive_mutex mu;
 std::string log_text;
 std::map<const void*, std::string> kernels;
 std::unordered_map<void*, size_t> device_blocks;
+std::map<uintptr_t, size_t> host_blocks;
+bool pinned_seen = false;  // whether pinned host memory is reported as such
 cudaError_t last_error = cudaSuccess;
 long malloc_good = -1, malloc_bad = 0, host_good = -1, host_bad = 0;  // so many succeed, then so many fail
 size_t device_total = (size_t)64 << 30, device_used = 0;
@@ -61,6 +63,7 @@ void fake_fail_host_malloc(long after, long times) {
   host_bad = times;
 }
 void fake_memory(size_t total) { device_total = total; }
+void fake_pinned(int on) { pinned_seen = on != 0; }
 void fake_capture(int on) { capturing = on != 0; }
 size_t fake_used() { return device_used; }
 void fake_clear_log() { log_text.clear(); }
@@ -126,12 +129,14 @@ cudaError_t cudaMallocHost(void** p, size_t bytes) {
   note(std::string("host_malloc ") + (no ? "fail" : "ok"));
   if (no) return set(cudaErrorMemoryAllocation);
   *p = calloc(1, bytes ? bytes : 1);
+  host_blocks[reinterpret_cast<uintptr_t>(*p)] = bytes;
   return cudaSuccess;
 }
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) { return cudaMallocHost(p, bytes); }
 cudaError_t cudaFreeHost(void* p) {
   std::lock_guard<std::recursive_mutex> l(mu);
   note("host_free");
+  host_blocks.erase(reinterpret_cast<uintptr_t>(p));
   free(p);
   return cudaSuccess;
 }
@@ -164,6 +169,11 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   memset(a, 0, sizeof *a);
   const bool device = device_blocks.count(const_cast<void*>(p)) != 0;
   a->type = device ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
+  auto it = host_blocks.upper_bound(reinterpret_cast<uintptr_t>(p));
+  if (pinned_seen && it != host_blocks.begin() && reinterpret_cast<uintptr_t>(p) < (--it)->first + it->second) {
+    a->type = cudaMemoryTypeHost;
+    a->devicePointer = a->hostPointer = const_cast<void*>(p);
+  }
   return cudaSuccess;
 }
 

@@ -111,6 +111,22 @@ def test_error_of_a_queued_walk_waits_for_its_own_report(ctx, oracle, rmat12, kw
     assert ctx.take_sampled_edges() == 0
 
 
+@pytest.mark.parametrize("kw", [dict(), dict(app=APP_PPR, tp=0.1), dict(flags=2)])
+def test_rows_of_a_failed_walk_are_not_written(ctx, oracle, rmat12, kw):
+    """A start vertex that does not exist fails the call; rows that are not to be filled keep what they held."""
+    import torch
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    bad = oracle.gen_starts(300, g.V, 3)
+    bad[7] = g.V + 7
+    paths = torch.full((300, 11), 5, dtype=torch.int32).pin_memory()
+    lengths = torch.zeros(300, dtype=torch.int32).pin_memory()
+    with pytest.raises(SkwError):
+        ctx.walk(bad, 11, seed=5, paths=paths, lengths=lengths, **kw)
+    assert (paths == 5).all()
+
+
 def test_class_counters_across_calls_and_streams(oracle, plaw):
     """Builds take zeroed counters from a few sets that the status kernel clears: more builds in one call than there are
     sets, queued builds whose call nothing waits for, and builds on another stream behind them."""

@@ -304,6 +304,26 @@ assert (paths == 5).all() and (lengths == 5).all()
 """ % (n, n, n))
 
 
+def test_rows_are_written_home_only_where_they_are_filled(fake_cudart):
+    """Without the flag that fills the rows no row is written before the whole batch is known to be good."""
+    _run(fake_cudart, """
+fake.fake_pinned(1)
+ctx = Context(0)
+ctx.upload(*ring())
+ctx.alias_build_offline()
+from skywalker_b200.api import _results
+paths, lengths = _results.array((300, 81)), _results.array((300,))
+for app in (0, 1):
+    for unbiased in (0, 2):
+        for fill in (0, 16):
+            calls()
+            ctx.walk(np.zeros(300, np.uint32), 81, app=app, tp=0.15, paths=paths, lengths=lengths, flags=unbiased | fill)
+            log = calls()
+            assert len(launches(log, "walk_home_kernel")) == (fill != 0), log
+            assert len(launches(log, "walk_offline_kernel")) == (fill == 0), log
+""")
+
+
 def test_freed_device_memory_waits_within_bounds(fake_cudart):
     """Freed blocks serve the next graph, up to a sixteenth of the memory, and are returned when an allocation fails
     without them, on request, and with the last context."""
