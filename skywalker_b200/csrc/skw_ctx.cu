@@ -269,12 +269,20 @@ static void free_graph(skw_ctx* ctx) {
   ctx->max_degree = 0;
   ctx->empty_lists = 0;
   ctx->long_lists = 0;
+  ctx->dead_ends = 0;
 }
 
-// out[0]: the largest degree, out[1]: the number of vertices of degree 0, longs: of those of degree 16385 to 65536
+// out[0]: the largest degree, out[1]: the number of vertices of degree 0, longs: of those of degree 16385 to 65536, ends: of
+// the sampled edges into vertices of degree 0
 __global__ void max_degree_kernel(const uint32_t* __restrict__ xadj, uint32_t V,
-                                  uint32_t* __restrict__ out, uint32_t* __restrict__ longs) {
+                                  uint32_t* __restrict__ out, uint32_t* __restrict__ longs,
+                                  const uint32_t* __restrict__ adjncy, uint64_t E, uint32_t* __restrict__ ends) {
   uint32_t m = 0, empty = 0;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < skw_ctx::kEdgeSample && E) {
+    const uint32_t to = adjncy[i * E / skw_ctx::kEdgeSample];
+    if (to < V && xadj[to] == xadj[to + 1]) atomicAdd(ends, 1u);
+  }
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < V;
        v += (size_t)gridDim.x * blockDim.x) {
     const uint32_t d = xadj[v + 1] - xadj[v];
@@ -430,7 +438,8 @@ int finish_graph(skw_ctx* ctx) {
   SKW_CUDA(ctx, cudaMemsetAsync(ctx->d_sum + 2, 0, sizeof(uint64_t), ctx->stream));
   if (ctx->V) {
     max_degree_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(
-        ctx->xadj, ctx->V, reinterpret_cast<uint32_t*>(ctx->d_sum), reinterpret_cast<uint32_t*>(ctx->d_sum + 2));
+        ctx->xadj, ctx->V, reinterpret_cast<uint32_t*>(ctx->d_sum), reinterpret_cast<uint32_t*>(ctx->d_sum + 2), ctx->adjncy, ctx->E,
+        reinterpret_cast<uint32_t*>(ctx->d_sum + 2) + 1);
     SKW_LAUNCHED(ctx);
   }
   SKW_CUDA(ctx, cudaMemcpyAsync(ctx->h_sum, ctx->d_sum, sizeof(uint64_t), cudaMemcpyDeviceToHost,
@@ -439,6 +448,7 @@ int finish_graph(skw_ctx* ctx) {
   SKW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->max_degree = (uint32_t)*ctx->h_sum;
   ctx->long_lists = (uint32_t)ctx->h_sum[2];
+  ctx->dead_ends = (uint32_t)(ctx->h_sum[2] >> 32);
   ctx->empty_lists = (uint32_t)(*ctx->h_sum >> 32);
   ctx->status_clean = false;
   return SKW_OK;

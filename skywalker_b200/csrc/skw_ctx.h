@@ -50,6 +50,8 @@ struct skw_ctx {
   uint32_t max_degree = 0;
   uint32_t empty_lists = 0;  // vertices without out-edges
   uint32_t long_lists = 0;   // vertices of degree 16385 to 65536
+  static constexpr uint32_t kEdgeSample = 4096;
+  uint32_t dead_ends = 0;    // of kEdgeSample edges spread over the list of all, those into vertices without out-edges
   uint32_t* xadj = nullptr;
   uint32_t* adjncy = nullptr;
   float* adjwgt = nullptr;
@@ -120,7 +122,7 @@ struct skw_ctx {
 namespace skw {
 
 int fail(skw_ctx* ctx, int code, const char* fmt, ...);
-// after the CSR pointers are set: compute max_degree and empty_lists
+// after the CSR pointers are set: compute max_degree, empty_lists, long_lists and dead_ends
 int finish_graph(skw_ctx* ctx);
 // allocate slots[E] / valid[V] if absent; a call that writes only a part of the table has the rest marked unusable
 enum class TableUse {

@@ -1475,10 +1475,22 @@ static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
 // walks at every call 40,000 424-467 / 369-385, 80,000 642-809 / 681-722; 200 steps, 4,096 305-379 / 245-275, 16,000 539-605 /
 // 356-410; 10 steps, 256 73-77 / 59-60, 5,000 84-88 / 72-74, 10,000 86-90 / 78-89, 20,000 97-102 / 106-115.  PPR of at most
 // 100 steps, tp 0.15: 256 walkers 94-98 / 79-82, 4,096 151-165 / 108-112, 29,600 344-365 / 321-330.
+// Beyond the end of the longest walk nothing hides the writes.  It is estimated from what ends a walk, the PPR draw and the
+// edges into vertices without out-edges: the rows go home this way as long as the cells behind it are at most 2.5 MB, which is
+// about what the copy's own launches cost, and at most 160 a row, which a warp writes one line after another.  Copied /
+// written: PPR, tp 0.15, R-MAT 18, 4,096 x 201 185 / 150, 29,600 x 81 325 / 321, but 10,000 x 501 491 / 563, 29,600 x 201
+// 579 / 626, 256 x 1,001 125 / 188; DeepWalk on a graph whose walks are over after a step 4,096 x 81 98 / 92, but
+// 29,600 x 81 266 / 329, 4,096 x 501 223 / 230, 29,600 x 33 164 / 178; on R-MAT 18, where one edge of a hundred (directed)
+// or none leads to such a vertex, 29,600 x 201 799 / 675 and 805 / 629, 4,096 x 1,001 1,194 / 943 and 1,316 / 1,089.
 // Only where the whole matrix comes home whatever happens, as it does where rows are filled.  Where they are not, cells past
 // a walk's end keep what the caller had there, and so do all of them when a walk meets a vertex that does not exist: rows are
 // not written before the whole batch is known to be good.
 static bool written_home(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
+  const double into_ends = (double)ctx->dead_ends / skw_ctx::kEdgeSample;
+  const double stop = prm->app == SKW_APP_PPR ? prm->tp + (1.0 - prm->tp) * into_ends : into_ends;  // a step's chance to be the last
+  const double longest = stop <= 0.0 ? prm->hop_num : stop >= 1.0 ? 0.0 : log((double)n) / -log1p(-stop);
+  const double behind = prm->hop_num - std::min<double>(prm->hop_num, longest);
+  if (behind > 160.0 || behind * (double)n * sizeof(u32) > 2.5e6) return false;
   return n != 0 && (prm->flags & SKW_WALK_FILL_ROWS) != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app != SKW_APP_NODE2VEC &&
          prm->hop_num <= (1u << 24) &&  // the kernel counts up to a line past the row's end in 32 bits
          (prm->mode != SKW_MODE_ONLINE || (prm->flags & SKW_WALK_UNBIASED)) && !follows_records(ctx, prm);

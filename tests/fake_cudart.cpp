@@ -98,6 +98,10 @@ cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cud
     const unsigned V = *static_cast<unsigned*>(args[1]);
     unsigned* out = *static_cast<unsigned**>(args[2]);
     for (unsigned v = 0; v < V; ++v) *out = xadj[v + 1] - xadj[v] > *out ? xadj[v + 1] - xadj[v] : *out;
+    const unsigned* adjncy = *static_cast<const unsigned**>(args[4]);
+    const unsigned long long E = *static_cast<unsigned long long*>(args[5]);
+    unsigned* ends = *static_cast<unsigned**>(args[6]);
+    for (unsigned i = 0; i < 4096 && E; ++i) *ends += xadj[adjncy[i * E / 4096]] == xadj[adjncy[i * E / 4096] + 1];
   }
   return cudaSuccess;
 }

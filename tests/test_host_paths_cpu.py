@@ -324,6 +324,31 @@ for app in (0, 1):
 """)
 
 
+@pytest.mark.parametrize("ends,app,tp,n,hop,home", [
+    (False, 0, 0.0, 29600, 201, True), (False, 0, 0.0, 4096, 1001, True), (False, 0, 0.0, 29601, 81, False),
+    (False, 0, 0.0, 5032, 32, True), (False, 0, 0.0, 5033, 32, False), (True, 0, 0.0, 4096, 81, True),
+    (True, 0, 0.0, 29600, 81, False), (True, 0, 0.0, 29600, 33, False), (True, 0, 0.0, 256, 161, False),
+    (False, 1, 0.15, 4096, 201, True), (False, 1, 0.15, 29600, 81, True), (True, 1, 0.15, 29600, 81, False),
+    (False, 1, 0.15, 29600, 201, False), (False, 1, 0.15, 10000, 501, False), (False, 1, 0.15, 256, 1001, False),
+    (False, 1, 0.0, 4096, 1001, True), (False, 1, 1.0, 4096, 101, True), (False, 1, 1.0, 10000, 101, False)])
+def test_rows_are_written_home_where_walks_hide_it(fake_cudart, ends, app, tp, n, hop, home):
+    """Walks hide the writes only while they last; matrices whose cells mostly lie behind the ends of all walks are copied."""
+    _run(fake_cudart, """
+fake.fake_pinned(1)
+ctx = Context(0)
+x, a, w = ring()
+if %r:                                  # every edge leads to a vertex without out-edges
+    x = np.concatenate([x, np.full(10, x[-1])]).astype(np.uint32)
+    a[:] = 1000
+ctx.upload(x, a, w)
+ctx.alias_build_offline()
+calls()
+ctx.walk(np.zeros(%d, np.uint32), %d, app=%d, tp=%g)
+log = calls()
+assert len(launches(log, "walk_home_kernel")) == %d and len(launches(log, "walk_offline_kernel")) == %d
+""" % (ends, n, hop, app, tp, home, not home))
+
+
 def test_freed_device_memory_waits_within_bounds(fake_cudart):
     """Freed blocks serve the next graph, up to a sixteenth of the memory, and are returned when an allocation fails
     without them, on request, and with the last context."""
