@@ -161,6 +161,13 @@ cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes) {
     drop_online_tables(ctx);
     e = DeviceMemory::get().alloc(p, bytes);
   }
+  if (e == cudaErrorMemoryAllocation && ctx->stage[skw_ctx::kHeadStage] && !ctx->heads_in_use) {
+    cudaGetLastError();
+    dev_free(ctx->stage[skw_ctx::kHeadStage]);
+    ctx->stage[skw_ctx::kHeadStage] = nullptr;
+    ctx->stage_bytes[skw_ctx::kHeadStage] = 0;
+    e = DeviceMemory::get().alloc(p, bytes);
+  }
   return e;
 }
 

@@ -117,6 +117,8 @@ struct skw_ctx {
   static constexpr int kStages = 14;
   void* stage[kStages] = {};
   size_t stage_bytes[kStages] = {};
+  static constexpr int kHeadStage = kStages - 1;  // for speed only: given up when another allocation fails
+  bool heads_in_use = false;
 };
 
 namespace skw {
@@ -145,7 +147,7 @@ void drop_online_tables(skw_ctx* ctx);
 // forget the fused walk records (they are derived from the table and die with it) and free their memory
 void drop_records(skw_ctx* ctx);
 // Device memory, from blocks freed earlier where one fits; gives up the memory of records that are no longer valid, then
-// that of an online call's tables, before it fails.  dev_free waits for the GPU.
+// that of an online call's tables, then that for heads of rows, before it fails.  dev_free waits for the GPU.
 cudaError_t dev_malloc_bytes(skw_ctx* ctx, void** p, size_t bytes);
 template <class T>
 cudaError_t dev_malloc(skw_ctx* ctx, T** p, size_t bytes) {

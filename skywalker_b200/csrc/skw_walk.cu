@@ -1549,10 +1549,10 @@ int skw_walk(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts,
 }  // extern "C"
 
 // The packed host entry points: lengths come home as 32-bit words (h_lengths) or, for walks of at
-// most 256 vertices, as bytes (h_lengths8); exactly one of the two is given.
+// most 256 vertices, as bytes (h_lengths8); exactly one of the two is given.  use_heads: where that pays and there is memory.
 static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t* h_starts, uint64_t n,
                             uint32_t* h_packed, uint64_t capacity_cells, uint32_t* h_lengths,
-                            uint8_t* h_lengths8, uint64_t* cells, float* ms, uint64_t* sampled_edges) {
+                            uint8_t* h_lengths8, uint64_t* cells, float* ms, uint64_t* sampled_edges, bool use_heads = true) {
   if (!ctx || !prm) return SKW_ERR_ARG;
   if (!cells) return fail(ctx, SKW_ERR_ARG, "skw_walk_packed: cells must not be null");
   *cells = 0;
@@ -1603,17 +1603,11 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
   if ((rc = ensure_bytes(ctx, &ctx->stage[2], &ctx->stage_bytes[2], sizeof(u32) * (size_t)n)) != SKW_OK) return rc;
   if ((rc = ensure_bytes(ctx, &ctx->stage[3], &ctx->stage_bytes[3], offs_bytes + tmp_bytes)) != SKW_OK) return rc;
   constexpr int kLen8Stage = 4 + skw_ctx::kPackSlices;
-  constexpr int kHeadStage = kLen8Stage + 1;
-  static_assert(skw_ctx::kStages > kHeadStage, "two more staging buffers for byte lengths and heads of rows");
+  constexpr int kHeadStage = skw_ctx::kHeadStage;
+  static_assert(kHeadStage > kLen8Stage, "two more staging buffers for byte lengths and heads of rows");
   if (h_lengths8 && (rc = ensure_bytes(ctx, &ctx->stage[kLen8Stage], &ctx->stage_bytes[kLen8Stage], (size_t)n)) != SKW_OK)
     return rc;
   uint8_t* d_len8 = h_lengths8 ? static_cast<uint8_t*>(ctx->stage[kLen8Stage]) : nullptr;
-  // PPR walks mostly end within the first cells of their rows.  Written to the rows, 404 bytes apart for 100 steps, these are
-  // isolated sectors, a third of the walk's time, and read back as such; side by side both are streams.
-  // (Without memory for them the rows will do.)
-  const bool heads = ppr_by_chunks(ctx, prm, n) && ensure_bytes(ctx, &ctx->stage[kHeadStage], &ctx->stage_bytes[kHeadStage],
-                                                                sizeof(u32) * kStage * (size_t)n) == SKW_OK;
-  if (!heads) cudaGetLastError();
   u32* d_starts = static_cast<u32*>(ctx->stage[0]);
   u32* d_rows = static_cast<u32*>(ctx->stage[1]);
   u32* d_len = static_cast<u32*>(ctx->stage[2]);
@@ -1636,6 +1630,18 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
     if ((rc = ensure_bytes(ctx, &ctx->stage[4 + c], &ctx->stage_bytes[4 + c], sizeof(u32) * (size_t)guess)) != SKW_OK) return rc;
     cap[c] = std::min<uint64_t>(ctx->stage_bytes[4 + c] / sizeof(u32), full);
   }
+  // PPR walks mostly end within the first cells of their rows.  Written to the rows, 404 bytes apart for 100 steps, these are
+  // isolated sectors, a third of the walk's time, and read back as such; side by side both are streams.
+  // Without memory for them the rows will do, so they come behind everything that the call cannot do without.
+  const bool heads = use_heads && ppr_by_chunks(ctx, prm, n) &&
+                     ensure_bytes(ctx, &ctx->stage[kHeadStage], &ctx->stage_bytes[kHeadStage],
+                                  sizeof(u32) * kStage * (size_t)n) == SKW_OK;
+  struct InUse {
+    bool& flag;
+    InUse(bool& f, bool used) : flag(f) { flag = used; }
+    ~InUse() { flag = false; }
+  } heads_in_use(ctx->heads_in_use, heads);
+  bool outgrown = false;  // a packed slice for which there is no memory
   if ((rc = err_reset(ctx)) != SKW_OK) return rc;
   unsigned long long* scratch_sum = reinterpret_cast<unsigned long long*>(ctx->d_sum) + 2;
   auto heads_of = [&](uint32_t c) -> u32* {
@@ -1714,7 +1720,10 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
         // still on the device).  Growing frees the old buffer, which waits for the device.
         const uint64_t roomy = std::min<uint64_t>(slice_cells + (slice_cells >> 3) + 4096, nc_of[c] * prm->hop_num);
         int r = ensure_bytes(ctx, &ctx->stage[4 + c], &ctx->stage_bytes[4 + c], sizeof(u32) * (size_t)roomy);
-        if (r != SKW_OK) return r;
+        if (r != SKW_OK) {
+          outgrown = true;
+          return r;
+        }
         cap[c] = roomy;
         if ((r = scan_and_pack(c)) != SKW_OK) return r;
         SKW_CUDA(ctx, cudaEventSynchronize(ctx->pk_ready[c]));
@@ -1752,6 +1761,10 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
     cudaStreamSynchronize(ctx->copy_stream);
     cudaStreamSynchronize(st);
     ctx->err = why;
+  }
+  if (rc != SKW_OK && outgrown && heads) {  // the memory of the heads may be what is missing: once more without them
+    ctx->heads_in_use = false;
+    return walk_packed_impl(ctx, prm, h_starts, n, h_packed, capacity_cells, h_lengths, h_lengths8, cells, ms, sampled_edges, false);
   }
   return rc;
 }

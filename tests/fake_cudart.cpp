@@ -22,6 +22,7 @@ std::map<uintptr_t, size_t> host_blocks;
 bool pinned_seen = false;  // whether pinned host memory is reported as such
 cudaError_t last_error = cudaSuccess;
 long malloc_good = -1, malloc_bad = 0, host_good = -1, host_bad = 0;  // so many succeed, then so many fail
+unsigned long long packed_total = 0;
 size_t device_total = (size_t)64 << 30, device_used = 0;
 bool capturing = false;
 struct Config {
@@ -63,6 +64,7 @@ void fake_fail_host_malloc(long after, long times) {
   host_bad = times;
 }
 void fake_memory(size_t total) { device_total = total; }
+void fake_packed(unsigned long long cells) { packed_total = cells; }
 void fake_pinned(int on) { pinned_seen = on != 0; }
 void fake_capture(int on) { capturing = on != 0; }
 size_t fake_used() { return device_used; }
@@ -103,6 +105,9 @@ cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cud
     unsigned* ends = *static_cast<unsigned**>(args[6]);
     for (unsigned i = 0; i < 4096 && E; ++i) *ends += xadj[adjncy[i * E / 4096]] == xadj[adjncy[i * E / 4096] + 1];
   }
+  // the number of cells that the packing kernels report, if a test wants some
+  if (packed_total && kernels[f].find("pack_rows_kernel") != std::string::npos) **static_cast<unsigned long long**>(args[7]) = packed_total;
+  if (packed_total && kernels[f].find("pack_heads_kernel") != std::string::npos) **static_cast<unsigned long long**>(args[8]) = packed_total;
   return cudaSuccess;
 }
 

@@ -349,6 +349,53 @@ assert len(launches(log, "walk_home_kernel")) == %d and len(launches(log, "walk_
 """ % (ends, n, hop, app, tp, home, not home))
 
 
+def test_packed_ppr_without_memory_for_heads(fake_cudart):
+    """The first cells of the rows travel apart from them where there is memory: it is asked for behind everything that
+    the call needs, and given up when another allocation fails, also in the middle of a call."""
+    _run(fake_cudart, """
+n, hop, MB = 200000, 101, 1 << 20
+kw = dict(app=1, tp=0.15)
+def context():
+    ctx = Context(0)
+    ctx.upload(*ring())
+    ctx.alias_build_offline()
+    ctx.walk_records_build()
+    ctx.walk(np.zeros(10, np.uint32), 5)
+    calls()
+    return ctx
+starts, packed, lengths = np.zeros(n, np.uint32), np.zeros(4000000, np.uint32), np.zeros(n, np.uint32)
+def walk(ctx):
+    used = fake.fake_used()
+    ctx.walk_packed(starts, hop, packed=packed, lengths=lengths, **kw)
+    log = calls()
+    return len(launches(log, "pack_heads")), len(launches(log, "pack_rows")), (fake.fake_used() - used) / MB
+ctx = context()
+heads, rows, need = walk(ctx)
+assert (heads, rows) == (1, 0) and need > 90
+ctx.close()
+# two megabytes less than all of it: enough without the heads
+ctx = context()
+fake.fake_memory(int(fake.fake_used() + (need - 2) * MB))
+assert walk(ctx)[:2] == (0, 1)
+fake.fake_memory(64 << 30)
+assert walk(ctx)[:2] == (1, 0)
+# kept for the next call, given up for another allocation
+fake.fake_memory(fake.fake_used() + MB)
+assert walk(ctx)[:2] == (1, 0)
+n += 10000                       # four megabytes of rows more
+starts, lengths = np.zeros(n, np.uint32), np.zeros(n, np.uint32)
+assert walk(ctx)[:2] == (0, 1)
+fake.fake_memory(64 << 30)
+assert walk(ctx)[:2] == (1, 0)
+# a result that outgrows its buffer in a call that holds the heads
+fake.fake_memory(fake.fake_used() + MB)
+fake.fake_packed(3600000)
+assert walk(ctx)[:2] == (1, 2)
+fake.fake_memory(64 << 30)
+assert walk(ctx)[:2] == (1, 0)
+""")
+
+
 def test_freed_device_memory_waits_within_bounds(fake_cudart):
     """Freed blocks serve the next graph, up to a sixteenth of the memory, and are returned when an allocation fails
     without them, on request, and with the last context."""
