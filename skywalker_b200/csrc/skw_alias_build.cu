@@ -54,7 +54,8 @@ constexpr u32 kListEpt = 16;
 constexpr u32 kGroupMax = 32 * kListEpt;      // 512: the longest list of a group of lanes
 constexpr u32 kMidSmemMax = 512 * kWideEpt;   // 8192: two CTAs of 512 threads an SM, 84 KB of lists each
 constexpr u32 kHugeSmemMax = 1024 * kWideEpt;  // 16384: one of 1024 threads; longer lists are in global memory
-constexpr u32 kAloneMax = 65536;              // longer ones are always built by clusters
+constexpr u32 kAloneMax = skw_ctx::kLongMost;  // longer ones are always built by clusters
+static_assert(kHugeSmemMax + 1 == skw_ctx::kLongLeast, "the graph's lists of class K_H are counted");
 static_assert(256 * kListEpt == kF64Max, "the classes up to 4096 end where the packed entries end");
 static_assert(2 * K_CLASSES <= skw_ctx::kClassWords, "class counters");
 
@@ -329,15 +330,18 @@ __host__ __device__ __forceinline__ u32 long_team(u32 count, u32 ctas) {
 }
 // More than 16384 weights, by teams of CL CTAs: those of up to 65536 (class h) if they are for teams of this size, the longer
 // ones (class g) if there are eight.  Each team has a slab of scratch for up to cap weights (cap even), 12 bytes each.
+// expected: how many lists of class h the host counts on, all of the graph's (whole) or at most so many.  Every number of them
+// is built, also one that the host does not expect: the team size follows from what decided on the launches.
 template <u32 CL>
 __global__ void __launch_bounds__(kLongThreads, 3) __cluster_dims__(CL, 1, 1)
     build_long_kernel(const u32* __restrict__ list_g, const u32* __restrict__ list_h, u32* __restrict__ cls, int g, int h,
-                      const __grid_constant__ ListBuild b, unsigned char* __restrict__ scratch, u64 cap, u32 ctas) {
+                      const __grid_constant__ ListBuild b, unsigned char* __restrict__ scratch, u64 cap, u32 ctas, u32 expected,
+                      bool whole) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ u32 s_it;
   const u32 rank = blockIdx.x % CL, team = blockIdx.x / CL;
   u64* A = reinterpret_cast<u64*>(scratch + team * cap * 12);
-  const u32 count_g = CL == kLongTeam ? cls[g] : 0u, count_h = long_team(cls[h], ctas) == CL ? cls[h] : 0u;
+  const u32 count_g = CL == kLongTeam ? cls[g] : 0u, count_h = long_team(whole ? expected : min(cls[h], expected), ctas) == CL ? cls[h] : 0u;
   // Teams of several have a list each, or little more; single CTAs many, and they start when there is room.
   for (u32 it = team;; it += gridDim.x / CL) {
     if constexpr (CL == 1) {
@@ -627,7 +631,7 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
     unsigned char* small = scratch + sc.cap * sc.teams * 12;
 #define LONG(CL, CTAS, SCRATCH, CAP, STREAM)                                                                                    \
   build_long_kernel<CL><<<CTAS, kLongThreads, sizeof(LongShared), STREAM>>>(lists.list[K_G], lists.list[K_H], cls, K_G, K_H, b, \
-                                                                            SCRATCH, CAP, ctas);                                \
+                                                                            SCRATCH, CAP, ctas, ctx->long_lists, whole);       \
   SKW_LAUNCHED(ctx)
     if (!whole || team == kLongTeam || ctx->max_degree > kAloneMax) {
       LONG(8, sc.teams * 8, scratch, sc.cap, ctx->bstream[4]);

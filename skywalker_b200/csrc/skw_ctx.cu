@@ -279,7 +279,7 @@ static void free_graph(skw_ctx* ctx) {
   ctx->dead_ends = 0;
 }
 
-// out[0]: the largest degree, out[1]: the number of vertices of degree 0, longs: of those of degree 16385 to 65536, ends: of
+// out[0]: the largest degree, out[1]: the number of vertices of degree 0, longs: of those of degree kLongLeast to kLongMost, ends: of
 // the sampled edges into vertices of degree 0
 __global__ void max_degree_kernel(const uint32_t* __restrict__ xadj, uint32_t V,
                                   uint32_t* __restrict__ out, uint32_t* __restrict__ longs,
@@ -295,7 +295,7 @@ __global__ void max_degree_kernel(const uint32_t* __restrict__ xadj, uint32_t V,
     const uint32_t d = xadj[v + 1] - xadj[v];
     m = max(m, d);
     empty += d == 0 ? 1u : 0u;
-    if (d > 16384u && d <= 65536u) atomicAdd(longs, 1u);  // (rare)
+    if (d >= skw_ctx::kLongLeast && d <= skw_ctx::kLongMost) atomicAdd(longs, 1u);  // (rare)
   }
   for (int o = 16; o; o >>= 1) {
     m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));

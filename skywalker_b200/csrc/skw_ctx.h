@@ -49,7 +49,8 @@ struct skw_ctx {
   uint64_t E = 0;
   uint32_t max_degree = 0;
   uint32_t empty_lists = 0;  // vertices without out-edges
-  uint32_t long_lists = 0;   // vertices of degree 16385 to 65536
+  static constexpr uint32_t kLongLeast = 16385, kLongMost = 65536;
+  uint32_t long_lists = 0;   // vertices of degree kLongLeast to kLongMost
   static constexpr uint32_t kEdgeSample = 4096;
   uint32_t dead_ends = 0;    // of kEdgeSample edges spread over the list of all, those into vertices without out-edges
   uint32_t* xadj = nullptr;

@@ -167,3 +167,33 @@ def test_alias_teams_of_long_lists(ctx, oracle, kind, quarters, more):
     ctx.alias_build_offline(0, cut)
     ctx.alias_build_offline(cut, len(lists))
     assert all(np.array_equal(a, b) for a, b in zip(whole, ctx.alias_export()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("before, after", [(60, 20), (20, 60), (240, 20), (20, 240)])
+def test_alias_offsets_of_a_borrowed_graph_change(ctx, oracle, before, after):
+    """The offsets of a borrowed graph are rewritten in place: another number of lists of 16385 to 65536 weights than the
+    teams were launched for.  All of them are built."""
+    import torch
+    E = 65536 + 240 * 16385
+    def offsets(lists):
+        sizes = [65536] + [16385 * (240 // lists) if 16385 * (240 // lists) <= 65536 else 49155] * lists
+        sizes += [1000] * 240
+        sizes[-240:] = [(E - sum(sizes[:-240])) // 240] * 239 + [(E - sum(sizes[:-240])) // 240 + (E - sum(sizes[:-240])) % 240]
+        assert sum(sizes) == E and all(n <= 16384 for n in sizes[-240:])
+        sizes += [0] * (500 - len(sizes))
+        return np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint32)
+    w = np.random.default_rng(before).uniform(1, 10, E).astype(np.float32)
+    x = torch.from_numpy(offsets(before).view(np.int32)).cuda()
+    a, d_w = torch.zeros(E, dtype=torch.int32, device="cuda"), torch.from_numpy(w).cuda()
+    torch.cuda.synchronize()
+    ctx.adopt_device(500, E, x, a, d_w)
+    ctx.alias_build_offline()
+    x.copy_(torch.from_numpy(offsets(after).view(np.int32)))
+    torch.cuda.synchronize()
+    for ranges in ([(0, 500)], [(0, 100), (100, 500)]):
+        for r in ranges:
+            ctx.alias_build_offline(*r)
+        prob, alias, valid = ctx.alias_export()
+        want_prob, want_alias, want_valid = oracle.alias_build(offsets(after), w)
+        assert np.array_equal(valid, want_valid) and np.array_equal(prob, want_prob) and np.array_equal(alias, want_alias)
