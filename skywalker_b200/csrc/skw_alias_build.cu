@@ -328,6 +328,19 @@ __host__ __device__ __forceinline__ u32 long_team(u32 count, u32 ctas) {
   while (team > 1 && count > ctas / team) team /= 2;
   return team;
 }
+// A few lists more than there are pairs: the pairs take as many as they are and larger teams the rest, since a CTA alone takes
+// longer than both one after the other.  So many lists of 33,000 / 63,000 weights, us, by single CTAs and this way (by CTAs of
+// 1024 threads, two waves of them, it was 216 to 235 / 370 to 402):
+//   223   228 / 404 -> 169 / 270          260   233 / 405 -> 180 / 299          278   234 / 408 -> 180 / 320
+struct LongPlan {
+  u32 team, lists;  // the first so many lists are for teams of this size,
+  u32 rest;         // the others for these
+};
+__host__ __device__ __forceinline__ LongPlan long_plan(u32 count, u32 ctas) {
+  const u32 pairs = ctas / 2;
+  if (count > pairs && count <= pairs + ctas / 6) return LongPlan{2, pairs, long_team(count - pairs, ctas)};
+  return LongPlan{long_team(count, ctas), 0xFFFFFFFFu, 0};
+}
 // More than 16384 weights, by teams of CL CTAs: those of up to 65536 (class h) if they are for teams of this size, the longer
 // ones (class g) if there are eight.  Each team has a slab of scratch for up to cap weights (cap even), 12 bytes each.
 // expected: how many lists of class h the host counts on, all of the graph's (whole) or at most so many.  Every number of them
@@ -341,7 +354,10 @@ __global__ void __launch_bounds__(kLongThreads, 3) __cluster_dims__(CL, 1, 1)
   __shared__ u32 s_it;
   const u32 rank = blockIdx.x % CL, team = blockIdx.x / CL;
   u64* A = reinterpret_cast<u64*>(scratch + team * cap * 12);
-  const u32 count_g = CL == kLongTeam ? cls[g] : 0u, count_h = long_team(whole ? expected : min(cls[h], expected), ctas) == CL ? cls[h] : 0u;
+  const LongPlan plan = long_plan(whole ? expected : min(cls[h], expected), ctas);
+  const u32 all_h = cls[h], first_h = CL == plan.rest ? min(all_h, plan.lists) : 0u;
+  const u32 count_g = CL == kLongTeam ? cls[g] : 0u;
+  const u32 count_h = CL == plan.rest ? all_h - first_h : CL == plan.team ? min(all_h, plan.lists) : 0u;
   // Teams of several have a list each, or little more; single CTAs many, and they start when there is room.
   for (u32 it = team;; it += gridDim.x / CL) {
     if constexpr (CL == 1) {
@@ -352,7 +368,7 @@ __global__ void __launch_bounds__(kLongThreads, 3) __cluster_dims__(CL, 1, 1)
       __syncthreads();
     }
     if (it >= count_g + count_h) break;
-    const u32 v = it < count_g ? list_g[it] : list_h[it - count_g];
+    const u32 v = it < count_g ? list_g[it] : list_h[first_h + it - count_g];
     const u32 off = b.xadj[v], n = b.xadj[v + 1] - off;
     if (n > cap || n == 0) {
       if (rank == 0 && threadIdx.x == 0) dev_fail(b.err, DEV_ERR_CAPACITY, v, n, (u32)cap);
@@ -623,26 +639,31 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
   for (int i = 0; i < streams; ++i) SKW_CUDA(ctx, cudaStreamWaitEvent(ctx->bstream[i], ctx->bfork, 0));
   const ListBuild b{ctx->xadj, ctx->adjwgt, slots, valid, ctx->launch_err};
   if (ctx->max_degree > kHugeSmemMax) {
-    // The size of the teams follows from the number of lists, which for all vertices is known here; for others it is at most
-    // that, and the kernels of teams that are not the ones find so.
+    // The sizes of the teams follow from the number of lists, which for all vertices is known here; for others it is at most
+    // that, and the kernels of teams that are not the ones find so.  Fours have the slabs behind those of pairs, since both may
+    // be at work.
     const LongScratch sc = long_scratch(ctx);
-    const u32 ctas = ctx->sm_count * 3, team = long_team(ctx->long_lists, ctas);
+    const u32 ctas = ctx->sm_count * 3;
+    const LongPlan plan = long_plan(ctx->long_lists, ctas);
     unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
     unsigned char* small = scratch + sc.cap * sc.teams * 12;
+    auto wanted = [&](u32 team) {
+      return whole ? team == plan.team || team == plan.rest : team == kLongTeam || team >= long_team(ctx->long_lists, ctas);
+    };
 #define LONG(CL, CTAS, SCRATCH, CAP, STREAM)                                                                                    \
   build_long_kernel<CL><<<CTAS, kLongThreads, sizeof(LongShared), STREAM>>>(lists.list[K_G], lists.list[K_H], cls, K_G, K_H, b, \
                                                                             SCRATCH, CAP, ctas, ctx->long_lists, whole);       \
   SKW_LAUNCHED(ctx)
-    if (!whole || team == kLongTeam || ctx->max_degree > kAloneMax) {
+    if (wanted(8) || ctx->max_degree > kAloneMax) {
       LONG(8, sc.teams * 8, scratch, sc.cap, ctx->bstream[4]);
     }
-    if (team == 4 || (!whole && team < 4)) {
-      LONG(4, ctas / 4 * 4, small, sc.cap_small, s_h);
+    if (wanted(4)) {
+      LONG(4, ctas / 4 * 4, small + sc.cap_small * (ctas / 2) * 12, sc.cap_small, ctx->bstream[4]);
     }
-    if (team == 2 || (!whole && team < 2)) {
+    if (wanted(2)) {
       LONG(2, ctas / 2 * 2, small, sc.cap_small, s_h);
     }
-    if (team == 1) {
+    if (wanted(1)) {
       LONG(1, ctas, small, sc.cap_small, s_h);
     }
 #undef LONG

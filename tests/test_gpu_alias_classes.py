@@ -170,6 +170,24 @@ def test_alias_teams_of_long_lists(ctx, oracle, kind, quarters, more):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("part, more", [(8, 0), (8, 1), (6, 0), (6, 1)])
+def test_alias_more_long_lists_than_pairs(ctx, oracle, part, more):
+    """A few lists of 16385 to 65536 weights more than there are pairs of CTAs go to teams of eight or four, which may be at
+    work beside the pairs; at the counts where that changes, all vertices at once and in two ranges."""
+    import torch
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count * 3
+    rng = np.random.default_rng(part)
+    lists = [_weights("uniform", 16385 + (i * 977) % 2000, rng) for i in range(ctas // 2 + ctas // part + more)]
+    lists[5] = _weights("one_heavy", 65536, rng)
+    lists[-1] = np.zeros(20000)
+    _check_lists(ctx, oracle, lists)
+    whole = ctx.alias_export()
+    ctx.alias_build_offline(0, 40)
+    ctx.alias_build_offline(40, len(lists))
+    assert all(np.array_equal(a, b) for a, b in zip(whole, ctx.alias_export()))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("before, after", [(60, 20), (20, 60), (240, 20), (20, 240)])
 def test_alias_offsets_of_a_borrowed_graph_change(ctx, oracle, before, after):
     """The offsets of a borrowed graph are rewritten in place: another number of lists of 16385 to 65536 weights than the
