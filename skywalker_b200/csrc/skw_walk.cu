@@ -126,12 +126,15 @@ static WalkGrid walk_grid(const skw_ctx* ctx, uint32_t app, u64 n, u32 warps, u3
 // Whether a draw fetches the neighbour of its column beside the slot: an access less in the chain of most steps, and one more
 // where the alias is taken.  It pays while walkers wait for memory and not for its rate.  80 steps, us, without / with:
 //   PPR        4,096 walkers 40 / 39 (R-MAT 22) and 45 / 44 (power law of 226 M edges), 40,000 75 / 68 and 101 / 92;
-//              1 M walkers of 20 steps on the power law 325 / 346
+//              1 M walkers of 20 steps on the power law 325 / 346; short walks over tables in the nearest caches take their
+//              neighbours from there and lose by it: at most 10 steps on R-MAT 14 with 6 MB, 16,000 38.9 / 40.2, 39,000 40.8 /
+//              42.8, 32 steps 39,000 55.6 / 57.3, but 40 steps and more, fewer walkers or larger tables 0.99 to 1.15 times as fast
 //   DeepWalk   tables out of cache: 1,000 walkers 96 / 89 and 111 / 98, 16,000 129 / 114 and 132 / 122, 100,000 170 / 190 and
 //              455 / 524; in cache (R-MAT 16, 4,096 walkers) 73 / 77
-static bool walk_ahead(const skw_ctx* ctx, uint32_t app, u64 n, bool unbiased) {
+static bool walk_ahead(const skw_ctx* ctx, uint32_t app, u64 n, u32 hop_num, bool unbiased) {
   if (unbiased) return false;
-  return app == SKW_APP_PPR ? n <= 270ull * ctx->sm_count : n <= 110ull * ctx->sm_count && ctx->E * 12 > (64u << 20);
+  const bool short_cached = hop_num <= 40 && ctx->E * 12 <= (8u << 20) && n > 40ull * ctx->sm_count;
+  return app == SKW_APP_PPR ? n <= 270ull * ctx->sm_count && !short_cached : n <= 110ull * ctx->sm_count && ctx->E * 12 > (64u << 20);
 }
 
 // All steps of all walkers in one launch.  The first `lanes` lanes of each warp own walkers w, w + T, w + 2T ...;
@@ -1294,7 +1297,7 @@ static int walk_launch(skw_ctx* ctx, const skw_walk_params* prm, const uint32_t*
   } else if (!online || whole_table) {
     const u64 read = ctx->E * (unbiased ? 4u : 12u);  // lists, and slots if they are drawn from
     const WalkGrid g = walk_grid(ctx, prm->app, n, prm->app == SKW_APP_DEEPWALK && read <= (8u << 20) ? 17 : 34, 1);
-    const bool ahead = walk_ahead(ctx, prm->app, n, unbiased);
+    const bool ahead = walk_ahead(ctx, prm->app, n, prm->hop_num, unbiased);
     const size_t rings = home ? sizeof(u32) * (kWalkCta / 32) * g.lanes * (kLineRing + 1) : 0;
     switch (prm->app) {
       case SKW_APP_DEEPWALK:

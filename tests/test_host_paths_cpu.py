@@ -349,6 +349,21 @@ assert len(launches(log, "walk_home_kernel")) == %d and len(launches(log, "walk_
 """ % (ends, n, hop, app, tp, home, not home))
 
 
+@pytest.mark.parametrize("V,n,hop,ahead", [(1000, 5920, 17, True), (1000, 5921, 17, False), (1000, 39000, 40, False),
+                                           (1000, 39000, 41, True), (60000, 39000, 17, True), (60000, 39961, 17, False)])
+def test_ppr_neighbours_beside_their_slots(fake_cudart, V, n, hop, ahead):
+    """Which kernel walks over slots take: the one that fetches neighbours ahead is for walks that wait for memory."""
+    _run(fake_cudart, """
+ctx = Context(0)
+ctx.upload(*ring(%d))
+ctx.alias_build_offline()
+s, p, l = Device(%d), Device(%d, %d), Device(%d)
+calls()
+ctx.walk(s, %d, app=1, tp=0.15, paths=p, lengths=l)
+assert len(launches(calls(), "walk_offline_kernelILi1ELb%dE")) == 1
+""" % (V, n, n, hop, n, hop, ahead))
+
+
 def test_packed_ppr_without_memory_for_heads(fake_cudart):
     """The first cells of the rows travel apart from them where there is memory: it is asked for behind everything that
     the call needs, and given up when another allocation fails, also in the middle of a call."""
