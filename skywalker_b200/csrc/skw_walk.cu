@@ -20,6 +20,8 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
+
 #include <cub/device/device_scan.cuh>
 #include <cub/iterator/transform_input_iterator.cuh>
 
@@ -1457,17 +1459,35 @@ static int walk_rows_by_scatter(skw_ctx* ctx, const skw_walk_params* prm, const 
   return SKW_OK;
 }
 
-// `count` words of host memory as the GPU sees them, or null where it does not (both ends are asked for, a part of an allocation
-// may be registered) or where they are not at a word boundary.
+// `count` words of host memory as the GPU sees them, or null where it does not or where they are not at a word boundary.  All of
+// them have to be in one pinned allocation or registration: parts of an array may be registered, with pages between them that
+// the GPU must not touch.
 static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
-  cudaPointerAttributes first, last;
-  if ((reinterpret_cast<uintptr_t>(h) & 3) == 0 && cudaPointerGetAttributes(&first, h) == cudaSuccess &&
-      cudaPointerGetAttributes(&last, h + (count - 1)) == cudaSuccess && first.type == cudaMemoryTypeHost &&
-      last.type == cudaMemoryTypeHost && first.devicePointer &&
-      static_cast<u32*>(last.devicePointer) == static_cast<u32*>(first.devicePointer) + (count - 1))
-    return static_cast<u32*>(first.devicePointer);
-  cudaGetLastError();
-  return nullptr;
+  using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<Query>(f);
+  }();
+  cudaPointerAttributes at;
+  if ((reinterpret_cast<uintptr_t>(h) & 3) != 0 || !query) return nullptr;
+  if (cudaPointerGetAttributes(&at, h) != cudaSuccess || at.type != cudaMemoryTypeHost || !at.devicePointer) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  const uint64_t d = reinterpret_cast<uint64_t>(at.devicePointer);
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS ||
+      query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS || d < start || d - start > size ||
+      (size - (d - start)) / sizeof(u32) < count)
+    return nullptr;
+  return static_cast<u32*>(at.devicePointer);
 }
 
 // Whether walk_home_kernel takes a batch: as long as the walks, a chain of hop_num dependent steps whatever their number, hide

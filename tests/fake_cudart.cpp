@@ -3,6 +3,7 @@
 // are noted down and (but for the one that finds the largest degree) not run.  Allocations fail on request, and fake_log() tells what was called, one call a line:
 //   malloc <bytes> <ok|fail>    free    host_malloc <ok|fail>    device_sync    launch <stream> <kernel>
 //   record <event> <stream>     wait <stream> <event>            sync <stream>  memset <stream>    copy <stream>
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -65,6 +66,7 @@ void fake_fail_host_malloc(long after, long times) {
 }
 void fake_memory(size_t total) { device_total = total; }
 void fake_packed(unsigned long long cells) { packed_total = cells; }
+void fake_register(void* p, size_t bytes) { host_blocks[reinterpret_cast<uintptr_t>(p)] = bytes; }
 void fake_pinned(int on) { pinned_seen = on != 0; }
 void fake_capture(int on) { capturing = on != 0; }
 size_t fake_used() { return device_used; }
@@ -183,6 +185,22 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     a->type = cudaMemoryTypeHost;
     a->devicePointer = a->hostPointer = const_cast<void*>(p);
   }
+  return cudaSuccess;
+}
+
+static CUresult pointer_attribute(void* out, CUpointer_attribute what, CUdeviceptr p) {
+  auto it = host_blocks.upper_bound(p);
+  if (it == host_blocks.begin() || p >= (--it)->first + it->second) return CUDA_ERROR_INVALID_VALUE;
+  if (what == CU_POINTER_ATTRIBUTE_RANGE_START_ADDR) *static_cast<CUdeviceptr*>(out) = it->first;
+  else if (what == CU_POINTER_ATTRIBUTE_RANGE_SIZE) *static_cast<size_t*>(out) = it->second;
+  else return CUDA_ERROR_INVALID_VALUE;
+  return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** f, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* found) {
+  const bool have = std::string(name) == "cuPointerGetAttribute";
+  *f = have ? reinterpret_cast<void*>(&pointer_attribute) : nullptr;
+  if (found) *found = have ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
   return cudaSuccess;
 }
 

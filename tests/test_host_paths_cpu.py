@@ -349,6 +349,28 @@ assert len(launches(log, "walk_home_kernel")) == %d and len(launches(log, "walk_
 """ % (ends, n, hop, app, tp, home, not home))
 
 
+def test_rows_of_which_only_parts_are_registered_are_copied(fake_cudart):
+    """The GPU writes a matrix of the caller's only if all of it is one pinned range: not one whose ends are pinned, with
+    other pages between them, or one that ends behind the range."""
+    _run(fake_cudart, """
+fake.fake_pinned(1)
+fake.fake_register.argtypes = [C.c_void_p, C.c_size_t]
+ctx = Context(0)
+ctx.upload(*ring())
+ctx.alias_build_offline()
+lengths = np.zeros(300, np.uint32)
+fake.fake_register(lengths.ctypes.data, lengths.nbytes)
+for parts, home in (([(0, 4096), (93104, 4096)], 0), ([(0, 97196)], 0), ([(4, 97196)], 0), ([(0, 97200)], 1)):
+    paths = np.zeros((300, 81), np.uint32)
+    for at, size in parts:
+        fake.fake_register(paths.ctypes.data + at, size)
+    calls()
+    ctx.walk(np.zeros(300, np.uint32), 81, paths=paths, lengths=lengths, flags=16)
+    assert len(launches(calls(), "walk_home_kernel")) == home, parts
+    globals().setdefault("keep", []).append(paths)      # (the addresses stay taken)
+""")
+
+
 @pytest.mark.parametrize("V,n,hop,ahead", [(1000, 5920, 17, True), (1000, 5921, 17, False), (1000, 39000, 40, False),
                                            (1000, 39000, 41, True), (60000, 39000, 17, True), (60000, 39961, 17, False)])
 def test_ppr_neighbours_beside_their_slots(fake_cudart, V, n, hop, ahead):
