@@ -584,25 +584,32 @@ static int class_counters(skw_ctx* ctx, u32** cls) {
 }
 
 // Scratch of the lists beyond 16384 weights: a slab with room for the longest for each team of eight, fewer of them when a
-// giant hub would make the slabs exceed 4 GB in total; then, if smaller teams may be used, as much as the smallest need.
+// giant hub would make the slabs exceed 4 GB in total, but eight at least; then, if smaller teams may be used, as much as the
+// smallest need (349 MB where there are lists of 65536).  Without memory for that the teams of eight build all of them.
 struct LongScratch {
   uint64_t cap = 0, cap_small = 0;  // entries of 12 bytes
   unsigned teams = 0, small = 0;
   uint64_t bytes() const { return (cap * teams + cap_small * small) * 12; }
 };
+// The number of lists that decides on the teams.
+static u32 long_lists(const skw_ctx* ctx) { return ctx->scratch_short ? 0 : ctx->long_lists; }
 static LongScratch long_scratch(const skw_ctx* ctx) {
   LongScratch s;
   if (ctx->max_degree > kHugeSmemMax) {
     s.cap = ((uint64_t)ctx->max_degree + 1) & ~1ull;
     s.teams = (unsigned)std::min<uint64_t>(ctx->sm_count * 3 / kLongTeam, std::max<uint64_t>((4ull << 30) / (s.cap * 12), 8));
     s.cap_small = std::min<uint64_t>(s.cap, kAloneMax);
-    s.small = long_team(ctx->long_lists, ctx->sm_count * 3) < kLongTeam ? ctx->sm_count * 3 : 0;
+    s.small = long_team(long_lists(ctx), ctx->sm_count * 3) < kLongTeam ? ctx->sm_count * 3 : 0;
   }
   return s;
 }
 static int reserve_scratch(skw_ctx* ctx) {
-  const uint64_t bytes = long_scratch(ctx).bytes();
-  return bytes ? ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, bytes) : SKW_OK;
+  const LongScratch s = long_scratch(ctx);
+  if (s.bytes() == 0) return SKW_OK;
+  const int rc = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, s.bytes());
+  if (rc == SKW_OK || s.small == 0) return rc;
+  ctx->scratch_short = true;
+  return ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, long_scratch(ctx).bytes());
 }
 
 // Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`; whole: all vertices of the
@@ -643,16 +650,16 @@ static int launch_builders(skw_ctx* ctx, const ClassLists& lists, u32* cls, Slot
     // that, and the kernels of teams that are not the ones find so.  Fours have the slabs behind those of pairs, since both may
     // be at work.
     const LongScratch sc = long_scratch(ctx);
-    const u32 ctas = ctx->sm_count * 3;
-    const LongPlan plan = long_plan(ctx->long_lists, ctas);
+    const u32 ctas = ctx->sm_count * 3, expected = long_lists(ctx);
+    const LongPlan plan = long_plan(expected, ctas);
     unsigned char* scratch = static_cast<unsigned char*>(ctx->cta_scratch);
     unsigned char* small = scratch + sc.cap * sc.teams * 12;
     auto wanted = [&](u32 team) {
-      return whole ? team == plan.team || team == plan.rest : team == kLongTeam || team >= long_team(ctx->long_lists, ctas);
+      return whole ? team == plan.team || team == plan.rest : team == kLongTeam || team >= long_team(expected, ctas);
     };
 #define LONG(CL, CTAS, SCRATCH, CAP, STREAM)                                                                                    \
   build_long_kernel<CL><<<CTAS, kLongThreads, sizeof(LongShared), STREAM>>>(lists.list[K_G], lists.list[K_H], cls, K_G, K_H, b, \
-                                                                            SCRATCH, CAP, ctas, ctx->long_lists, whole);       \
+                                                                            SCRATCH, CAP, ctas, expected, whole);              \
   SKW_LAUNCHED(ctx)
     if (wanted(8) || ctx->max_degree > kAloneMax) {
       LONG(8, sc.teams * 8, scratch, sc.cap, ctx->bstream[4]);

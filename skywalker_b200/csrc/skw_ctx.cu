@@ -277,6 +277,7 @@ static void free_graph(skw_ctx* ctx) {
   ctx->empty_lists = 0;
   ctx->long_lists = 0;
   ctx->dead_ends = 0;
+  ctx->scratch_short = false;
 }
 
 // out[0]: the largest degree, out[1]: the number of vertices of degree 0, longs: of those of degree kLongLeast to kLongMost, ends: of

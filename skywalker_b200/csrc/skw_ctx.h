@@ -95,6 +95,7 @@ struct skw_ctx {
   unsigned cls_used = 0;  // sets that are not zero; the last one belongs to graphs
   void* cta_scratch = nullptr;       // slabs of the global-memory CTA builder
   size_t cta_scratch_bytes = 0;
+  bool scratch_short = false;        // no memory for those of this graph's smaller teams: the largest do without
 
   // online mode: per-frontier work lists (one per degree class) and the claim stamps that make
   // every distinct frontier vertex be built once per round

@@ -101,7 +101,12 @@ cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cud
     const unsigned* xadj = *static_cast<const unsigned**>(args[0]);
     const unsigned V = *static_cast<unsigned*>(args[1]);
     unsigned* out = *static_cast<unsigned**>(args[2]);
-    for (unsigned v = 0; v < V; ++v) *out = xadj[v + 1] - xadj[v] > *out ? xadj[v + 1] - xadj[v] : *out;
+    unsigned* longs = *static_cast<unsigned**>(args[3]);
+    for (unsigned v = 0; v < V; ++v) {
+      const unsigned d = xadj[v + 1] - xadj[v];
+      *out = d > *out ? d : *out;
+      *longs += d > 16384 && d <= 65536;
+    }
     const unsigned* adjncy = *static_cast<const unsigned**>(args[4]);
     const unsigned long long E = *static_cast<unsigned long long*>(args[5]);
     unsigned* ends = *static_cast<unsigned**>(args[6]);

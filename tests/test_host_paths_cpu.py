@@ -349,6 +349,42 @@ assert len(launches(log, "walk_home_kernel")) == %d and len(launches(log, "walk_
 """ % (ends, n, hop, app, tp, home, not home))
 
 
+@pytest.mark.parametrize("call", ["alias_build_offline()", "walk(s, 20, mode=1, paths=p, lengths=l)",
+                                  "sample_khop(np.zeros(2000, np.uint32), [5, 3], mode=1)"])
+def test_long_lists_without_memory_for_small_teams(fake_cudart, call):
+    """Lists of more than 16384 weights beyond what teams of eight CTAs take at a time go to smaller teams, with more
+    scratch; without memory for that the teams of eight take them all."""
+    _run(fake_cudart, """
+def context():
+    ctx = Context(0)
+    d = np.full(1000, 12)
+    d[:60] = 20000
+    x = np.concatenate([[0], np.cumsum(d)]).astype(np.uint32)
+    ctx.upload(x, np.arange(x[-1], dtype=np.uint32) %% 1000, np.ones(x[-1], np.float32))
+    return ctx
+MB = 1 << 20
+s, p, l = Device(1 << 18), Device(1 << 18, 20), Device(1 << 18)
+ctx = context()
+idle = fake.fake_used()
+ctx.%s
+log = calls()
+need = fake.fake_used() - idle
+assert need > 110 * MB and launches(log, "build_long_kernelILj4E") and not launches(log, "direct")
+ctx.close()
+ctx = context()
+fake.fake_memory(fake.fake_used() + need - 60 * MB)
+for _ in range(2):
+    ctx.%s
+    log = calls()
+    assert launches(log, "build_long_kernelILj8E") and not launches(log, "build_long_kernelILj4E")
+assert not [x for x in log if x[0] == "malloc"]
+fake.fake_memory(64 << 30)
+ctx.upload(*ring(hub=20000))
+ctx.alias_build_offline()
+assert ctx.alias_export()[0].size == 32000
+""" % (call, call))
+
+
 def test_rows_of_which_only_parts_are_registered_are_copied(fake_cudart):
     """The GPU writes a matrix of the caller's only if all of it is one pinned range: not one whose ends are pinned, with
     other pages between them, or one that ends behind the range."""
