@@ -109,9 +109,8 @@ def _check_lists(ctx, oracle, lists):
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("more_than_clusters", [-1, 0, 1, 150])
 def test_alias_many_giant_lists(ctx, oracle, kind, more_than_clusters):
-    """Lists of more than 16384 weights by clusters of CTAs, and by one CTA each from one list more than there are
-    clusters on: around the tiles and windows of 8192, of all kinds of weights, and a list without usable weights
-    between others."""
+    """Lists of more than 16384 weights of all kinds by teams of eight CTAs, by teams of four from one list more than there are
+    teams of eight on, and by pairs, with a list without usable weights between others."""
     import torch
     rng = np.random.default_rng(len(kind))
     clusters = torch.cuda.get_device_properties(0).multi_processor_count * 3 // 8
@@ -126,7 +125,8 @@ def test_alias_many_giant_lists(ctx, oracle, kind, more_than_clusters):
 @pytest.mark.parametrize("kind", ["lognormal", "one_heavy"])
 @pytest.mark.parametrize("others", [0, 60])
 def test_alias_list_of_many_windows(ctx, oracle, kind, others):
-    """A list that takes more than one round of merge windows, alone (a cluster) and among others (one CTA)."""
+    """A list that takes more than one round of merge windows, alone and behind others that take more teams than there are of
+    eight CTAs: a list of more than 65536 weights always has a team of eight."""
     rng = np.random.default_rng(others)
     _check_lists(ctx, oracle, [_weights(kind, 20000, rng) for _ in range(others)] + [_weights(kind, 1024 * 8192 + 5, rng)])
 
@@ -167,6 +167,24 @@ def test_alias_teams_of_long_lists(ctx, oracle, kind, quarters, more):
     ctx.alias_build_offline(0, cut)
     ctx.alias_build_offline(cut, len(lists))
     assert all(np.array_equal(a, b) for a, b in zip(whole, ctx.alias_export()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["uniform", "one_heavy", "unusable"])
+@pytest.mark.parametrize("team", [8, 4, 2, 1])
+def test_alias_edges_of_tiles_and_windows(ctx, oracle, kind, team):
+    """Lists around whole numbers of tiles of 4096 weights a CTA, chunks that end in few weights, and merge windows of whole and of
+    other sizes, by teams of each size."""
+    import torch
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count * 3
+    rng = np.random.default_rng(team)
+    sizes = [team * t * 4096 + d for t in (1, 2, 3, 5) for d in (-257, -256, -1, 0, 1, 255, 256, 257)]
+    sizes += [team * 256 * k + d for k in (9, 15, 17, 33, 65) for d in (0, 1)] + [65535]
+    sizes = [n for n in sizes if 16384 < n <= 65536]
+    while len(sizes) <= {8: 0, 4: ctas // 8, 2: ctas // 4, 1: ctas // 2 + ctas // 6}[team]:
+        sizes.append(16385 + len(sizes))
+    assert len(sizes) <= {8: ctas // 8, 4: ctas // 4, 2: ctas // 2, 1: ctas}[team]
+    _check_lists(ctx, oracle, [_weights(kind, n, rng) for n in sizes])
 
 
 @pytest.mark.gpu

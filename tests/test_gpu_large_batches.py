@@ -219,6 +219,62 @@ def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, app, hop, n, off, 
     assert np.array_equal(odd.reshape(n, hop)[live], rows[live])
 
 
+@pytest.fixture(scope="module")
+def rmat19(ctx):
+    """Tables out of cache (72 MB), on the host as well."""
+    ctx.generate_rmat(19, 12 << 19, graph_seed=2, weight_seed=3)
+    x, a, w = ctx.download()
+    assert len(a) * 12 > 64 << 20
+    return x, a, w
+
+
+@pytest.mark.parametrize("app,hop,n,off,flags", [
+    (APP_DEEPWALK, 81, 4099, 7, 16), (APP_DEEPWALK, 81, 4099, 7, 0), (APP_DEEPWALK, 11, 2500, 31, 16), (APP_DEEPWALK, 70, 16281, 1, 16),
+    (APP_PPR, 81, 4099, 5, 16), (APP_PPR, 33, 9999, 3, 16)])
+def test_rows_written_into_pinned_memory_of_a_large_graph(ctx, oracle, rmat19, app, hop, n, off, flags):
+    """The same where draws fetch their neighbours ahead, into an array that the caller has registered."""
+    import mmap
+    import torch
+    x, a, w = rmat19
+    ctx.upload(x, a, w)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, len(x) - 1, 12)
+    cells = np.frombuffer(mmap.mmap(-1, (n * hop + 64 + n) * 4), np.uint32)
+    cells[:] = 0x5A5A5A5A
+    rows, lengths = cells[off:off + n * hop].reshape(n, hop), cells[n * hop + 64:]
+    kw = dict(app=app, tp=0.1, seed=6, walker_base=9)
+    runtime = torch.cuda.cudart()
+    assert int(runtime.cudaHostRegister(cells.ctypes.data, cells.nbytes, 0)) == 0
+    try:
+        ctx.walk(starts, hop, paths=rows, lengths=lengths, flags=flags, **kw)
+    finally:
+        runtime.cudaHostUnregister(cells.ctypes.data)
+    want, want_len = oracle.walk(x, a, w, ctx.alias_export(), starts, hop, **kw)
+    live = np.arange(hop)[None, :] <= want_len[:, None]
+    assert np.array_equal(lengths, want_len) and np.array_equal(rows[live], want[live])
+    assert (rows[~live] == (0xFFFFFFFF if flags else 0x5A5A5A5A)).all()
+    assert (cells[:off] == 0x5A5A5A5A).all() and (cells[off + n * hop:n * hop + 64] == 0x5A5A5A5A).all()
+
+
+@pytest.mark.parametrize("hop", [1, 2, 31, 32, 33, 40])
+@pytest.mark.parametrize("app", [APP_DEEPWALK, APP_PPR])
+@pytest.mark.parametrize("n,flags", [(4097, 18), (9999, 16)])
+def test_short_rows_written_into_pinned_memory(ctx, oracle, rmat12, app, hop, n, flags):
+    """Rows of a line or less with uniform draws (2), and those a little longer of draws from tables in cache."""
+    import torch
+    g = rmat12
+    ctx.upload(g.xadj, g.adjncy, g.adjwgt)
+    ctx.alias_build_offline()
+    starts = oracle.gen_starts(n, g.V, 11)
+    paths, lengths = torch.zeros((n, hop), dtype=torch.int32).pin_memory(), torch.zeros(n, dtype=torch.int32).pin_memory()
+    kw = dict(app=app, tp=0.1, seed=6, flags=flags)
+    _, _, _, edges = ctx.walk(starts, hop, paths=paths, lengths=lengths, **kw)
+    want, want_len = np.zeros((n, hop), np.uint32), np.zeros(n, np.uint32)
+    _, _, _, want_edges = ctx.walk(starts, hop, paths=want, lengths=want_len, **kw)      # pageable: copied
+    assert np.array_equal(lengths.numpy().view(np.uint32), want_len) and edges == want_edges
+    assert np.array_equal(paths.numpy().view(np.uint32), want)
+
+
 @pytest.mark.parametrize("fanout", [[4, 3, 2], [5, 3]])
 @pytest.mark.parametrize("per_sm,more", [(6, 0), (6, 1), (8, 0), (8, 1)])
 def test_weighted_trees_around_whole_waves(ctx, oracle, rmat12, fanout, per_sm, more):
