@@ -26,8 +26,8 @@
 // Work distribution: vertices are binned by degree with warp ballots and shared-memory prefix sums (classify_*
 // kernels), one work list per class.  Lists of up to 4096 weights are built in double precision by a lane, a group of
 // lanes, a warp or a CTA that holds the whole list in registers (skw_alias_f64.cuh), up to 16384 by a CTA alike
-// (skw_alias_wide.cuh); longer ones by CTAs that work
-// through it in tiles (skw_alias_long.cuh), the few giant ones by clusters of CTAs.
+// (skw_alias_wide.cuh); longer ones are worked through in tiles (skw_alias_long.cuh) by teams of CTAs, clusters of eight, four
+// or two or CTAs alone by the number of lists, and beyond 65536 always by eight.
 #include <math_constants.h>
 
 #include <algorithm>

@@ -1599,7 +1599,9 @@ static int walk_packed_impl(skw_ctx* ctx, const skw_walk_params* prm, const uint
   static_assert(skw_ctx::kPackSlices >= 8 && skw_ctx::kStages >= 4 + 8, "one event set and one packing buffer per slice");
   // Slice sizes in the ratio 1 : 2 : 4 : 4 ... (three: 1 : 2 : 2): the first results are on the bus early (the call is
   // as long as the time to the first packed slice plus the copy of everything), the later slices are
-  // large enough to walk efficiently.  2 M PPR walks: 926 us in two slices of 1 : 2, 880 in these three, 893 in four.
+  // large enough to walk efficiently.  2 M PPR walks: 926 us in two slices of 1 : 2, 880 in these three, 893 in four;
+  // in two / three on R-MAT 20, 1.05, 1.3, 1.6 and 2 M walkers: PPR of 30 steps, tp 0.03, 1247 / 1178, 1506 / 1428, 1797 / 1777 and
+  // 2257 / 2144, DeepWalk of ten steps 841 / 773, 916 / 912, 1098 / 1067 and 1414 / 1341.
   uint64_t base_of[skw_ctx::kPackSlices + 1] = {};
   uint64_t per = n;  // the largest slice
   if (slices > 1) {
