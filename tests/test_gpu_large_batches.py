@@ -192,9 +192,10 @@ def test_packed_ppr_over_records(ctx, oracle, request, graph, hop, tp, n):
 @pytest.mark.parametrize("app", [APP_DEEPWALK, APP_PPR])
 @pytest.mark.parametrize("n,off,flags", [(1, 0, 0), (37, 5, 16), (4096, 31, 16), (4097, 2, 0), (9999, 1, 18)])
 def test_rows_written_into_pinned_memory(ctx, oracle, rmat12, app, hop, n, off, flags):
-    """DeepWalk and PPR write their rows into the caller's pinned matrix a 128-byte line at a time, wherever in a line a row starts (off
-    words).  Cells past a walk's end keep their contents or (16, fill rows) get the invalid vertex, words around the matrix
-    keep theirs, and all of it equals the rows of pageable memory; 2: uniform draws."""
+    """Rows in the caller's pinned matrix, wherever in a 128-byte line a row starts (off words).  16, fill rows: DeepWalk and PPR write
+    them there, a line at a time, and cells past a walk's end get the invalid vertex; otherwise the cells of the walks are
+    copied, and those past their ends keep their contents.  Words around the matrix keep theirs, and all of it equals the rows of
+    pageable memory; 2: uniform draws."""
     import torch
     g = rmat12
     ctx.upload(g.xadj, g.adjncy, g.adjwgt)
