@@ -194,14 +194,22 @@ __global__ void __launch_bounds__(256, 8) khop_weighted_tree_kernel(const KhopAr
   khop_trees<false>(a, per_cta);
 }
 
-// Whether trees of weighted draws take 64 warps an SM.  Trees of one or two hops do where 48 do not hold all CTAs (40 / 32
-// registers, us: 65,536 x 25, 10 on R-MAT and power-law graphs 126-212 / 117-199, 30,000 x 25, 10 60-98 / 59-89, 65,536 x 40
-// 33-42 / 31-40).  From three hops on the short hops between barriers are bound by instructions, and fewer registers
-// take more of them (65,536 x 5, 5, 3 100-128 / 105-138, 8,191 x 15, 10, 5 114-121 / 120-122), unless the eight CTAs an SM make
-// the difference between one wave and two (1,000 x 15, 10, 5 20-28 / 19-22, x 5, 5, 3 14-18 / 13-14).  Up to 48 warps an SM
-// more registers are never worse (380 x 15, 10, 5 16-18 / 16-18).
-static bool weighted_tree_warps(const skw_ctx* ctx, uint32_t nhops, uint64_t ctas) {
-  return ctas > ctx->sm_count * 6ull && (nhops <= 2 || ctas <= ctx->sm_count * 8ull);
+// Whether trees of weighted draws take 64 warps an SM, eight CTAs, or 48, six.  With eight each CTA is slower, so they pay where
+// they save a wave of CTAs (40 / 32 registers, us, with replacement, power law of 57 M edges: 20,000 x 25, 10, 2,000 CTAs, 110 / 102,
+// but 13,645, 1,365 CTAs and two waves either way, 75 / 86; 1,100 x 25, 10 17 / 15; 65,536 x 40 46 / 43).  By what binds instead:
+//   three hops and more, more than a wave   instructions, in the short hops between barriers, and fewer registers take more of
+//                                           them (65,536 x 5, 5, 3 100-128 / 105-138, 8,191 x 15, 10, 5 114-121 / 120-122)
+//   two hops, tables of up to 24 MB         instructions too (R-MAT 16 of 0.5 M edges, 30,000 x 25, 10 58 / 63); one tree a CTA is
+//                                           short enough to gain all the same (power law of 1 M edges, 2,000 x 10, 5 15.7 / 14.9)
+//   two hops, small trees, many seeds       memory, whatever the waves (R-MAT 22, 65 M edges, 4,000 x 10, 5 with the take-all rule
+//   without out-edges                       15.1 / 13.6, 17,000 23.4 / 21.6; larger trees 13,645 x 25, 10 37.4 / 37.1)
+static bool weighted_tree_warps(const skw_ctx* ctx, const KhopArgs& a, uint64_t ctas) {
+  const uint64_t six = ctx->sm_count * 6ull, eight = ctx->sm_count * 8ull, table = ctx->E * 12;
+  const bool fewer_waves = (ctas + eight - 1) / eight < (ctas + six - 1) / six;
+  if (ctas <= eight || a.nhops == 1) return fewer_waves;
+  if (a.nhops > 2) return false;
+  if (table <= (24u << 20)) return fewer_waves && a.n <= 2 * eight;
+  return fewer_waves || (ctx->empty_lists * 4ull > ctx->V && table > (40u << 20) && a.cells <= 128);
 }
 
 // One hop of every tree (online mode, whose tables are built hop by hop, and trees that are too large for a CTA).  64 warps an SM,
@@ -401,7 +409,7 @@ static int khop_launch(skw_ctx* ctx, const skw_khop_params* prm, const uint32_t*
     const uint64_t ctas = (n + per_cta - 1) / per_cta;
     if (ctas <= 0x7FFFFFFFull) {
       if (distinct) khop_tree_kernel<true><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
-      else if ((a.flags & SKW_KHOP_UNBIASED) || !weighted_tree_warps(ctx, prm->nhops, ctas))
+      else if ((a.flags & SKW_KHOP_UNBIASED) || !weighted_tree_warps(ctx, a, ctas))
         khop_tree_kernel<false><<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
       else khop_weighted_tree_kernel<<<(unsigned)ctas, 256, 0, st>>>(a, per_cta);
       SKW_LAUNCHED(ctx);

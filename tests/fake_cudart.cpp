@@ -105,6 +105,7 @@ cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cud
     for (unsigned v = 0; v < V; ++v) {
       const unsigned d = xadj[v + 1] - xadj[v];
       *out = d > *out ? d : *out;
+      out[1] += d == 0;
       *longs += d > 16384 && d <= 65536;
     }
     const unsigned* adjncy = *static_cast<const unsigned**>(args[4]);

@@ -407,6 +407,27 @@ for parts, home in (([(0, 4096), (93104, 4096)], 0), ([(0, 97196)], 0), ([(4, 97
 """)
 
 
+@pytest.mark.parametrize("V,ends,fanout,n,more", [
+    (1000, 0, [25, 10], 888, False), (1000, 0, [25, 10], 889, True), (1000, 0, [25, 10], 1184, True), (1000, 0, [25, 10], 1300, False),
+    (1000, 0, [25, 10], 2000, True), (1000, 0, [25, 10], 20000, False), (200000, 0, [25, 10], 20000, True),
+    (200000, 0, [25, 10], 13645, False), (400000, 0, [10, 5], 13645, False), (400000, 200000, [10, 5], 13645, True),
+    (400000, 200000, [25, 10], 13645, False), (1000, 0, [40], 65536, True), (1000, 0, [15, 10, 5], 1000, True),
+    (400000, 0, [15, 10, 5], 2000, False)])
+def test_warps_of_weighted_trees(fake_cudart, V, ends, fanout, n, more):
+    """Which of its two kernels a batch of trees takes: eight CTAs an SM where they save a wave and the tables are large."""
+    _run(fake_cudart, """
+ctx = Context(0)
+x, a, w = ring(%d)
+ctx.upload(np.concatenate([x, np.full(%d, x[-1])]).astype(np.uint32), a, w)
+ctx.alias_build_offline()
+cells, lens = ctx.khop_layout(%r)
+calls()
+ctx.sample_khop(Device(%d), %r, mode=0, data=Device(%d, cells), sample_lengths=Device(%d, lens))
+log = calls()
+assert len(launches(log, "khop_weighted_tree_kernel")) == %d and len(launches(log, "khop_tree_kernelILb0")) == %d
+""" % (V, ends, fanout, n, fanout, n, n, more, not more))
+
+
 @pytest.mark.parametrize("V,n,hop,ahead", [(1000, 5920, 17, True), (1000, 5921, 17, False), (1000, 39000, 40, False),
                                            (1000, 39000, 41, True), (60000, 39000, 17, True), (60000, 39961, 17, False)])
 def test_ppr_neighbours_beside_their_slots(fake_cudart, V, n, hop, ahead):
