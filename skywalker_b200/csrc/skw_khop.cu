@@ -216,7 +216,9 @@ static bool weighted_tree_warps(const skw_ctx* ctx, const KhopArgs& a, uint64_t 
 // as above: hop 2 of 65,536 x 25, 10 (16.4 M cells, 9 M draws) waited for memory 18 of every 25 cycles with 40 warps; the
 // whole batch 672 -> 640 us, by distinct draws 834 -> 813.  Unlike those of whole trees, hops of their own gain with uniform
 // and distinct draws as well (32 registers here, 48 before): offline trees of 2,000 x 25, 20, 20 uniform 191 -> 177 us, distinct
-// 287 -> 269, of 2,000 x 100, 100 150 / 150 and 199 -> 190, 500 seeds 2 % more to 3 % less.  (A warp that takes 32 parents, reads their offsets once and deals
+// 287 -> 269, of 2,000 x 100, 100 150 / 150 and 199 -> 190, 500 seeds 2 % more to 3 % less.  What loses are offline trees of 90
+// children a parent over small tables, uniform or with the take-all rule (R-MAT 16, 3,000 x 100, 90 186 -> 192 and 132 -> 139 us),
+// where those of 30, 30, 10 gain (3,000: 5 and 7 %).  (A warp that takes 32 parents, reads their offsets once and deals
 // out the children of those that have any: 677.)
 __global__ void __launch_bounds__(256) khop_init_kernel(const u32* __restrict__ seeds, u64 n,
                                                         u32 cells, u32* __restrict__ data) {
