@@ -609,7 +609,9 @@ static int reserve_scratch(skw_ctx* ctx) {
   const int rc = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, s.bytes());
   if (rc == SKW_OK || s.small == 0) return rc;
   ctx->scratch_short = true;
-  return ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, long_scratch(ctx).bytes());
+  const int less = ensure_bytes(ctx, &ctx->cta_scratch, &ctx->cta_scratch_bytes, long_scratch(ctx).bytes());
+  if (less != SKW_OK) ctx->scratch_short = false;  // the next call asks for all of it again
+  return less;
 }
 
 // Launch the class builders over the work lists of cls (see ClassLists) into `slots` and `valid`; whole: all vertices of the

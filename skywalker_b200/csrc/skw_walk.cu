@@ -136,7 +136,8 @@ static WalkGrid walk_grid(const skw_ctx* ctx, uint32_t app, u64 n, u32 warps, u3
 static bool walk_ahead(const skw_ctx* ctx, uint32_t app, u64 n, u32 hop_num, bool unbiased) {
   if (unbiased) return false;
   const bool short_cached = hop_num <= 40 && ctx->E * 12 <= (8u << 20) && n > 40ull * ctx->sm_count;
-  return app == SKW_APP_PPR ? n <= 270ull * ctx->sm_count && !short_cached : n <= 110ull * ctx->sm_count && ctx->E * 12 > (64u << 20);
+  if (app == SKW_APP_PPR) return n <= 270ull * ctx->sm_count && !short_cached;
+  return n <= 110ull * ctx->sm_count && ctx->E * 12 > (64u << 20);
 }
 
 // All steps of all walkers in one launch.  The first `lanes` lanes of each warp own walkers w, w + T, w + 2T ...;
@@ -1509,12 +1510,13 @@ static u32* seen_by_gpu(uint32_t* h, uint64_t count) {
 // a walk's end keep what the caller had there, and so do all of them when a walk meets a vertex that does not exist: rows are
 // not written before the whole batch is known to be good.
 static bool written_home(const skw_ctx* ctx, const skw_walk_params* prm, uint64_t n) {
+  if (n == 0 || !(prm->flags & SKW_WALK_FILL_ROWS) || prm->app == SKW_APP_NODE2VEC) return false;
   const double into_ends = (double)ctx->dead_ends / skw_ctx::kEdgeSample;
   const double stop = prm->app == SKW_APP_PPR ? prm->tp + (1.0 - prm->tp) * into_ends : into_ends;  // a step's chance to be the last
   const double longest = stop <= 0.0 ? prm->hop_num : stop >= 1.0 ? 0.0 : log((double)n) / -log1p(-stop);
   const double behind = prm->hop_num - std::min<double>(prm->hop_num, longest);
   if (behind > 160.0 || behind * (double)n * sizeof(u32) > 2.5e6) return false;
-  return n != 0 && (prm->flags & SKW_WALK_FILL_ROWS) != 0 && n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count && prm->app != SKW_APP_NODE2VEC &&
+  return n <= (prm->hop_num > kLineCells ? 200ull : 34ull) * ctx->sm_count &&
          prm->hop_num <= (1u << 24) &&  // the kernel counts up to a line past the row's end in 32 bits
          (prm->mode != SKW_MODE_ONLINE || (prm->flags & SKW_WALK_UNBIASED)) && !follows_records(ctx, prm);
 }

@@ -378,11 +378,23 @@ for _ in range(2):
     log = calls()
     assert launches(log, "build_long_kernelILj8E") and not launches(log, "build_long_kernelILj4E")
 assert not [x for x in log if x[0] == "malloc"]
+ctx.close()
+# without memory for either the call fails (walks compute their slots), and the next one has all of it
+ctx = context()
+fake.fake_memory(fake.fake_used() + 4 * MB)
+try:
+    ctx.%s
+    assert launches(calls(), "direct")
+except SkwError as e:
+    assert "out of memory" in str(e)
 fake.fake_memory(64 << 30)
+calls()
+ctx.%s
+assert launches(calls(), "build_long_kernelILj4E")
 ctx.upload(*ring(hub=20000))
 ctx.alias_build_offline()
 assert ctx.alias_export()[0].size == 32000
-""" % (call, call))
+""" % (call, call, call, call))
 
 
 def test_rows_of_which_only_parts_are_registered_are_copied(fake_cudart):
